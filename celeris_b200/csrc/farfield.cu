@@ -8,14 +8,14 @@
 // throughfocus.cpp:105-118 (CPU caustic loop).
 //
 // Layout in HBM
-//   pillar records  f64 form: double4 {x, y, Re t, Im t}            32 B/pillar
+//   pillar records  f64 form: double4 {x, y, |t|, arg t (polar_record)} 32 B/pillar
 //                   f32 form: float4  {x - ox, y - oy, |t|, arg t/2pi} 16 B/pillar
 //   partial sums    double2 [nchunk][npix] (pillar-chunk split of the sum)
 //   outputs         double2 field [npix] and/or double |E|^2 [npix]
 //
 // Kernels
 //   ff_pack_*        FP64 inputs -> pillar records (one pass over the pillars)
-//   rs_f64_kernel    plain form: FP64 terms exactly as focal.cpp:229-233
+//   rs_f64_kernel    plain form: FP64 terms of focal.cpp:229-233 (term64)
 //   rs_f32c_kernel   precision form: FP32 terms; R - z refined by one Newton
 //                    step on (R - z)(R + z) = dx^2 + dy^2 so the large k*z part
 //                    of the phase never enters FP32; phase reduced in turns;
@@ -59,9 +59,8 @@ constexpr int kThreads = 256;
 constexpr int kTile64 = 256;  // pillars (or pixels) per stage, 32 B records -> 8 KB
 constexpr int kTile32 = 512;  // pillars per stage, 16 B records -> 8 KB
 constexpr int kStages = 4;
-constexpr int kPPT64 = 2;     // pixels per thread, plain form
+constexpr int kPPT64 = 4;     // most pixels per thread, plain form (pillars, in the adjoint); 1 or 2 where that fills the chip better
 constexpr int kPPT32 = 6;     // pixels per thread, precision form: 3 packed pixel pairs share each pillar record
-constexpr int kAdjPPT = 2;    // pillars per thread, adjoint
 constexpr int kAdjPPT32 = 6;  // pillars per thread, precision-form adjoint (3 packed pairs)
 
 enum { GEOM_PSF = 0, GEOM_ZX = 1 };
@@ -114,6 +113,28 @@ __global__ void ff_pack_f64(const double* __restrict__ px, const double* __restr
     rec[j] = make_double4(px[j], py[j], t.x, t.y);
 }
 
+// Polar records of the FP64 sums: {x, y, |t|, psi}, the phase psi = arg t in
+// units of 1/kTab turn, split into its nearest integer and a remainder. The
+// remainder (|.| <= 1/2) is stored with the integer mod kTab in the low 9 bits
+// of its mantissa, which moves it by at most 2^-45 units (2^-54 turns).
+constexpr int kTab = 512;
+constexpr double kTabPerRad = 81.487330863050411914;  // kTab / (2 pi)
+__device__ __forceinline__ double4 polar_record(double x, double y, double re, double im) {
+    const double u = atan2(im, re) * kTabPerRad;
+    const double n = rint(u);
+    const long long b = __double_as_longlong(u - n);
+    const long long q = (long long)((int)n & (kTab - 1));
+    return make_double4(x, y, hypot(re, im), __longlong_as_double((b & ~(long long)(kTab - 1)) | q));
+}
+__global__ void ff_pack_f64p(const double* __restrict__ px, const double* __restrict__ py,
+                             const double2* __restrict__ pt, int npil, int slot, double4* __restrict__ rec) {
+    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= npil) return;
+    const double2 t = pt[j];
+    flag_nonfinite(slot, px[j], py[j], t.x, t.y);
+    rec[j] = polar_record(px[j], py[j], t.x, t.y);
+}
+
 // ---- pixel grid of the precision form ----------------------------------------------
 // Pillar coordinates are rounded to FP32 relative to the FP32 origin (ulp <=
 // G below). A pixel is split into a base on the grid of step G = 2^(ilogb(L) -
@@ -156,7 +177,7 @@ __global__ void ff_pack_f32(const double* __restrict__ px, const double* __restr
     rec[j] = make_float4((float)(px[j] - ox), (float)(py[j] - oy), (float)A, (float)psi);
 }
 
-// pixel records for the adjoint: {fx, fy, Re v, Im v}
+// pixel records for the adjoint: {fx, fy, |v|, arg v} as polar_record
 __global__ void ff_pack_pix(Geom g, const double2* __restrict__ v, double4* __restrict__ rec) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     int npix = g.nx * g.ny;
@@ -166,7 +187,7 @@ __global__ void ff_pack_pix(Geom g, const double2* __restrict__ v, double4* __re
     pixel_pos(g, i, j, fx, fy, fz);
     double2 vv = v[p];
     flag_nonfinite(g.slot, vv.x, vv.y, 0.0, 0.0);
-    rec[p] = make_double4(fx, fy, vv.x, vv.y);
+    rec[p] = polar_record(fx, fy, vv.x, vv.y);
 }
 
 // precision-form adjoint: float4 {fx - ox, fy - oy, Re v, Im v} per pixel
@@ -233,62 +254,197 @@ struct TilePipe {
 };
 
 // ---- plain FP64 form ----------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) rs_f64_kernel(const double4* __restrict__ rec,
-                                                          int npil, int chunk_len, Geom g,
-                                                          double k, double2* __restrict__ partial) {
-    __shared__ __align__(128) double4 buf[kStages][kTile64];
+// One term |t| e^{i (k R + psi)} / R in FP64. The FP64 pipe bounds these sums (64
+// FMA lanes per SM), so the term is arranged to need few FP64 operations: 27
+// against the ~70 issue slots of sqrt + sincos + division + complex product.
+//  * 1/R and R together from one hardware reciprocal square root of
+//    S = dx^2 + dy^2 + z^2 and one third-order step (the binomial series of
+//    (1 - e)^(-1/2), e = 1 - S y0^2): 6 operations, R within ~0.75 ulp.
+//  * The phase in units of 1/512 turn: n = rint(R il), g = R il - n exactly by
+//    FMA (il + il_lo = 512 k / 2 pi as a double pair), plus the record's
+//    remainder: |g| <= 1. The integer parts add as integers, so the rounding of
+//    k R of the direct form (half an ulp of ~1e4 rad) does not occur.
+//  * e^{2 pi i g / 512} by short polynomials (sine on Chebyshev nodes in g^2, cosine
+//    minimax; |error| < 2e-16) and e^{2 pi i n / 512} from a table in shared memory. Each
+//    lane of a quarter-warp reads its own copy of the table (8 copies, 16 B x 8 =
+//    one full bank row per entry), so the 16-byte lookups never conflict.
+// Domain: all coordinates and z within 1e9 um, |k| <= 4e3 rad/um (R il < 2^50) and
+// |z| >= 1e-100; outside it (or for NaN) tile_general evaluates the direct form.
+// Measured (B200, 70,688 pillars x 161^2): 7.35 ms with sqrt, sincos and a division
+// per term, 3.41 ms (5.4e11 terms/s) here, the FP64 pipe 84 % busy; 125,676 pillars x
+// 321^2: 5.65e11 terms/s. Four pixels per thread at two CTAs per SM; three CTAs, two
+// pixels, or the pillar loop unrolled by two measured 1-10 % slower. Error against
+// long double on lattice apertures (2-norm, relative): 5.8e-15, 4.0e-15, 2.3e-15 at
+// 1,085 / 11,304 / 70,688 pillars; the direct form 6.8e-15, 4.3e-15, 2.6e-15.
+constexpr int kTabCopies = 8;
+constexpr double kMagic64 = 6755399441055744.0;  // 1.5 * 2^52: x + M - M rounds x to an integer
+constexpr double kS1 = 0.01227184630308513, kS3 = -3.080196845514468e-07, kS5 = 2.3193482082506783e-12;
+constexpr double kC2 = -7.529910584122855e-05, kC4 = 9.44985951974752e-10;
+// (1 - e)^(-1/2) - 1 = e / 2 + 3 e^2 / 8 + 5 e^3 / 16 + ...: the seed's e lies in
+// [-1.14e-6, 1.86e-6] (measured over every high word), where the cubic term moves
+// a phase of 1e4 rad by up to 2e-14 rad, the same way for many pillars. Its
+// quadratic Chebyshev part on that interval is folded into the two coefficients;
+// what remains is below 5e-19.
+constexpr double kF0 = 0.5 + 4.03e-13, kF1 = 0.375 + 3.39e-7;
+constexpr double kCoordMax = 1e9, kWaveMax = 4e3, kZMin = 1e-100;
+
+// Phase constants of a launch: 512 k / 2 pi = il + il_lo (the adjoint negates
+// both), and whether z and k are in the domain above.
+struct Phase64 {
+    double il, il_lo, k;
+    int ok;
+};
+
+__device__ __forceinline__ double rsqrt_seed(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+
+// The table: entry n, copy l & 7 of lane l at tab[n * 8 + copy].
+__device__ __forceinline__ void fill_phase_table(double2* tab) {
+    for (int n = threadIdx.x; n < kTab; n += blockDim.x) {
+        double s, c;
+        sincospi(n * (2.0 / kTab), &s, &c);
+        for (int r = 0; r < kTabCopies; ++r) tab[n * kTabCopies + r] = make_double2(c, s);
+    }
+}
+
+// er + i ei += amp e^{i (2 pi / 512) (R il + ph)} / R, R = sqrt(S); ph: the record's
+// phase word, pn its integer part (low word), tab the lane's copy of the table.
+__device__ __forceinline__ void term64(double S, double amp, double ph, int pn, const double2* tab, double il,
+                                       double il_lo, double& er, double& ei) {
+    const double y0 = rsqrt_seed(S);
+    const double t = S * y0;
+    const double e = fma(-t, y0, 1.0);
+    const double f = e * fma(e, kF1, kF0);
+    const double R = fma(t, f, t);
+    const double a = amp * fma(y0, f, y0);
+    const double m = fma(R, il, kMagic64);
+    const double v = m - kMagic64;
+    const double g = fma(R, il, -v) + fma(R, il_lo, ph);
+    const double2 cs = tab[((__double2loint(m) + pn) & (kTab - 1)) * kTabCopies];
+    const double w = g * g;
+    const double sg = g * fma(w, fma(w, kS5, kS3), kS1);
+    const double cg = fma(w, fma(w, kC4, kC2), 1.0);
+    er = fma(a, fma(cs.x, cg, -(cs.y * sg)), er);
+    ei = fma(a, fma(cs.y, cg, cs.x * sg), ei);
+}
+
+// The direct form of the same sum over one tile (any finite range, NaN and Inf
+// propagate): the expression of focal.cpp:229-233. sgn = +1 (field) or -1 (adjoint).
+template <int PPT>
+__device__ __noinline__ void tile_general(const double4* tile, int cnt, const double* fx, const double* fy, double z2,
+                                          double k, double sgn, double* er, double* ei) {
+    for (int p = 0; p < cnt; ++p) {
+        const double4 r = tile[p];
+        double ts, tc;
+        sincospi((r.w + (double)(__double2loint(r.w) & (kTab - 1))) * (2.0 / kTab), &ts, &tc);
+        const double tr = r.z * tc, ti = r.z * ts;
+#pragma unroll
+        for (int q = 0; q < PPT; ++q) {
+            const double dx = fx[q] - r.x, dy = fy[q] - r.y;
+            const double R = sqrt(dx * dx + dy * dy + z2);
+            double s, c;
+            sincos(k * R, &s, &c);
+            const double inv = 1.0 / R;
+            const double pr = inv * c, pim = sgn * (inv * s);
+            er[q] += tr * pr - ti * pim;
+            ei[q] += tr * pim + ti * pr;
+        }
+    }
+}
+
+// dynamic shared memory of the FP64 sums: the phase table, then the tile stages
+constexpr size_t kSmem64 = (size_t)kTab * kTabCopies * sizeof(double2) + (size_t)kStages * kTile64 * sizeof(double4);
+
+// Every thread looks at the tile's record of its own index; the block takes the
+// direct form for the tile if any is out of the domain.
+__device__ __forceinline__ bool tile_in_domain(const double4* tile, int cnt, bool ok) {
+    bool in = ok;
+    for (int p = threadIdx.x; p < cnt; p += blockDim.x)
+        in = in && fabs(tile[p].x) <= kCoordMax && fabs(tile[p].y) <= kCoordMax;
+    return __syncthreads_and(in);
+}
+
+// PPT pixels of one row per thread share each pillar's record and dy^2.
+template <int PPT>
+__global__ void __launch_bounds__(kThreads, 2) rs_f64_kernel(const double4* __restrict__ rec, int npil,
+                                                             int chunk_len, Geom g, Phase64 ph,
+                                                             double2* __restrict__ partial) {
+    extern __shared__ __align__(128) unsigned char smem64[];
     __shared__ __align__(8) uint64_t full[kStages];
+    double2* tab = reinterpret_cast<double2*>(smem64);
+    double4(*buf)[kTile64] = reinterpret_cast<double4(*)[kTile64]>(tab + kTab * kTabCopies);
 
     const int npix = g.nx * g.ny;
-    const int spr = (g.nx + kPPT64 - 1) / kPPT64;
+    const int spr = (g.nx + PPT - 1) / PPT;
     const int strip = blockIdx.x * kThreads + threadIdx.x;
     const int j = strip / spr;
-    const int i0 = (strip - j * spr) * kPPT64;
+    const int i0 = (strip - j * spr) * PPT;
     const int jj = min(j, g.ny - 1);
 
-    double fx[kPPT64], fy = 0.0, fz = 0.0;
+    double fx[PPT], fy = 0.0, fz = 0.0;
 #pragma unroll
-    for (int q = 0; q < kPPT64; ++q) pixel_pos(g, min(i0 + q, g.nx - 1), jj, fx[q], fy, fz);
+    for (int q = 0; q < PPT; ++q) pixel_pos(g, min(i0 + q, g.nx - 1), jj, fx[q], fy, fz);
     const double z2 = fz * fz;
+    bool ok = ph.ok && fabs(fz) >= kZMin && fabs(fz) <= kCoordMax && fabs(fy) <= kCoordMax;
+#pragma unroll
+    for (int q = 0; q < PPT; ++q) ok = ok && fabs(fx[q]) <= kCoordMax;
 
     TilePipe<double4, kTile64> pipe;
     const int lo = blockIdx.y * chunk_len;
     pipe.init(buf, full, rec, lo, min(npil, lo + chunk_len), g.slot);
+    fill_phase_table(tab);
+    const double2* tl = tab + (threadIdx.x & (kTabCopies - 1));
 
-    double er[kPPT64], ei[kPPT64];
+    double er[PPT], ei[PPT];
 #pragma unroll
-    for (int q = 0; q < kPPT64; ++q) er[q] = ei[q] = 0.0;
+    for (int q = 0; q < PPT; ++q) er[q] = ei[q] = 0.0;
 
     for (int t = 0; t < pipe.ntiles; ++t) {
         const bool got = pipe.wait(t);
-        if (got) {
-            const double4* tile = buf[t % kStages];
-            const int cnt = pipe.count(t);
+        const double4* tile = buf[t % kStages];
+        const int cnt = got ? pipe.count(t) : 0;
+        if (tile_in_domain(tile, cnt, ok)) {  // (also orders the table before its first use)
+#pragma unroll 1
             for (int p = 0; p < cnt; ++p) {
                 const double4 r = tile[p];
+                const int pn = __double2loint(r.w);
                 const double dy = fy - r.y;
                 const double dy2 = dy * dy;
 #pragma unroll
-                for (int q = 0; q < kPPT64; ++q) {
+                for (int q = 0; q < PPT; ++q) {
+                    // z^2 is added last: a rounding of dy^2 + z^2 would be the
+                    // same for every pillar of a lattice row
                     const double dx = fx[q] - r.x;
-                    const double R = sqrt(dx * dx + dy2 + z2);
-                    double s, c;
-                    sincos(k * R, &s, &c);
-                    const double inv = 1.0 / R;
-                    const double pr = inv * c, pim = inv * s;  // std::polar(1/R, kR)
-                    er[q] += r.z * pr - r.w * pim;             // t * polar
-                    ei[q] += r.z * pim + r.w * pr;
+                    term64(fma(dx, dx, dy2) + z2, r.z, r.w, pn, tl, ph.il, ph.il_lo, er[q], ei[q]);
                 }
+            }
+        } else {
+            // copies, so that the loop above keeps its own values in registers
+            double xq[PPT], yq[PPT], e1[PPT], e2[PPT];
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) {
+                xq[q] = fx[q];
+                yq[q] = fy;
+                e1[q] = er[q];
+                e2[q] = ei[q];
+            }
+            tile_general<PPT>(tile, cnt, xq, yq, z2, ph.k, 1.0, e1, e2);
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) {
+                er[q] = e1[q];
+                ei[q] = e2[q];
             }
         }
         if (!pipe.release(t, got)) return;
     }
     if (j < g.ny) {
 #pragma unroll
-        for (int q = 0; q < kPPT64; ++q)
+        for (int q = 0; q < PPT; ++q)
             if (i0 + q < g.nx)
-                partial[(size_t)blockIdx.y * npix + (size_t)j * g.nx + i0 + q] =
-                    make_double2(er[q], ei[q]);
+                partial[(size_t)blockIdx.y * npix + (size_t)j * g.nx + i0 + q] = make_double2(er[q], ei[q]);
     }
 }
 
@@ -581,17 +737,53 @@ __global__ void adj_f32c_reduce(const double2* __restrict__ partial, int nchunk,
 }
 
 // ---- chunk reduction + epilogue ---------------------------------------------
+// Sum of output p over the chunks. blockDim (32, 8): eight threads take an eighth of
+// the chunks each and thread y = 0 adds their sums in order (true there only).
+// With one thread per output, 64 chunks are a chain of 64 dependent sums behind
+// 16 round trips to L2, and a small grid has too few threads to hide them.
+constexpr int kSplitY = 8;
+__device__ __forceinline__ bool split_chunk_sum(const double2* __restrict__ partial, int nchunk, int n, int p,
+                                                double& er, double& ei) {
+    __shared__ double2 part[kSplitY][33];
+    const int per = (nchunk + kSplitY - 1) / kSplitY;
+    const int c0 = threadIdx.y * per, c1 = min(nchunk, c0 + per);
+    double sr = 0.0, si = 0.0;
+    if (p < n) {
+#pragma unroll 8
+        for (int c = c0; c < c1; ++c) {
+            const double2 v = partial[(size_t)c * n + p];
+            sr += v.x;
+            si += v.y;
+        }
+    }
+    part[threadIdx.y][threadIdx.x] = make_double2(sr, si);
+    __syncthreads();
+    if (threadIdx.y != 0 || p >= n) return false;
+    er = ei = 0.0;
+#pragma unroll
+    for (int y = 0; y < kSplitY; ++y) {
+        er += part[y][threadIdx.x].x;
+        ei += part[y][threadIdx.x].y;
+    }
+    return true;
+}
+
+template <bool SPLIT>
 __global__ void rs_reduce_kernel(const double2* __restrict__ partial, int nchunk, Geom g,
                                  double k, int apply_phase, double2* __restrict__ field,
                                  double* __restrict__ intensity) {
     const int npix = g.nx * g.ny;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npix) return;
     double er = 0.0, ei = 0.0;
-    for (int c = 0; c < nchunk; ++c) {
-        const double2 v = partial[(size_t)c * npix + p];
-        er += v.x;
-        ei += v.y;
+    if constexpr (SPLIT) {
+        if (!split_chunk_sum(partial, nchunk, npix, p, er, ei)) return;
+    } else {
+        if (p >= npix) return;
+        for (int c = 0; c < nchunk; ++c) {
+            const double2 v = partial[(size_t)c * npix + p];
+            er += v.x;
+            ei += v.y;
+        }
     }
     if (apply_phase) {
         const int j = p / g.nx;
@@ -611,73 +803,84 @@ __global__ void rs_reduce_kernel(const double2* __restrict__ partial, int nchunk
 }
 
 // ---- adjoint: out_j = sum_p conj(g_pj) v_p ----------------------------------
-__global__ void __launch_bounds__(kThreads) rs_adj_f64_kernel(const double4* __restrict__ pix,
-                                                              int npix, int chunk_len,
-                                                              const double* __restrict__ px,
-                                                              const double* __restrict__ py,
-                                                              int npil, double z, double k, int slot,
-                                                              double2* __restrict__ partial) {
-    __shared__ __align__(128) double4 buf[kStages][kTile64];
+// conj(g) v = |v| e^{i (arg v - k R)} / R: the field's term with the phase's sign
+// turned (ph.il, ph.il_lo negative), pixels as records and pillars as outputs.
+template <int PPT>
+__global__ void __launch_bounds__(kThreads, 2) rs_adj_f64_kernel(const double4* __restrict__ pix, int npix,
+                                                                 int chunk_len, const double* __restrict__ px,
+                                                                 const double* __restrict__ py, int npil, double z,
+                                                                 Phase64 ph, int slot,
+                                                                 double2* __restrict__ partial) {
+    extern __shared__ __align__(128) unsigned char smem64[];
     __shared__ __align__(8) uint64_t full[kStages];
+    double2* tab = reinterpret_cast<double2*>(smem64);
+    double4(*buf)[kTile64] = reinterpret_cast<double4(*)[kTile64]>(tab + kTab * kTabCopies);
 
-    const int j0 = (blockIdx.x * kThreads + threadIdx.x) * kAdjPPT;
-    double x[kAdjPPT], y[kAdjPPT];
+    const int j0 = (blockIdx.x * kThreads + threadIdx.x) * PPT;
+    double x[PPT], y[PPT];
+    bool ok = ph.ok && fabs(z) >= kZMin && fabs(z) <= kCoordMax;
 #pragma unroll
-    for (int q = 0; q < kAdjPPT; ++q) {
+    for (int q = 0; q < PPT; ++q) {
         const int jq = min(j0 + q, npil - 1);
         x[q] = px[jq];
         y[q] = py[jq];
+        ok = ok && fabs(x[q]) <= kCoordMax && fabs(y[q]) <= kCoordMax;
     }
     const double z2 = z * z;
 
     TilePipe<double4, kTile64> pipe;
     const int lo = blockIdx.y * chunk_len;
     pipe.init(buf, full, pix, lo, min(npix, lo + chunk_len), slot);
+    fill_phase_table(tab);
+    const double2* tl = tab + (threadIdx.x & (kTabCopies - 1));
 
-    double gr[kAdjPPT], gi[kAdjPPT];
+    double gr[PPT], gi[PPT];
 #pragma unroll
-    for (int q = 0; q < kAdjPPT; ++q) gr[q] = gi[q] = 0.0;
+    for (int q = 0; q < PPT; ++q) gr[q] = gi[q] = 0.0;
 
     for (int t = 0; t < pipe.ntiles; ++t) {
         const bool got = pipe.wait(t);
-        if (got) {
-            const double4* tile = buf[t % kStages];
-            const int cnt = pipe.count(t);
+        const double4* tile = buf[t % kStages];
+        const int cnt = got ? pipe.count(t) : 0;
+        if (tile_in_domain(tile, cnt, ok)) {
+#pragma unroll 1
             for (int p = 0; p < cnt; ++p) {
-                const double4 r = tile[p];  // {fx, fy, Re v, Im v}
+                const double4 r = tile[p];  // {fx, fy, |v|, arg v}
+                const int pn = __double2loint(r.w);
 #pragma unroll
-                for (int q = 0; q < kAdjPPT; ++q) {
-                    const double dx = r.x - x[q];
-                    const double dy = r.y - y[q];
-                    const double R = sqrt(dx * dx + dy * dy + z2);
-                    double s, c;
-                    sincos(k * R, &s, &c);
-                    const double inv = 1.0 / R;
-                    const double pr = inv * c, pim = inv * s;
-                    gr[q] += pr * r.z + pim * r.w;  // conj(g) * v
-                    gi[q] += pr * r.w - pim * r.z;
+                for (int q = 0; q < PPT; ++q) {
+                    const double dx = r.x - x[q], dy = r.y - y[q];
+                    term64(fma(dx, dx, dy * dy) + z2, r.z, r.w, pn, tl, ph.il, ph.il_lo, gr[q], gi[q]);
                 }
+            }
+        } else {
+            double xq[PPT], yq[PPT], e1[PPT], e2[PPT];
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) {
+                xq[q] = x[q];
+                yq[q] = y[q];
+                e1[q] = gr[q];
+                e2[q] = gi[q];
+            }
+            tile_general<PPT>(tile, cnt, xq, yq, z2, ph.k, -1.0, e1, e2);
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) {
+                gr[q] = e1[q];
+                gi[q] = e2[q];
             }
         }
         if (!pipe.release(t, got)) return;
     }
 #pragma unroll
-    for (int q = 0; q < kAdjPPT; ++q)
-        if (j0 + q < npil)
-            partial[(size_t)blockIdx.y * npil + j0 + q] = make_double2(gr[q], gi[q]);
+    for (int q = 0; q < PPT; ++q)
+        if (j0 + q < npil) partial[(size_t)blockIdx.y * npil + j0 + q] = make_double2(gr[q], gi[q]);
 }
 
 __global__ void chunk_sum_kernel(const double2* __restrict__ partial, int nchunk, int n,
                                  double2* __restrict__ out) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
     double r = 0.0, i = 0.0;
-    for (int c = 0; c < nchunk; ++c) {
-        const double2 v = partial[(size_t)c * n + j];
-        r += v.x;
-        i += v.y;
-    }
-    out[j] = make_double2(r, i);
+    if (split_chunk_sum(partial, nchunk, n, j, r, i)) out[j] = make_double2(r, i);
 }
 
 // ---- stated error of the precision form ------------------------------------------
@@ -906,6 +1109,79 @@ void plan_chunks(int ctas_other, int nrec, int tile, int resident_per_sm, int* n
     if (*nchunk < 1) *nchunk = 1;
 }
 
+// Plan of the FP64 sums: `ppt` outputs per thread (ctas CTAs over the outputs) and
+// chunks of records. Four outputs per thread share a record's loads; grids whose
+// CTAs, even with chunks of 64 records, do not fill the chip twice take fewer.
+struct Plan64 {
+    int ppt, ctas, nchunk, chunk_len;
+};
+template <class Ctas>
+Plan64 plan64(Ctas ctas_of, int nrec) {
+    const long slots = (long)sm_count() * 2;
+    const long pieces = std::max(1, (nrec + 63) / 64);
+    Plan64 p;
+    for (p.ppt = kPPT64; p.ppt > 1; p.ppt /= 2)
+        if (ctas_of(p.ppt) * pieces >= 2 * slots) break;
+    p.ctas = (int)ctas_of(p.ppt);
+    plan_chunks(p.ctas, nrec, p.ppt == 1 ? 32 : 64, 2, &p.nchunk, &p.chunk_len);
+    return p;
+}
+Plan64 plan_field64(const Geom& g, int npil) {
+    return plan64([&](int ppt) { return ((long)((g.nx + ppt - 1) / ppt) * g.ny + kThreads - 1) / kThreads; }, npil);
+}
+
+Phase64 phase64(double z, double k, bool adjoint) {
+    Phase64 p;
+    // 512 k / 2 pi as a pair: the product's rounding by FMA, and 512 / 2 pi's own
+    const double c_lo = -5.037741228846716e-15;  // 512 / (2 pi) - kTabPerRad
+    const double il = k * kTabPerRad;
+    const double lo = std::fma(k, kTabPerRad, -il) + k * c_lo;
+    p.il = adjoint ? -il : il;
+    p.il_lo = adjoint ? -lo : lo;
+    p.k = k;
+    p.ok = std::fabs(k) <= kWaveMax && std::fabs(z) <= kCoordMax;
+    return p;
+}
+
+// The dynamic shared memory of the FP64 kernels exceeds the 48 KB default; the
+// limit is raised once per device.
+int prepare64() {
+    static std::mutex mu;
+    static bool done[64] = {};
+    int dev = 0;
+    CEL_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev >= 0 && dev < 64 && done[dev]) return CELERIS_OK;
+    const void* fn[] = {reinterpret_cast<const void*>(rs_f64_kernel<1>), reinterpret_cast<const void*>(rs_f64_kernel<2>),
+                        reinterpret_cast<const void*>(rs_f64_kernel<4>),
+                        reinterpret_cast<const void*>(rs_adj_f64_kernel<1>),
+                        reinterpret_cast<const void*>(rs_adj_f64_kernel<2>),
+                        reinterpret_cast<const void*>(rs_adj_f64_kernel<4>)};
+    for (const void* f : fn) CEL_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem64));
+    if (dev >= 0 && dev < 64) done[dev] = true;
+    return CELERIS_OK;
+}
+
+void launch_f64(const Plan64& p, cudaStream_t st, const double4* rec, int npil, const Geom& g, double k,
+                double2* partial) {
+    const dim3 grid(p.ctas, p.nchunk);
+    const Phase64 ph = phase64(g.mode == GEOM_PSF ? g.z : 0.0, k, false);  // ZX: the kernel checks each row's z
+    if (p.ppt == 4) rs_f64_kernel<4><<<grid, kThreads, kSmem64, st>>>(rec, npil, p.chunk_len, g, ph, partial);
+    else if (p.ppt == 2) rs_f64_kernel<2><<<grid, kThreads, kSmem64, st>>>(rec, npil, p.chunk_len, g, ph, partial);
+    else rs_f64_kernel<1><<<grid, kThreads, kSmem64, st>>>(rec, npil, p.chunk_len, g, ph, partial);
+}
+
+void launch_reduce(const double2* partial, int nchunk, const Geom& g, double k, int apply_phase, double2* field,
+                   double* intensity, cudaStream_t st) {
+    const long npix = (long)g.nx * g.ny;
+    if (nchunk >= 2 * kSplitY)
+        rs_reduce_kernel<true><<<(int)((npix + 31) / 32), dim3(32, kSplitY), 0, st>>>(partial, nchunk, g, k,
+                                                                                      apply_phase, field, intensity);
+    else
+        rs_reduce_kernel<false><<<(int)((npix + 255) / 256), 256, 0, st>>>(partial, nchunk, g, k, apply_phase, field,
+                                                                           intensity);
+}
+
 // Status word of a stream: the legacy default stream in slot 0, other streams
 // hashed over the remaining slots.
 int status_slot(cudaStream_t st) {
@@ -1037,13 +1313,17 @@ int ff_run(int form, const double* d_px, const double* d_py, const double* d_pt,
         return CELERIS_OK;
     }
     const bool f32 = (form == CELERIS_FORM_F32C);
-    const int ppt = f32 ? kPPT32 : kPPT64;
-    const int tile = f32 ? kTile32 : kTile64;
-    const long spr = (g.nx + ppt - 1) / ppt;
-    const long strips = spr * g.ny;
-    const int ctas_pix = (int)((strips + kThreads - 1) / kThreads);
-    int nchunk = 1, chunk_len = npil;
-    plan_chunks(ctas_pix, npil, tile, f32 ? 3 : 2, &nchunk, &chunk_len);
+    int ctas_pix = 0, nchunk = 1, chunk_len = npil;
+    Plan64 p64{};
+    if (f32) {
+        const long strips = (long)((g.nx + kPPT32 - 1) / kPPT32) * g.ny;
+        ctas_pix = (int)((strips + kThreads - 1) / kThreads);
+        plan_chunks(ctas_pix, npil, kTile32, 3, &nchunk, &chunk_len);
+    } else {
+        CEL_TRY(prepare64());
+        p64 = plan_field64(g, npil);
+        nchunk = p64.nchunk;
+    }
 
     Workspace& ws = Workspace::for_stream(st);
     const size_t rec_bytes = (size_t)npil * (f32 ? sizeof(float4) : sizeof(double4));
@@ -1062,8 +1342,8 @@ int ff_run(int form, const double* d_px, const double* d_py, const double* d_pt,
                                         g.ox, g.oy, g.slot, static_cast<float4*>(rec));
         count_launch(1);
     } else {
-        ff_pack_f64<<<pb, 256, 0, st>>>(d_px, d_py, reinterpret_cast<const double2*>(d_pt), npil,
-                                        g.slot, static_cast<double4*>(rec));
+        ff_pack_f64p<<<pb, 256, 0, st>>>(d_px, d_py, reinterpret_cast<const double2*>(d_pt), npil,
+                                         g.slot, static_cast<double4*>(rec));
     }
     dim3 grid(ctas_pix, nchunk);
     timer_begin(st);
@@ -1073,12 +1353,10 @@ int ff_run(int form, const double* d_px, const double* d_py, const double* d_pt,
         const float lo = (float)(il - (double)hi);
         launch_f32c(grid, st, static_cast<const float4*>(rec), npil, chunk_len, g, hi, lo, ext, wmax, partial);
     } else {
-        rs_f64_kernel<<<grid, kThreads, 0, st>>>(static_cast<const double4*>(rec), npil,
-                                                 chunk_len, g, k, partial);
+        launch_f64(p64, st, static_cast<const double4*>(rec), npil, g, k, partial);
     }
     timer_end(st);
-    rs_reduce_kernel<<<(int)((npix + 255) / 256), 256, 0, st>>>(
-        partial, nchunk, g, k, f32 ? 1 : 0, reinterpret_cast<double2*>(d_field), d_int);
+    launch_reduce(partial, nchunk, g, k, f32 ? 1 : 0, reinterpret_cast<double2*>(d_field), d_int, st);
     count_launch(3);
     CEL_CUDA(cudaGetLastError());
     return CELERIS_OK;
@@ -1119,23 +1397,30 @@ int ff_adjoint(const double* d_px, const double* d_py, int npil, const Geom& g0,
         CEL_CUDA(cudaGetLastError());
         return CELERIS_OK;
     }
-    const int ctas = (int)(((long)npil + kThreads * kAdjPPT - 1) / (kThreads * kAdjPPT));
-    int nchunk = 1, chunk_len = (int)npix;
-    plan_chunks(ctas, (int)npix, kTile64, 2, &nchunk, &chunk_len);
+    CEL_TRY(prepare64());
+    const Plan64 p64 = plan64([&](int ppt) { return ((long)npil + kThreads * ppt - 1) / (kThreads * ppt); }, (int)npix);
     Workspace& ws = Workspace::for_stream(st);
     const size_t rec_bytes = (size_t)npix * sizeof(double4);
-    const size_t part_bytes = (size_t)nchunk * npil * sizeof(double2);
+    const size_t part_bytes = (size_t)p64.nchunk * npil * sizeof(double2);
     CEL_TRY(ws.reserve(st, celeris_rt::align256(rec_bytes) + celeris_rt::align256(part_bytes)));
     double4* rec = static_cast<double4*>(ws.take(rec_bytes));
     double2* partial = static_cast<double2*>(ws.take(part_bytes));
     ff_pack_pix<<<(int)((npix + 255) / 256), 256, 0, st>>>(g, reinterpret_cast<const double2*>(d_v), rec);
-    dim3 grid(ctas, nchunk);
+    const dim3 grid(p64.ctas, p64.nchunk);
+    const Phase64 ph = phase64(g.z, k, true);
     timer_begin(st);
-    rs_adj_f64_kernel<<<grid, kThreads, 0, st>>>(rec, (int)npix, chunk_len, d_px, d_py, npil, g.z, k, g.slot,
-                                                 partial);
+    if (p64.ppt == 4)
+        rs_adj_f64_kernel<4><<<grid, kThreads, kSmem64, st>>>(rec, (int)npix, p64.chunk_len, d_px, d_py, npil, g.z, ph,
+                                                              g.slot, partial);
+    else if (p64.ppt == 2)
+        rs_adj_f64_kernel<2><<<grid, kThreads, kSmem64, st>>>(rec, (int)npix, p64.chunk_len, d_px, d_py, npil, g.z, ph,
+                                                              g.slot, partial);
+    else
+        rs_adj_f64_kernel<1><<<grid, kThreads, kSmem64, st>>>(rec, (int)npix, p64.chunk_len, d_px, d_py, npil, g.z, ph,
+                                                              g.slot, partial);
     timer_end(st);
-    chunk_sum_kernel<<<(npil + 255) / 256, 256, 0, st>>>(partial, nchunk, npil,
-                                                         reinterpret_cast<double2*>(d_out));
+    chunk_sum_kernel<<<(npil + 31) / 32, dim3(32, kSplitY), 0, st>>>(partial, p64.nchunk, npil,
+                                                                     reinterpret_cast<double2*>(d_out));
     count_launch(3);
     CEL_CUDA(cudaGetLastError());
     return CELERIS_OK;
@@ -1496,10 +1781,6 @@ int ff_run_noalloc(int form, const double* d_px, const double* d_py, const doubl
         return CELERIS_OK;
     }
     const bool f32 = (form == CELERIS_FORM_F32C);
-    const int ppt = f32 ? kPPT32 : kPPT64;
-    const int tile = f32 ? kTile32 : kTile64;
-    const long spr = (g.nx + ppt - 1) / ppt;
-    const int ctas_pix = (int)((spr * g.ny + kThreads - 1) / kThreads);
     // scratch: pillar records | the coordinate extent word (256 B) | partial sums
     const size_t rec_bytes =
         celeris_rt::align256((size_t)npil * (f32 ? sizeof(float4) : sizeof(double4))) + 256;
@@ -1508,15 +1789,28 @@ int ff_run_noalloc(int form, const double* d_px, const double* d_py, const doubl
         return set_error(CELERIS_ERR_TOO_LARGE,
                          "no-alloc far-field: %d pillars x %ld pixels need %zu bytes of scratch, limit %zu",
                          npil, npix, rec_bytes + part_one, kNoAllocScratchBytes);
-    int nchunk = 1, chunk_len = npil;
-    plan_chunks(ctas_pix, npil, tile, f32 ? 3 : 2, &nchunk, &chunk_len);
+    int ctas_pix = 0, nchunk = 1, chunk_len = npil;
+    Plan64 p64{};
+    if (f32) {
+        const long spr = (g.nx + kPPT32 - 1) / kPPT32;
+        ctas_pix = (int)((spr * g.ny + kThreads - 1) / kThreads);
+        plan_chunks(ctas_pix, npil, kTile32, 3, &nchunk, &chunk_len);
+    } else {
+        CEL_TRY(prepare64());
+        p64 = plan_field64(g, npil);
+        nchunk = p64.nchunk;
+        chunk_len = p64.chunk_len;
+    }
     // fewer chunks (longer ones) until the partial sums fit beside the records
+    const int tile = f32 ? kTile32 : kTile64;
     const int ntiles = (npil + tile - 1) / tile;
     while ((size_t)nchunk * part_one + rec_bytes > kNoAllocScratchBytes) {
         const int tiles_per = (chunk_len / tile) + 1;
         chunk_len = tiles_per * tile;
         nchunk = (ntiles + tiles_per - 1) / tiles_per;
     }
+    p64.nchunk = nchunk;
+    p64.chunk_len = chunk_len;
     void* rec = base;
     unsigned long long* ext = reinterpret_cast<unsigned long long*>(static_cast<char*>(base) + rec_bytes - 256);
     double2* partial = reinterpret_cast<double2*>(static_cast<char*>(base) + rec_bytes);
@@ -1529,8 +1823,8 @@ int ff_run_noalloc(int form, const double* d_px, const double* d_py, const doubl
                                         g.slot, static_cast<float4*>(rec));
         count_launch(1);
     } else
-        ff_pack_f64<<<pb, 256, 0, st>>>(d_px, d_py, reinterpret_cast<const double2*>(d_pt), npil, g.slot,
-                                        static_cast<double4*>(rec));
+        ff_pack_f64p<<<pb, 256, 0, st>>>(d_px, d_py, reinterpret_cast<const double2*>(d_pt), npil, g.slot,
+                                         static_cast<double4*>(rec));
     dim3 grid(ctas_pix, nchunk);
     if (f32) {
         const double il = k / (2.0 * 3.14159265358979323846);
@@ -1538,10 +1832,9 @@ int ff_run_noalloc(int form, const double* d_px, const double* d_py, const doubl
         const float lo = (float)(il - (double)hi);
         launch_f32c(grid, st, static_cast<const float4*>(rec), npil, chunk_len, g, hi, lo, ext, wmax, partial);
     } else {
-        rs_f64_kernel<<<grid, kThreads, 0, st>>>(static_cast<const double4*>(rec), npil, chunk_len, g, k, partial);
+        launch_f64(p64, st, static_cast<const double4*>(rec), npil, g, k, partial);
     }
-    rs_reduce_kernel<<<(int)((npix + 255) / 256), 256, 0, st>>>(partial, nchunk, g, k, f32 ? 1 : 0,
-                                                                 reinterpret_cast<double2*>(d_field), d_int);
+    launch_reduce(partial, nchunk, g, k, f32 ? 1 : 0, reinterpret_cast<double2*>(d_field), d_int, st);
     count_launch(3);
     CEL_CUDA(cudaGetLastError());
     return CELERIS_OK;
