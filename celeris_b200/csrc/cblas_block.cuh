@@ -748,20 +748,6 @@ __device__ __forceinline__ bool gj_step(int n, int ncol, cplx* M, int ld, int k,
     return true;
 }
 
-// [A | B] (n x (n + nrhs), shared; an odd ld keeps column walks free of bank
-// conflicts) -> B <- A^-1 B by Gauss-Jordan with partial pivoting (A is
-// destroyed). scratch: 2 (n + nrhs) + 1 complex and one int of shared memory.
-// Returns 0 or the 1-based column of a zero pivot.
-__device__ int blk_gj_solve_smem(int n, int nrhs, cplx* M, int ld, cplx* scratch, int* sp) {
-    cplx* rowv = scratch;
-    cplx* colv = scratch + n + nrhs;
-    cplx* sd = colv + n + nrhs;
-    __syncthreads();
-    for (int k = 0; k < n; ++k)
-        if (!gj_step<false>(n, n + nrhs, M, ld, k, rowv, colv, sp, sd)) return k + 1;
-    return 0;
-}
-
 // A (n x n, shared, ld) <- A^-1 in place by Gauss-Jordan with partial pivoting
 // (rows swapped during the sweep, the inverse's columns swapped back after it).
 // scratch: 2 n + 1 complex; piv: n ints of shared memory.

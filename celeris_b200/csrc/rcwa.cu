@@ -6,10 +6,24 @@
 //
 // One unit cell = one patterned layer between the incident and substrate
 // half-spaces (the library-sweep stack). Cells are bucketed by (Mx, My, raster
-// size); a bucket runs as a fixed sequence of kernels with one CTA per cell:
+// size, symmetry); a bucket runs as a fixed sequence of kernels with one CTA per cell or
+// parity class:
 //   rcwa_fourier_rect / rcwa_fourier_laurent  eps operators (analytic Li rule,
 //                 or 4x4-supersampled raster -> centred DFT -> Laurent Toeplitz)
 //                 and Einv (LU inverse for the Laurent path)
+//   rcwa_sym_build  M = ep2 kp - kkT and kp of the excited parity classes
+//                 (mirror-symmetric cells)
+//   rcwa_slab     the layer as a two-port without an eigendecomposition (slab.cuh),
+//                 then the amplitudes between the half-spaces
+//   rcwa_sym_expand  class amplitudes into the order basis
+//   rcwa_epilogue Poynting flux and order-0 field for each requested excitation
+// Stacks run rcwa_slab per layer and rcwa_stack_port (one CTA per stack).
+// Measured (one B200, whole calls, against the eigendecomposition's sequence below):
+//   one M = 5 cell 4.6 -> 0.9 ms; 64 cells M = 3 0.99 -> 0.49 ms; 512 rasterised cells M = 3..7
+//   37 -> 13 ms; 96 oblique cells M = 4 26 -> 7 ms; 64 two-layer stacks M = 3 15.5 -> 3.4 ms
+//
+// The eigendecomposition's sequence remains for what the two-port does not take (needs_qr)
+// or flags (kInfoRedo), and for celeris_eig_general; it runs in the order basis:
 //   rcwa_build_M  M = ep2 kp - kkT using the diagonal Kx, Ky (two N^3 GEMMs)
 //   rcwa_hess     Householder reduction to Hessenberg form H = Q^H M Q (in
 //                 shared memory for n <= 112, blocked compact-WY panels above)
@@ -20,13 +34,13 @@
 //   rcwa_smat1    A = kp W, T11/T12 of interface 0, S12 and u = T11^{-1} a0
 //   rcwa_smat2    W^{-1}, A^{-1}, T11'/T12' of interface 1, B = T11' - D S12 T12',
 //                 aN = B^{-1} D u, b0 = T12 u + S22 T12' aN
-//   rcwa_epilogue Poynting flux and order-0 field for each requested excitation
-// The algebra is that of the reference's grcwa recursion specialised to
+// Its algebra is that of the reference's grcwa recursion specialised to
 // phi = I in the half-spaces and to the two excitation columns actually read
 // (a0 has two non-zeros), so only 2 columns of the global S11/S21 are formed.
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <atomic>
 #include <cmath>
 
 #include <algorithm>
@@ -43,6 +57,7 @@
 
 #include "cblas_block.cuh"
 #include "schur_aed.cuh"
+#include "slab.cuh"
 #include "runtime.cuh"
 
 namespace {
@@ -66,7 +81,8 @@ struct CellDev {
     cplx n_inc, n_sub;
     cplx ex0, ey0;  // excitation of result slot 0 (batch: X = (1, 0))
     int shape, nexc;
-    int pad0, pad1;
+    int real_mat;  // M is real in exact arithmetic (real permittivities and in-plane wavevector)
+    int pad1;
 };
 
 struct Bucket {
@@ -84,20 +100,22 @@ struct Bucket {
     const cplx* phy;  // [(4My+1) x ng]
     long long* dbg;   // optional per-cell counters, kDbgSlots each (CELERIS_RCWA_STAGE_CLOCKS=1), else NULL
     double* ord;      // optional per-order efficiencies: per cell and excitation [N][2] = (de_t, de_r), else NULL
-    // mirror-symmetric cells (sym != 0): the eigenproblem solved in its four
-    // parity classes; size class k (0: classes (+,+) and (-,-), 1: (+,-) and
-    // (-,+)) holds two m[k] x m[k] matrices per cell, matrix 2 cell + j
+    // mirror-symmetric cells (sym != 0): the layer problem in its excited parity
+    // classes
     int sym;         // 0: full path; 1: both excited classes; 2: also C4-symmetric (one class)
     int ncls, cls0;  // excited classes solved per cell (2, or 1 = class 1 only) and the first one
     double sym_tol;  // largest asymmetry of M (relative to max |M|) the class split accepts
-    int m[2];
-    cplx *sH[2], *sZ[2], *sX[2], *sW[2], *sA[2], *sq[2];
-    int* sinfo[2];
-    // S-matrix in the two excited classes, matrix 2 cell + c (c = 0: (+,+), the
-    // Y excitation; c = 1: (-,-), the X excitation), order m[0]: layer kp,
-    // incident diag(kz) kp^-1, substrate kp diag(1/kz), and the work matrices
-    cplx *cKp, *cC0, *cKs, *cA, *cT11, *cT11lu, *cT12, *cS12, *cQ, *cSQ, *cCm, *cvec;
-    int* cpiv;
+    int m;           // order of a class
+    // per solved class (matrix ncls * cell + class): M and kp in the class basis,
+    // and the amplitudes aN | b0 (2 m)
+    cplx *cM, *cKp, *cvec;
+    // the layer two-port (slab.cuh): work area of a full-order cell (s_w complex), kp
+    cplx *slab, *Kp;
+    size_t s_w;
+    // layers of a stack: A, B and kp of cell i go to slot lslot[i] (s_nn each)
+    cplx *lA, *lB, *lK;
+    const int* lslot;
+    int* lrest;  // log2 of the slabs (A, B) the layer consists of
 };
 
 __device__ __forceinline__ cplx* at(cplx* base, size_t stride, int c) { return base + stride * c; }
@@ -105,6 +123,9 @@ __device__ __forceinline__ cplx* at(cplx* base, size_t stride, int c) { return b
 // Mirror-symmetric cells (Bucket::sym != 0): per-cell info code of a cell found
 // not symmetric to the tolerance, which is solved again by the full path.
 constexpr int kInfoAsym = 1 << 29;
+// A cell whose two-port was ill conditioned (slab.cuh), which is solved again
+// through the eigendecomposition.
+constexpr int kInfoRedo = 1 << 28;
 
 // Parity classes under the two mirrors p -> -p, q -> -q.
 // class c: 0 = (+,+), 1 = (-,-), 2 = (+,-), 3 = (-,+)
@@ -1183,7 +1204,7 @@ __global__ void __launch_bounds__(kRT) rcwa_epilogue(Bucket b) {
     }
 }
 
-// ---- mirror-symmetric cells: the eigenproblem in four parity classes -------------------------
+// ---- mirror-symmetric cells: the layer problem in its parity classes -------------------------
 // A cell whose pattern is symmetric under x -> -x and under y -> -y (every
 // unrotated shape of rcwa2d.cpp:37-72) at normal incidence (kx0 = ky0 = 0) has
 // Kx odd and Ky even under the order map p -> -p (Px), and Einv, Exx, Eyy
@@ -1195,16 +1216,14 @@ __global__ void __launch_bounds__(kRT) rcwa_epilogue(Bucket b) {
 // orthonormal basis of orbit vectors (the orders (+-p, +-q) of one orbit
 // combined with signs a, b and weight 1/sqrt(count)). With P_c that basis,
 //   M = sum_c P_c M_c P_c^T,  M_c = P_c^T M P_c,
-// so the eigenpairs of M are those of the M_c mapped by P_c: W = [P_c W_c]_c.
-// The eigen-stages then run on matrices of order ~n/4 (16x fewer QR
-// rotations per class, 64x fewer flops each); the S-matrix stages use the
-// full W unchanged, so t, R and T are those of the full eigensolve up to
-// rounding. M_c is built straight from the scalar parity blocks of Exx, Eyy
+// so the layer problem splits into one of order ~n/4 per class, each excitation lies
+// in one class, and the amplitudes of the excited classes are those of the full problem
+// up to rounding. M_c is built straight from the scalar parity blocks of Exx, Eyy
 // and Einv (rcwa_sym_build; the Laurent Einv itself comes from four block
 // inverses), never forming M. A cell whose eps operators are not mirror
 // symmetric to rounding (a raster sample falling exactly on a shape boundary
-// one way and not the other) is flagged kInfoAsym and solved again by the full
-// eigensolve. When the cell is
+// one way and not the other) is flagged kInfoAsym and solved again at full order.
+// When the cell is
 // also symmetric under the 90 degree rotation R (square period, Mx = My,
 // fill_x = fill_y), R commutes with every operator and maps the X excitation
 // onto the Y excitation, so only the X class is solved and the Y solution is R
@@ -1240,30 +1259,6 @@ __device__ int sym_vector(int Mx, int My, int c, int i, int* idx, double* coef) 
             ++k;
         }
     return k;
-}
-
-// Entry (k, l) of a per-order block operator of a homogeneous half-space
-// (non-zero only within one order: the 2 x 2 block of indices i, N + i).
-// which = 0: incident diag(kz) kp^-1 (rcwa2d.cpp:376-388, P1 of the first
-// interface); which = 1: substrate kp diag(1/kz) (K of the last interface).
-__device__ cplx halfspace_entry(const Bucket& b, const CellDev& c, int which, int k, int l) {
-    const int N = b.N;
-    const int ok = k % N, ol = l % N;
-    if (ok != ol) return C(0.0, 0.0);
-    const cplx nr = which == 0 ? c.n_inc : c.n_sub;
-    const cplx er = cmul(nr, nr), ier = cinv(er);
-    const cplx kx = kx_of(b, c, ok), ky = ky_of(b, c, ok);
-    cplx ka, kb, kc, kd;
-    kp_uniform(ier, c.omega, kx, ky, ka, kb, kc, kd);
-    const cplx kz = kz_uniform(er, c.omega, kx, ky);
-    const int r = k / N, s = l / N;
-    if (which == 0) {  // kz [[kd, -kb], [-kc, ka]] / det
-        const cplx idet = cmul(kz, cinv(csub(cmul(ka, kd), cmul(kb, kc))));
-        const cplx v = r == 0 ? (s == 0 ? kd : cneg(kb)) : (s == 0 ? cneg(kc) : ka);
-        return cmul(v, idet);
-    }
-    const cplx v = r == 0 ? (s == 0 ? ka : kb) : (s == 0 ? kc : kd);
-    return cmul(v, cinv(kz));
 }
 
 // Orbit (p, q) >= 0 of index i in scalar parity class (a, bb).
@@ -1315,9 +1310,7 @@ __device__ cplx scalar_block_entry(const cplx* E, int N, int Mx, int My, int a, 
 //   M(v,v) = w^2 Ev[l][m] - Yb[l][s(m)] kx(m) - [l = m] ky^2
 // (the order-space M of rcwa_build_M), the layer kp = w^2 - J Einv J^T
 // (rcwa2d.cpp:346-352) as kp(u,u) = w^2 [i = j] - ky G ky, kp(u,v) = ky G kx,
-// kp(v,u) = kx G ky, kp(v,v) = w^2 [i = j] - kx G kx, and each half-space
-// operator as the 2 x 2 block of an orbit's representative order (|p|, |q|) (its
-// u-v entries are odd in p and in q, the u-u and v-v entries even).
+// kp(v,u) = kx G ky, kp(v,v) = w^2 [i = j] - kx G kx.
 // Flags kInfoAsym when Exx, Eyy or Einv is not mirror symmetric to the
 // tolerance, or, for a C4 bucket (ncls = 1), when Eyy[k][l] != Exx[rho k][rho l]
 // or Einv[rho k][rho l] != Einv[k][l] (rho: order (p, q) -> (-q, p)); these
@@ -1378,7 +1371,7 @@ __global__ void __launch_bounds__(kRT) rcwa_sym_build(Bucket b) {
         if (asym && b.info[cell] == 0) b.info[cell] = kInfoAsym;
     }
     const double w2 = cd.omega * cd.omega;
-    const int m = b.m[0];
+    const int m = b.m;
     cplx* Zs = at(b.Z, b.s_nn, cell);
     cplx* Xs = at(b.X, b.s_nn, cell);
     for (int cc = 0; cc < b.ncls; ++cc) {
@@ -1419,10 +1412,8 @@ __global__ void __launch_bounds__(kRT) rcwa_sym_build(Bucket b) {
         blk_gemm(sv, st, st, C(1.0, 0.0), Lb, st, G, st, C(0.0, 0.0), Yb, st, &gs);
         __syncthreads();
         const size_t mi = (size_t)(b.ncls * cell + cc) * m * m;
-        cplx* Mc = b.sH[0] + mi;
+        cplx* Mc = b.cM + mi;
         cplx* Kp = b.cKp + mi;
-        cplx* C0 = b.cC0 + mi;
-        cplx* Ks = b.cKs + mi;
         for (int e = tid; e < m * m; e += nt) {
             const int i = e / m, j = e % m;
             const bool ui = i < su, uj = j < su;
@@ -1459,197 +1450,470 @@ __global__ void __launch_bounds__(kRT) rcwa_sym_build(Bucket b) {
             }
             Mc[e] = mv;
             Kp[e] = kv;
-            cplx h0 = C(0.0, 0.0), hs = C(0.0, 0.0);
-            if (same) {  // the representative order (|p|, |q|) of the orbit, in each field block
-                const int o = (pi + Mx) * ny + (qi + My);
-                const int k = (ui ? 0 : N) + o, l = (uj ? 0 : N) + o;
-                h0 = halfspace_entry(b, cd, 0, k, l);
-                hs = halfspace_entry(b, cd, 1, k, l);
+        }
+    }
+}
+
+// ---- single layers through their two-port (slab.cuh) ----------------------------------------
+// A half-space's relation h = Y e of an outgoing field (h = a, e = kp q^-1 a, phi = I):
+// Y = diag(kz) kp^-1 couples only the two field components of one order (of one orbit in
+// a parity class): row i of Y holds d at i and o at `pair` (-1: none).
+struct HalfEntry {
+    cplx d, o;
+    int pair;
+};
+// c: parity class, or -1 for the order basis.
+__device__ HalfEntry half_entry(int Mx, int My, const CellDev& cd, cplx nreg, int c, int i) {
+    const int N = (2 * Mx + 1) * (2 * My + 1);
+    HalfEntry h;
+    int p, q;
+    bool u;
+    if (c < 0) {
+        u = i < N;
+        const int o = u ? i : i - N;
+        p = o / (2 * My + 1) - Mx;
+        q = o % (2 * My + 1) - My;
+        h.pair = u ? N + o : o;
+    } else {
+        const int a = sym_class_a(c), b = sym_class_b(c);
+        const int su = sym_count(Mx, a) * sym_count(My, b);
+        u = i < su;
+        // the representative order (|p|, |q|) of the orbit
+        scalar_orbit(My, u ? a : -a, u ? b : -b, u ? i : i - su, p, q);
+        const int j = u ? scalar_orbit_index(My, -a, -b, p, q) : scalar_orbit_index(My, a, b, p, q);
+        h.pair = j < 0 ? -1 : (u ? su + j : j);
+    }
+    const cplx er = cmul(nreg, nreg);
+    const cplx kx = csub(cd.kx0, C(2.0 * PI * (double)p / cd.px, 0.0));
+    const cplx ky = csub(cd.ky0, C(2.0 * PI * (double)q / cd.py, 0.0));
+    cplx ka, kb, kc, kd;
+    kp_uniform(cinv(er), cd.omega, kx, ky, ka, kb, kc, kd);
+    const cplx f = cmul(kz_uniform(er, cd.omega, kx, ky), cinv(csub(cmul(ka, kd), cmul(kb, kc))));
+    h.d = cmul(f, u ? kd : ka);
+    h.o = cneg(cmul(f, u ? kb : kc));
+    return h;
+}
+// The table of a half-space in shared memory (over the panel's region, free outside
+// gauss_jordan); starts and ends on a barrier.
+struct HalfTable {
+    cplx *d, *o;
+    int* pair;
+    __device__ cplx times(const cplx* K, int ld, int r, int c) const {  // (Y K)[r][c]
+        const cplx v = cmul(d[r], K[(size_t)r * ld + c]);
+        return pair[r] < 0 ? v : cfma(o[r], K[(size_t)pair[r] * ld + c], v);
+    }
+};
+__device__ HalfTable half_table(int Mx, int My, const CellDev& cd, cplx nreg, int c, int n, const slab::Shared& s) {
+    HalfTable t;
+    t.d = s.pan;
+    t.o = t.d + n;
+    t.pair = reinterpret_cast<int*>(t.o + n);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const HalfEntry h = half_entry(Mx, My, cd, nreg, c, i);
+        t.d[i] = h.d;
+        t.o[i] = h.o;
+        t.pair[i] = h.pair;
+    }
+    __syncthreads();
+    return t;
+}
+
+// out[r][k] = sum_c A[row(r)][c] v[c][k], k < nr <= 2 (v, out: [n][2]); one warp per row.
+template <class Row>
+__device__ void matvec_rows2(int n, int nr, const cplx* A, int ld, const Row& row, const cplx* v, cplx* out) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    for (int r = warp; r < n; r += nwarp) {
+        const cplx* a = A + (size_t)row(r) * ld;
+        cplx s0 = C(0.0, 0.0), s1 = s0;
+        for (int c = lane; c < n; c += 32) {
+            s0 = cfma(a[c], v[2 * c], s0);
+            if (nr > 1) s1 = cfma(a[c], v[2 * c + 1], s1);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            s0.x += __shfl_down_sync(0xffffffffu, s0.x, o);
+            s0.y += __shfl_down_sync(0xffffffffu, s0.y, o);
+            s1.x += __shfl_down_sync(0xffffffffu, s1.x, o);
+            s1.y += __shfl_down_sync(0xffffffffu, s1.y, o);
+        }
+        if (lane == 0) {
+            out[2 * r] = s0;
+            out[2 * r + 1] = s1;
+        }
+    }
+}
+
+// The excitation a0 of column k at index i: order basis (c < 0) X: e_{N+i0}, Y: -e_{i0}
+// (rcwa2d.cpp:403-411); a class has one column (class 0: Y, class 1: X).
+__device__ double excitation(int Mx, int My, int c, int i, int k) {
+    const int N = (2 * Mx + 1) * (2 * My + 1), i0 = Mx * (2 * My + 1) + My;
+    if (c < 0) return k == 0 ? (i == N + i0 ? 1.0 : 0.0) : (i == i0 ? -1.0 : 0.0);
+    int idx[4];
+    double coef[4];
+    const int cnt = sym_vector(Mx, My, c, i, idx, coef), want = c == 1 ? N + i0 : i0;
+    double v = 0.0;
+    for (int u = 0; u < cnt; ++u)
+        if (idx[u] == want) v += (c == 1 ? 1.0 : -1.0) * coef[u];
+    return v;
+}
+
+// The layer, `slabs` equal slabs (A, B), between its half-spaces. With e = kp g on both
+// sides of an interface,
+//   substrate:  i h = i Ys kp g            ->  load L = -i Ys kp of the last slab,
+//   each slab:  X = (A + L)^-1 B (g at its far side from its near side), Yin = A - B X,
+//               the load of the slab before it,
+//   incident:   i h(0) = -Yin g_0;  2 a0 = (i Yin + Yi kp) g_0,
+//   b0 = a0 - Yi kp g_0,  aN = Ys kp X .. X g_0,
+// Gauss-Jordan solves and products, for the excitation columns only. aN, b0: column k
+// at + k * stride. Returns false at a zero or non-finite pivot.
+template <class T>
+__device__ __noinline__ bool slab_port(int Mx, int My, const CellDev& cd, int c, int n, int slabs, const T* A,
+                                       const T* B, const cplx* Kp, const slab::Work& w, const slab::Shared& s,
+                                       cplx* aN, cplx* b0, size_t stride) {
+    const int tid = threadIdx.x, nt = blockDim.x, nr = c < 0 ? 2 : 1, n2 = 2 * n, ldg = n + 2;
+    cplx *Q = w.q, *G = w.w2, *L = w.e[0], *P = w.e[1], *Pn = w.e[2];
+    HalfTable ys = half_table(Mx, My, cd, cd.n_sub, c, n, s);
+    HalfTable yi;
+    for (int k = slabs; k >= 1; --k) {
+        for (int e = tid; e < n * n; e += nt) {
+            const int r = e / n, j = e - r * n;
+            cplx a = slab::as_cplx(A[e]);
+            if (k == slabs) {
+                const cplx y = ys.times(Kp, n, r, j);
+                a = C(a.x + y.y, a.y - y.x);
+            } else {
+                a = cadd(a, L[e]);
             }
-            C0[e] = h0;
-            Ks[e] = hs;
+            Q[(size_t)r * n2 + j] = a;
+            Q[(size_t)r * n2 + n + j] = slab::as_cplx(B[e]);
+        }
+        if (!slab::gauss_jordan(n, n2, Q, n2, false, s)) return false;
+        for (int i = tid; i < n; i += nt) s.perm2[i] = s.perm[i];
+        yi = half_table(Mx, My, cd, cd.n_inc, c, n, s);
+        if (k > 1) {
+            slab::gemm(n, n, n, B, n, Q + n, n2, s.perm2, [=](int r, int j, cplx v) {
+                const size_t e = (size_t)r * n + j;
+                L[e] = csub(slab::as_cplx(A[e]), v);
+            });
+            // product of the X of the slabs below the first
+            if (k == slabs) {
+                for (int e = tid; e < n * n; e += nt) P[e] = Q[(size_t)s.perm2[e / n] * n2 + n + e % n];
+            } else {
+                slab::gemm(n, n, n, (const cplx*)P, n, (const cplx*)(Q + n), n2, s.perm2,
+                           [=](int r, int j, cplx v) { Pn[(size_t)r * n + j] = v; });
+                cplx* t = P;
+                P = Pn;
+                Pn = t;
+            }
+            __syncthreads();
         }
     }
+    slab::gemm(n, n, n, B, n, Q + n, n2, s.perm2, [=](int r, int j, cplx v) {
+        const cplx yin = csub(slab::as_cplx(A[(size_t)r * n + j]), v), y = yi.times(Kp, n, r, j);
+        G[(size_t)r * ldg + j] = C(y.x - yin.y, y.y + yin.x);
+    });
+    for (int e = tid; e < n * nr; e += nt) {
+        const int r = e / nr, k = e - r * nr;
+        G[(size_t)r * ldg + n + k] = C(2.0 * excitation(Mx, My, c, r, k), 0.0);
+    }
+    if (!slab::gauss_jordan(n, n + nr, G, ldg, false, s)) return false;
+    cplx *g0 = w.v, *gh = g0 + n2, *kg = gh + n2, *kh = kg + n2;
+    for (int e = tid; e < 2 * n; e += nt) {
+        const int r = e >> 1, k = e & 1;
+        g0[e] = k < nr ? G[(size_t)s.perm[r] * ldg + n + k] : C(0.0, 0.0);
+    }
+    __syncthreads();
+    auto same = [](int r) { return r; };
+    const int* xp = s.perm2;
+    matvec_rows2(n, nr, Kp, n, same, g0, kg);
+    matvec_rows2(n, nr, Q + n, n2, [=](int r) { return xp[r]; }, g0, gh);
+    yi = half_table(Mx, My, cd, cd.n_inc, c, n, s);
+    for (int e = tid; e < n * nr; e += nt) {
+        const int r = e / nr, k = e - r * nr;
+        const cplx y = yi.times(kg, 2, r, k);
+        b0[(size_t)k * stride + r] = C(excitation(Mx, My, c, r, k) - y.x, -y.y);
+    }
+    if (slabs > 1) {
+        matvec_rows2(n, nr, P, n, same, gh, g0);
+        gh = g0;
+        __syncthreads();
+    }
+    matvec_rows2(n, nr, Kp, n, same, gh, kh);
+    ys = half_table(Mx, My, cd, cd.n_sub, c, n, s);
+    for (int e = tid; e < n * nr; e += nt) {
+        const int r = e / nr, k = e - r * nr;
+        aN[(size_t)k * stride + r] = ys.times(kh, 2, r, k);
+    }
+    __syncthreads();
+    return true;
 }
 
-// Class S-matrix solves by Gauss-Jordan in shared memory when the widest
-// augmented system [T11 | -T12 D | a0] (m x (2m + 1)) fits in 128 KB (classes
-// up to m = 61, M <= 5 on square cells); larger classes use the blocked LU.
-__host__ __device__ constexpr size_t sym_gj_bytes(int m) {
-    return ((size_t)m * (2 * m + 2) + 2 * (2 * m + 1) + 1) * 16 + 16;
+// M = ep2 kp - kk^T and kp of a layer in the order basis (rcwa2d.cpp:346-352), from
+// Einv, Exx, Eyy: one 2N x N x N product (the layer's Y of rcwa_build_M) whose epilogue
+// writes M. tmp: 2 N^2 complex.
+__device__ void slab_build_full(const Bucket& b, const CellDev& c, int cell, cplx* M, cplx* Kp, cplx* tmp) {
+    const int N = b.N, n = b.n, tid = threadIdx.x, nt = blockDim.x;
+    const cplx* Einv = at(b.Einv, b.s_NN, cell);
+    const cplx* Exx = at(b.Exx, b.s_NN, cell);
+    const cplx* Eyy = b.ng > 0 ? Exx : at(b.Eyy, b.s_NN, cell);
+    const double w2 = c.omega * c.omega;
+    for (int e = tid; e < N * N; e += nt) {
+        const int i = e / N, j = e - i * N;
+        const cplx kxi = kx_of(b, c, i), kyi = ky_of(b, c, i), kxj = kx_of(b, c, j), kyj = ky_of(b, c, j);
+        tmp[e] = cneg(cmul(Eyy[e], kyj));
+        tmp[(size_t)N * N + e] = cmul(Exx[e], kxj);
+        // kp = w^2 - J Einv J^T, J = [-Ky; Kx]
+        const cplx ey = cmul(Einv[e], kyj), ex = cmul(Einv[e], kxj);
+        const cplx d = C(i == j ? w2 : 0.0, 0.0);
+        Kp[(size_t)i * n + j] = csub(d, cmul(kyi, ey));
+        Kp[(size_t)i * n + N + j] = cmul(kyi, ex);
+        Kp[(size_t)(N + i) * n + j] = cmul(kxi, ey);
+        Kp[(size_t)(N + i) * n + N + j] = csub(d, cmul(kxi, ex));
+    }
+    __syncthreads();
+    slab::gemm(2 * N, N, N, (const cplx*)tmp, N, Einv, N, nullptr, [=](int r, int j, cplx y) {
+        const int i = r < N ? r : r - N;
+        const cplx kxj = kx_of(b, c, j), kyj = ky_of(b, c, j);
+        cplx mu = cmul(y, kyj), mv = cneg(cmul(y, kxj));
+        const cplx e = r < N ? Eyy[(size_t)i * N + j] : Exx[(size_t)i * N + j];
+        if (r < N) mu = C(fma(w2, e.x, mu.x), fma(w2, e.y, mu.y));
+        else mv = C(fma(w2, e.x, mv.x), fma(w2, e.y, mv.y));
+        if (i == j) {
+            const cplx ki = r < N ? kxj : kyj;
+            mu = csub(mu, cmul(ki, kxj));
+            mv = csub(mv, cmul(ki, kyj));
+        }
+        M[(size_t)r * n + j] = mu;
+        M[(size_t)r * n + N + j] = mv;
+    });
+    __syncthreads();
 }
-__host__ __device__ constexpr bool sym_gj_fits(int m) { return sym_gj_bytes(m) <= 128 * 1024; }
 
-// The S-matrix of one excited class: rcwa_smat1 and rcwa_smat2 restricted to
-// the class, with the class's one excitation (class 0: Y, a0 = -e_i0; class 1:
-// X, a0 = e_{N+i0}, rcwa2d.cpp:403-411). In the class basis the half-spaces'
-// phi stays I and their kz stays diagonal (kz is even in p and q), so the
-// reference's recursion carries over with every matrix of order m:
-//   A = kp W,  P = C0 A diag(1/q),  T11 = (W + P)/2,  T12 = (W - P)/2,
-//   [S12 | u] = T11^-1 [-T12 D | a0],
-//   Q = diag(q) A^-1 Ks W,  (I + Q - D S12 + D S12 Q) y = 2 D u,
-//   aN = W y,  y2 = (y - Q y)/2,  b0 = T12 (u + S12 y2) + T11 D y2.
-// Writes aN and b0 (class basis) to the class vector area.
-// dynamic smem: sym_smat_smem(m) (LU staging, or the Gauss-Jordan systems)
-__global__ void __launch_bounds__(kRT) rcwa_sym_smat(Bucket b) {
+// One block per cell (order basis) or per solved parity class: the layer's two-port
+// and, unless the cell is a layer of a stack (b.lA), its amplitudes between the
+// half-spaces. 512 threads where a launch has no more matrices than SMs or the order
+// exceeds 128 (the panel's columns then take all sixteen warps), else 256 threads with
+// two blocks per SM.
+template <int NT>
+__global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) rcwa_slab(Bucket b) {
     extern __shared__ __align__(16) unsigned char smem[];
-    cplx* stg = reinterpret_cast<cplx*>(smem);
-    __shared__ GemmSmem gs;
-    __shared__ RedScratch rs;
-    const int mi = blockIdx.x, cell = mi / b.ncls, c = b.cls0 + mi % b.ncls;
+    __shared__ int skip;
+    const int mi = blockIdx.x;
+    const int cell = b.sym ? mi / b.ncls : mi, cc = b.sym ? mi - cell * b.ncls : 0;
+    const int c = b.sym ? b.cls0 + cc : -1, n = b.sym ? b.m : b.n;
     const CellDev cd = b.cells[cell];
-    const int m = b.m[0], N = b.N, Mx = b.Mx, My = b.My;
+    if (threadIdx.x == 0) skip = b.info[cell] != 0;  // flagged by an earlier stage
+    __syncthreads();
+    if (skip) return;
+    cplx *M, *Kp, *base;
+    if (b.sym) {
+        M = b.cM + (size_t)mi * n * n;
+        Kp = b.cKp + (size_t)mi * n * n;
+        base = at(cc ? b.X : b.Z, b.s_nn, cell);  // the class build's scratch, free now
+    } else {
+        M = at(b.H, b.s_nn, cell);
+        Kp = at(b.Kp, b.s_nn, cell);
+        base = b.slab + b.s_w * cell;
+    }
+    slab::Shared s = slab::carve(smem, n);
+    if (b.dbg) s.prof = b.dbg + kDbgSlots * (size_t)mi;
+    const long long t0 = clock64();
+    const slab::Work w = slab::carve_work(base, n);
+    if (!b.sym) slab_build_full(b, cd, cell, M, Kp, w.p);
+    // real arithmetic where M is real up to rounding (a raster that is not inversion
+    // symmetric leaves imaginary parts ~1e-8 of the largest entry)
+    bool real = cd.real_mat != 0;
+    if (real) {
+        double re = 0.0, im = 0.0;
+        for (int e = threadIdx.x; e < n * n; e += NT) {
+            re = fmax(re, fabs(M[e].x));
+            im = fmax(im, fabs(M[e].y));
+        }
+        re = slab::block_max(re, s.red);
+        im = slab::block_max(im, s.red);
+        real = im <= 1e-12 * re;
+    }
+    cplx *aN, *b0;
+    size_t stride;
+    if (b.sym) {
+        aN = b.cvec + (size_t)mi * 2 * n;
+        b0 = aN + n;
+        stride = 0;
+    } else {
+        aN = at(b.vec, 10 * b.s_n, cell);
+        b0 = aN + 2 * b.s_n;
+        stride = b.s_n;
+    }
+    const double qmax = cd.omega * sqrt(fmax(cabs(cd.eps_p), cabs(cd.eps_b)));
+    bool ok;
+    int rest = 0;
+    long long t1 = 0;
+    auto finish = [&](auto* A, auto* B) {
+        t1 = clock64();
+        if (!b.lA) return slab_port(b.Mx, b.My, cd, c, n, 1 << rest, A, B, Kp, w, s, aN, b0, stride);
+        if (threadIdx.x == 0) b.lrest[b.lslot[cell]] = rest;
+        const size_t o = b.s_nn * b.lslot[cell];
+        for (int e = threadIdx.x; e < n * n; e += NT) {
+            b.lA[o + e] = slab::as_cplx(A[e]);
+            b.lB[o + e] = slab::as_cplx(B[e]);
+            b.lK[o + e] = Kp[e];
+        }
+        return true;
+    };
+    if (real) {
+        double *A = nullptr, *B = nullptr;
+        ok = slab::two_port<double>(n, M, cd.h, qmax, w, s, &A, &B, &rest);
+        if (ok) ok = finish(A, B);
+    } else {
+        cplx *A = nullptr, *B = nullptr;
+        ok = slab::two_port<cplx>(n, M, cd.h, qmax, w, s, &A, &B, &rest);
+        if (ok) ok = finish(A, B);
+    }
+    if (!ok && threadIdx.x == 0) atomicCAS(&b.info[cell], 0, kInfoRedo);
+    if (s.prof && threadIdx.x == 0) {
+        s.prof[2] += clock64() - t0;
+        s.prof[3] += clock64() - t1;
+        s.prof[4] += rest;
+    }
+}
+
+// A stack from the two-ports of its layers, from the substrate up: layer l's load L
+// (i h = -L g at its far side) gives X_l = (A + L)^-1 B and the input relation
+// Yin_l = A - B X_l; with e = kp g continuous, g_l(0) = Z_l g_{l-1}(h), Z_l = kp_l^-1 kp_{l-1},
+// the next load is Yin_l Z_l. Then the fields go down: g_l(h) = X_l g_l(0). One block per
+// stack; X_l and Z_l replace A_l and B_l in the layer store. work: slab::work_size(n)
+// complex per stack.
+struct StackPort {
+    int Mx, My, n, nstack;
+    const CellDev* cells;  // shared parameters of each stack (its first layer's descriptor)
+    const int2* stacks;    // (layers, first slot)
+    cplx *lA, *lB, *lK, *work, *vec;
+    const int* lrest;
+    int* info;
+    size_t s_nn, s_w, s_n;
+};
+__global__ void __launch_bounds__(512, 1) rcwa_stack_port(StackPort sp) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int skip;
+    const int st = blockIdx.x, n = sp.n, n2 = 2 * n, ldg = n + 2;
     const int tid = threadIdx.x, nt = blockDim.x;
-    const size_t o2 = (size_t)mi * m * m;
-    const cplx* W = b.sW[0] + o2;
-    const cplx* q = b.sq[0] + (size_t)mi * m;
-    const cplx *Kp = b.cKp + o2, *C0 = b.cC0 + o2, *Ks = b.cKs + o2;
-    cplx *A = b.cA + o2, *T11 = b.cT11 + o2, *T11lu = b.cT11lu + o2, *T12 = b.cT12 + o2;
-    cplx *Q = b.cQ + o2, *SQ = b.cSQ + o2, *Cm = b.cCm + o2;
-    cplx* S = b.cS12 + (size_t)mi * m * (m + 1);
-    cplx* vec = b.cvec + (size_t)mi * 8 * m;  // aN | b0 | y | Q y | y2 | u + S12 y2 | D y2
-    int* piv = b.cpiv + (size_t)mi * m;
-    const int ld = m + 1;
-    const cplx one = C(1.0, 0.0), zero = C(0.0, 0.0);
-    // stage clocks: per-phase clock64 sums in slots 16.. of the cell's counters
-    long long* pf = (b.dbg && tid == 0) ? b.dbg + kDbgSlots * (size_t)mi + 16 : nullptr;
-    long long tp = clock64();
-    auto phase = [&](int k) {
-        if (pf) {
-            const long long t = clock64();
-            pf[k] += t - tp;
-            tp = t;
+    if (tid == 0) skip = sp.info[st] != 0;
+    __syncthreads();
+    if (skip) return;
+    const CellDev cd = sp.cells[st];
+    const int nl = sp.stacks[st].x, slot0 = sp.stacks[st].y;
+    const slab::Shared s = slab::carve(smem, n);
+    const slab::Work w = slab::carve_work(sp.work + sp.s_w * st, n);
+    cplx *Q = w.q, *G = w.w2, *Yin = w.w0, *L = w.w1;
+    bool ok = true;
+    for (int l = nl - 1; l >= 0; --l) {
+        cplx *A = sp.lA + sp.s_nn * (slot0 + l), *B = sp.lB + sp.s_nn * (slot0 + l);
+        const cplx* K = sp.lK + sp.s_nn * (slot0 + l);
+        if (l == nl - 1) {
+            const HalfTable ys = half_table(sp.Mx, sp.My, cd, cd.n_sub, -1, n, s);
+            for (int e = tid; e < n * n; e += nt) {
+                const cplx y = ys.times(K, n, e / n, e % n);
+                L[e] = C(y.y, -y.x);
+            }
+            __syncthreads();
         }
-    };
-    // A = kp W, then P = C0 A (into T12), T11 = (W + P diag(1/q))/2, T12 = (W - P diag(1/q))/2
-    blk_gemm(m, m, m, one, Kp, m, W, m, zero, A, m, &gs);
-    blk_gemm(m, m, m, one, C0, m, A, m, zero, T12, m, &gs);
-    for (int e = tid; e < m * m; e += nt) {
-        const cplx p = cmul(T12[e], cinv(q[e % m]));
-        const cplx w = W[e];
-        const cplx t = cscale(cadd(w, p), 0.5);
-        T11[e] = t;
-        T11lu[e] = t;
-        T12[e] = cscale(csub(w, p), 0.5);
-    }
-    __syncthreads();
-    // [-T12 D | a0]: a0 of the class's excitation in the class basis
-    const int i0 = Mx * (2 * My + 1) + My;
-    const int k0 = c == 1 ? N + i0 : i0;
-    const double s0 = c == 1 ? 1.0 : -1.0;
-    for (int e = tid; e < m * ld; e += nt) {
-        const int i = e / ld, j = e % ld;
-        cplx v;
-        if (j < m) {
-            v = cneg(cmul(T12[(size_t)i * m + j], cexpi(cscale(q[j], cd.h))));
-        } else {
-            int ii[4];
-            double ci[4];
-            const int ni = sym_vector(Mx, My, c, i, ii, ci);
-            double a = 0.0;
-            for (int u = 0; u < ni; ++u)
-                if (ii[u] == k0) a += s0 * ci[u];
-            v = C(a, 0.0);
+        const int slabs = 1 << sp.lrest[slot0 + l];
+        cplx *P = w.e[0], *Pn = w.e[1];
+        for (int k = slabs; k >= 1; --k) {
+            const cplx* load = k == slabs ? L : Yin;
+            for (int e = tid; e < n * n; e += nt) {
+                const int r = e / n, j = e - r * n;
+                Q[(size_t)r * n2 + j] = cadd(A[e], load[e]);
+                Q[(size_t)r * n2 + n + j] = B[e];
+            }
+            ok = slab::gauss_jordan(n, n2, Q, n2, false, s);
+            if (!ok) break;
+            slab::gemm(n, n, n, (const cplx*)B, n, (const cplx*)(Q + n), n2, s.perm,
+                       [=](int r, int j, cplx v) { Yin[(size_t)r * n + j] = csub(A[(size_t)r * n + j], v); });
+            // product of the slabs' X
+            if (k == slabs) {
+                for (int e = tid; e < n * n; e += nt) P[e] = Q[(size_t)s.perm[e / n] * n2 + n + e % n];
+            } else {
+                slab::gemm(n, n, n, (const cplx*)P, n, (const cplx*)(Q + n), n2, s.perm,
+                           [=](int r, int j, cplx v) { Pn[(size_t)r * n + j] = v; });
+                cplx* t = P;
+                P = Pn;
+                Pn = t;
+            }
+            __syncthreads();
         }
-        S[e] = v;
-    }
-    __syncthreads();
-    phase(0);
-    const bool gj = sym_gj_fits(m);
-    const int lg = 2 * m + 1;  // the augmented systems' row stride in shared memory (odd)
-    cplx* gscr = stg + (size_t)m * lg;
-    int* gsp = reinterpret_cast<int*>(gscr + 2 * (2 * m + 1) + 1);
-    // [A | X] (X: nx columns of a global row-major array, ldx) -> X <- A^-1 X in shared memory
-    auto gj_solve = [&](const cplx* Am, int lda, cplx* X, int ldx, int nx) {
-        const int w = m + nx;
-        for (int e = tid; e < m * w; e += nt) {
-            const int i = e / w, j = e % w;
-            stg[i * lg + j] = j < m ? Am[(size_t)i * lda + j] : X[(size_t)i * ldx + j - m];
+        if (!ok) break;
+        for (int e = tid; e < n * n; e += nt) A[e] = P[e];  // X_l
+        __syncthreads();
+        if (l > 0) {
+            const cplx* Ku = sp.lK + sp.s_nn * (slot0 + l - 1);
+            for (int e = tid; e < n * n; e += nt) {
+                const int r = e / n, j = e - r * n;
+                Q[(size_t)r * n2 + j] = K[e];
+                Q[(size_t)r * n2 + n + j] = Ku[e];
+            }
+            ok = slab::gauss_jordan(n, n2, Q, n2, false, s);
+            if (!ok) break;
+            for (int e = tid; e < n * n; e += nt) B[e] = Q[(size_t)s.perm[e / n] * n2 + n + e % n];  // Z_l
+            slab::gemm(n, n, n, (const cplx*)Yin, n, (const cplx*)(Q + n), n2, s.perm,
+                       [=](int r, int j, cplx v) { L[(size_t)r * n + j] = v; });
+            __syncthreads();
         }
-        const int inf = blk_gj_solve_smem(m, nx, stg, lg, gscr, gsp);
-        if (tid == 0 && inf) atomicCAS(&b.info[cell], 0, -inf);
-        for (int e = tid; e < m * nx; e += nt) X[(size_t)(e / nx) * ldx + e % nx] = stg[(e / nx) * lg + m + e % nx];
-        __syncthreads();
-    };
-    int info = 0;
-    if (gj) {
-        gj_solve(T11, m, S, ld, m + 1);  // [S12 | u]
-        phase(1);
-    } else {
-        info = blk_lu_blocked(m, T11lu, m, piv, &rs, stg, &gs);
-        if (tid == 0 && info) atomicCAS(&b.info[cell], 0, -info);
-        __syncthreads();
-        phase(1);
-        blk_lu_solve_blocked(m, T11lu, m, piv, ld, S, ld, stg, &gs);  // [S12 | u]
     }
-    __syncthreads();
-    phase(2);
-    // interface to the substrate: Q = diag(q) A^-1 Ks W
-    blk_gemm(m, m, m, one, Ks, m, W, m, zero, Q, m, &gs);
-    __syncthreads();
-    phase(3);
-    if (gj) {
-        gj_solve(A, m, Q, m, m);
-        phase(4);
-    } else {
-        info = blk_lu_blocked(m, A, m, piv, &rs, stg, &gs);
-        if (tid == 0 && info) atomicCAS(&b.info[cell], 0, -info);
-        __syncthreads();
-        phase(4);
-        blk_lu_solve_blocked(m, A, m, piv, m, Q, m, stg, &gs);
+    if (ok) {
+        const cplx* K0 = sp.lK + sp.s_nn * slot0;
+        HalfTable yi = half_table(sp.Mx, sp.My, cd, cd.n_inc, -1, n, s);
+        for (int e = tid; e < n * n; e += nt) {
+            const int r = e / n, j = e - r * n;
+            const cplx y = yi.times(K0, n, r, j);
+            G[(size_t)r * ldg + j] = C(y.x - Yin[e].y, y.y + Yin[e].x);
+        }
+        for (int e = tid; e < n2; e += nt)
+            G[(size_t)(e >> 1) * ldg + n + (e & 1)] = C(2.0 * excitation(sp.Mx, sp.My, -1, e >> 1, e & 1), 0.0);
+        ok = slab::gauss_jordan(n, n + 2, G, ldg, false, s);
+        if (ok) {
+            cplx *g = w.v, *gn = g + n2, *kg = gn + n2;
+            cplx* aN = sp.vec + 10 * sp.s_n * st;
+            cplx* b0 = aN + 2 * sp.s_n;
+            auto same = [](int r) { return r; };
+            for (int e = tid; e < n2; e += nt) g[e] = G[(size_t)s.perm[e >> 1] * ldg + n + (e & 1)];
+            __syncthreads();
+            matvec_rows2(n, 2, K0, n, same, g, kg);
+            yi = half_table(sp.Mx, sp.My, cd, cd.n_inc, -1, n, s);
+            for (int e = tid; e < n2; e += nt) {
+                const int r = e >> 1, k = e & 1;
+                const cplx y = yi.times(kg, 2, r, k);
+                b0[(size_t)k * sp.s_n + r] = C(excitation(sp.Mx, sp.My, -1, r, k) - y.x, -y.y);
+            }
+            for (int l = 0; l < nl; ++l) {
+                __syncthreads();
+                matvec_rows2(n, 2, sp.lA + sp.s_nn * (slot0 + l), n, same, g, gn);
+                __syncthreads();
+                const bool last = l + 1 == nl;
+                matvec_rows2(n, 2, last ? sp.lK + sp.s_nn * (slot0 + l) : sp.lB + sp.s_nn * (slot0 + l + 1), n, same, gn, g);
+            }
+            const HalfTable ys = half_table(sp.Mx, sp.My, cd, cd.n_sub, -1, n, s);
+            for (int e = tid; e < n2; e += nt) {
+                const int r = e >> 1, k = e & 1;
+                aN[(size_t)k * sp.s_n + r] = ys.times(g, 2, r, k);
+            }
+        }
     }
-    __syncthreads();
-    phase(5);
-    for (int e = tid; e < m * m; e += nt) Q[e] = cmul(q[e / m], Q[e]);
-    blk_gemm(m, m, m, one, S, ld, Q, m, zero, SQ, m, &gs);  // S12 Q
-    __syncthreads();
-    phase(6);
-    cplx *aN = vec, *b0 = vec + m, *y = vec + 2 * m, *Qy = vec + 3 * m, *y2 = vec + 4 * m, *zz = vec + 5 * m,
-         *dy2 = vec + 6 * m;
-    for (int e = tid; e < m * m; e += nt) {
-        const int i = e / m, j = e % m;
-        const cplx d = cexpi(cscale(q[i], cd.h));
-        cplx v = cadd(Q[e], cmul(d, csub(SQ[e], S[(size_t)i * ld + j])));
-        if (i == j) v.x += 1.0;
-        Cm[e] = v;
-    }
-    for (int i = tid; i < m; i += nt) y[i] = cscale(cmul(cexpi(cscale(q[i], cd.h)), S[(size_t)i * ld + m]), 2.0);
-    __syncthreads();
-    if (gj) {
-        gj_solve(Cm, m, y, 1, 1);  // y
-    } else {
-        info = blk_lu_blocked(m, Cm, m, piv, &rs, stg, &gs);
-        if (tid == 0 && info) atomicCAS(&b.info[cell], 0, -info);
-        blk_lu_solve_blocked(m, Cm, m, piv, 1, y, 1, stg, &gs);  // y
-    }
-    blk_gemm(m, 1, m, one, W, m, y, 1, zero, aN, 1, &gs);    // aN = W y
-    blk_gemm(m, 1, m, one, Q, m, y, 1, zero, Qy, 1, &gs);    // Q y
-    for (int i = tid; i < m; i += nt) {
-        const cplx v = cscale(csub(y[i], Qy[i]), 0.5);
-        y2[i] = v;
-        zz[i] = S[(size_t)i * ld + m];                              // u
-        dy2[i] = cmul(cexpi(cscale(q[i], cd.h)), v);                // D y2
-    }
-    blk_gemm(m, 1, m, one, S, ld, y2, 1, one, zz, 1, &gs);    // u + S12 y2
-    blk_gemm(m, 1, m, one, T12, m, zz, 1, zero, b0, 1, &gs);  // T12 (u + S12 y2)
-    blk_gemm(m, 1, m, one, T11, m, dy2, 1, one, b0, 1, &gs);  // + T11 D y2
-    __syncthreads();
-    phase(7);
+    if (!ok && tid == 0) sp.info[st] = kInfoRedo;
 }
 
 // aN and b0 of both excitations into the full basis (the vector area the
-// epilogue reads: aN_X, aN_Y, b0_X, b0_Y); a class eigensolve failure becomes
-// the cell's info (it is the cause of any later singular pivot).
+// epilogue reads: aN_X, aN_Y, b0_X, b0_Y).
 __global__ void __launch_bounds__(kRT) rcwa_sym_expand(Bucket b) {
     const int cell = blockIdx.x;
-    const int N = b.N, n = b.n, Mx = b.Mx, My = b.My, m = b.m[0], ny = 2 * My + 1;
+    const int N = b.N, n = b.n, Mx = b.Mx, My = b.My, m = b.m, ny = 2 * My + 1;
     const int tid = threadIdx.x, nt = blockDim.x;
     cplx* vec = at(b.vec, 10 * b.s_n, cell);
     for (int e = tid; e < 4 * (int)b.s_n; e += nt) vec[e] = C(0.0, 0.0);
     __syncthreads();
     for (int cc = 0; cc < b.ncls; ++cc) {
         const int c = b.cls0 + cc, mi = b.ncls * cell + cc;
-        const cplx* cv = b.cvec + (size_t)mi * 8 * m;
+        const cplx* cv = b.cvec + (size_t)mi * 2 * m;
         cplx* dst_a = vec + (c == 1 ? 0 : b.s_n);       // aN_X : aN_Y
         cplx* dst_b = vec + (c == 1 ? 2 : 3) * b.s_n;   // b0_X : b0_Y
         for (int i = tid; i < m; i += nt) {
@@ -1676,38 +1940,6 @@ __global__ void __launch_bounds__(kRT) rcwa_sym_expand(Bucket b) {
             vec[3 * b.s_n + rk] = cscale(vec[2 * b.s_n + k], sg);
         }
     }
-    if (tid == 0 && b.info[cell] != kInfoAsym) {
-        for (int cc = 0; cc < b.ncls; ++cc) {
-            const int e = b.sinfo[0][b.ncls * cell + cc];
-            if (e != 0) {
-                b.info[cell] = e;
-                break;
-            }
-        }
-    }
-}
-
-// The eigen-stage bucket of size class k of a mirror-symmetric bucket.
-Bucket sym_eig_bucket(const Bucket& b, int k) {
-    Bucket e;
-    std::memset(&e, 0, sizeof(e));
-    e.Mx = b.Mx;
-    e.My = b.My;
-    e.n = b.m[k];
-    e.N = e.n / 2;
-    e.ncell = b.ncls * b.ncell;
-    e.cells = b.cells;
-    e.H = b.sH[k];
-    e.Z = b.sZ[k];
-    e.X = b.sX[k];
-    e.W = b.sW[k];
-    e.A = b.sA[k];
-    e.q1 = b.sq[k];
-    e.info = b.sinfo[k];
-    e.dbg = b.dbg;  // the stage-clock counters hold 2 slots per cell
-    e.s_nn = (size_t)e.n * e.n;
-    e.s_n = (size_t)e.n;
-    return e;
 }
 
 // ---- host side ------------------------------------------------------------------------------------
@@ -1715,10 +1947,11 @@ struct HostCell {
     CellDev d;
     int Mx, My, ng;  // ng = 0: analytic rect path
     int index;       // position in the caller's array
-    int sym;         // 1: mirror-symmetric cell at normal incidence (eigenproblem in parity classes)
+    int sym;         // 1: mirror-symmetric cell at normal incidence (solved in its parity classes); 2: and C4
+    int qr;          // 1: through the eigendecomposition (QR) instead of the layer two-port
 };
 
-// The parity-class eigensolve applies to unrotated shapes (all mirror
+// The parity classes apply to unrotated shapes (all mirror
 // symmetric, rcwa2d.cpp:37-72) at normal incidence with at least one order on
 // each side of 0 in x and y; CELERIS_RCWA_SYMMETRY=0 turns it off.
 bool symmetry_enabled() {
@@ -1729,13 +1962,28 @@ bool symmetry_enabled() {
 // of each eps operator (Exx, Eyy, Einv and the Laurent coefficients): rounding
 // leaves ~1e-15; one raster sample on the other side of a shape boundary
 // ~1e-6. CELERIS_RCWA_SYM_TOL overrides it (the test is strict, so 0 sends
-// every cell to the full eigensolve through the fallback, for tests of that path).
+// every cell to the full order through the fallback, for tests of that path).
 double symmetry_tolerance() {
     const char* e = std::getenv("CELERIS_RCWA_SYM_TOL");
     return e ? std::atof(e) : 1e-9;
 }
 bool sym_eligible(const celeris_rcwa_cell& c) {
     return c.theta_rad == 0.0 && c.rotation_rad == 0.0 && c.Mx >= 1 && c.My >= 1 && symmetry_enabled();
+}
+
+// Cells the two-port does not take: orders above its limit; layers thinner than k0 h =
+// 0.01 (~1 nm in the visible; A and B are ~1 / h and only their difference counts, so
+// digits go as 1 / (k0 h)), zero and negative thicknesses with them; layers of more than
+// 100 rad of optical phase (every doubling past pi / 2 may meet a mode's pole); and every
+// cell while the QR iteration cap of the failure-path tests is set (the cap is about
+// the eigendecomposition).
+std::atomic<int> g_qr_cap_set{0};
+bool needs_qr(const celeris_rcwa_cell& c) {
+    const int n = 2 * (2 * c.Mx + 1) * (2 * c.My + 1);
+    const int order = sym_eligible(c) ? sym_class_size(c.Mx, c.My, 0) : n;
+    const double kh = 2.0 * PI / c.wavelength_um * c.thickness_um;
+    const double eps = std::max(std::hypot(c.eps_pillar[0], c.eps_pillar[1]), std::hypot(c.eps_bg[0], c.eps_bg[1]));
+    return order > slab::kMaxOrder || !(kh >= 0.01) || !(kh * std::sqrt(eps) <= 100.0) || g_qr_cap_set.load() != 0;
 }
 
 int validate(const celeris_rcwa_cell& c) {
@@ -1786,6 +2034,7 @@ HostCell make_cell(const celeris_rcwa_cell& c, int index, double ex_re, double e
     d.ey0 = make_double2(ey_re, ey_im);
     d.shape = c.shape;
     d.nexc = nexc;
+    d.real_mat = c.eps_pillar[1] == 0.0 && c.eps_bg[1] == 0.0 && d.kx0.y == 0.0 && d.ky0.y == 0.0;
     h.Mx = c.Mx;
     h.My = c.My;
     const bool plain_rect = c.shape == CELERIS_SHAPE_RECT && c.rotation_rad == 0.0 && !c.force_laurent;
@@ -1797,6 +2046,8 @@ HostCell make_cell(const celeris_rcwa_cell& c, int index, double ex_re, double e
     // the Y solution is the rotated X solution and one class is solved
     h.sym = !sym_eligible(c) ? 0
             : (c.period_x_um == c.period_y_um && c.Mx == c.My && c.fill_x == c.fill_y) ? 2 : 1;
+    h.qr = needs_qr(c) ? 1 : 0;
+    if (h.qr) h.sym = 0;
     return h;
 }
 
@@ -1827,9 +2078,16 @@ size_t hess_stage_bytes(int n) { return (size_t)(n + LNB * LNB + 2 * LNB) * size
 // staging of blk_lu_blocked and the matvecs of the S-matrix kernels
 size_t lu_stage_bytes(int n) { return (size_t)(2 * n + LNB * LNB) * sizeof(cplx); }
 
-// dynamic shared memory of rcwa_sym_smat for class order m
-size_t sym_smat_smem(int m) {
-    return std::max(lu_stage_bytes(m), sym_gj_fits(m) ? sym_gj_bytes(m) : (size_t)0);
+// Threads of rcwa_slab for `count` matrices of order n.
+int slab_threads(int n, int count) {
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (sms <= 0) sms = 1;
+    }
+    return n > 128 || count <= sms ? 512 : 256;
 }
 
 size_t laurent_smem(int Mx, int My, int ng) {
@@ -1874,7 +2132,7 @@ bool tuning_enabled() {
 }
 
 struct BucketPlan {
-    int Mx, My, ng, N, n, sym;
+    int Mx, My, ng, N, n, sym, qr;
     std::vector<int> ids;  // indices into the cell list
     size_t per_cell = 0, bytes = 0;
     Bucket b;
@@ -1888,41 +2146,45 @@ size_t per_cell_bytes(int n, int nexc) {
            celeris_rt::align256(sizeof(CellDev)) + 14 * 256;
 }
 
-// Device memory of one mirror-symmetric cell: of the full-order buffers only
-// H (M, and the Laurent LU scratch), Z, X (build_M's products), the Fourier
-// operators, the vector area and pivots; per excited class (two per cell) the
-// eigen-stage matrices H, Z, X, W, scratch, q and info, and the class S-matrix's
-// ten m x m matrices, S12 (m x (m + 1)), 8 m vector entries and m pivots.
+// Device memory of one order-basis cell solved through its two-port: M, kp, the
+// two-port's work area, the Fourier operators, the vector area and pivots.
+size_t slab_per_cell_bytes(int n, int nexc) {
+    const size_t N = n / 2, s_nn = (size_t)n * n;
+    return (2 * s_nn + slab::work_size(n) + 3 * N * N + 10 * (size_t)n) * sizeof(cplx) + (size_t)n * sizeof(int) +
+           sizeof(int) + sizeof(celeris_rcwa_result) * nexc + sizeof(CellDev) + 16 * 256;
+}
+
+// Device memory of one mirror-symmetric cell: the full-order H (the Laurent inverse's
+// blocks), Z and X (the class build's scratch, then the two-port's work areas), the
+// Fourier operators, the vector area and pivots; per solved class M, kp and 2 m
+// amplitudes.
 size_t sym_per_cell_bytes(int Mx, int My, int nexc, int ncls) {
     const int N = (2 * Mx + 1) * (2 * My + 1), n = 2 * N;
     const size_t m = (size_t)sym_class_size(Mx, My, 0);
     const size_t full = (3 * (size_t)n * n + 3 * (size_t)N * N + 10 * (size_t)n) * sizeof(cplx) +
                         (size_t)n * sizeof(int) + sizeof(int) + sizeof(celeris_rcwa_result) * nexc + sizeof(CellDev);
-    const size_t cls = ncls * (((5 * m * m + m) * sizeof(cplx) + sizeof(int)) +
-                               ((10 * m * m + m * (m + 1) + 8 * m) * sizeof(cplx) + m * sizeof(int)));
-    return full + cls + 32 * 256;
+    return full + ncls * (2 * m * m + 2 * m) * sizeof(cplx) + 20 * 256;
 }
 
 // The largest dynamic shared memory each stage kernel needs over a wave's
 // buckets; raised once per wave, outside any capture.
 struct SmemNeeds {
-    size_t laurent = 0, rect = 0, hess_s = 0, hess_g = 0, smat = 0, smat_sym = 0;
+    size_t laurent = 0, rect = 0, hess_s = 0, hess_g = 0, smat = 0, slab = 0;
     bool aed = false;
     void add_eig(int n) {
         if (n <= kSmemEigMaxN) hess_s = std::max(hess_s, ((size_t)n * n + 2 * n) * sizeof(cplx));
         else hess_g = std::max(hess_g, hess_stage_bytes(n));
         aed = true;
     }
-    void add(int Mx, int My, int ng, int n, int sym = 0) {
+    void add(int Mx, int My, int ng, int n, int sym = 0, int qr = 1) {
         if (ng > 0) {
             laurent = std::max(laurent, laurent_smem(Mx, My, ng));
         } else {
             const int nx = 2 * Mx + 1, ny = 2 * My + 1;
             rect = std::max(rect, ((size_t)2 * (nx * nx + ny * ny) + 2 * std::max(nx, ny)) * sizeof(cplx));
         }
-        if (sym) {
-            add_eig(sym_class_size(Mx, My, 0));
-            smat_sym = std::max(smat_sym, sym_smat_smem(sym_class_size(Mx, My, 0)));
+        if (!qr) {
+            slab = std::max(slab, slab::shared_bytes(sym ? sym_class_size(Mx, My, 0) : n));
         } else {
             add_eig(n);
             smat = std::max(smat, lu_stage_bytes(n));
@@ -1963,14 +2225,19 @@ int set_smem_limits(const SmemNeeds& s) {
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_smat1), s.smat));
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_smat2), s.smat));
     }
-    if (s.smat_sym) CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_sym_smat), s.smat_sym));
+    if (s.slab) {
+        CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_slab<256>), s.slab));
+        CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_slab<512>), s.slab));
+    }
     return CELERIS_OK;
 }
 
 // Launch the stage sequence of one bucket on `st`. ev (ST_COUNT + 1 events) is
 // optional: stage boundaries are recorded into it.
 // eig_only: stop after the eigenvectors (the layers of a multi-layer stack).
-void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEvent_t* ev, bool eig_only = false) {
+// qr: through the eigendecomposition (order basis), else through the layer two-port.
+void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEvent_t* ev, bool qr,
+                   bool eig_only = false) {
     const int nc = b.ncell, n = b.n;
     const int* T = cfg.threads;
     if (ev) cudaEventRecord(ev[0], st);
@@ -1988,32 +2255,23 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
         count_launch(1);
     }
     if (ev) cudaEventRecord(ev[1], st);
-    if (b.sym) {
-        // the excited parity classes: their operators (in place of build_M),
-        // eigen-stages (ncls matrices of order m[0] per cell), the class
-        // S-matrix, expand into the epilogue's vectors
-        rcwa_sym_build<<<nc, T[ST_BUILD], 0, st>>>(b);
-        if (ev) cudaEventRecord(ev[2], st);
-        const Bucket e = sym_eig_bucket(b, 0);
-        cudaMemsetAsync(e.info, 0, sizeof(int) * e.ncell, st);
-        const int m = e.n;
-        if (m <= kSmemEigMaxN)
-            rcwa_hess<true><<<e.ncell, hess_smem_threads(m, T[ST_HESS]), ((size_t)m * m + 2 * m) * sizeof(cplx),
-                              st>>>(e);
+    if (!qr) {
+        // the layer two-port: class operators first for mirror-symmetric cells, then one
+        // kernel (timed as smat1), the amplitudes into the order basis, the outputs
+        if (b.sym) rcwa_sym_build<<<nc, T[ST_BUILD], 0, st>>>(b);
+        if (ev)
+            for (int i = 2; i <= 5; ++i) cudaEventRecord(ev[i], st);
+        const int m = b.sym ? b.m : n, count = b.sym ? b.ncls * nc : nc;
+        if (slab_threads(m, count) == 512)
+            rcwa_slab<512><<<count, 512, slab::shared_bytes(m), st>>>(b);
         else
-            rcwa_hess<false><<<e.ncell, T[ST_HESS], hess_stage_bytes(m), st>>>(e);
-        if (ev) cudaEventRecord(ev[3], st);
-        rcwa_schur<<<e.ncell, kSchurThreads, schur_smem(e.ncell), st>>>(e);
-        if (ev) cudaEventRecord(ev[4], st);
-        rcwa_vec<<<e.ncell, T[ST_VEC], 0, st>>>(e);
-        if (ev) cudaEventRecord(ev[5], st);
-        rcwa_sym_smat<<<e.ncell, T[ST_SMAT1], sym_smat_smem(m), st>>>(b);
+            rcwa_slab<256><<<count, 256, slab::shared_bytes(m), st>>>(b);
         if (ev) cudaEventRecord(ev[6], st);
-        rcwa_sym_expand<<<nc, T[ST_SMAT2], 0, st>>>(b);
+        if (b.sym) rcwa_sym_expand<<<nc, T[ST_SMAT2], 0, st>>>(b);
         if (ev) cudaEventRecord(ev[7], st);
-        rcwa_epilogue<<<nc, T[ST_EPI], 0, st>>>(b);
+        if (!b.lA) rcwa_epilogue<<<nc, T[ST_EPI], 0, st>>>(b);
         if (ev) cudaEventRecord(ev[8], st);
-        count_launch(7);
+        count_launch((b.sym ? 3 : 1) + (b.lA ? 0 : 1));
         return;
     }
     rcwa_build_M<<<nc, T[ST_BUILD], 0, st>>>(b, b.ng > 0 ? 1 : 0);
@@ -2058,7 +2316,7 @@ int autotune(const BucketPlan& p, cudaStream_t st, StageCfg* out) {
     float best[ST_COUNT];
     StageCfg cfg = uniform_cfg(256);
     for (int c = 0; c < 2; ++c) {
-        launch_bucket(t, uniform_cfg(kCand[c]), st, ev);
+        launch_bucket(t, uniform_cfg(kCand[c]), st, ev, p.qr != 0);
         CEL_CUDA(cudaStreamSynchronize(st));
         for (int s = 0; s < ST_COUNT; ++s) {
             float ms = 0.f;
@@ -2176,9 +2434,9 @@ size_t cached_free_memory(int dev) {
 int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_out, int nexc) {
     CEL_TRY(celeris_rt::require_device());
     // ---- plan: buckets by (Mx, My, raster), largest first so they start first
-    std::map<std::tuple<int, int, int, int>, std::vector<int>> by;
+    std::map<std::tuple<int, int, int, int, int>, std::vector<int>> by;
     for (int i = 0; i < (int)cells.size(); ++i)
-        by[std::make_tuple(cells[i].Mx, cells[i].My, cells[i].ng, cells[i].sym)].push_back(i);
+        by[std::make_tuple(cells[i].Mx, cells[i].My, cells[i].ng, cells[i].sym, cells[i].qr)].push_back(i);
     std::vector<BucketPlan> plans;
     std::vector<std::vector<int>> waves;
     CEL_TRY(ensure_streams(1));
@@ -2206,11 +2464,14 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             p.My = std::get<1>(kv.first);
             p.ng = std::get<2>(kv.first);
             p.sym = std::get<3>(kv.first);
+            p.qr = std::get<4>(kv.first);
             p.N = (2 * p.Mx + 1) * (2 * p.My + 1);
             p.n = 2 * p.N;
             if (p.ng > 0 && laurent_smem(p.Mx, p.My, p.ng) + 1024 > (size_t)smem_optin)
                 return set_error(CELERIS_ERR_TOO_LARGE, "raster %d with M=(%d,%d) exceeds shared memory", p.ng, p.Mx, p.My);
-            p.per_cell = p.sym ? sym_per_cell_bytes(p.Mx, p.My, nexc, p.sym == 2 ? 1 : 2) : per_cell_bytes(p.n, nexc);
+            p.per_cell = p.qr    ? per_cell_bytes(p.n, nexc)
+                         : p.sym ? sym_per_cell_bytes(p.Mx, p.My, nexc, p.sym == 2 ? 1 : 2)
+                                 : slab_per_cell_bytes(p.n, nexc);
             // split buckets that alone exceed the budget
             const size_t max_cells = std::max<size_t>(1, budget / std::max<size_t>(1, p.per_cell));
             for (size_t c0 = 0; c0 < kv.second.size(); c0 += max_cells) {
@@ -2308,15 +2569,23 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             b.s_n = (size_t)p.n;
             CellDev* dcells = static_cast<CellDev*>(ws.take(sizeof(CellDev) * nc));
             b.cells = dcells;
-            // full-order buffers: the class path needs only H, Z, X (M and
-            // build_M's products) besides the Fourier operators and vectors
-            cplx** mats[] = {&b.H, &b.Z, &b.X, &b.W, &b.A, &b.T11, &b.T11lu, &b.T12};
-            for (int k = 0; k < (p.sym ? 3 : 8); ++k) *mats[k] = static_cast<cplx*>(ws.take(sizeof(cplx) * b.s_nn * nc));
-            if (!p.sym) b.S12 = static_cast<cplx*>(ws.take(sizeof(cplx) * b.s_ns * nc));
+            auto take = [&](size_t count) { return static_cast<cplx*>(ws.take(sizeof(cplx) * count)); };
+            if (p.qr) {
+                cplx** mats[] = {&b.H, &b.Z, &b.X, &b.W, &b.A, &b.T11, &b.T11lu, &b.T12};
+                for (cplx** m : mats) *m = take(b.s_nn * nc);
+                b.S12 = take(b.s_ns * nc);
+                b.q1 = take(b.s_n * nc);
+            } else if (p.sym) {
+                for (cplx** m : {&b.H, &b.Z, &b.X}) *m = take(b.s_nn * nc);
+            } else {
+                b.H = take(b.s_nn * nc);
+                b.Kp = take(b.s_nn * nc);
+                b.s_w = slab::work_size(p.n);
+                b.slab = take(b.s_w * nc);
+            }
             b.Einv = static_cast<cplx*>(ws.take(sizeof(cplx) * b.s_NN * nc));
             b.Exx = static_cast<cplx*>(ws.take(sizeof(cplx) * b.s_NN * nc));
             b.Eyy = static_cast<cplx*>(ws.take(sizeof(cplx) * b.s_NN * nc));
-            if (!p.sym) b.q1 = static_cast<cplx*>(ws.take(sizeof(cplx) * b.s_n * nc));
             b.vec = static_cast<cplx*>(ws.take(sizeof(cplx) * 10 * b.s_n * nc));
             b.piv = static_cast<int*>(ws.take(sizeof(int) * b.s_n * nc));
             b.info = static_cast<int*>(ws.take(sizeof(int) * nc));
@@ -2328,22 +2597,14 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             b.sym = p.sym;
             b.sym_tol = symmetry_tolerance();
             if (p.sym) {
-                // the two excited classes (order m[0]), two matrices per cell
+                // the excited classes of order m
                 b.ncls = p.sym == 2 ? 1 : 2;
                 b.cls0 = p.sym == 2 ? 1 : 0;
-                const size_t nm = (size_t)b.ncls * nc;  // class matrices in the bucket
-                const size_t m = (size_t)sym_class_size(p.Mx, p.My, 0), mm = m * m * nm;
-                b.m[0] = (int)m;
-                b.m[1] = sym_class_size(p.Mx, p.My, 2);
-                cplx** sm[] = {&b.sH[0], &b.sZ[0], &b.sX[0], &b.sW[0], &b.sA[0]};
-                for (cplx** x : sm) *x = static_cast<cplx*>(ws.take(sizeof(cplx) * mm));
-                b.sq[0] = static_cast<cplx*>(ws.take(sizeof(cplx) * m * nm));
-                b.sinfo[0] = static_cast<int*>(ws.take(sizeof(int) * nm));
-                cplx** cm[] = {&b.cKp, &b.cC0, &b.cKs, &b.cA, &b.cT11, &b.cT11lu, &b.cT12, &b.cQ, &b.cSQ, &b.cCm};
-                for (cplx** x : cm) *x = static_cast<cplx*>(ws.take(sizeof(cplx) * mm));
-                b.cS12 = static_cast<cplx*>(ws.take(sizeof(cplx) * m * (m + 1) * nm));
-                b.cvec = static_cast<cplx*>(ws.take(sizeof(cplx) * 8 * m * nm));
-                b.cpiv = static_cast<int*>(ws.take(sizeof(int) * m * nm));
+                b.m = sym_class_size(p.Mx, p.My, 0);
+                const size_t nm = (size_t)b.ncls * nc, m = (size_t)b.m;  // class matrices in the bucket
+                b.cM = take(m * m * nm);
+                b.cKp = take(m * m * nm);
+                b.cvec = take(2 * m * nm);
             }
             hdesc[w] = reinterpret_cast<CellDev*>(pin);
             pin += celeris_rt::align256(sizeof(CellDev) * nc);
@@ -2352,9 +2613,9 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             hinfo_pin[w] = reinterpret_cast<int*>(pin);
             pin += celeris_rt::align256(sizeof(int) * nc);
             for (int i = 0; i < nc; ++i) hdesc[w][i] = cells[p.ids[i]].d;
-            needs.add(p.Mx, p.My, p.ng, p.n, p.sym);
+            needs.add(p.Mx, p.My, p.ng, p.n, p.sym, p.qr);
             sig += "|" + std::to_string(p.Mx) + "," + std::to_string(p.My) + "," + std::to_string(p.ng) + "," +
-                   std::to_string(p.sym) + "," + std::to_string(nc) + "," + std::to_string(b.sym_tol);
+                   std::to_string(p.sym) + "," + std::to_string(p.qr) + "," + std::to_string(nc) + "," + std::to_string(b.sym_tol);
         }
         CEL_TRY(set_smem_limits(needs));
         // ---- tune unseen bucket shapes (descriptors must be on the device)
@@ -2364,7 +2625,7 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             // key: shape and batch class (fewer than, or at least, one cell per SM)
             int sms = 148;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            const auto key = std::make_tuple(p.Mx, p.My, 4 * p.ng + 2 * p.sym + ((int)p.ids.size() >= sms ? 1 : 0));
+            const auto key = std::make_tuple(p.Mx, p.My, 8 * p.ng + (p.qr ? 0 : 4) + 2 * (p.sym != 0) + ((int)p.ids.size() >= sms ? 1 : 0));
             bool have = false;
             {
                 std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -2396,7 +2657,7 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                 p.b.dbg = dbg;
                 cudaEvent_t ev[ST_COUNT + 1];
                 for (auto& e : ev) cudaEventCreate(&e);
-                launch_bucket(p.b, cfgs[w], st, ev);
+                launch_bucket(p.b, cfgs[w], st, ev, p.qr != 0);
                 CEL_CUDA(cudaMemcpyAsync(hres_pin[w], p.b.res, sizeof(celeris_rcwa_result) * nexc * nc,
                                          cudaMemcpyDeviceToHost, st));
                 CEL_CUDA(cudaMemcpyAsync(hinfo_pin[w], p.b.info, sizeof(int) * nc, cudaMemcpyDeviceToHost, st));
@@ -2415,6 +2676,17 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                     char buf[64];
                     std::snprintf(buf, sizeof(buf), " %s %.2f", kStageNames[s], ms);
                     line += buf;
+                }
+                if (!p.qr) {
+                    char b3[256];
+                    std::snprintf(b3, sizeof(b3), " | two-port Mcycles/cell: %.3f (between the half-spaces %.3f); panels %.3f, their updates %.3f; "
+                                  "left-out doublings %.3f\n",
+                                  ph[2] / nc * 1e-6, ph[3] / nc * 1e-6, ph[0] / nc * 1e-6, ph[1] / nc * 1e-6, ph[4] / nc);
+                    std::fprintf(stderr, "%s%s", line.c_str(), b3);
+                    for (auto& e : ev) cudaEventDestroy(e);
+                    cudaFree(dbg);
+                    p.b.dbg = nullptr;
+                    continue;
                 }
                 char buf[64];
                 std::snprintf(buf, sizeof(buf), " | sweeps/cell %.1f", sw / nc);
@@ -2454,8 +2726,8 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                     cudaStreamWaitEvent(bs, ctx.fork[w], 0);
                     cudaMemcpyAsync(const_cast<CellDev*>(p.b.cells), hdesc[w], sizeof(CellDev) * nc,
                                     cudaMemcpyHostToDevice, bs);
-                    launch_bucket(p.b, cfgs[w], bs, nullptr);
-                    nk += (p.ng > 0 ? 3 : 1) + 7;
+                    launch_bucket(p.b, cfgs[w], bs, nullptr, p.qr != 0);
+                    nk += (p.ng > 0 ? 3 : 1) + (p.qr ? 7 : p.sym ? 4 : 2);
                     cudaMemcpyAsync(hres_pin[w], p.b.res, sizeof(celeris_rcwa_result) * nexc * nc,
                                     cudaMemcpyDeviceToHost, bs);
                     cudaMemcpyAsync(hinfo_pin[w], p.b.info, sizeof(int) * nc, cudaMemcpyDeviceToHost, bs);
@@ -2488,11 +2760,11 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             }
         }
     }
-    // cells flagged as not mirror symmetric to rounding: solve again with the
-    // full eigensolve
+    // cells flagged as not mirror symmetric to rounding are solved again at full order,
+    // cells whose two-port was ill conditioned through the eigendecomposition
     std::vector<int> redo;
     for (size_t i = 0; i < hinfo.size(); ++i)
-        if (hinfo[i] == kInfoAsym) redo.push_back((int)i);
+        if (hinfo[i] == kInfoAsym || hinfo[i] == kInfoRedo) redo.push_back((int)i);
     if (!redo.empty()) {
         std::vector<int> pos(cells.size(), -1);
         for (int i = 0; i < (int)cells.size(); ++i) pos[cells[i].index] = i;
@@ -2500,6 +2772,7 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
         for (size_t j = 0; j < redo.size(); ++j) {
             HostCell h = cells[pos[redo[j]]];
             h.sym = 0;
+            h.qr = h.qr || hinfo[redo[j]] == kInfoRedo || 2 * (2 * h.Mx + 1) * (2 * h.My + 1) > slab::kMaxOrder;
             h.index = (int)j;
             sub.push_back(h);
         }
@@ -2548,8 +2821,9 @@ size_t a256(size_t b) { return celeris_rt::align256(std::max<size_t>(b, 1)); }
 // stacks[s] = (first layer index, layer count) into `layers`; exc holds 4 doubles
 // (Ex0 re, im, Ey0 re, im) per stack; results nexc per stack.
 // ord_out (may be NULL): per stack and excitation N x (de_t, de_r).
-int run_stacks(const celeris_rcwa_cell* layers, const std::vector<std::pair<int, int>>& stacks,
-               const double* exc, celeris_rcwa_result* out, int* info_out, int nexc, double* ord_out = nullptr) {
+// Through the eigendecompositions of the layers (rcwa_stack_smat).
+int run_stacks_qr(const celeris_rcwa_cell* layers, const std::vector<std::pair<int, int>>& stacks,
+                  const double* exc, celeris_rcwa_result* out, int* info_out, int nexc, double* ord_out) {
     CEL_TRY(celeris_rt::require_device());
     int dev = 0, smem_optin = 0;
     cudaGetDevice(&dev);
@@ -2675,7 +2949,7 @@ int run_stacks(const celeris_rcwa_cell* layers, const std::vector<std::pair<int,
                 SmemNeeds needs;
                 needs.add(Mx, My, ng, n);
                 CEL_TRY(set_smem_limits(needs));
-                launch_bucket(b, uniform_cfg(256), st, nullptr, true);
+                launch_bucket(b, uniform_cfg(256), st, nullptr, true, true);
                 rcwa_layer_out<<<nc, kRT, 0, st>>>(b, LW, LA, Lq, Lh, dslot);
                 count_launch(1);
                 CEL_CUDA(cudaGetLastError());
@@ -2774,6 +3048,275 @@ int run_stacks(const celeris_rcwa_cell* layers, const std::vector<std::pair<int,
                         return set_error(CELERIS_ERR_SINGULAR, "singular interface system (stack %d)", ids[k]);
                 }
         }
+    }
+    return CELERIS_OK;
+}
+
+// The same through the layers' two-ports (rcwa_slab, rcwa_stack_port). info_out (required):
+// 0 or kInfoRedo per stack; results of flagged stacks are not written.
+int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair<int, int>>& stacks, const double* exc,
+                    celeris_rcwa_result* out, int* info_out, int nexc, double* ord_out) {
+    CEL_TRY(celeris_rt::require_device());
+    int dev = 0, smem_optin = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    static thread_local celeris_rt::ThreadStream t_slab_st;
+    cudaStream_t st = nullptr;
+    CEL_TRY(t_slab_st.get(&st));
+    Workspace& ws = Workspace::for_stream(st);
+    // stacks grouped by (Mx, My): one layer store and one recursion launch per group
+    std::map<std::pair<int, int>, std::vector<int>> groups;
+    for (int s = 0; s < (int)stacks.size(); ++s) {
+        const celeris_rcwa_cell& f = layers[stacks[s].first];
+        groups[{f.Mx, f.My}].push_back(s);
+    }
+    size_t free_b = 0, total_b = 0;
+    CEL_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const size_t budget = (free_b + ws.capacity()) / 2;
+    const size_t c16 = sizeof(cplx);
+    for (auto& g : groups) {
+        const int Mx = g.first.first, My = g.first.second;
+        const int N = (2 * Mx + 1) * (2 * My + 1), n = 2 * N;
+        const size_t s_nn = (size_t)n * n, s_n = (size_t)n, s_NN = (size_t)N * N, s_w = slab::work_size(n);
+        const size_t per_layer = (5 * s_nn + s_w + 3 * s_NN) * c16 + 4096;
+        const size_t per_stack = (s_w + 10 * s_n) * c16 + (size_t)nexc * N * 2 * sizeof(double) + 4096;
+        size_t c0 = 0;
+        while (c0 < g.second.size()) {
+            std::vector<int> ids;
+            size_t bytes = 0;
+            while (c0 < g.second.size()) {
+                const size_t need = per_stack + per_layer * stacks[g.second[c0]].second;
+                if (!ids.empty() && bytes + need > budget) break;
+                ids.push_back(g.second[c0++]);
+                bytes += need;
+            }
+            const int ns = (int)ids.size();
+            std::vector<HostCell> sub;
+            std::vector<int2> hs(ns);
+            std::vector<CellDev> hc(ns);
+            std::vector<int> hinfo(ns, 0);
+            for (int k = 0; k < ns; ++k) {
+                const auto& sp = stacks[ids[k]];
+                const double* e = exc + 4 * (size_t)ids[k];
+                hs[k] = make_int2(sp.second, (int)sub.size());
+                hc[k] = make_cell(layers[sp.first], ids[k], e[0], e[1], e[2], e[3], nexc).d;
+                for (int l = 0; l < sp.second; ++l)
+                    sub.push_back(make_cell(layers[sp.first + l], (int)sub.size(), 1.0, 0.0, 0.0, 0.0, 2));
+            }
+            const int nslot = (int)sub.size();
+            // buckets by raster: (ng, cells)
+            std::map<int, std::vector<int>> by_ng;
+            for (int i = 0; i < nslot; ++i) by_ng[sub[i].ng].push_back(i);
+            size_t fixed = 3 * a256(s_nn * nslot * c16) + a256(s_w * ns * c16) + a256(10 * s_n * ns * c16) +
+                           a256(ns * sizeof(int)) + a256(nslot * sizeof(int)) + a256(ns * sizeof(CellDev)) +
+                           a256(ns * sizeof(int2)) +
+                           a256(ns * nexc * sizeof(celeris_rcwa_result));
+            if (ord_out) fixed += a256((size_t)ns * nexc * N * 2 * sizeof(double));
+            for (auto& kv : by_ng) {
+                const size_t nc = kv.second.size(), ng = (size_t)std::max(kv.first, 0);
+                fixed += a256(nc * sizeof(CellDev)) + 2 * a256(s_nn * nc * c16) + a256(s_w * nc * c16) +
+                         3 * a256(s_NN * nc * c16) + a256(s_n * nc * sizeof(int)) + 2 * a256(nc * sizeof(int));
+                if (ng > 0) fixed += a256((4 * Mx + 1) * ng * c16) + a256((4 * My + 1) * ng * c16);
+            }
+            CEL_TRY(ws.reserve(st, fixed));
+            Bump mem{static_cast<char*>(ws.take(fixed)), fixed};
+            StackPort sp;
+            std::memset(&sp, 0, sizeof(sp));
+            sp.Mx = Mx;
+            sp.My = My;
+            sp.n = n;
+            sp.nstack = ns;
+            sp.s_nn = s_nn;
+            sp.s_w = s_w;
+            sp.s_n = s_n;
+            CEL_TRY(mem.get(&sp.lA, s_nn * nslot));
+            CEL_TRY(mem.get(&sp.lB, s_nn * nslot));
+            CEL_TRY(mem.get(&sp.lK, s_nn * nslot));
+            CEL_TRY(mem.get(&sp.work, s_w * ns));
+            CEL_TRY(mem.get(&sp.vec, 10 * s_n * ns));
+            CEL_TRY(mem.get(&sp.info, (size_t)ns));
+            int* lrest;
+            CEL_TRY(mem.get(&lrest, (size_t)nslot));
+            sp.lrest = lrest;
+            CellDev* scells;
+            int2* sstacks;
+            celeris_rcwa_result* dres;
+            CEL_TRY(mem.get(&scells, (size_t)ns));
+            CEL_TRY(mem.get(&sstacks, (size_t)ns));
+            CEL_TRY(mem.get(&dres, (size_t)ns * nexc));
+            sp.cells = scells;
+            sp.stacks = sstacks;
+            CEL_CUDA(cudaMemcpyAsync(scells, hc.data(), sizeof(CellDev) * ns, cudaMemcpyHostToDevice, st));
+            CEL_CUDA(cudaMemcpyAsync(sstacks, hs.data(), sizeof(int2) * ns, cudaMemcpyHostToDevice, st));
+            CEL_CUDA(cudaMemsetAsync(sp.info, 0, sizeof(int) * ns, st));
+            CEL_CUDA(cudaMemsetAsync(lrest, 0, sizeof(int) * nslot, st));
+            // the layers, one bucket per raster class
+            std::vector<std::vector<CellDev>> hd;
+            std::vector<std::vector<int>> hlinfo;
+            std::vector<int*> dlinfo;
+            for (auto& kv : by_ng) {
+                const int ng = kv.first, nc = (int)kv.second.size();
+                if (ng > 0 && laurent_smem(Mx, My, ng) + 1024 > (size_t)smem_optin)
+                    return set_error(CELERIS_ERR_TOO_LARGE, "raster %d with M=(%d,%d) exceeds shared memory", ng,
+                                     Mx, My);
+                Bucket b;
+                std::memset(&b, 0, sizeof(b));
+                b.Mx = Mx;
+                b.My = My;
+                b.N = N;
+                b.n = n;
+                b.ng = ng;
+                b.ncell = nc;
+                b.s_nn = s_nn;
+                b.s_NN = s_NN;
+                b.s_n = s_n;
+                b.s_w = s_w;
+                b.lA = sp.lA;
+                b.lB = sp.lB;
+                b.lK = sp.lK;
+                b.lrest = lrest;
+                CellDev* dcells;
+                int* dslot;
+                CEL_TRY(mem.get(&dcells, (size_t)nc));
+                CEL_TRY(mem.get(&b.H, s_nn * nc));
+                CEL_TRY(mem.get(&b.Kp, s_nn * nc));
+                CEL_TRY(mem.get(&b.slab, s_w * nc));
+                CEL_TRY(mem.get(&b.Einv, s_NN * nc));
+                CEL_TRY(mem.get(&b.Exx, s_NN * nc));
+                CEL_TRY(mem.get(&b.Eyy, s_NN * nc));
+                CEL_TRY(mem.get(&b.piv, s_n * nc));
+                CEL_TRY(mem.get(&b.info, (size_t)nc));
+                CEL_TRY(mem.get(&dslot, (size_t)nc));
+                if (ng > 0) {
+                    cplx *phx, *phy;
+                    CEL_TRY(mem.get(&phx, (size_t)(4 * Mx + 1) * ng));
+                    CEL_TRY(mem.get(&phy, (size_t)(4 * My + 1) * ng));
+                    b.phx = phx;
+                    b.phy = phy;
+                }
+                b.cells = dcells;
+                b.lslot = dslot;
+                hd.emplace_back(nc);
+                for (int i = 0; i < nc; ++i) hd.back()[i] = sub[kv.second[i]].d;
+                CEL_CUDA(cudaMemcpyAsync(dcells, hd.back().data(), sizeof(CellDev) * nc, cudaMemcpyHostToDevice, st));
+                CEL_CUDA(cudaMemcpyAsync(dslot, kv.second.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
+                SmemNeeds needs;
+                needs.add(Mx, My, ng, n, 0, 0);
+                CEL_TRY(set_smem_limits(needs));
+                launch_bucket(b, uniform_cfg(256), st, nullptr, false);
+                CEL_CUDA(cudaGetLastError());
+                dlinfo.push_back(b.info);
+                hlinfo.emplace_back(nc);
+            }
+            CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_stack_port), slab::shared_bytes(n)));
+            rcwa_stack_port<<<ns, 512, slab::shared_bytes(n), st>>>(sp);
+            Bucket eb;
+            std::memset(&eb, 0, sizeof(eb));
+            eb.Mx = Mx;
+            eb.My = My;
+            eb.N = N;
+            eb.n = n;
+            eb.ncell = ns;
+            eb.cells = scells;
+            eb.vec = sp.vec;
+            eb.info = sp.info;
+            eb.res = dres;
+            eb.s_n = s_n;
+            eb.s_nn = s_nn;
+            if (ord_out) CEL_TRY(mem.get(&eb.ord, (size_t)ns * nexc * N * 2));
+            rcwa_epilogue<<<ns, kRT, 0, st>>>(eb);
+            count_launch(2);
+            CEL_CUDA(cudaGetLastError());
+            std::vector<celeris_rcwa_result> hres((size_t)ns * nexc);
+            CEL_CUDA(cudaMemcpyAsync(hres.data(), dres, sizeof(celeris_rcwa_result) * ns * nexc,
+                                     cudaMemcpyDeviceToHost, st));
+            CEL_CUDA(cudaMemcpyAsync(hinfo.data(), sp.info, sizeof(int) * ns, cudaMemcpyDeviceToHost, st));
+            for (size_t k = 0; k < dlinfo.size(); ++k)
+                CEL_CUDA(cudaMemcpyAsync(hlinfo[k].data(), dlinfo[k], sizeof(int) * hlinfo[k].size(),
+                                         cudaMemcpyDeviceToHost, st));
+            std::vector<double> hord;
+            if (ord_out) {
+                hord.resize((size_t)ns * nexc * N * 2);
+                CEL_CUDA(cudaMemcpyAsync(hord.data(), eb.ord, sizeof(double) * hord.size(), cudaMemcpyDeviceToHost,
+                                         st));
+            }
+            CEL_CUDA(cudaStreamSynchronize(st));
+            // a flagged layer flags its stack (its part of the layer store was not written)
+            std::vector<char> bad(nslot, 0);
+            size_t k = 0;
+            for (auto& kv : by_ng) {
+                for (size_t i = 0; i < kv.second.size(); ++i) bad[kv.second[i]] = hlinfo[k][i] != 0;
+                ++k;
+            }
+            for (int i = 0; i < ns; ++i) {
+                int f = hinfo[i];
+                for (int l = 0; l < hs[i].x; ++l)
+                    if (bad[hs[i].y + l]) f = kInfoRedo;
+                info_out[ids[i]] = f;
+                if (f != 0) continue;
+                for (int e = 0; e < nexc; ++e) out[(size_t)ids[i] * nexc + e] = hres[(size_t)i * nexc + e];
+                if (ord_out)
+                    std::memcpy(ord_out + (size_t)ids[i] * nexc * N * 2, hord.data() + (size_t)i * nexc * N * 2,
+                                sizeof(double) * nexc * N * 2);
+            }
+        }
+    }
+    return CELERIS_OK;
+}
+
+// Stacks through the two-ports; those it does not take (needs_qr of a layer) and those
+// it flags through the eigendecompositions.
+int run_stacks(const celeris_rcwa_cell* layers, const std::vector<std::pair<int, int>>& stacks, const double* exc,
+               celeris_rcwa_result* out, int* info_out, int nexc, double* ord_out = nullptr) {
+    const int ns = (int)stacks.size();
+    std::vector<int> info(ns, 0), direct, rest;
+    for (int s = 0; s < ns; ++s) {
+        bool qr = false;
+        for (int l = 0; l < stacks[s].second; ++l) {
+            const celeris_rcwa_cell& c = layers[stacks[s].first + l];
+            qr = qr || needs_qr(c) || 2 * (2 * c.Mx + 1) * (2 * c.My + 1) > slab::kMaxOrder;
+        }
+        (qr ? rest : direct).push_back(s);
+    }
+    // a subset of the stacks through one of the two, results back at their places
+    auto run = [&](const std::vector<int>& sel, bool qr) -> int {
+        if (sel.empty()) return CELERIS_OK;
+        const int k = (int)sel.size();
+        std::vector<std::pair<int, int>> st(k);
+        std::vector<double> ex(4 * (size_t)k);
+        std::vector<celeris_rcwa_result> res((size_t)k * nexc);
+        std::vector<int> inf(k, 0);
+        size_t per = 0;  // order records per stack: one stack at a time is asked for them
+        if (ord_out) {
+            const celeris_rcwa_cell& f = layers[stacks[0].first];
+            per = (size_t)nexc * (2 * f.Mx + 1) * (2 * f.My + 1) * 2;
+        }
+        std::vector<double> ord(per * k);
+        for (int i = 0; i < k; ++i) {
+            st[i] = stacks[sel[i]];
+            std::memcpy(&ex[4 * (size_t)i], exc + 4 * (size_t)sel[i], 4 * sizeof(double));
+        }
+        double* o = ord_out ? ord.data() : nullptr;
+        CEL_TRY(qr ? run_stacks_qr(layers, st, ex.data(), res.data(), inf.data(), nexc, o)
+                   : run_stacks_slab(layers, st, ex.data(), res.data(), inf.data(), nexc, o));
+        for (int i = 0; i < k; ++i) {
+            info[sel[i]] = inf[i];
+            if (!qr && inf[i] != 0) continue;
+            for (int e = 0; e < nexc; ++e) out[(size_t)sel[i] * nexc + e] = res[(size_t)i * nexc + e];
+            if (o) std::memcpy(ord_out + per * sel[i], o + per * i, per * sizeof(double));
+        }
+        return CELERIS_OK;
+    };
+    CEL_TRY(run(direct, false));
+    for (int s : direct)
+        if (info[s] != 0) rest.push_back(s);
+    CEL_TRY(run(rest, true));
+    for (int s = 0; s < ns; ++s) {
+        if (info_out) info_out[s] = info[s];
+        else if (info[s] > 0)
+            return set_error(CELERIS_ERR_EIG_NOCONV, "eigensolve did not converge (a layer of stack %d)", s);
+        else if (info[s] < 0)
+            return set_error(CELERIS_ERR_SINGULAR, "singular interface system (stack %d)", s);
     }
     return CELERIS_OK;
 }
@@ -2881,7 +3424,8 @@ int celeris_rcwa_tuning_report(char* buf, int len) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     for (const auto& kv : tune_table()) {
         s += "Mx=" + std::to_string(std::get<0>(kv.first)) + " My=" + std::to_string(std::get<1>(kv.first)) +
-             " grid=" + std::to_string(std::get<2>(kv.first) / 4) +
+             " grid=" + std::to_string(std::get<2>(kv.first) / 8) +
+             ((std::get<2>(kv.first) & 4) ? "" : " eigensolve") +
              ((std::get<2>(kv.first) & 2) ? " parity-classes" : "") +
              ((std::get<2>(kv.first) & 1) ? " batch>=SMs:" : " batch<SMs:");
         for (int st = 0; st < ST_COUNT; ++st)
@@ -3003,6 +3547,7 @@ int celeris_debug_qr_iteration_cap(int cap) {
     if (cap < 0) return set_error(CELERIS_ERR_INVALID_ARG, "cap < 0");
     CEL_TRY(celeris_rt::require_device());
     CEL_CUDA(cudaMemcpyToSymbol(g_qr_iter_cap, &cap, sizeof(int)));
+    g_qr_cap_set.store(cap);
     return CELERIS_OK;
 }
 

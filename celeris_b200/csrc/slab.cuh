@@ -1,0 +1,684 @@
+// One uniform-in-z layer as a two-port, without an eigendecomposition.
+//
+// Inside a layer the tangential fields follow g'' = -M g with g = W q^-1 (a - b) (the
+// amplitude vector of e = kp g) and i h = g' (h = W (a + b)), M = ep2 kp - kk^T the
+// matrix whose eigenvalues are q^2. A slab of thickness x therefore maps the two
+// boundary values of g to the two of i h by functions of M alone:
+//     i h(0) = -A g(0) + B g(x),   i h(x) = -B g(0) + A g(x),
+//     A = Q cot(Q x),  B = Q / sin(Q x),  Q = M^(1/2),
+// both even in Q, so no square root and no eigenvector is needed:
+//   * C = cos(Q y), S = sin(Q y) / Q by their Taylor series in M y^2 (degree 11 in
+//     groups of four, Paterson and Stockmeyer's scheme, Higham, Functions of Matrices,
+//     sec. 4.2) at a y where the spectral radius of Q y is at most 2.2; up to two
+//     double-angle steps (while no propagating mode reaches the zero of sin at pi);
+//     B = S^-1, A = S^-1 C. A smaller y loses digits of the slow modes in I - M y^2 / 2
+//     (radius 1.1: five times the error), a larger one to cosh of the evanescent ones;
+//   * the slab is then put together with itself until it has the layer's thickness
+//     (the doubling of layer theory): X = A^-1 B, B <- B X / 2, A <- A - B.
+// Everything is matrix products and Gauss-Jordan solves, which run on the FP64 tensor
+// cores; for a layer with real M (real permittivities, real in-plane wavevector) in
+// real arithmetic. The evanescent orders decay in B multiplicatively, so nothing
+// overflows however thick the layer is.
+//
+// A doubling is ill conditioned where A has a small eigenvalue, i.e. where a mode has
+// cos(q x) ~ 0; max |X| ~ 1 / |cos(q x)| shows it, and the error of the result grows as
+// eps max |X|. The last doublings (q x of a propagating mode reaches pi / 2 only there)
+// are then left out: the slab of h / 2^r is used 2^r times in the caller's recursion
+// from the substrate up, whose systems A + load are damped by the radiation and have
+// no such poles. Each step of that recursion is a complex solve, so it costs about
+// four times the real doubling it replaces.
+//
+// One thread block per matrix. Matrices are row-major in global memory (the working
+// set of a block stays in L1 / L2); panels of the Gauss-Jordan steps live in registers.
+#pragma once
+
+#include "cblas_block.cuh"
+
+namespace cb {
+namespace slab {
+
+constexpr int kMaxOrder = 512;        // largest order of the routines here
+constexpr int kNB = 16;               // Gauss-Jordan panel width
+constexpr int kGs = 20;               // row stride of the staged panel (4 mod 16: fragment reads do not conflict)
+constexpr double kSpectral = 2.2;     // largest spectral radius of Q y of the series
+constexpr double kPhaseMax = 2.5;     // largest q x of a propagating mode at S^-1 (sin q x = 0 at pi)
+constexpr int kMaxAngles = 2;         // double-angle steps
+constexpr int kMaxDoublings = 40;
+// Largest max |X| of the doubling that leaves r more (r >= 0): beyond it the doublings
+// stop (r + 1 <= kMaxRest), or the layer is given up. 64 keeps the error at the level of
+// the eigendecomposition's (1e-14 to 1e-13 against long double); a stop further from the
+// end costs more, so it waits for a larger loss.
+constexpr int kMaxRest = 3;
+__device__ __forceinline__ double growth_limit(int rest) {
+    return rest <= 1 ? 64.0 : rest == 2 ? 128.0 : rest == 3 ? 512.0 : 5e3;
+}
+
+// ---- scalars: double or complex ---------------------------------------------------------
+__device__ __forceinline__ double zero_of(double) { return 0.0; }
+__device__ __forceinline__ cplx zero_of(cplx) { return C(0.0, 0.0); }
+__device__ __forceinline__ double mul(double a, double b) { return a * b; }
+__device__ __forceinline__ cplx mul(cplx a, cplx b) { return cmul(a, b); }
+__device__ __forceinline__ double fms(double a, double b, double c) { return fma(-a, b, c); }  // c - a b
+__device__ __forceinline__ cplx fms(cplx a, cplx b, cplx c) { return cfms(a, b, c); }
+__device__ __forceinline__ double add(double a, double b) { return a + b; }
+__device__ __forceinline__ cplx add(cplx a, cplx b) { return cadd(a, b); }
+__device__ __forceinline__ double sub(double a, double b) { return a - b; }
+__device__ __forceinline__ cplx sub(cplx a, cplx b) { return csub(a, b); }
+__device__ __forceinline__ double scale(double a, double s) { return a * s; }
+__device__ __forceinline__ cplx scale(cplx a, double s) { return cscale(a, s); }
+__device__ __forceinline__ double neg(double a) { return -a; }
+__device__ __forceinline__ cplx neg(cplx a) { return cneg(a); }
+__device__ __forceinline__ double recip(double a) { return 1.0 / a; }
+__device__ __forceinline__ cplx recip(cplx a) {
+    const double s = 1.0 / cnorm2(a);
+    return C(a.x * s, -a.y * s);
+}
+__device__ __forceinline__ double size1(double a) { return fabs(a); }
+__device__ __forceinline__ double size1(cplx a) { return cabs1(a); }
+__device__ __forceinline__ double real_part(double a) { return a; }
+__device__ __forceinline__ double real_part(cplx a) { return a.x; }
+__device__ __forceinline__ double plus_real(double a, double r) { return a + r; }
+__device__ __forceinline__ cplx plus_real(cplx a, double r) { return C(a.x + r, a.y); }
+__device__ __forceinline__ double shfl_of(double a, int l) { return __shfl_sync(0xffffffffu, a, l); }
+__device__ __forceinline__ cplx shfl_of(cplx a, int l) {
+    return C(__shfl_sync(0xffffffffu, a.x, l), __shfl_sync(0xffffffffu, a.y, l));
+}
+__device__ __forceinline__ cplx as_cplx(double a) { return C(a, 0.0); }
+__device__ __forceinline__ cplx as_cplx(cplx a) { return a; }
+
+// Accumulator of one 8 x 8 tile: the lane's two entries (rows g, columns 2 t, 2 t + 1).
+template <bool CPLX>
+struct Acc {
+    double r[2], i[CPLX ? 2 : 1];
+    __device__ void clear() {
+        r[0] = r[1] = 0.0;
+        i[0] = 0.0;
+        if constexpr (CPLX) i[1] = 0.0;
+    }
+    __device__ void set(int h, double v) { r[h] = v; }
+    __device__ void set(int h, cplx v) {
+        r[h] = v.x;
+        if constexpr (CPLX) i[h] = v.y;
+    }
+    __device__ __forceinline__ void get(int h, double& v) const { v = r[h]; }
+    __device__ __forceinline__ void get(int h, cplx& v) const { v = C(r[h], CPLX ? i[CPLX ? h : 0] : 0.0); }
+};
+__device__ __forceinline__ void mma(Acc<false>& c, double a, double b) { dmma(c.r[0], c.r[1], a, b); }
+__device__ __forceinline__ void mma(Acc<true>& c, double a, cplx b) {
+    dmma(c.r[0], c.r[1], a, b.x);
+    dmma(c.i[0], c.i[1], a, b.y);
+}
+__device__ __forceinline__ void mma(Acc<true>& c, cplx a, cplx b) {
+    dmma(c.r[0], c.r[1], a.x, b.x);
+    dmma(c.i[0], c.i[1], a.x, b.y);
+    dmma(c.r[0], c.r[1], -a.y, b.y);
+    dmma(c.i[0], c.i[1], a.y, b.x);
+}
+template <class TA, class TB>
+struct Prod {
+    typedef cplx type;
+};
+template <>
+struct Prod<double, double> {
+    typedef double type;
+};
+
+// ---- product: epi(row, col, (A B)[row][col]) for every entry, A m x k, B k x n -----------------
+// Each warp takes units of 8 rows x 8 W columns; fragments come straight from memory
+// (L1 holds the rows the warps share), so no staging and no barrier inside. The width
+// W in {1, 2, 4} is the one that leaves the least work to the busiest warp. bmap (shared, may be
+// NULL): row r of B is stored at row bmap[r].
+template <class TA, class TB, int W, class Epi>
+__device__ __forceinline__ void gemm_units(int m, int n, int k, const TA* A, int lda, const TB* B, int ldb,
+                                           const int* bmap, const Epi& epi) {
+    typedef typename Prod<TA, TB>::type TC;
+    constexpr bool CP = sizeof(TC) == sizeof(cplx);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int rt = (m + 7) >> 3, units = rt * ((n + 8 * W - 1) / (8 * W));
+    for (int u = warp; u < units; u += nwarp) {
+        const int i0 = (u % rt) * 8, j0 = (u / rt) * (8 * W);
+        const TA* ap = A + (size_t)min(i0 + g, m - 1) * lda;
+        int col[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) col[j] = min(j0 + 8 * j + g, n - 1);
+        Acc<CP> acc[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) acc[j].clear();
+        auto load = [&](int k0, TA& a, TB (&b)[W]) {
+            const int kk = k0 + t4, kc = min(kk, k - 1);
+            a = ap[kc];
+            if (kk >= k) a = zero_of(TA());
+            const TB* bp = B + (size_t)(bmap ? bmap[kc] : kc) * ldb;
+#pragma unroll
+            for (int j = 0; j < W; ++j) b[j] = bp[col[j]];
+        };
+        TA a0, a1;
+        TB b0[W], b1[W];
+        load(0, a0, b0);
+        int k0 = 0;
+        for (; k0 + 4 < k; k0 += 8) {  // two steps per round, the next step's loads ahead of the products
+            load(k0 + 4, a1, b1);
+#pragma unroll
+            for (int j = 0; j < W; ++j) mma(acc[j], a0, b0[j]);
+            if (k0 + 8 < k) load(k0 + 8, a0, b0);
+#pragma unroll
+            for (int j = 0; j < W; ++j) mma(acc[j], a1, b1[j]);
+        }
+        if (k0 < k) {
+#pragma unroll
+            for (int j = 0; j < W; ++j) mma(acc[j], a0, b0[j]);
+        }
+        const int row = i0 + g;
+        if (row < m) {
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int c = j0 + 8 * j + 2 * t4 + h;
+                    if (c < n) {
+                        TC v;
+                        acc[j].get(h, v);
+                        epi(row, c, v);
+                    }
+                }
+        }
+    }
+}
+// Column width (in 8-column tiles) of the warps' units for `rt` row tiles and `ct` column tiles.
+__device__ __forceinline__ int unit_width(int rt, int ct) {
+    const int nwarp = blockDim.x >> 5;
+    int best = 1, cost = 1 << 30;
+#pragma unroll
+    for (int w = 1; w <= 4; w *= 2) {
+        const int rounds = (rt * ((ct + w - 1) / w) + nwarp - 1) / nwarp;
+        const int c = rounds * (4 * w + 1);
+        if (c <= cost) {
+            cost = c;
+            best = w;
+        }
+    }
+    return best;
+}
+template <class TA, class TB, class Epi>
+__device__ void gemm(int m, int n, int k, const TA* A, int lda, const TB* B, int ldb, const int* bmap, const Epi& epi) {
+    const int w = unit_width((m + 7) >> 3, (n + 7) >> 3);
+    if (w == 4) gemm_units<TA, TB, 4>(m, n, k, A, lda, B, ldb, bmap, epi);
+    else if (w == 2) gemm_units<TA, TB, 2>(m, n, k, A, lda, B, ldb, bmap, epi);
+    else gemm_units<TA, TB, 1>(m, n, k, A, lda, B, ldb, bmap, epi);
+}
+
+// ---- Gauss-Jordan ------------------------------------------------------------------------
+// Shared memory of the routines (dynamic): see carve().
+struct Shared {
+    cplx* fcol;   // [2][rows_of(n)]: multipliers of the current and the next column
+    cplx* pan;    // staged panel [n][kGs]
+    cplx* prow;   // staged pivot rows [kNB][chunk + pad]
+    int* perm;    // [n] row that holds variable k
+    int* pos;     // [n] variable of row r, -1 while it has none
+    int* perm2;   // [n] a kept copy of perm
+    cplx* piv;    // [2] reciprocal pivots
+    int* pidx;    // [2] pivot rows (-1: zero or non-finite pivot)
+    double* red;  // [32]
+    int chunk;    // columns staged at a time
+    long long* prof;  // optional clock64 sums: [0] panels, [1] updates of the other columns, [2] whole kernel
+};
+__host__ __device__ inline size_t pad16(size_t b) { return (b + 15) & ~size_t(15); }
+// Rows the panel's lanes cover: 32 times a power of two.
+__host__ __device__ inline int rows_of(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512; }
+// Columns of a staged chunk of pivot rows: as wide as 64 KB allows, and the whole
+// augmented matrix when it is narrower.
+__host__ __device__ inline int chunk_of(int n) {
+    const int all = (2 * n + 31) & ~31;
+    const int cap = n <= 256 ? 256 : 64;
+    return all < cap ? all : cap;
+}
+__host__ __device__ inline size_t shared_bytes(int n) {
+    return pad16(2 * (size_t)rows_of(n) * 16) + pad16((size_t)n * kGs * 16) +
+           pad16((size_t)kNB * (chunk_of(n) + 4) * 16) + 3 * pad16((size_t)n * 4) + 32 + 16 + 256;
+}
+__device__ __forceinline__ Shared carve(unsigned char* p, int n) {
+    Shared s;
+    s.prof = nullptr;
+    s.chunk = chunk_of(n);
+    s.fcol = reinterpret_cast<cplx*>(p);
+    p += pad16(2 * (size_t)rows_of(n) * 16);
+    s.pan = reinterpret_cast<cplx*>(p);
+    p += pad16((size_t)n * kGs * 16);
+    s.prow = reinterpret_cast<cplx*>(p);
+    p += pad16((size_t)kNB * (s.chunk + 4) * 16);
+    s.perm = reinterpret_cast<int*>(p);
+    p += pad16((size_t)n * 4);
+    s.pos = reinterpret_cast<int*>(p);
+    p += pad16((size_t)n * 4);
+    s.perm2 = reinterpret_cast<int*>(p);
+    p += pad16((size_t)n * 4);
+    s.piv = reinterpret_cast<cplx*>(p);
+    p += 32;
+    s.pidx = reinterpret_cast<int*>(p);
+    p += 16;
+    s.red = reinterpret_cast<double*>(p);
+    return s;
+}
+template <class T>
+__device__ __forceinline__ T* as(cplx* p) {
+    return reinterpret_cast<T*>(p);
+}
+
+// Largest value over the block, the same in every thread.
+__device__ __forceinline__ double block_max(double v, double* red) {
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double m = red[0];
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
+    return m;
+}
+
+// One panel of kb <= kNB columns (k0 ..) of the n-row matrix Wm, in registers: lane l
+// of every warp holds rows l + 32 r, warp w columns w + NW q. In-place Gauss-Jordan with
+// partial pivoting over the rows that have no variable yet (rows are not moved:
+// perm / pos record which row serves which variable). Per column one barrier: the
+// owner warp finds the pivot with one warp reduction over the magnitudes' high words
+// (the row in the low bits: a pivot within 0.1 % of the largest) and hands the
+// column, the pivot's row and its reciprocal to the others. The finished panel G goes
+// to s.pan: the update of every other column is row <- row + G (old pivot rows), with
+// the pivot rows themselves replaced (trailing()).
+template <class T, int RA, int NW>
+__device__ __noinline__ bool panel(int n, int k0, int kb, const T* Wm, int ld, const Shared& s, unsigned& used) {
+    constexpr int CPW = kNB / NW;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int nr = 32 * RA;
+    T* fcol = as<T>(s.fcol);
+    T* pivs = as<T>(s.piv);
+    T a[CPW][RA];
+#pragma unroll
+    for (int q = 0; q < CPW; ++q) {
+        const int c = warp + NW * q;
+#pragma unroll
+        for (int r = 0; r < RA; ++r) {
+            const int row = lane + 32 * r;
+            a[q][r] = (c < kb && row < n) ? Wm[(size_t)row * ld + k0 + c] : zero_of(T());
+        }
+    }
+    bool ok = true;
+#pragma unroll
+    for (int qo = 0; qo < CPW; ++qo) {
+        for (int wo = 0; wo < NW; ++wo) {
+            const int j = qo * NW + wo;
+            if (j >= kb) break;
+            const int buf = j & 1;
+            if (warp == wo) {
+                unsigned key = 0u;
+#pragma unroll
+                for (int r = 0; r < RA; ++r) {
+                    const int row = lane + 32 * r;
+                    const unsigned hi = (unsigned)__double2hiint(size1(a[qo][r]));
+                    if (row < n && !((used >> r) & 1u)) key = max(key, (hi & ~(unsigned)(kMaxOrder - 1)) | (unsigned)row);
+                }
+                key = __reduce_max_sync(0xffffffffu, key);
+                const int p = (int)(key & (unsigned)(kMaxOrder - 1)), pr = p >> 5;
+                T v = a[qo][0];
+#pragma unroll
+                for (int r = 1; r < RA; ++r)
+                    if (r == pr) v = a[qo][r];
+                v = shfl_of(v, p & 31);
+                const T d = recip(v);
+                const bool good = (key & ~(unsigned)(kMaxOrder - 1)) != 0u && isfinite(size1(d));
+#pragma unroll
+                for (int r = 0; r < RA; ++r) {
+                    const int row = lane + 32 * r;
+                    fcol[buf * nr + row] = row == p ? zero_of(T()) : a[qo][r];
+                }
+                if (lane == 0) {
+                    pivs[buf] = d;
+                    s.pidx[buf] = good ? p : -1;
+                    s.perm[k0 + j] = p;
+                    s.pos[p] = k0 + j;
+                }
+            }
+            __syncthreads();
+            const int p = s.pidx[buf];
+            if (p < 0) {
+                ok = false;
+                break;
+            }
+            const T d = pivs[buf];
+            const int pl = p & 31, pr = p >> 5;
+#pragma unroll
+            for (int q = 0; q < CPW; ++q) {
+                T v = a[q][0];
+#pragma unroll
+                for (int r = 1; r < RA; ++r)
+                    if (r == pr) v = a[q][r];
+                v = mul(shfl_of(v, pl), d);  // the scaled pivot row's entry in this column
+                const bool own = warp == wo && q == qo;
+#pragma unroll
+                for (int r = 0; r < RA; ++r) {
+                    const T f = fcol[buf * nr + lane + 32 * r];
+                    const T e = own ? neg(mul(f, d)) : fms(f, v, a[q][r]);
+                    a[q][r] = (lane == pl && r == pr) ? (own ? d : v) : e;
+                }
+            }
+            if (lane == pl) used |= 1u << pr;
+        }
+        if (!ok) break;
+    }
+    if (!ok) return false;
+    T* pan = as<T>(s.pan);
+#pragma unroll
+    for (int q = 0; q < CPW; ++q)
+#pragma unroll
+        for (int r = 0; r < RA; ++r) {
+            const int row = lane + 32 * r;
+            if (row < n) pan[row * kGs + warp + NW * q] = a[q][r];  // zero in the columns past kb
+        }
+    return true;
+}
+
+// Columns [c0, c0 + cn) of Wm after a panel: row i <- (pivot row of this panel ? 0 : row i) + G[i] . old
+// pivot rows (staged in s.prow from c0). K = kNB, on the tensor cores.
+template <class T, int W>
+__device__ __forceinline__ void trailing_units(int n, int c0, int cn, T* Wm, int ld, const Shared& s, int k0, int ldp) {
+    constexpr bool CP = sizeof(T) == sizeof(cplx);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const T* pan = as<T>(s.pan);
+    const T* pr = as<T>(s.prow);
+    const int rt = (n + 7) >> 3, units = rt * ((cn + 8 * W - 1) / (8 * W));
+    for (int u = warp; u < units; u += nwarp) {
+        const int row = (u % rt) * 8 + g, j0 = (u / rt) * (8 * W);
+        const int rowc = min(row, n - 1);
+        const bool keep = row < n && s.pos[rowc] < k0;  // pos >= k0: a pivot row of this panel
+        T* wrow = Wm + (size_t)rowc * ld + c0;
+        Acc<CP> acc[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = j0 + 8 * j + 2 * t4 + h;
+                acc[j].set(h, (keep && c < cn) ? wrow[c] : zero_of(T()));
+            }
+#pragma unroll
+        for (int ks = 0; ks < kNB; ks += 4) {
+            const T av = pan[rowc * kGs + ks + t4];
+#pragma unroll
+            for (int j = 0; j < W; ++j) mma(acc[j], av, pr[(ks + t4) * ldp + j0 + 8 * j + g]);
+        }
+        if (row < n) {
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int c = j0 + 8 * j + 2 * t4 + h;
+                    if (c < cn) {
+                        T v;
+                        acc[j].get(h, v);
+                        wrow[c] = v;
+                    }
+                }
+        }
+    }
+}
+template <class T>
+__device__ void trailing(int n, int c0, int c1, T* Wm, int ld, const Shared& s, int k0, int kb) {
+    constexpr bool CP = sizeof(T) == sizeof(cplx);
+    T* pr = as<T>(s.prow);
+    const int cmax = CP ? s.chunk : 2 * s.chunk;  // staged columns
+    for (int c = c0; c < c1; c += cmax) {
+        const int cn = min(cmax, c1 - c);
+        const int ldp = cmax + (CP ? 2 : 4);  // fragment reads of the staged rows do not conflict
+        for (int e = threadIdx.x; e < kNB * cn; e += blockDim.x) {
+            const int l = e / cn, j = e - l * cn;
+            pr[l * ldp + j] = l < kb ? Wm[(size_t)s.perm[k0 + l] * ld + c + j] : zero_of(T());
+        }
+        __syncthreads();
+        const int w = unit_width((n + 7) >> 3, (cn + 7) >> 3);
+        if (w == 4) trailing_units<T, 4>(n, c, cn, Wm, ld, s, k0, ldp);
+        else if (w == 2) trailing_units<T, 2>(n, c, cn, Wm, ld, s, k0, ldp);
+        else trailing_units<T, 1>(n, c, cn, Wm, ld, s, k0, ldp);
+        __syncthreads();
+    }
+}
+
+// Gauss-Jordan on the n x ncol matrix Wm = [A | R] (A its first n columns): afterwards row
+// s.perm[k] of the right part holds row k of A^-1 R. inverse: A's part becomes A^-1 in
+// place, its entry (k, perm[l]) stored at (row perm[k], column l). Returns false (in
+// every thread) at a zero or non-finite pivot. Starts and ends on a barrier.
+template <class T>
+__device__ bool gauss_jordan(int n, int ncol, T* Wm, int ld, bool inverse, const Shared& s) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) s.pos[i] = -1;
+    __syncthreads();
+    unsigned used = 0u;
+    const bool wide = blockDim.x >= 512;
+    for (int k0 = 0; k0 < n; k0 += kNB) {
+        const int kb = min(kNB, n - k0);
+        const long long t0 = clock64();
+        bool ok;
+        if (wide) {
+            if (n <= 32) ok = panel<T, 1, 16>(n, k0, kb, Wm, ld, s, used);
+            else if (n <= 64) ok = panel<T, 2, 16>(n, k0, kb, Wm, ld, s, used);
+            else if (n <= 128) ok = panel<T, 4, 16>(n, k0, kb, Wm, ld, s, used);
+            else if (n <= 256) ok = panel<T, 8, 16>(n, k0, kb, Wm, ld, s, used);
+            else ok = panel<T, 16, 16>(n, k0, kb, Wm, ld, s, used);
+        } else {
+            if (n <= 32) ok = panel<T, 1, 8>(n, k0, kb, Wm, ld, s, used);
+            else if (n <= 64) ok = panel<T, 2, 8>(n, k0, kb, Wm, ld, s, used);
+            else ok = panel<T, 4, 8>(n, k0, kb, Wm, ld, s, used);
+        }
+        __syncthreads();
+        if (!ok) return false;
+        const long long t1 = clock64();
+        const int c1 = k0 + kb;
+        if (inverse) {
+            if (k0 > 0) trailing(n, 0, k0, Wm, ld, s, k0, kb);
+            const T* pan = as<T>(s.pan);
+            for (int e = threadIdx.x; e < n * kb; e += blockDim.x) {
+                const int i = e / kb, j = e - i * kb;
+                Wm[(size_t)i * ld + k0 + j] = pan[i * kGs + j];
+            }
+        }
+        if (c1 < ncol) trailing(n, c1, ncol, Wm, ld, s, k0, kb);
+        __syncthreads();
+        if (s.prof && threadIdx.x == 0) {
+            s.prof[0] += t1 - t0;
+            s.prof[1] += clock64() - t1;
+        }
+    }
+    return true;
+}
+
+// ---- the layer's two-port ------------------------------------------------------------------
+// Work area of one matrix: kAreas buffers of order^2 complex plus 10 order (the
+// third carries two right-hand-side columns; four vectors of two columns). In real
+// arithmetic the same buffers hold doubles.
+constexpr int kAreas = 10;
+__host__ __device__ inline size_t work_size(int n) { return (size_t)kAreas * n * n + 10 * (size_t)n; }
+struct Work {
+    cplx *w0, *w1, *w2, *p, *q, *v;  // w2: n (n + 2); p, q: 2 n^2 each; v: 8 n
+    cplx* e[3];                      // n^2 each: the recursion's load and products
+};
+__device__ __forceinline__ Work carve_work(cplx* base, int n) {
+    const size_t nn = (size_t)n * n;
+    Work w;
+    w.w0 = base;
+    w.w1 = w.w0 + nn;
+    w.w2 = w.w1 + nn;
+    w.p = w.w2 + nn + 2 * (size_t)n;
+    w.q = w.p + 2 * nn;
+    w.e[0] = w.q + 2 * nn;
+    w.e[1] = w.e[0] + nn;
+    w.e[2] = w.e[1] + nn;
+    w.v = w.e[2] + nn;
+    return w;
+}
+
+// max |.|_inf (row sums of |re| + |im|) of an n x n matrix.
+template <class T>
+__device__ double norm_inf(int n, const T* A, int ld, double* red) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    double best = 0.0;
+    for (int i = warp; i < n; i += nwarp) {
+        double t = 0.0;
+        for (int j = lane; j < n; j += 32) t += size1(A[(size_t)i * ld + j]);
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        best = t > best || t != t ? t : best;  // NaN sticks
+    }
+    return block_max(best, red);
+}
+
+// max |re| + |im| of the entries (row i < n, column c0 + j, j < n).
+template <class T>
+__device__ double max_entry(int n, const T* A, int ld, int c0, double* red) {
+    double best = 0.0;
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+        const int i = e / n, j = e - i * n;
+        const double v = size1(A[(size_t)i * ld + c0 + j]);
+        best = v > best || v != v ? v : best;
+    }
+    return block_max(best, red);
+}
+
+// A, B of the slab of thickness h / 2^*rest from M (n x n), *rest = 0 unless the last
+// doublings are ill conditioned. In real arithmetic (T double) M's real part is used.
+// qmax bounds the propagating modes' q. Returns false (in every thread) when an earlier
+// doubling is ill conditioned too. A and B point into the work area (w.q, w.w2 and w.e free). M may be overwritten.
+template <class T>
+__device__ __noinline__ bool two_port(int n, cplx* Mc, double h, double qmax, const Work& w, const Shared& s, T** Aout, T** Bout,
+                                      int* rest) {
+    const int tid = threadIdx.x, nt = blockDim.x, n2 = 2 * n;
+    T* M1;
+    if constexpr (sizeof(T) == sizeof(double)) {
+        M1 = as<T>(w.w0);
+        for (int e = tid; e < n * n; e += nt) M1[e] = Mc[e].x;
+    } else {
+        M1 = Mc;
+    }
+    T *M2 = as<T>(w.w1), *M34 = as<T>(w.e[0]), *P = as<T>(w.p), *Q = as<T>(w.q);
+    T* A = P;
+    T* B0 = P + (size_t)n * n;
+    __syncthreads();
+    // M^2, then [M^3 | M^4] (side by side, ld 2 n)
+    gemm(n, n, n, M1, n, M1, n, nullptr, [=](int r, int c, T v) { M2[(size_t)r * n + c] = v; });
+    __syncthreads();
+    gemm(n, n, n, M2, n, M1, n, nullptr, [=](int r, int c, T v) { M34[(size_t)r * n2 + c] = v; });
+    gemm(n, n, n, M2, n, M2, n, nullptr, [=](int r, int c, T v) { M34[(size_t)r * n2 + n + c] = v; });
+    __syncthreads();
+    // spectral radius of Q: from ||M||, or ||M^2||, ||M^4|| (every power's root bounds it)
+    const double b1 = norm_inf(n, M1, n, s.red), b2 = norm_inf(n, M2, n, s.red),
+                 b4 = norm_inf(n, M34 + n, n2, s.red);
+    const double rho = sqrt(fmin(b1, fmin(sqrt(b2), sqrt(sqrt(b4)))));
+    if (!isfinite(b1 + b2 + b4) || !(h > 0.0)) return false;
+    int ns = 0;  // halvings of h
+    double y = h;
+    while (rho * y > kSpectral && ns < kMaxDoublings) {
+        y *= 0.5;
+        ++ns;
+    }
+    if (rho * y > kSpectral) return false;
+    int angles = 0;
+    double x = y;
+    while (angles < min(kMaxAngles, ns) && 2.0 * qmax * x <= kPhaseMax) {
+        x *= 2.0;
+        ++angles;
+    }
+    ns -= angles;
+    // S / y and C: sum_k (-M y^2)^k / (2k + 1)!, / (2k)!, k = 0 .. 11, as three groups in
+    // M^4; [S | C] side by side
+    const double y2 = y * y, y4 = y2 * y2, y6 = y4 * y2, y8 = y4 * y4;
+    auto group = [=](int r, int c, double f0, double f1, double f2, double f3) {
+        // f0 I + f1 M y^2 + f2 M^2 y^4 + f3 M^3 y^6
+        const size_t e = (size_t)r * n + c;
+        T v = scale(M1[e], f1 * y2);
+        v = add(v, scale(M2[e], f2 * y4));
+        v = add(v, scale(M34[(size_t)r * n2 + c], f3 * y6));
+        return r == c ? plus_real(v, f0) : v;
+    };
+    auto group_s = [=](int r, int c, int k) {
+        return k == 0   ? group(r, c, 1.0, -1.0 / 6.0, 1.0 / 120.0, -1.0 / 5040.0)
+               : k == 1 ? group(r, c, 1.0 / 362880.0, -1.0 / 39916800.0, 1.0 / 6227020800.0, -1.0 / 1307674368000.0)
+                        : group(r, c, 1.0 / 355687428096000.0, -1.0 / 121645100408832000.0,
+                                1.0 / 51090942171709440000.0, -1.0 / 25852016738884976640000.0);
+    };
+    auto group_c = [=](int r, int c, int k) {
+        return k == 0   ? group(r, c, 1.0, -0.5, 1.0 / 24.0, -1.0 / 720.0)
+               : k == 1 ? group(r, c, 1.0 / 40320.0, -1.0 / 3628800.0, 1.0 / 479001600.0, -1.0 / 87178291200.0)
+                        : group(r, c, 1.0 / 20922789888000.0, -1.0 / 6402373705728000.0, 1.0 / 2432902008176640000.0,
+                                -1.0 / 1124000727777607680000.0);
+    };
+    for (int e = tid; e < n * n; e += nt) {
+        const int r = e / n, c = e - r * n;
+        P[(size_t)r * n2 + c] = group_s(r, c, 2);
+        P[(size_t)r * n2 + n + c] = group_c(r, c, 2);
+    }
+    __syncthreads();
+    gemm(n, n2, n, M34 + n, n2, P, n2, nullptr, [=](int r, int c, T v) {
+        const T g = c < n ? group_s(r, c, 1) : group_c(r, c - n, 1);
+        Q[(size_t)r * n2 + c] = add(scale(v, y8), g);
+    });
+    __syncthreads();
+    gemm(n, n2, n, M34 + n, n2, Q, n2, nullptr, [=](int r, int c, T v) {
+        const T g = add(scale(v, y8), c < n ? group_s(r, c, 0) : group_c(r, c - n, 0));
+        P[(size_t)r * n2 + c] = c < n ? scale(g, y) : g;
+    });
+    __syncthreads();
+    // double angle: S(2y) = 2 C S, C(2y) = 2 C^2 - I
+    T *X = P, *Xn = Q;
+    for (int a = 0; a < angles; ++a) {
+        gemm(n, n2, n, X + n, n2, X, n2, nullptr, [=](int r, int c, T v) {
+            const T d = scale(v, 2.0);
+            Xn[(size_t)r * n2 + c] = c == r + n ? plus_real(d, -1.0) : d;
+        });
+        __syncthreads();
+        T* t = X;
+        X = Xn;
+        Xn = t;
+    }
+    if (X != Q) {
+        for (size_t e = tid; e < (size_t)n * n2; e += nt) Q[e] = X[e];
+        __syncthreads();
+    }
+    if (!gauss_jordan(n, n2, Q, n2, true, s)) return false;  // [S^-1 | S^-1 C]
+    for (int e = tid; e < n * n; e += nt) {
+        const int k = e / n, c = e - k * n;
+        const size_t row = (size_t)s.perm[k] * n2;
+        B0[(size_t)k * n + s.perm[c]] = Q[row + c];
+        A[(size_t)k * n + c] = Q[row + n + c];
+    }
+    T *B = B0, *Bn = M2;
+    *rest = 0;
+    for (int i = 0; i < ns; ++i) {
+        __syncthreads();
+        for (int e = tid; e < n * n; e += nt) {
+            const int r = e / n, c = e - r * n;
+            Q[(size_t)r * n2 + c] = A[e];
+            Q[(size_t)r * n2 + n + c] = B[e];
+        }
+        // X = A^-1 B in the right half of Q (rows by s.perm)
+        const bool ok = gauss_jordan(n, n2, Q, n2, false, s);
+        const int left = ns - 1 - i;
+        if (!ok || !(max_entry(n, Q, n2, n, s.red) <= growth_limit(left))) {  // NaN too
+            if (left + 1 > kMaxRest) return false;
+            *rest = left + 1;
+            break;
+        }
+        gemm(n, n, n, B, n, Q + n, n2, s.perm, [=](int r, int c, T v) {
+            const size_t e = (size_t)r * n + c;
+            const T b = scale(v, 0.5);
+            Bn[e] = b;
+            A[e] = sub(A[e], b);
+        });
+        T* t = B;
+        B = Bn;
+        Bn = t;
+    }
+    __syncthreads();
+    *Aout = A;
+    *Bout = B;
+    return true;
+}
+
+}  // namespace slab
+}  // namespace cb

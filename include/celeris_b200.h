@@ -298,7 +298,7 @@ int celeris_solve_rcwa_2d(const celeris_rcwa_cell* cell, const double* Ex0,
 /* Every real field of a cell must be finite: a NaN or Inf returns
  * CELERIS_ERR_INVALID_ARG (naming the cell in a batch) before any device work. */
 
-/* New: batched uneven cells. Each cell is solved once (one eigensolve, one
+/* New: batched uneven cells. Each cell is solved once (one layer solution, one
  * S-matrix) for BOTH the X (Ex0=1, Ey0=0) and Y (Ex0=0, Ey0=1) excitations;
  * out receives 2*ncell results: out[2c] = X, out[2c+1] = Y. Cells are bucketed
  * by harmonic count internally. info (ncell ints, may be NULL) receives 0 or the
@@ -307,9 +307,9 @@ int celeris_solve_rcwa_2d(const celeris_rcwa_cell* cell, const double* Ex0,
  * and reports failures there only, without info a failure returns
  * CELERIS_ERR_EIG_NOCONV / CELERIS_ERR_SINGULAR naming the first failing cell.
  * Cells symmetric under both mirrors at normal incidence (every unrotated
- * shape, theta = 0) solve the eigenproblem in its four parity classes (the same
- * eigenpairs at a quarter of the order; CELERIS_RCWA_SYMMETRY=0 turns it off),
- * only the two excited classes, and only one of them when the cell is also
+ * shape, theta = 0) are solved in their parity classes (the same fields at a
+ * quarter of the order; CELERIS_RCWA_SYMMETRY=0 turns it off), only the two
+ * excited classes, and only one of them when the cell is also
  * symmetric under a 90-degree rotation (square period, Mx = My, fill_x =
  * fill_y). A cell whose Fourier operators are not symmetric to within
  * CELERIS_RCWA_SYM_TOL (default 1e-9) of their largest entry is solved again at
