@@ -1570,14 +1570,15 @@ template <class T>
 __device__ __noinline__ bool slab_port(int Mx, int My, const CellDev& cd, int c, int n, int slabs, const T* A,
                                        const T* B, const cplx* Kp, const slab::Work& w, const slab::Shared& s,
                                        cplx* aN, cplx* b0, size_t stride) {
-    const int tid = threadIdx.x, nt = blockDim.x, nr = c < 0 ? 2 : 1, n2 = 2 * n, ldg = n + 2;
+    const int tid = threadIdx.x, nt = blockDim.x, nr = c < 0 ? 2 : 1, n2 = 2 * n, ldg = n + 2,
+              ln = slab::ld_of(n);
     cplx *Q = w.q, *G = w.w2, *L = w.e[0], *P = w.e[1], *Pn = w.e[2];
     HalfTable ys = half_table(Mx, My, cd, cd.n_sub, c, n, s);
     HalfTable yi;
     for (int k = slabs; k >= 1; --k) {
         for (int e = tid; e < n * n; e += nt) {
             const int r = e / n, j = e - r * n;
-            cplx a = slab::as_cplx(A[e]);
+            cplx a = slab::as_cplx(A[(size_t)r * ln + j]);
             if (k == slabs) {
                 const cplx y = ys.times(Kp, n, r, j);
                 a = C(a.x + y.y, a.y - y.x);
@@ -1585,15 +1586,15 @@ __device__ __noinline__ bool slab_port(int Mx, int My, const CellDev& cd, int c,
                 a = cadd(a, L[e]);
             }
             Q[(size_t)r * n2 + j] = a;
-            Q[(size_t)r * n2 + n + j] = slab::as_cplx(B[e]);
+            Q[(size_t)r * n2 + n + j] = slab::as_cplx(B[(size_t)r * ln + j]);
         }
         if (!slab::gauss_jordan(n, n2, Q, n2, false, s)) return false;
         for (int i = tid; i < n; i += nt) s.perm2[i] = s.perm[i];
         yi = half_table(Mx, My, cd, cd.n_inc, c, n, s);
         if (k > 1) {
-            slab::gemm(n, n, n, B, n, Q + n, n2, s.perm2, [=](int r, int j, cplx v) {
+            slab::gemm(n, n, n, B, ln, (const cplx*)(Q + n), n2, s.perm2, [=](int r, int j, cplx v) {
                 const size_t e = (size_t)r * n + j;
-                L[e] = csub(slab::as_cplx(A[e]), v);
+                L[e] = csub(slab::as_cplx(A[(size_t)r * ln + j]), v);
             });
             // product of the X of the slabs below the first
             if (k == slabs) {
@@ -1608,8 +1609,8 @@ __device__ __noinline__ bool slab_port(int Mx, int My, const CellDev& cd, int c,
             __syncthreads();
         }
     }
-    slab::gemm(n, n, n, B, n, Q + n, n2, s.perm2, [=](int r, int j, cplx v) {
-        const cplx yin = csub(slab::as_cplx(A[(size_t)r * n + j]), v), y = yi.times(Kp, n, r, j);
+    slab::gemm(n, n, n, B, ln, (const cplx*)(Q + n), n2, s.perm2, [=](int r, int j, cplx v) {
+        const cplx yin = csub(slab::as_cplx(A[(size_t)r * ln + j]), v), y = yi.times(Kp, n, r, j);
         G[(size_t)r * ldg + j] = C(y.x - yin.y, y.y + yin.x);
     });
     for (int e = tid; e < n * nr; e += nt) {
@@ -1754,8 +1755,9 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) rcwa_slab(Bucket b) {
         if (threadIdx.x == 0) b.lrest[b.lslot[cell]] = rest;
         const size_t o = b.s_nn * b.lslot[cell];
         for (int e = threadIdx.x; e < n * n; e += NT) {
-            b.lA[o + e] = slab::as_cplx(A[e]);
-            b.lB[o + e] = slab::as_cplx(B[e]);
+            const size_t p = (size_t)(e / n) * slab::ld_of(n) + e % n;
+            b.lA[o + e] = slab::as_cplx(A[p]);
+            b.lB[o + e] = slab::as_cplx(B[p]);
             b.lK[o + e] = Kp[e];
         }
         return true;

@@ -50,7 +50,7 @@ constexpr int kMaxDoublings = 40;
 // end costs more, so it waits for a larger loss.
 constexpr int kMaxRest = 3;
 __device__ __forceinline__ double growth_limit(int rest) {
-    return rest <= 1 ? 64.0 : rest == 2 ? 128.0 : rest == 3 ? 512.0 : 5e3;
+    return rest == 0 ? 64.0 : rest == 1 ? 1e3 : 5e3;
 }
 
 // ---- scalars: double or complex ---------------------------------------------------------
@@ -75,6 +75,9 @@ __device__ __forceinline__ cplx recip(cplx a) {
 }
 __device__ __forceinline__ double size1(double a) { return fabs(a); }
 __device__ __forceinline__ double size1(cplx a) { return cabs1(a); }
+// A size whose high word (sign aside) ranks pivots: |a|, or |re| + |im|.
+__device__ __forceinline__ double pivot_size(double a) { return a; }
+__device__ __forceinline__ double pivot_size(cplx a) { return cabs1(a); }
 __device__ __forceinline__ double real_part(double a) { return a; }
 __device__ __forceinline__ double real_part(cplx a) { return a.x; }
 __device__ __forceinline__ double plus_real(double a, double r) { return a + r; }
@@ -124,10 +127,104 @@ struct Prod<double, double> {
 };
 
 // ---- product: epi(row, col, (A B)[row][col]) for every entry, A m x k, B k x n -----------------
-// Each warp takes units of 8 rows x 8 W columns; fragments come straight from memory
-// (L1 holds the rows the warps share), so no staging and no barrier inside. The width
-// W in {1, 2, 4} is the one that leaves the least work to the busiest warp. bmap (shared, may be
-// NULL): row r of B is stored at row bmap[r].
+// Fragments come straight from memory (L1 holds the rows the warps share), so no
+// staging and no barrier inside; what bounds the real products is L1's throughput
+// (8-byte fragments: 56 % of L1 and 25 % of the tensor pipe busy at order 162), so they
+// load 16 bytes per lane: two k of A at a time (the order of k within a step of 8
+// is free) and two columns of B, and a warp's unit is 8 R x 8 W with the R, W that leave
+// the least to the busiest warp (96 oblique cells of order 162: 7.0 -> 5.6 ms a call). Real operands have even leading dimensions and
+// 16-byte-aligned bases. bmap (shared, may be NULL): row r of B is stored at row bmap[r].
+template <class TB, int R, int W, class Epi>
+__device__ __forceinline__ void gemm_units_real(int m, int n, int k, const double* A, int lda, const TB* B, int ldb,
+                                                const int* bmap, const Epi& epi) {
+    constexpr bool CP = sizeof(TB) == sizeof(cplx);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int rt = (m + 8 * R - 1) / (8 * R), units = rt * ((n + 8 * W - 1) / (8 * W));
+    for (int u = warp; u < units; u += nwarp) {
+        const int i0 = (u % rt) * (8 * R), j0 = (u / rt) * (8 * W);
+        const double* ap[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) ap[r] = A + (size_t)min(i0 + 8 * r + g, m - 1) * lda + 2 * t4;
+        Acc<CP> acc[R][W];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int j = 0; j < W; ++j) acc[r][j].clear();
+        // real B: columns j0 + 16 q + 2 g (+ 1) feed tiles 2 q (+ 1); complex B: column j0 + 8 j + g
+        constexpr int NB = CP ? W : W / 2;
+        int col[NB];
+#pragma unroll
+        for (int q = 0; q < NB; ++q)
+            col[q] = CP ? min(j0 + 8 * q + g, n - 1) : min(j0 + 16 * q + 2 * g, (n - 1) & ~1);
+        struct Step {
+            double2 a[R], b[2][NB];
+        };
+        auto load = [&](int k0, Step& st) {
+            const int kk = k0 + 2 * t4;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                double2 v = make_double2(0.0, 0.0);
+                if (kk < k) {
+                    v = *reinterpret_cast<const double2*>(ap[r] + k0);
+                    if (kk + 1 >= k) v.y = 0.0;
+                }
+                st.a[r] = v;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int kc = min(kk + h, k - 1);
+                const TB* bp = B + (size_t)(bmap ? bmap[kc] : kc) * ldb;
+#pragma unroll
+                for (int q = 0; q < NB; ++q) st.b[h][q] = *reinterpret_cast<const double2*>(bp + col[q]);
+            }
+        };
+        auto product = [&](const Step& st) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const double a = h == 0 ? st.a[r].x : st.a[r].y;
+#pragma unroll
+                    for (int q = 0; q < NB; ++q) {
+                        if constexpr (CP) {
+                            mma(acc[r][q], a, st.b[h][q]);
+                        } else {
+                            mma(acc[r][2 * q], a, st.b[h][q].x);
+                            mma(acc[r][2 * q + 1], a, st.b[h][q].y);
+                        }
+                    }
+                }
+        };
+        Step s0, s1;
+        load(0, s0);
+        int k0 = 0;
+        for (; k0 + 8 < k; k0 += 16) {
+            load(k0 + 8, s1);
+            product(s0);
+            if (k0 + 16 < k) load(k0 + 16, s0);
+            product(s1);
+        }
+        if (k0 < k) product(s0);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int row = i0 + 8 * r + g;
+            if (row >= m) continue;
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int c = CP ? j0 + 8 * j + 2 * t4 + h : j0 + 16 * (j >> 1) + 4 * t4 + 2 * h + (j & 1);
+                    if (c < n) {
+                        typename Prod<double, TB>::type v;
+                        acc[r][j].get(h, v);
+                        epi(row, c, v);
+                    }
+                }
+        }
+    }
+}
+// Complex A: units of 8 rows x 8 W columns, W in {1, 2, 4}.
 template <class TA, class TB, int W, class Epi>
 __device__ __forceinline__ void gemm_units(int m, int n, int k, const TA* A, int lda, const TB* B, int ldb,
                                            const int* bmap, const Epi& epi) {
@@ -200,25 +297,45 @@ __device__ __forceinline__ int unit_width(int rt, int ct) {
     }
     return best;
 }
-template <class TA, class TB, class Epi>
-__device__ void gemm(int m, int n, int k, const TA* A, int lda, const TB* B, int ldb, const int* bmap, const Epi& epi) {
+// Cost of the busiest warp with units of 8 r x 8 w: tensor work and fragment loads.
+__device__ __forceinline__ int unit_cost(int m, int n, int r, int w) {
+    const int units = ((m + 8 * r - 1) / (8 * r)) * ((n + 8 * w - 1) / (8 * w)), nwarp = blockDim.x >> 5;
+    return ((units + nwarp - 1) / nwarp) * (2 * r * w + r + w);
+}
+template <class TB, class Epi>
+__device__ void gemm(int m, int n, int k, const double* A, int lda, const TB* B, int ldb, const int* bmap,
+                     const Epi& epi) {
+    const int c12 = unit_cost(m, n, 1, 2), c14 = unit_cost(m, n, 1, 4), c22 = unit_cost(m, n, 2, 2),
+              c24 = unit_cost(m, n, 2, 4);
+    const int best = min(min(c12, c14), min(c22, c24));
+    if (((m + 7) >> 3) * ((n + 7) >> 3) <= (int)(blockDim.x >> 5)) {  // one 8 x 8 tile per warp
+        gemm_units<double, TB, 1>(m, n, k, A, lda, B, ldb, bmap, epi);
+        return;
+    }
+    if (sizeof(TB) == sizeof(double) && best == c24) gemm_units_real<TB, 2, 4>(m, n, k, A, lda, B, ldb, bmap, epi);
+    else if (best == c22 || best == c24) gemm_units_real<TB, 2, 2>(m, n, k, A, lda, B, ldb, bmap, epi);
+    else if (best == c14) gemm_units_real<TB, 1, 4>(m, n, k, A, lda, B, ldb, bmap, epi);
+    else gemm_units_real<TB, 1, 2>(m, n, k, A, lda, B, ldb, bmap, epi);
+}
+template <class Epi>
+__device__ void gemm(int m, int n, int k, const cplx* A, int lda, const cplx* B, int ldb, const int* bmap,
+                     const Epi& epi) {
     const int w = unit_width((m + 7) >> 3, (n + 7) >> 3);
-    if (w == 4) gemm_units<TA, TB, 4>(m, n, k, A, lda, B, ldb, bmap, epi);
-    else if (w == 2) gemm_units<TA, TB, 2>(m, n, k, A, lda, B, ldb, bmap, epi);
-    else gemm_units<TA, TB, 1>(m, n, k, A, lda, B, ldb, bmap, epi);
+    if (w == 4) gemm_units<cplx, cplx, 4>(m, n, k, A, lda, B, ldb, bmap, epi);
+    else if (w == 2) gemm_units<cplx, cplx, 2>(m, n, k, A, lda, B, ldb, bmap, epi);
+    else gemm_units<cplx, cplx, 1>(m, n, k, A, lda, B, ldb, bmap, epi);
 }
 
 // ---- Gauss-Jordan ------------------------------------------------------------------------
 // Shared memory of the routines (dynamic): see carve().
 struct Shared {
-    cplx* fcol;   // [2][rows_of(n)]: multipliers of the current and the next column
-    cplx* pan;    // staged panel [n][kGs]
+    cplx* pan;    // staged panel [n][kGs]; during a panel its columns [kNB][rows_of(n)]
     cplx* prow;   // staged pivot rows [kNB][chunk + pad]
     int* perm;    // [n] row that holds variable k
     int* pos;     // [n] variable of row r, -1 while it has none
     int* perm2;   // [n] a kept copy of perm
-    cplx* piv;    // [2] reciprocal pivots
-    int* pidx;    // [2] pivot rows (-1: zero or non-finite pivot)
+    int* flag;    // [kNB] of a panel's columns: 0, or 1 + the pivot's row, or -1 (no pivot)
+    int* bad;     // set when a column had no pivot
     double* red;  // [32]
     int chunk;    // columns staged at a time
     long long* prof;  // optional clock64 sums: [0] panels, [1] updates of the other columns, [2] whole kernel
@@ -233,18 +350,19 @@ __host__ __device__ inline int chunk_of(int n) {
     const int cap = n <= 256 ? 256 : 64;
     return all < cap ? all : cap;
 }
+__host__ __device__ inline size_t panel_elems(int n) {
+    const size_t g = (size_t)n * kGs, c = (size_t)kNB * rows_of(n);
+    return g > c ? g : c;
+}
 __host__ __device__ inline size_t shared_bytes(int n) {
-    return pad16(2 * (size_t)rows_of(n) * 16) + pad16((size_t)n * kGs * 16) +
-           pad16((size_t)kNB * (chunk_of(n) + 4) * 16) + 3 * pad16((size_t)n * 4) + 32 + 16 + 256;
+    return panel_elems(n) * 16 + pad16((size_t)kNB * (chunk_of(n) + 4) * 16) + 3 * pad16((size_t)n * 4) + 64 + 16 + 256;
 }
 __device__ __forceinline__ Shared carve(unsigned char* p, int n) {
     Shared s;
     s.prof = nullptr;
     s.chunk = chunk_of(n);
-    s.fcol = reinterpret_cast<cplx*>(p);
-    p += pad16(2 * (size_t)rows_of(n) * 16);
     s.pan = reinterpret_cast<cplx*>(p);
-    p += pad16((size_t)n * kGs * 16);
+    p += panel_elems(n) * 16;
     s.prow = reinterpret_cast<cplx*>(p);
     p += pad16((size_t)kNB * (s.chunk + 4) * 16);
     s.perm = reinterpret_cast<int*>(p);
@@ -253,9 +371,9 @@ __device__ __forceinline__ Shared carve(unsigned char* p, int n) {
     p += pad16((size_t)n * 4);
     s.perm2 = reinterpret_cast<int*>(p);
     p += pad16((size_t)n * 4);
-    s.piv = reinterpret_cast<cplx*>(p);
-    p += 32;
-    s.pidx = reinterpret_cast<int*>(p);
+    s.flag = reinterpret_cast<int*>(p);
+    p += 64;
+    s.bad = reinterpret_cast<int*>(p);
     p += 16;
     s.red = reinterpret_cast<double*>(p);
     return s;
@@ -276,105 +394,151 @@ __device__ __forceinline__ double block_max(double v, double* red) {
     return m;
 }
 
-// One panel of kb <= kNB columns (k0 ..) of the n-row matrix Wm, in registers: lane l
-// of every warp holds rows l + 32 r, warp w columns w + NW q. In-place Gauss-Jordan with
-// partial pivoting over the rows that have no variable yet (rows are not moved:
-// perm / pos record which row serves which variable). Per column one barrier: the
-// owner warp finds the pivot with one warp reduction over the magnitudes' high words
-// (the row in the low bits: a pivot within 0.1 % of the largest) and hands the
-// column, the pivot's row and its reciprocal to the others. The finished panel G goes
-// to s.pan: the update of every other column is row <- row + G (old pivot rows), with
-// the pivot rows themselves replaced (trailing()).
-template <class T, int RA, int NW>
-__device__ __noinline__ bool panel(int n, int k0, int kb, const T* Wm, int ld, const Shared& s, unsigned& used) {
-    constexpr int CPW = kNB / NW;
+// One panel of kb <= kNB columns (k0 ..) of the n-row matrix Wm, in registers of the
+// first PW = kNB / CPW warps: lane l holds rows l + 32 r, warp w columns w + PW q. In-place
+// Gauss-Jordan with partial pivoting over the rows that have no variable yet (rows are
+// not moved: perm / pos record which row serves which variable). What bounds a panel is
+// the chain from one pivot to the next, so a column is handed over without a barrier:
+// its owner stores the raw column in a buffer of its own, finds the pivot with one warp
+// reduction over the magnitudes' high words (the row in the low bits: a pivot within
+// 0.1 % of the largest) and raises the column's flag with the row; every warp then
+// forms the reciprocal itself. The owner of the next column brings that one up to date and
+// hands it over before it touches its others. Cycles per column at 25 / 61 / 113 / 162
+// rows, real: 565, 682, 880, 1241 (complex 763, 878, 1195, 2030); one column per warp
+// behind block-wide barriers took 830, 1109, 1537, 2065 (1006, 1477, 2166, 2926). The
+// finished panel G goes to s.pan (over the column buffers): the update of every other
+// column is row <- row + G (old pivot rows), with the pivot rows themselves replaced
+// (trailing()).
+constexpr unsigned kFlagPolls = 1u << 22;  // bound of a wait for a column
+__device__ __forceinline__ int wait_column(const int* flag) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(flag);
+    int v = 0;
+    for (unsigned i = 0; i < kFlagPolls && v == 0; ++i)
+        asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v == 0 ? -1 : v;
+}
+__device__ __forceinline__ void raise_column(int* flag, int v) {
+    asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(flag)), "r"(v) : "memory");
+}
+template <int THREADS>
+__device__ __forceinline__ void panel_barrier() {
+    asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+}
+template <class T, int RA, int CPW>
+__device__ __noinline__ void panel(int n, int k0, int kb, const T* Wm, int ld, const Shared& s, unsigned& used) {
+    constexpr int PW = kNB / CPW, nr = 32 * RA;
+    constexpr unsigned kRow = kMaxOrder - 1;  // row bits of a pivot key
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int nr = 32 * RA;
-    T* fcol = as<T>(s.fcol);
-    T* pivs = as<T>(s.piv);
+    if (warp >= PW) return;
+    T* col = as<T>(s.pan);  // [kNB][nr]
+    int* flag = s.flag;
+    int *perm = s.perm + k0, *pos = s.pos;
     T a[CPW][RA];
 #pragma unroll
     for (int q = 0; q < CPW; ++q) {
-        const int c = warp + NW * q;
+        const int c = warp + PW * q;
 #pragma unroll
         for (int r = 0; r < RA; ++r) {
             const int row = lane + 32 * r;
             a[q][r] = (c < kb && row < n) ? Wm[(size_t)row * ld + k0 + c] : zero_of(T());
         }
     }
+    // row candidates: the sign and the row bits cleared from a magnitude's high word, all
+    // of it once the row has a variable (or past the matrix)
+    unsigned mask = used, keep[RA];
+#pragma unroll
+    for (int r = 0; r < RA; ++r) keep[r] = (lane + 32 * r < n && !((mask >> r) & 1u)) ? 0x7fffffffu & ~kRow : 0u;
+    auto hand_over = [&](const T(&c)[RA], int j) {
+        unsigned key = 0u;
+#pragma unroll
+        for (int r = 0; r < RA; ++r) {
+            const int row = lane + 32 * r;
+            col[j * nr + row] = c[r];
+            key = max(key, ((unsigned)__double2hiint(pivot_size(c[r])) & keep[r]) | (unsigned)row);
+        }
+        key = __reduce_max_sync(0xffffffffu, key);
+        if (lane == 0) {
+            const int p = (int)(key & kRow);
+            // zero (or denormal), infinite and NaN pivots: the high word's exponent field
+            const unsigned e = (key >> 20) & 0x7ffu;
+            raise_column(flag + j, e == 0u || e == 0x7ffu ? -1 : p + 1);
+            perm[j] = p;
+            pos[p] = k0 + j;
+        }
+    };
+    if (warp == 0) hand_over(a[0], 0);
     bool ok = true;
 #pragma unroll
     for (int qo = 0; qo < CPW; ++qo) {
-        for (int wo = 0; wo < NW; ++wo) {
-            const int j = qo * NW + wo;
+        for (int wo = 0; wo < PW; ++wo) {
+            const int j = qo * PW + wo;
             if (j >= kb) break;
-            const int buf = j & 1;
-            if (warp == wo) {
-                unsigned key = 0u;
-#pragma unroll
-                for (int r = 0; r < RA; ++r) {
-                    const int row = lane + 32 * r;
-                    const unsigned hi = (unsigned)__double2hiint(size1(a[qo][r]));
-                    if (row < n && !((used >> r) & 1u)) key = max(key, (hi & ~(unsigned)(kMaxOrder - 1)) | (unsigned)row);
-                }
-                key = __reduce_max_sync(0xffffffffu, key);
-                const int p = (int)(key & (unsigned)(kMaxOrder - 1)), pr = p >> 5;
-                T v = a[qo][0];
-#pragma unroll
-                for (int r = 1; r < RA; ++r)
-                    if (r == pr) v = a[qo][r];
-                v = shfl_of(v, p & 31);
-                const T d = recip(v);
-                const bool good = (key & ~(unsigned)(kMaxOrder - 1)) != 0u && isfinite(size1(d));
-#pragma unroll
-                for (int r = 0; r < RA; ++r) {
-                    const int row = lane + 32 * r;
-                    fcol[buf * nr + row] = row == p ? zero_of(T()) : a[qo][r];
-                }
-                if (lane == 0) {
-                    pivs[buf] = d;
-                    s.pidx[buf] = good ? p : -1;
-                    s.perm[k0 + j] = p;
-                    s.pos[p] = k0 + j;
-                }
-            }
-            __syncthreads();
-            const int p = s.pidx[buf];
-            if (p < 0) {
+            const int got = wait_column(flag + j);
+            if (got < 0) {
                 ok = false;
                 break;
             }
-            const T d = pivs[buf];
-            const int pl = p & 31, pr = p >> 5;
+            const int p = got - 1, pl = p & 31, pr = p >> 5;
+            const T* cj = col + j * nr;
+            const T d = recip(cj[p]);
+            if (lane == pl) mask |= 1u << pr;
 #pragma unroll
-            for (int q = 0; q < CPW; ++q) {
-                T v = a[q][0];
+            for (int r = 0; r < RA; ++r)
+                if (lane == pl && r == pr) keep[r] = 0u;
+            // column j + 1's slot in its owner: qo, or qo + 1 after the last warp
+            const bool wrap = wo == PW - 1;
+            const bool next = warp == (wrap ? 0 : wo + 1) && j + 1 < kb;
+            auto update = [&](T(&c)[RA]) {
+                T v = c[0];
 #pragma unroll
                 for (int r = 1; r < RA; ++r)
-                    if (r == pr) v = a[q][r];
+                    if (r == pr) v = c[r];
                 v = mul(shfl_of(v, pl), d);  // the scaled pivot row's entry in this column
-                const bool own = warp == wo && q == qo;
 #pragma unroll
                 for (int r = 0; r < RA; ++r) {
-                    const T f = fcol[buf * nr + lane + 32 * r];
-                    const T e = own ? neg(mul(f, d)) : fms(f, v, a[q][r]);
-                    a[q][r] = (lane == pl && r == pr) ? (own ? d : v) : e;
+                    const T e = fms(cj[lane + 32 * r], v, c[r]);
+                    c[r] = (lane == pl && r == pr) ? v : e;
+                }
+            };
+            if (next) {
+                if (!wrap) {
+                    update(a[qo]);
+                    hand_over(a[qo], j + 1);
+                } else if (qo + 1 < CPW) {
+                    update(a[qo + 1 < CPW ? qo + 1 : qo]);
+                    hand_over(a[qo + 1 < CPW ? qo + 1 : qo], j + 1);
                 }
             }
-            if (lane == pl) used |= 1u << pr;
+#pragma unroll
+            for (int q = 0; q < CPW; ++q) {
+                if (next && q == (wrap ? qo + 1 : qo)) continue;
+                if (warp == wo && q == qo) {
+#pragma unroll
+                    for (int r = 0; r < RA; ++r) {
+                        const T e = neg(mul(a[q][r], d));
+                        a[q][r] = (lane == pl && r == pr) ? d : e;
+                    }
+                } else {
+                    update(a[q]);
+                }
+            }
         }
         if (!ok) break;
     }
-    if (!ok) return false;
+    used = mask;
+    panel_barrier<PW * 32>();  // the column buffers are read; G overlays them
+    if (!ok) {
+        if (threadIdx.x == 0) *s.bad = 1;
+        return;
+    }
     T* pan = as<T>(s.pan);
 #pragma unroll
     for (int q = 0; q < CPW; ++q)
 #pragma unroll
         for (int r = 0; r < RA; ++r) {
             const int row = lane + 32 * r;
-            if (row < n) pan[row * kGs + warp + NW * q] = a[q][r];  // zero in the columns past kb
+            if (row < n) pan[row * kGs + warp + PW * q] = a[q][r];  // zero in the columns past kb
         }
-    return true;
 }
 
 // Columns [c0, c0 + cn) of Wm after a panel: row i <- (pivot row of this panel ? 0 : row i) + G[i] . old
@@ -450,26 +614,21 @@ template <class T>
 __device__ bool gauss_jordan(int n, int ncol, T* Wm, int ld, bool inverse, const Shared& s) {
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) s.pos[i] = -1;
+    if (threadIdx.x < kNB) s.flag[threadIdx.x] = 0;
+    if (threadIdx.x == 0) *s.bad = 0;
     __syncthreads();
     unsigned used = 0u;
-    const bool wide = blockDim.x >= 512;
     for (int k0 = 0; k0 < n; k0 += kNB) {
         const int kb = min(kNB, n - k0);
         const long long t0 = clock64();
-        bool ok;
-        if (wide) {
-            if (n <= 32) ok = panel<T, 1, 16>(n, k0, kb, Wm, ld, s, used);
-            else if (n <= 64) ok = panel<T, 2, 16>(n, k0, kb, Wm, ld, s, used);
-            else if (n <= 128) ok = panel<T, 4, 16>(n, k0, kb, Wm, ld, s, used);
-            else if (n <= 256) ok = panel<T, 8, 16>(n, k0, kb, Wm, ld, s, used);
-            else ok = panel<T, 16, 16>(n, k0, kb, Wm, ld, s, used);
-        } else {
-            if (n <= 32) ok = panel<T, 1, 8>(n, k0, kb, Wm, ld, s, used);
-            else if (n <= 64) ok = panel<T, 2, 8>(n, k0, kb, Wm, ld, s, used);
-            else ok = panel<T, 4, 8>(n, k0, kb, Wm, ld, s, used);
-        }
+        if (n <= 32) panel<T, 1, 2>(n, k0, kb, Wm, ld, s, used);
+        else if (n <= 64) panel<T, 2, 2>(n, k0, kb, Wm, ld, s, used);
+        else if (n <= 128) panel<T, 4, 2>(n, k0, kb, Wm, ld, s, used);
+        else if (n <= 256) panel<T, 8, 2>(n, k0, kb, Wm, ld, s, used);
+        else panel<T, 16, 1>(n, k0, kb, Wm, ld, s, used);
         __syncthreads();
-        if (!ok) return false;
+        if (*s.bad) return false;
+        if (threadIdx.x < kNB) s.flag[threadIdx.x] = 0;  // a barrier follows before the next panel
         const long long t1 = clock64();
         const int c1 = k0 + kb;
         if (inverse) {
@@ -491,17 +650,19 @@ __device__ bool gauss_jordan(int n, int ncol, T* Wm, int ld, bool inverse, const
 }
 
 // ---- the layer's two-port ------------------------------------------------------------------
-// Work area of one matrix: kAreas buffers of order^2 complex plus 10 order (the
+// Work area of one matrix: kAreas buffers of order x ld_of(order) complex plus 10 order (the
 // third carries two right-hand-side columns; four vectors of two columns). In real
 // arithmetic the same buffers hold doubles.
 constexpr int kAreas = 10;
-__host__ __device__ inline size_t work_size(int n) { return (size_t)kAreas * n * n + 10 * (size_t)n; }
+// Leading dimension of the n x n matrices in the work area (real products load pairs).
+__host__ __device__ inline int ld_of(int n) { return (n + 1) & ~1; }
+__host__ __device__ inline size_t work_size(int n) { return (size_t)kAreas * n * ld_of(n) + 10 * (size_t)n; }
 struct Work {
     cplx *w0, *w1, *w2, *p, *q, *v;  // w2: n (n + 2); p, q: 2 n^2 each; v: 8 n
     cplx* e[3];                      // n^2 each: the recursion's load and products
 };
 __device__ __forceinline__ Work carve_work(cplx* base, int n) {
-    const size_t nn = (size_t)n * n;
+    const size_t nn = (size_t)n * ld_of(n);
     Work w;
     w.w0 = base;
     w.w1 = w.w0 + nn;
@@ -548,27 +709,30 @@ __device__ double max_entry(int n, const T* A, int ld, int c0, double* red) {
 template <class T>
 __device__ __noinline__ bool two_port(int n, cplx* Mc, double h, double qmax, const Work& w, const Shared& s, T** Aout, T** Bout,
                                       int* rest) {
-    const int tid = threadIdx.x, nt = blockDim.x, n2 = 2 * n;
+    // matrices of leading dimension ln; pairs [. | .] side by side, the right one from column ln
+    const int tid = threadIdx.x, nt = blockDim.x, ln = ld_of(n), n2 = 2 * ln, nw = ln + n;
     T* M1;
+    int l1 = ln;  // M1's
     if constexpr (sizeof(T) == sizeof(double)) {
         M1 = as<T>(w.w0);
-        for (int e = tid; e < n * n; e += nt) M1[e] = Mc[e].x;
+        for (int e = tid; e < n * n; e += nt) M1[(e / n) * ln + e % n] = Mc[e].x;
     } else {
         M1 = Mc;
+        l1 = n;
     }
     T *M2 = as<T>(w.w1), *M34 = as<T>(w.e[0]), *P = as<T>(w.p), *Q = as<T>(w.q);
     T* A = P;
-    T* B0 = P + (size_t)n * n;
+    T* B0 = P + (size_t)n * ln;
     __syncthreads();
     // M^2, then [M^3 | M^4] (side by side, ld 2 n)
-    gemm(n, n, n, M1, n, M1, n, nullptr, [=](int r, int c, T v) { M2[(size_t)r * n + c] = v; });
+    gemm(n, n, n, M1, l1, M1, l1, nullptr, [=](int r, int c, T v) { M2[(size_t)r * ln + c] = v; });
     __syncthreads();
-    gemm(n, n, n, M2, n, M1, n, nullptr, [=](int r, int c, T v) { M34[(size_t)r * n2 + c] = v; });
-    gemm(n, n, n, M2, n, M2, n, nullptr, [=](int r, int c, T v) { M34[(size_t)r * n2 + n + c] = v; });
+    gemm(n, n, n, M2, ln, M1, l1, nullptr, [=](int r, int c, T v) { M34[(size_t)r * n2 + c] = v; });
+    gemm(n, n, n, M2, ln, M2, ln, nullptr, [=](int r, int c, T v) { M34[(size_t)r * n2 + ln + c] = v; });
     __syncthreads();
     // spectral radius of Q: from ||M||, or ||M^2||, ||M^4|| (every power's root bounds it)
-    const double b1 = norm_inf(n, M1, n, s.red), b2 = norm_inf(n, M2, n, s.red),
-                 b4 = norm_inf(n, M34 + n, n2, s.red);
+    const double b1 = norm_inf(n, M1, l1, s.red), b2 = norm_inf(n, M2, ln, s.red),
+                 b4 = norm_inf(n, M34 + ln, n2, s.red);
     const double rho = sqrt(fmin(b1, fmin(sqrt(b2), sqrt(sqrt(b4)))));
     if (!isfinite(b1 + b2 + b4) || !(h > 0.0)) return false;
     int ns = 0;  // halvings of h
@@ -590,9 +754,8 @@ __device__ __noinline__ bool two_port(int n, cplx* Mc, double h, double qmax, co
     const double y2 = y * y, y4 = y2 * y2, y6 = y4 * y2, y8 = y4 * y4;
     auto group = [=](int r, int c, double f0, double f1, double f2, double f3) {
         // f0 I + f1 M y^2 + f2 M^2 y^4 + f3 M^3 y^6
-        const size_t e = (size_t)r * n + c;
-        T v = scale(M1[e], f1 * y2);
-        v = add(v, scale(M2[e], f2 * y4));
+        T v = scale(M1[(size_t)r * l1 + c], f1 * y2);
+        v = add(v, scale(M2[(size_t)r * ln + c], f2 * y4));
         v = add(v, scale(M34[(size_t)r * n2 + c], f3 * y6));
         return r == c ? plus_real(v, f0) : v;
     };
@@ -611,25 +774,28 @@ __device__ __noinline__ bool two_port(int n, cplx* Mc, double h, double qmax, co
     for (int e = tid; e < n * n; e += nt) {
         const int r = e / n, c = e - r * n;
         P[(size_t)r * n2 + c] = group_s(r, c, 2);
-        P[(size_t)r * n2 + n + c] = group_c(r, c, 2);
+        P[(size_t)r * n2 + ln + c] = group_c(r, c, 2);
     }
     __syncthreads();
-    gemm(n, n2, n, M34 + n, n2, P, n2, nullptr, [=](int r, int c, T v) {
-        const T g = c < n ? group_s(r, c, 1) : group_c(r, c - n, 1);
+    // (column n of an odd order is padding: nothing reads what lands there)
+    gemm(n, nw, n, M34 + ln, n2, P, n2, nullptr, [=](int r, int c, T v) {
+        if (c >= n && c < ln) return;
+        const T g = c < n ? group_s(r, c, 1) : group_c(r, c - ln, 1);
         Q[(size_t)r * n2 + c] = add(scale(v, y8), g);
     });
     __syncthreads();
-    gemm(n, n2, n, M34 + n, n2, Q, n2, nullptr, [=](int r, int c, T v) {
-        const T g = add(scale(v, y8), c < n ? group_s(r, c, 0) : group_c(r, c - n, 0));
+    gemm(n, nw, n, M34 + ln, n2, Q, n2, nullptr, [=](int r, int c, T v) {
+        if (c >= n && c < ln) return;
+        const T g = add(scale(v, y8), c < n ? group_s(r, c, 0) : group_c(r, c - ln, 0));
         P[(size_t)r * n2 + c] = c < n ? scale(g, y) : g;
     });
     __syncthreads();
     // double angle: S(2y) = 2 C S, C(2y) = 2 C^2 - I
     T *X = P, *Xn = Q;
     for (int a = 0; a < angles; ++a) {
-        gemm(n, n2, n, X + n, n2, X, n2, nullptr, [=](int r, int c, T v) {
+        gemm(n, nw, n, X + ln, n2, X, n2, nullptr, [=](int r, int c, T v) {
             const T d = scale(v, 2.0);
-            Xn[(size_t)r * n2 + c] = c == r + n ? plus_real(d, -1.0) : d;
+            Xn[(size_t)r * n2 + c] = c == r + ln ? plus_real(d, -1.0) : d;
         });
         __syncthreads();
         T* t = X;
@@ -640,12 +806,12 @@ __device__ __noinline__ bool two_port(int n, cplx* Mc, double h, double qmax, co
         for (size_t e = tid; e < (size_t)n * n2; e += nt) Q[e] = X[e];
         __syncthreads();
     }
-    if (!gauss_jordan(n, n2, Q, n2, true, s)) return false;  // [S^-1 | S^-1 C]
+    if (!gauss_jordan(n, nw, Q, n2, true, s)) return false;  // [S^-1 | S^-1 C]
     for (int e = tid; e < n * n; e += nt) {
         const int k = e / n, c = e - k * n;
         const size_t row = (size_t)s.perm[k] * n2;
-        B0[(size_t)k * n + s.perm[c]] = Q[row + c];
-        A[(size_t)k * n + c] = Q[row + n + c];
+        B0[(size_t)k * ln + s.perm[c]] = Q[row + c];
+        A[(size_t)k * ln + c] = Q[row + ln + c];
     }
     T *B = B0, *Bn = M2;
     *rest = 0;
@@ -653,19 +819,19 @@ __device__ __noinline__ bool two_port(int n, cplx* Mc, double h, double qmax, co
         __syncthreads();
         for (int e = tid; e < n * n; e += nt) {
             const int r = e / n, c = e - r * n;
-            Q[(size_t)r * n2 + c] = A[e];
-            Q[(size_t)r * n2 + n + c] = B[e];
+            Q[(size_t)r * n2 + c] = A[(size_t)r * ln + c];
+            Q[(size_t)r * n2 + ln + c] = B[(size_t)r * ln + c];
         }
         // X = A^-1 B in the right half of Q (rows by s.perm)
-        const bool ok = gauss_jordan(n, n2, Q, n2, false, s);
+        const bool ok = gauss_jordan(n, nw, Q, n2, false, s);
         const int left = ns - 1 - i;
-        if (!ok || !(max_entry(n, Q, n2, n, s.red) <= growth_limit(left))) {  // NaN too
+        if (!ok || !(max_entry(n, Q, n2, ln, s.red) <= growth_limit(left))) {  // NaN too
             if (left + 1 > kMaxRest) return false;
             *rest = left + 1;
             break;
         }
-        gemm(n, n, n, B, n, Q + n, n2, s.perm, [=](int r, int c, T v) {
-            const size_t e = (size_t)r * n + c;
+        gemm(n, n, n, B, ln, Q + ln, n2, s.perm, [=](int r, int c, T v) {
+            const size_t e = (size_t)r * ln + c;
             const T b = scale(v, 0.5);
             Bn[e] = b;
             A[e] = sub(A[e], b);
