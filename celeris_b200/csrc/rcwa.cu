@@ -11,8 +11,9 @@
 //   rcwa_fourier_rect / rcwa_fourier_laurent  eps operators (analytic Li rule,
 //                 or 4x4-supersampled raster -> centred DFT -> Laurent Toeplitz)
 //                 and Einv (LU inverse for the Laurent path)
-//   rcwa_sym_build  M = ep2 kp - kkT and kp of the excited parity classes
-//                 (mirror-symmetric cells)
+//                 (order basis)
+//   rcwa_sym_ops  the same for the excited parity classes of a mirror-symmetric cell:
+//                 their blocks of the eps operators, M = ep2 kp - kkT and kp
 //   rcwa_slab     the layer as a two-port without an eigendecomposition (slab.cuh),
 //                 then the amplitudes between the half-spaces
 //   rcwa_sym_expand  class amplitudes into the order basis
@@ -98,6 +99,9 @@ struct Bucket {
     size_t s_nn, s_ns, s_NN, s_n;
     const cplx* phx;  // [(4Mx+1) x ng] centred DFT phase table (x)
     const cplx* phy;  // [(4My+1) x ng]
+    const cplx* pcx;  // class path: [(2Mx+1) x (ng+1)] prefix sums of phx (there phx, phy hold m >= 0)
+    cplx* G1;         // class path, per cell s_g1: the raster's row transform, or the 1D inverses
+    size_t s_g1;
     long long* dbg;   // optional per-cell counters, kDbgSlots each (CELERIS_RCWA_STAGE_CLOCKS=1), else NULL
     double* ord;      // optional per-order efficiencies: per cell and excitation [N][2] = (de_t, de_r), else NULL
     // mirror-symmetric cells (sym != 0): the layer problem in its excited parity
@@ -277,134 +281,6 @@ __global__ void rcwa_phase_table(int ng, int mmax, cplx* ph) {
     ph[e] = C(co / ng, s / ng);
 }
 
-// 1 / sqrt(cnt) for cnt = 2^e, e in 0..4: the product of two orbit-vector
-// weights (1, 1/sqrt2 or 1/2 each) with no rounding beyond the one constant.
-__device__ __forceinline__ double orbit_weight(int e) {
-    return (e & 1) ? ldexp(0.70710678118654752440, -(e >> 1)) : ldexp(1.0, -(e >> 1));
-}
-
-// Position of order (p, q) in scalar parity class c: its index in the class
-// basis (orbit vectors of (|p|, |q|)) and the sign of its entry there, or
-// -1 when the orbit has no vector in that class (p = 0 in an odd-x class, or
-// q = 0 in an odd-y class). *e gains log2 of the orbit size.
-__device__ __forceinline__ int scalar_class_index(int My, int c, int p, int q, double* sgn, int* e) {
-    const int a = sym_class_a(c), bb = sym_class_b(c);
-    if ((p == 0 && a < 0) || (q == 0 && bb < 0)) return -1;
-    const int ap = abs(p), aq = abs(q);
-    *sgn = (p < 0 && a < 0 ? -1.0 : 1.0) * (q < 0 && bb < 0 ? -1.0 : 1.0);
-    *e += (ap > 0) + (aq > 0);
-    return (ap - (a > 0 ? 0 : 1)) * sym_count(My, bb) + (aq - (bb > 0 ? 0 : 1));
-}
-
-// Einv = epsT^-1 of a mirror-symmetric cell (Bucket::sym != 0). The Laurent
-// matrix epsT[(p,q)][(p',q')] = Ge[p-p'][q-q'] commutes with both mirrors when
-// Ge is even in dp and in dq, so in the scalar parity basis (unit orbit vectors
-// of (|p|, |q|) with signs a^[p<0] b^[q<0]) it is block diagonal with four blocks
-// of orders (Mx + [a>0]) (My + [b>0]). Each block is inverted on its own, in
-// place in shared memory by Gauss-Jordan with partial pivoting (about N^3/16 of
-// the work of the full inverse, and no triangular solves), and Einv assembled:
-//   Einv[k][l] = sum_c s_c(k) s_c(l) B_c^-1[i_c(k)][i_c(l)].
-// A Ge that is not even to the symmetry tolerance flags the cell kInfoAsym (it
-// is solved again by the full path). work: 2 N^2 complex (blocks, then their
-// inverses); smem: the kernel's dynamic shared memory, Ge's region included.
-__device__ void laurent_inverse_by_class(const Bucket& b, int cell, const cplx* Ge, cplx* work, cplx* Einv,
-                                         unsigned char* smem, RedScratch* rs) {
-    const int Mx = b.Mx, My = b.My, N = b.N, my4 = 4 * My + 1, mx4 = 4 * Mx + 1;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    double dev = 0.0, mag = 0.0;
-    for (int e = tid; e < mx4 * my4; e += nt) {
-        const int pi = e / my4, qi = e % my4;
-        const cplx v = Ge[e];
-        dev = fmax(dev, fmax(cabs(csub(v, Ge[(mx4 - 1 - pi) * my4 + qi])), cabs(csub(v, Ge[pi * my4 + (my4 - 1 - qi)]))));
-        mag = fmax(mag, cabs(v));
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        dev = fmax(dev, __shfl_down_sync(0xffffffffu, dev, o));
-        mag = fmax(mag, __shfl_down_sync(0xffffffffu, mag, o));
-    }
-    if ((tid & 31) == 0) {
-        rs->d[tid >> 5] = dev;
-        rs->d[32 + (tid >> 5)] = mag;
-    }
-    // assemble the four blocks B_c = S_c^T epsT S_c and identity right-hand sides
-    size_t off = 0;
-    for (int c = 0; c < 4; ++c) {
-        const int a = sym_class_a(c), bb = sym_class_b(c);
-        const int nb = sym_count(My, bb), s = sym_count(Mx, a) * nb;
-        cplx* B = work + off;
-        for (int e = tid; e < s * s; e += nt) {
-            const int i = e / s, j = e % s;
-            const int pi = i / nb + (a > 0 ? 0 : 1), qi = i % nb + (bb > 0 ? 0 : 1);
-            const int pj = j / nb + (a > 0 ? 0 : 1), qj = j % nb + (bb > 0 ? 0 : 1);
-            const double w = orbit_weight((pi > 0) + (qi > 0) + (pj > 0) + (qj > 0));
-            cplx v = C(0.0, 0.0);
-            for (int sp = 1; sp >= (pi > 0 ? -1 : 1); sp -= 2)
-                for (int sq = 1; sq >= (qi > 0 ? -1 : 1); sq -= 2)
-                    for (int tp = 1; tp >= (pj > 0 ? -1 : 1); tp -= 2)
-                        for (int tq = 1; tq >= (qj > 0 ? -1 : 1); tq -= 2) {
-                            const double sg = (sp < 0 ? a : 1) * (sq < 0 ? bb : 1) * (tp < 0 ? a : 1) * (tq < 0 ? bb : 1);
-                            const cplx g = Ge[(sp * pi - tp * pj + 2 * Mx) * my4 + (sq * qi - tq * qj + 2 * My)];
-                            v = cadd(v, cscale(g, sg));
-                        }
-            B[e] = cscale(v, w);
-        }
-        off += (size_t)s * s;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double d = 0.0, m = 0.0;
-        for (int w = 0; w < nt / 32; ++w) {
-            d = fmax(d, rs->d[w]);
-            m = fmax(m, rs->d[32 + w]);
-        }
-        if (!(d < b.sym_tol * m) && b.info[cell] == 0) b.info[cell] = kInfoAsym;  // strict: tolerance 0 flags all
-    }
-    // Ge is dead: each block is inverted in place in shared memory over the
-    // raster region (Gauss-Jordan, laurent_smem() reserves the largest block)
-    off = 0;
-    for (int c = 0; c < 4; ++c) {
-        const int s = sym_count(Mx, sym_class_a(c)) * sym_count(My, sym_class_b(c));
-        if (s == 0) continue;
-        const int ld = s | 1;  // odd: the pivot search's column walk spreads over the banks
-        cplx* Ms = reinterpret_cast<cplx*>(smem);
-        cplx* scr = Ms + (size_t)s * ld;
-        int* gpiv = reinterpret_cast<int*>(scr + 2 * s + 1);
-        int* sp = gpiv + s;
-        const cplx* B = work + off;
-        for (int e = tid; e < s * s; e += nt) Ms[(e / s) * ld + e % s] = B[e];
-        const int info = blk_gj_inverse_smem(s, Ms, ld, scr, gpiv, sp);
-        if (info != 0 && tid == 0 && b.info[cell] == 0) b.info[cell] = -info;
-        cplx* R = work + (size_t)N * N + off;
-        for (int e = tid; e < s * s; e += nt) R[e] = Ms[(e / s) * ld + e % s];
-        __syncthreads();
-        off += (size_t)s * s;
-    }
-    size_t offs[4];
-    off = 0;
-    for (int c = 0; c < 4; ++c) {
-        offs[c] = off;
-        const int s = sym_count(Mx, sym_class_a(c)) * sym_count(My, sym_class_b(c));
-        off += (size_t)s * s;
-    }
-    for (int e = tid; e < N * N; e += nt) {
-        int p, q, pp, qq;
-        order_pq(b, e / N, p, q);
-        order_pq(b, e % N, pp, qq);
-        cplx v = C(0.0, 0.0);
-        for (int c = 0; c < 4; ++c) {
-            double si, sj;
-            int ex = 0;
-            const int i = scalar_class_index(My, c, p, q, &si, &ex);
-            const int j = scalar_class_index(My, c, pp, qq, &sj, &ex);
-            if (i < 0 || j < 0) continue;
-            const int s = sym_count(Mx, sym_class_a(c)) * sym_count(My, sym_class_b(c));
-            const cplx r = work[(size_t)N * N + offs[c] + (size_t)i * s + j];
-            v = cadd(v, cscale(r, si * sj * orbit_weight(ex)));
-        }
-        Einv[e] = v;
-    }
-}
-
 // Rows of G1 in shared memory: at least 4, so that the per-axis sample tables
 // of the raster (2 x 4 ng doubles) fit in the same region.
 __host__ __device__ __forceinline__ int laurent_g1_rows(int Mx) { return 4 * Mx + 1 > 4 ? 4 * Mx + 1 : 4; }
@@ -524,14 +400,8 @@ __global__ void __launch_bounds__(kRT) rcwa_fourier_laurent(Bucket b) {
         order_pq(b, col, pp, qq);
         const cplx v = Ge[(p - pp + 2 * b.Mx) * my4 + (q - qq + 2 * b.My)];
         Exx[e] = v;
-        if (!b.sym) {
-            lu[e] = v;
-            Einv[e] = C(r == col ? 1.0 : 0.0, 0.0);
-        }
-    }
-    if (b.sym) {
-        laurent_inverse_by_class(b, cell, Ge, lu, Einv, smem, &rs);
-        return;
+        lu[e] = v;
+        Einv[e] = C(r == col ? 1.0 : 0.0, 0.0);
     }
     __syncthreads();
     // the raster, G1 and Ge are dead: the LU staging and GEMM tiles overlay them
@@ -1219,8 +1089,7 @@ __global__ void __launch_bounds__(kRT) rcwa_epilogue(Bucket b) {
 // so the layer problem splits into one of order ~n/4 per class, each excitation lies
 // in one class, and the amplitudes of the excited classes are those of the full problem
 // up to rounding. M_c is built straight from the scalar parity blocks of Exx, Eyy
-// and Einv (rcwa_sym_build; the Laurent Einv itself comes from four block
-// inverses), never forming M. A cell whose eps operators are not mirror
+// and Einv (rcwa_sym_ops), never forming M. A cell whose eps operators are not mirror
 // symmetric to rounding (a raster sample falling exactly on a shape boundary
 // one way and not the other) is flagged kInfoAsym and solved again at full order.
 // When the cell is
@@ -1272,37 +1141,13 @@ __device__ __forceinline__ int scalar_orbit_index(int My, int a, int bb, int p, 
     if ((p == 0 && a < 0) || (q == 0 && bb < 0)) return -1;
     return (p - (a > 0 ? 0 : 1)) * sym_count(My, bb) + (q - (bb > 0 ? 0 : 1));
 }
-// Entry (i, j) of S^T E S for the unit orbit vectors S of scalar class (a, bb)
-// and an N x N order-space operator E that commutes with both mirrors.
-__device__ cplx scalar_block_entry(const cplx* E, int N, int Mx, int My, int a, int bb, int i, int j) {
-    const int ny = 2 * My + 1;
-    int pi, qi, pj, qj;
-    scalar_orbit(My, a, bb, i, pi, qi);
-    scalar_orbit(My, a, bb, j, pj, qj);
-    cplx v = C(0.0, 0.0);
-    for (int sp = 1; sp >= (pi > 0 ? -1 : 1); sp -= 2)
-        for (int sq = 1; sq >= (qi > 0 ? -1 : 1); sq -= 2) {
-            const cplx* row = E + (size_t)((sp * pi + Mx) * ny + (sq * qi + My)) * N;
-            const int si = (sp < 0 ? a : 1) * (sq < 0 ? bb : 1);
-            for (int tp = 1; tp >= (pj > 0 ? -1 : 1); tp -= 2)
-                for (int tq = 1; tq >= (qj > 0 ? -1 : 1); tq -= 2) {
-                    const int sg = si * (tp < 0 ? a : 1) * (tq < 0 ? bb : 1);
-                    v = cadd(v, cscale(row[(tp * pj + Mx) * ny + (tq * qj + My)], (double)sg));
-                }
-        }
-    return cscale(v, orbit_weight((pi > 0) + (qi > 0) + (pj > 0) + (qj > 0)));
-}
-
-// The class operators of a mirror-symmetric cell, built from the scalar parity
-// blocks of its eps operators (on the class path this replaces the full
-// M = [Eyy; Exx] J Einv J' + ... of rcwa_build_M and its projection).
-// Vector class c = (a, b) has its u field block in scalar class (a, b) and its
-// v block in (-a, -b). Every operator of M maps parity classes onto parity
-// classes: with kx0 = ky0 = 0, Kx takes the unit orbit vector of (|p|, |q|) in
-// class (a, b) to kx = -2 pi |p| / px times the orbit vector of the same orbit
-// in (-a, b), and Ky likewise in q. So with Eu = Eyy^(a,b), Ev = Exx^(-a,-b)
-// and G = Einv^(a,-b), the one block of Einv that the class meets, and s(j) the
-// index in (a, -b) of the orbit of j (its k is 0 where it has none):
+// ---- class operators of mirror-symmetric cells ------------------------------------------------
+// Vector class c = (a, b) has its u field block in scalar class (a, b) and its v block in
+// (-a, -b). Every operator of M maps parity classes onto parity classes: with kx0 =
+// ky0 = 0, Kx takes the unit orbit vector of (|p|, |q|) in class (a, b) to kx = -2 pi |p| / px
+// times the orbit vector of the same orbit in (-a, b), and Ky likewise in q. So with
+// Eu = Eyy^(a,b), Ev = Exx^(-a,-b) and G = Einv^(a,-b), the one block of Einv that the class
+// meets, and s(j) the index in (a, -b) of the orbit of j (its k is 0 where it has none):
 //   Yt = Lt G, Lt[i][t] = Eu[i][t] (-ky(t));   Yb = Lb G, Lb[l][t] = Ev[l][t] kx(t)
 //   M(u,u) = Yt[i][s(j)] ky(j) + w^2 Eu[i][j] - [i = j] kx^2
 //   M(u,v) = -Yt[i][s(j)] kx(j) - [same orbit] kx ky
@@ -1311,69 +1156,272 @@ __device__ cplx scalar_block_entry(const cplx* E, int N, int Mx, int My, int a, 
 // (the order-space M of rcwa_build_M), the layer kp = w^2 - J Einv J^T
 // (rcwa2d.cpp:346-352) as kp(u,u) = w^2 [i = j] - ky G ky, kp(u,v) = ky G kx,
 // kp(v,u) = kx G ky, kp(v,v) = w^2 [i = j] - kx G kx.
-// Flags kInfoAsym when Exx, Eyy or Einv is not mirror symmetric to the
-// tolerance, or, for a C4 bucket (ncls = 1), when Eyy[k][l] != Exx[rho k][rho l]
-// or Einv[rho k][rho l] != Einv[k][l] (rho: order (p, q) -> (-q, p)); these
-// make M commute with the mirrors (and with R).
-// Scratch: the cell's full-order Z and X (free on the class path).
-__global__ void __launch_bounds__(kRT) rcwa_sym_build(Bucket b) {
-    __shared__ GemmSmem gs;
-    __shared__ double red[6][32];
+//
+// The scalar blocks come straight from the 1D tables (analytic rectangle) or from the
+// Laurent coefficients Ge; no N x N operator is formed:
+//   a Toeplitz or parity-even operator T[p][p'] between the unit orbit vectors of parity
+//   a is f (T[p][p'] + a T[p][-p']), f = 1, 1/sqrt2, 1/2 by how many of p, p' are 0, times 2;
+//   Laurent: B^(a,b) is the sum of the four Ge[p -+ p'][q -+ q'] with those signs, and
+//   G its inverse (Gauss-Jordan of slab.cuh): one block per solved class, order ~N/4.
+
+// factor of (T[p][p'] + a T[p][-p']) between unit orbit vectors (p, p' >= 0; p' = 0 has
+// one term only, so both terms are equal there and half the sum counts)
+__device__ __forceinline__ double orbit_factor(int p, int pp) {
+    return p == 0 ? (pp == 0 ? 0.5 : 0.70710678118654752440) : (pp == 0 ? 0.70710678118654752440 : 1.0);
+}
+
+// ---- rasterised shapes: Fourier coefficients from sample intervals
+// The samples of a raster row (one of four per pixel row, rcwa2d.cpp:74-95) that lie inside
+// an unrotated shape form an interval, less an inner one for a ring: the tests compare a
+// function of |x| that does not decrease away from x = 0 (with the reference's own
+// roundings) with a bound. So a row is two binary searches, and its sum over the samples is a
+// difference of prefix sums of the phase factors: nothing is summed over the pixels. 512
+// cells on 256^2 rasters, M = 3..7, 11.9 -> 6.9 ms a call; the operators of 102 M = 7 cells
+// 2.1 -> 0.2 ms, of one M = 5 rectangle 0.30 -> 0.08 ms.
+//
+// Tables of a bucket, m = 0 .. 2 M: ph[m][i] = exp(-2 pi i m xf_i) / ng of pixel i, and
+// pc[m][i] = sum of ph[m][0 .. i), the geometric series in closed form.
+__global__ void rcwa_prefix_table(int ng, int mmax, cplx* ph, cplx* pc) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (mmax + 1) * (ng + 1)) return;
+    const int m = e / (ng + 1), i = e - m * (ng + 1);
+    double s, c;
+    if (i < ng) {
+        sincospi(-2.0 * m * ((i + 0.5) / ng - 0.5), &s, &c);
+        ph[(size_t)m * ng + i] = C(c / ng, s / ng);
+    }
+    if (m % ng == 0) {  // every pixel has the same phase
+        sincospi(-2.0 * m * (0.5 / ng - 0.5), &s, &c);
+        pc[e] = C(c * i / ng, s * i / ng);
+        return;
+    }
+    // e^{i pi m} e^{-i pi m i / ng} sin(pi m i / ng) / (ng sin(pi m / ng))
+    const double r = sinpi((double)m * i / ng) / (ng * sinpi((double)m / ng));
+    sincospi(m - (double)m * i / ng, &s, &c);
+    pc[e] = C(r * c, r * s);
+}
+
+// First index in [0, cnt) at which pred holds (cnt if none); pred is monotone.
+template <class Pred>
+__device__ __forceinline__ int first_true(int cnt, const Pred& pred) {
+    int lo = 0, hi = cnt;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (pred(mid)) hi = mid;
+        else lo = mid + 1;
+    }
+    return lo;
+}
+// The samples t in [0, 2 half) with pred(t), pred true on an interval around the middle
+// (monotone on either half): [lo, hi).
+template <class Pred>
+__device__ __forceinline__ void centred_interval(int half, const Pred& pred, int& lo, int& hi) {
+    lo = first_true(half, pred);
+    hi = half + first_true(half, [&](int t) { return !pred(half + t); });
+}
+
+// Shared memory of rcwa_sym_ops: a region for the raster tables (or the 1D rectangle
+// tables), later the Gauss-Jordan routine's, then the coefficients.
+__host__ __device__ inline size_t sym_ops_tables(int ng) { return (size_t)4 * ng * (2 * 8 + 4 * 2); }
+__host__ __device__ inline size_t sym_ops_smem(int Mx, int My, int ng) {
+    const int big = (Mx + 1) * (My + 1) > 2 * (Mx > My ? Mx : My) + 1 ? (Mx + 1) * (My + 1) : 2 * (Mx > My ? Mx : My) + 1;
+    const size_t a = slab::shared_bytes(big), t = ng > 0 ? sym_ops_tables(ng) : 0;
+    const size_t coef = ng > 0 ? (size_t)(2 * Mx + 1) * (4 * My + 1) * 16
+                               : ((size_t)(4 * Mx + 1) + (4 * My + 1)) * 8 + 16;
+    return ((a > t ? a : t) + 15) / 16 * 16 + coef;
+}
+
+struct RasterCoef {  // Ge from the count transform F (dp >= 0; F[-d] = conj F[d])
+    const cplx* F;
+    cplx eb, dE;
+    int My;
+    __device__ cplx operator()(int dp, int dq) const {
+        const cplx f = dp >= 0 ? F[dp * (4 * My + 1) + dq + 2 * My] : cconj(F[-dp * (4 * My + 1) - dq + 2 * My]);
+        const cplx v = cmul(dE, f);
+        return dp == 0 && dq == 0 ? cadd(v, eb) : v;
+    }
+};
+
+// F[dp][dq], dp = 0 .. 2 Mx, of the cell's inside fractions into smem (F); G1 (global):
+// (2 Mx + 1) x ng. tabs: the shared tables.
+__device__ void raster_transform(const Bucket& b, const CellDev& c, cplx* G1, unsigned char* tabs, cplx* F) {
+    const int ng = b.ng, Mx = b.Mx, My = b.My, tid = threadIdx.x, nt = blockDim.x;
+    double* tx = reinterpret_cast<double*>(tabs);
+    double* ty = tx + 4 * ng;
+    short* iv = reinterpret_cast<short*>(ty + 4 * ng);  // per sample row: lo, hi, inner lo, inner hi
+    const double ax = c.fill_x * 0.5, ay = c.fill_y * 0.5;
+    const bool round_shape = c.shape == CELERIS_SHAPE_ELLIPSE || c.shape == CELERIS_SHAPE_RING;
+    const bool empty = round_shape && (ax <= 0.0 || ay <= 0.0);
+    for (int t = tid; t < 4 * ng; t += nt) {
+        const double xf = raster_coord(t >> 2, t & 3, ng);
+        if (round_shape) {
+            const double u = xf / ax, v = xf / ay;
+            tx[t] = __dmul_rn(u, u);
+            ty[t] = __dmul_rn(v, v);
+        } else {
+            tx[t] = ty[t] = fabs(xf);
+        }
+    }
+    __syncthreads();
+    const double hx = ax * c.shape_param, hy = ay * c.shape_param, ri2 = __dmul_rn(c.shape_param, c.shape_param);
+    const int half = 2 * ng;
+    for (int t = tid; t < 4 * ng; t += nt) {
+        int lo = 0, hi = 0, ilo = 0, ihi = 0;
+        const double y = ty[t];
+        if (empty) {
+        } else if (round_shape) {
+            centred_interval(half, [&](int i) { return __dadd_rn(tx[i], y) <= 1.0; }, lo, hi);
+            if (c.shape == CELERIS_SHAPE_RING)
+                centred_interval(half, [&](int i) { return !(__dadd_rn(tx[i], y) >= ri2); }, ilo, ihi);
+        } else {
+            double bound = -1.0;
+            if (y <= ay) bound = c.shape == CELERIS_SHAPE_RECT ? ax : hx;
+            if (c.shape == CELERIS_SHAPE_CROSS && y <= hy) bound = fmax(bound, ax);
+            if (bound >= 0.0) centred_interval(half, [&](int i) { return tx[i] <= bound; }, lo, hi);
+        }
+        ilo = max(ilo, lo);
+        ihi = max(min(ihi, hi), ilo);
+        if (ilo >= hi) ilo = ihi = hi;
+        iv[4 * t] = (short)lo;
+        iv[4 * t + 1] = (short)hi;
+        iv[4 * t + 2] = (short)ilo;
+        iv[4 * t + 3] = (short)ihi;
+    }
+    __syncthreads();
+    // G1[dp][iy] = sum over the row's samples of ph[dp][pixel] (a sixteenth each)
+    for (int e = tid; e < (2 * Mx + 1) * ng; e += nt) {
+        const int dp = e / ng, iy = e - dp * ng;
+        const cplx* ph = b.phx + (size_t)dp * ng;
+        const cplx* pc = b.pcx + (size_t)dp * (ng + 1);
+        cplx s = C(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const short4 v = reinterpret_cast<const short4*>(iv)[4 * iy + k];
+            const int end[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {  // + hi - lo, - (inner hi - inner lo)
+                const double sg = (j == 1 || j == 2) ? 1.0 : -1.0;
+                const int px = end[j] >> 2, rest = end[j] & 3;
+                s = cadd(s, cscale(pc[px], sg * 4.0));  // four samples a pixel
+                if (rest) s = cadd(s, cscale(ph[px], sg * rest));
+            }
+        }
+        G1[e] = cscale(s, 0.0625);
+    }
+    __syncthreads();
+    // F[dp][dq] = sum_iy G1[dp][iy] ph[dq][iy]
+    const int nq = 4 * My + 1;
+    for (int e = tid; e < (2 * Mx + 1) * nq; e += nt) {
+        const int dp = e / nq, dq = e - dp * nq - 2 * My;
+        const cplx* g = G1 + (size_t)dp * ng;
+        const cplx* ph = b.phy + (size_t)abs(dq) * ng;
+        const double sg = dq < 0 ? -1.0 : 1.0;
+        cplx s[4] = {C(0.0, 0.0), C(0.0, 0.0), C(0.0, 0.0), C(0.0, 0.0)};
+        int i = 0;
+        for (; i + 4 <= ng; i += 4)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[u] = cfma(g[i + u], C(ph[i + u].x, sg * ph[i + u].y), s[u]);
+        for (; i < ng; ++i) s[0] = cfma(g[i], C(ph[i].x, sg * ph[i].y), s[0]);
+        F[e] = cadd(cadd(s[0], s[1]), cadd(s[2], s[3]));
+    }
+    __syncthreads();
+}
+
+// The operators M and kp of a cell's solved classes. Flags kInfoAsym when the Laurent
+// coefficients are not even in dp and in dq to the tolerance (or, for a C4 bucket, Ge(dp, dq)
+// != Ge(-dq, dp)); those symmetries make M commute with the mirrors (and with the rotation).
+// The analytic rectangle has them exactly. Scratch: the cell's Z and X.
+template <int NT>
+__global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) rcwa_sym_ops(Bucket b) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double red[32];
     const int cell = blockIdx.x;
     const CellDev cd = b.cells[cell];
-    const int N = b.N, Mx = b.Mx, My = b.My, ny = 2 * My + 1;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const cplx* Exx = at(b.Exx, b.s_NN, cell);
-    const cplx* Eyy = b.ng > 0 ? Exx : at(b.Eyy, b.s_NN, cell);
-    const cplx* Einv = at(b.Einv, b.s_NN, cell);
-    // symmetry of the ingredients: deviation and magnitude of Exx, Eyy, Einv
-    double dv[3] = {0.0, 0.0, 0.0}, mg[3] = {0.0, 0.0, 0.0};
-    for (int e = tid; e < N * N; e += nt) {
-        const int k = e / N, l = e % N;
-        const int pk = k / ny - Mx, qk = k % ny - My, pl = l / ny - Mx, ql = l % ny - My;
-        const size_t ex = (size_t)((-pk + Mx) * ny + qk + My) * N + (-pl + Mx) * ny + ql + My;
-        const size_t ey = (size_t)((pk + Mx) * ny - qk + My) * N + (pl + Mx) * ny - ql + My;
-        const cplx* X[3] = {Exx, Eyy, Einv};
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const cplx v = X[t][e];
-            dv[t] = fmax(dv[t], fmax(cabs(csub(v, X[t][ex])), cabs(csub(v, X[t][ey]))));
-            mg[t] = fmax(mg[t], cabs(v));
-        }
-        if (b.ncls == 1) {  // rho k = (-qk, pk): Mx = My, so ny indexes both axes
-            const size_t er = (size_t)((-qk + Mx) * ny + pk + My) * N + (-ql + Mx) * ny + pl + My;
-            dv[1] = fmax(dv[1], cabs(csub(Eyy[e], Exx[er])));
-            dv[2] = fmax(dv[2], cabs(csub(Einv[e], Einv[er])));
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < 3; ++t)
-        for (int o = 16; o > 0; o >>= 1) {
-            dv[t] = fmax(dv[t], __shfl_down_sync(0xffffffffu, dv[t], o));
-            mg[t] = fmax(mg[t], __shfl_down_sync(0xffffffffu, mg[t], o));
-        }
-    if ((tid & 31) == 0)
-        for (int t = 0; t < 3; ++t) {
-            red[t][tid >> 5] = dv[t];
-            red[3 + t][tid >> 5] = mg[t];
-        }
-    __syncthreads();
-    if (tid == 0) {
-        bool asym = false;
-        for (int t = 0; t < 3; ++t) {
-            double d = 0.0, m = 0.0;
-            for (int w = 0; w < nt / 32; ++w) {
-                d = fmax(d, red[t][w]);
-                m = fmax(m, red[3 + t][w]);
-            }
-            asym = asym || !(d < b.sym_tol * m);  // strict: tolerance 0 flags every cell
-        }
-        if (asym && b.info[cell] == 0) b.info[cell] = kInfoAsym;
-    }
-    const double w2 = cd.omega * cd.omega;
-    const int m = b.m;
+    const int Mx = b.Mx, My = b.My, tid = threadIdx.x, nt = NT, m = b.m;
+    const int nx = 2 * Mx + 1, ny = 2 * My + 1;
+    const int big = max((Mx + 1) * (My + 1), max(nx, ny));
+    unsigned char* coef = smem + sym_ops_smem(Mx, My, b.ng) -
+                          (b.ng > 0 ? (size_t)nx * (4 * My + 1) * 16 : ((size_t)(4 * Mx + 1) + (4 * My + 1)) * 8 + 16);
     cplx* Zs = at(b.Z, b.s_nn, cell);
     cplx* Xs = at(b.X, b.s_nn, cell);
+    const double w2 = cd.omega * cd.omega;
+    const cplx ep = cd.eps_p, eb = cd.eps_b, ibe = cinv(eb), dI = csub(cinv(ep), ibe);
+    cplx* F = reinterpret_cast<cplx*>(coef);
+    double* sx = reinterpret_cast<double*>(coef);  // rect1d(d, fill_x), d = 0 .. 4 Mx
+    double* sy = sx + 4 * Mx + 1;
+    cplx* ax = b.G1 + b.s_g1 * cell;  // rectangle: the inverses of the 1D reciprocal Toeplitz matrices
+    cplx* ay = ax + nx * nx;
+    const RasterCoef Ge{F, eb, csub(ep, eb), My};
+    bool asym;
+    if (b.ng > 0) {
+        raster_transform(b, cd, ax, smem, F);
+        double dev = 0.0, mag = 0.0;
+        for (int e = tid; e < (4 * Mx + 1) * (4 * My + 1); e += nt) {
+            const int dp = e / (4 * My + 1) - 2 * Mx, dq = e % (4 * My + 1) - 2 * My;
+            const cplx v = Ge(dp, dq);
+            dev = fmax(dev, fmax(cabs(csub(v, Ge(-dp, dq))), cabs(csub(v, Ge(dp, -dq)))));
+            if (b.ncls == 1) dev = fmax(dev, cabs(csub(v, Ge(-dq, dp))));
+            mag = fmax(mag, cabs(v));
+        }
+        dev = slab::block_max(dev, red);
+        mag = slab::block_max(mag, red);
+        asym = !(dev < b.sym_tol * mag);  // strict: tolerance 0 flags every cell
+    } else {
+        for (int d = tid; d <= 4 * Mx; d += nt) sx[d] = rect1d(d, cd.fill_x);
+        for (int d = tid; d <= 4 * My; d += nt) sy[d] = rect1d(d, cd.fill_y);
+        __syncthreads();
+        asym = !(0.0 < b.sym_tol);
+        // Hx, Hy (rcwa2d.cpp:299-303, 317-321), inverted
+        const slab::Shared s = slab::carve(smem, big);
+        for (int axis = 0; axis < 2; ++axis) {
+            const int n1 = axis ? ny : nx;
+            const double* t1 = axis ? sy : sx;
+            cplx* W = Zs;
+            for (int e = tid; e < n1 * n1; e += nt) {
+                const int i = e / n1, j = e - i * n1;
+                const cplx v = cscale(dI, t1[abs(i - j)]);
+                W[e] = i == j ? cadd(v, ibe) : v;
+            }
+            if (!slab::gauss_jordan(n1, n1, W, n1, true, s)) {
+                if (tid == 0) b.info[cell] = -(axis + 1);
+                return;
+            }
+            for (int e = tid; e < n1 * n1; e += nt) {
+                const int k = e / n1, c = e - k * n1;
+                (axis ? ay : ax)[(size_t)k * n1 + s.perm[c]] = W[(size_t)s.perm[k] * n1 + c];
+            }
+            __syncthreads();
+        }
+    }
+    if (asym) {
+        if (tid == 0) b.info[cell] = kInfoAsym;
+        return;
+    }
+    // entry (i, j) of an operator's block in scalar class (a, bb): which = 0 Exx, 1 Eyy,
+    // 2 Einv (rectangle only)
+    auto entry = [&](int which, int a, int bb, int i, int j) -> cplx {
+        int p, q, pp, qq;
+        scalar_orbit(My, a, bb, i, p, q);
+        scalar_orbit(My, a, bb, j, pp, qq);
+        const double f = orbit_factor(p, pp) * orbit_factor(q, qq);
+        if (b.ng > 0) {
+            const cplx u = cadd(Ge(p - pp, q - qq), cscale(Ge(p + pp, q - qq), (double)a));
+            const cplx v = cadd(Ge(p - pp, q + qq), cscale(Ge(p + pp, q + qq), (double)a));
+            return cscale(cadd(u, cscale(v, (double)bb)), f);
+        }
+        const double tx = sx[abs(p - pp)] + a * sx[p + pp], ty = sy[abs(q - qq)] + bb * sy[q + qq];
+        const double dx = p == pp ? 1.0 : 0.0, dy = q == qq ? 1.0 : 0.0;
+        if (which == 2) {
+            cplx v = cscale(dI, tx * ty * f);
+            return i == j ? cadd(v, ibe) : v;
+        }
+        if (which == 0) {  // Ax (x) Sy + eb I (x) (I - Sy)
+            const cplx A = cadd(ax[(p + Mx) * nx + pp + Mx], cscale(ax[(p + Mx) * nx - pp + Mx], (double)a));
+            return cadd(cscale(A, ty * f), cscale(eb, dx * (dy - ty * orbit_factor(q, qq))));
+        }
+        const cplx A = cadd(ay[(q + My) * ny + qq + My], cscale(ay[(q + My) * ny - qq + My], (double)bb));
+        return cadd(cscale(A, tx * f), cscale(eb, dy * (dx - tx * orbit_factor(p, pp))));
+    };
     for (int cc = 0; cc < b.ncls; ++cc) {
         const int c = b.cls0 + cc;
         const int a = sym_class_a(c), bb = sym_class_b(c);
@@ -1388,10 +1436,23 @@ __global__ void __launch_bounds__(kRT) rcwa_sym_build(Bucket b) {
         cplx* Yt = Lb + (size_t)sv * st;
         cplx* Yb = Yt + (size_t)su * st;
         __syncthreads();  // the previous class's readers of the scratch are done
-        for (int e = tid; e < su * su; e += nt) Eu[e] = scalar_block_entry(Eyy, N, Mx, My, a, bb, e / su, e % su);
-        for (int e = tid; e < sv * sv; e += nt) Ev[e] = scalar_block_entry(Exx, N, Mx, My, -a, -bb, e / sv, e % sv);
-        for (int e = tid; e < st * st; e += nt) G[e] = scalar_block_entry(Einv, N, Mx, My, a, -bb, e / st, e % st);
+        for (int e = tid; e < su * su; e += nt) Eu[e] = entry(1, a, bb, e / su, e % su);
+        for (int e = tid; e < sv * sv; e += nt) Ev[e] = entry(0, -a, -bb, e / sv, e % sv);
+        cplx* Gb = b.ng > 0 ? Xs : G;  // the Laurent block is inverted on the way
+        for (int e = tid; e < st * st; e += nt) Gb[e] = entry(2, a, -bb, e / st, e % st);
         __syncthreads();
+        if (b.ng > 0 && st > 0) {
+            const slab::Shared s = slab::carve(smem, big);  // the raster tables are dead
+            if (!slab::gauss_jordan(st, st, Gb, st, true, s)) {
+                if (tid == 0 && b.info[cell] == 0) b.info[cell] = -1;
+                return;
+            }
+            for (int e = tid; e < st * st; e += nt) {
+                const int k = e / st, l = e - k * st;
+                G[(size_t)k * st + s.perm[l]] = Gb[(size_t)s.perm[k] * st + l];
+            }
+            __syncthreads();
+        }
         // Lt[i][t] = Eu[i][orbit t in (a, b)] (-ky(t)), Lb[l][t] = Ev[l][orbit t in (-a, -b)] kx(t)
         for (int e = tid; e < (su + sv) * st; e += nt) {
             const int r = e / st, t = e % st;
@@ -1408,8 +1469,13 @@ __global__ void __launch_bounds__(kRT) rcwa_sym_build(Bucket b) {
                 Lb[(size_t)l * st + t] = j < 0 ? C(0.0, 0.0) : cscale(Ev[(size_t)l * sv + j], kx);
             }
         }
-        blk_gemm(su, st, st, C(1.0, 0.0), Lt, st, G, st, C(0.0, 0.0), Yt, st, &gs);
-        blk_gemm(sv, st, st, C(1.0, 0.0), Lb, st, G, st, C(0.0, 0.0), Yb, st, &gs);
+        __syncthreads();
+        if (su > 0 && st > 0)
+            slab::gemm(su, st, st, (const cplx*)Lt, st, (const cplx*)G, st, nullptr,
+                       [=](int r, int j, cplx v) { Yt[(size_t)r * st + j] = v; });
+        if (sv > 0 && st > 0)
+            slab::gemm(sv, st, st, (const cplx*)Lb, st, (const cplx*)G, st, nullptr,
+                       [=](int r, int j, cplx v) { Yb[(size_t)r * st + j] = v; });
         __syncthreads();
         const size_t mi = (size_t)(b.ncls * cell + cc) * m * m;
         cplx* Mc = b.cM + mi;
@@ -2096,11 +2162,7 @@ size_t laurent_smem(int Mx, int My, int ng) {
     const size_t mx4 = 4 * Mx + 1, my4 = 4 * My + 1;
     const int N = (2 * Mx + 1) * (2 * My + 1);
     const size_t raster = ((size_t)laurent_g1_rows(Mx) * ng + mx4 * my4) * sizeof(cplx) + (size_t)ng * ng;
-    // the class path inverts its largest scalar parity block in place: s x (s + 1)
-    // + 2 s + 1 complex, s + 1 ints
-    const size_t sb = (size_t)(Mx + 1) * (My + 1);
-    const size_t gj = (sb * (sb + 1) + 2 * sb + 1) * sizeof(cplx) + (sb + 1) * sizeof(int);
-    return std::max(std::max(raster, gj), lu_stage_bytes(N) + sizeof(GemmSmem));
+    return std::max(raster, lu_stage_bytes(N) + sizeof(GemmSmem));
 }
 
 // ---- stage configuration and autotuning -------------------------------------------------
@@ -2156,22 +2218,25 @@ size_t slab_per_cell_bytes(int n, int nexc) {
            sizeof(int) + sizeof(celeris_rcwa_result) * nexc + sizeof(CellDev) + 16 * 256;
 }
 
-// Device memory of one mirror-symmetric cell: the full-order H (the Laurent inverse's
-// blocks), Z and X (the class build's scratch, then the two-port's work areas), the
-// Fourier operators, the vector area and pivots; per solved class M, kp and 2 m
-// amplitudes.
-size_t sym_per_cell_bytes(int Mx, int My, int nexc, int ncls) {
-    const int N = (2 * Mx + 1) * (2 * My + 1), n = 2 * N;
+// Row transform of a raster (or the two 1D inverses) of one mirror-symmetric cell.
+size_t sym_g1_size(int Mx, int My, int ng) {
+    const size_t nx = 2 * Mx + 1, ny = 2 * My + 1;
+    return std::max(nx * (size_t)ng, nx * nx + ny * ny);
+}
+// Device memory of one mirror-symmetric cell: Z and X of full order (the class build's
+// scratch, then the two-port's work areas), the raster's row transform, the vector
+// area; per solved class M, kp and 2 m amplitudes.
+size_t sym_per_cell_bytes(int Mx, int My, int ng, int nexc, int ncls) {
+    const size_t n = 2 * (size_t)(2 * Mx + 1) * (2 * My + 1);
     const size_t m = (size_t)sym_class_size(Mx, My, 0);
-    const size_t full = (3 * (size_t)n * n + 3 * (size_t)N * N + 10 * (size_t)n) * sizeof(cplx) +
-                        (size_t)n * sizeof(int) + sizeof(int) + sizeof(celeris_rcwa_result) * nexc + sizeof(CellDev);
-    return full + ncls * (2 * m * m + 2 * m) * sizeof(cplx) + 20 * 256;
+    return (2 * n * n + sym_g1_size(Mx, My, ng) + 10 * n + ncls * (2 * m * m + 2 * m)) * sizeof(cplx) + sizeof(int) +
+           sizeof(celeris_rcwa_result) * nexc + sizeof(CellDev) + 16 * 256;
 }
 
 // The largest dynamic shared memory each stage kernel needs over a wave's
 // buckets; raised once per wave, outside any capture.
 struct SmemNeeds {
-    size_t laurent = 0, rect = 0, hess_s = 0, hess_g = 0, smat = 0, slab = 0;
+    size_t laurent = 0, rect = 0, hess_s = 0, hess_g = 0, smat = 0, slab = 0, ops = 0;
     bool aed = false;
     void add_eig(int n) {
         if (n <= kSmemEigMaxN) hess_s = std::max(hess_s, ((size_t)n * n + 2 * n) * sizeof(cplx));
@@ -2179,7 +2244,9 @@ struct SmemNeeds {
         aed = true;
     }
     void add(int Mx, int My, int ng, int n, int sym = 0, int qr = 1) {
-        if (ng > 0) {
+        if (sym) {
+            ops = std::max(ops, sym_ops_smem(Mx, My, ng));
+        } else if (ng > 0) {
             laurent = std::max(laurent, laurent_smem(Mx, My, ng));
         } else {
             const int nx = 2 * Mx + 1, ny = 2 * My + 1;
@@ -2227,6 +2294,10 @@ int set_smem_limits(const SmemNeeds& s) {
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_smat1), s.smat));
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_smat2), s.smat));
     }
+    if (s.ops) {
+        CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_sym_ops<256>), s.ops));
+        CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_sym_ops<512>), s.ops));
+    }
     if (s.slab) {
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_slab<256>), s.slab));
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_slab<512>), s.slab));
@@ -2244,7 +2315,14 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
     const int* T = cfg.threads;
     if (ev) cudaEventRecord(ev[0], st);
     cudaMemsetAsync(b.info, 0, sizeof(int) * nc, st);
-    if (b.ng > 0) {
+    if (b.sym) {
+        if (b.ng > 0) {
+            const int mmax = 2 * std::max(b.Mx, b.My);
+            rcwa_prefix_table<<<((mmax + 1) * (b.ng + 1) + 255) / 256, 256, 0, st>>>(
+                b.ng, mmax, const_cast<cplx*>(b.phx), const_cast<cplx*>(b.pcx));
+        }
+        count_launch(b.ng > 0 ? 1 : 0);
+    } else if (b.ng > 0) {
         const int Mx = b.Mx, My = b.My, ng = b.ng;
         rcwa_phase_table<<<((4 * Mx + 1) * ng + 255) / 256, 256, 0, st>>>(ng, 2 * Mx, const_cast<cplx*>(b.phx));
         rcwa_phase_table<<<((4 * My + 1) * ng + 255) / 256, 256, 0, st>>>(ng, 2 * My, const_cast<cplx*>(b.phy));
@@ -2260,7 +2338,11 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
     if (!qr) {
         // the layer two-port: class operators first for mirror-symmetric cells, then one
         // kernel (timed as smat1), the amplitudes into the order basis, the outputs
-        if (b.sym) rcwa_sym_build<<<nc, T[ST_BUILD], 0, st>>>(b);
+        if (b.sym) {
+            const size_t sm = sym_ops_smem(b.Mx, b.My, b.ng);
+            if (slab_threads(1, nc) == 512) rcwa_sym_ops<512><<<nc, 512, sm, st>>>(b);
+            else rcwa_sym_ops<256><<<nc, 256, sm, st>>>(b);
+        }
         if (ev)
             for (int i = 2; i <= 5; ++i) cudaEventRecord(ev[i], st);
         const int m = b.sym ? b.m : n, count = b.sym ? b.ncls * nc : nc;
@@ -2472,7 +2554,7 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             if (p.ng > 0 && laurent_smem(p.Mx, p.My, p.ng) + 1024 > (size_t)smem_optin)
                 return set_error(CELERIS_ERR_TOO_LARGE, "raster %d with M=(%d,%d) exceeds shared memory", p.ng, p.Mx, p.My);
             p.per_cell = p.qr    ? per_cell_bytes(p.n, nexc)
-                         : p.sym ? sym_per_cell_bytes(p.Mx, p.My, nexc, p.sym == 2 ? 1 : 2)
+                         : p.sym ? sym_per_cell_bytes(p.Mx, p.My, p.ng, nexc, p.sym == 2 ? 1 : 2)
                                  : slab_per_cell_bytes(p.n, nexc);
             // split buckets that alone exceed the budget
             const size_t max_cells = std::max<size_t>(1, budget / std::max<size_t>(1, p.per_cell));
@@ -2578,23 +2660,29 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                 b.S12 = take(b.s_ns * nc);
                 b.q1 = take(b.s_n * nc);
             } else if (p.sym) {
-                for (cplx** m : {&b.H, &b.Z, &b.X}) *m = take(b.s_nn * nc);
+                for (cplx** m : {&b.Z, &b.X}) *m = take(b.s_nn * nc);
+                b.s_g1 = sym_g1_size(p.Mx, p.My, p.ng);
+                b.G1 = take(b.s_g1 * nc);
             } else {
                 b.H = take(b.s_nn * nc);
                 b.Kp = take(b.s_nn * nc);
                 b.s_w = slab::work_size(p.n);
                 b.slab = take(b.s_w * nc);
             }
-            b.Einv = static_cast<cplx*>(ws.take(sizeof(cplx) * b.s_NN * nc));
-            b.Exx = static_cast<cplx*>(ws.take(sizeof(cplx) * b.s_NN * nc));
-            b.Eyy = static_cast<cplx*>(ws.take(sizeof(cplx) * b.s_NN * nc));
-            b.vec = static_cast<cplx*>(ws.take(sizeof(cplx) * 10 * b.s_n * nc));
-            b.piv = static_cast<int*>(ws.take(sizeof(int) * b.s_n * nc));
+            if (!p.sym) {
+                for (cplx** m : {&b.Einv, &b.Exx, &b.Eyy}) *m = take(b.s_NN * nc);
+                b.piv = static_cast<int*>(ws.take(sizeof(int) * b.s_n * nc));
+            }
+            b.vec = take(10 * b.s_n * nc);
             b.info = static_cast<int*>(ws.take(sizeof(int) * nc));
             b.res = static_cast<celeris_rcwa_result*>(ws.take(sizeof(celeris_rcwa_result) * nexc * nc));
-            if (p.ng > 0) {
-                b.phx = static_cast<cplx*>(ws.take(sizeof(cplx) * (4 * p.Mx + 1) * p.ng));
-                b.phy = static_cast<cplx*>(ws.take(sizeof(cplx) * (4 * p.My + 1) * p.ng));
+            if (p.ng > 0 && p.sym) {  // one table for both axes
+                const size_t mt = 2 * std::max(p.Mx, p.My) + 1;
+                b.phx = b.phy = take(mt * p.ng);
+                b.pcx = take(mt * (p.ng + 1));
+            } else if (p.ng > 0) {
+                b.phx = take((size_t)(4 * p.Mx + 1) * p.ng);
+                b.phy = take((size_t)(4 * p.My + 1) * p.ng);
             }
             b.sym = p.sym;
             b.sym_tol = symmetry_tolerance();
@@ -2729,7 +2817,7 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                     cudaMemcpyAsync(const_cast<CellDev*>(p.b.cells), hdesc[w], sizeof(CellDev) * nc,
                                     cudaMemcpyHostToDevice, bs);
                     launch_bucket(p.b, cfgs[w], bs, nullptr, p.qr != 0);
-                    nk += (p.ng > 0 ? 3 : 1) + (p.qr ? 7 : p.sym ? 4 : 2);
+                    nk += p.sym ? (p.ng > 0 ? 5 : 4) : (p.ng > 0 ? 3 : 1) + (p.qr ? 7 : 2);
                     cudaMemcpyAsync(hres_pin[w], p.b.res, sizeof(celeris_rcwa_result) * nexc * nc,
                                     cudaMemcpyDeviceToHost, bs);
                     cudaMemcpyAsync(hinfo_pin[w], p.b.info, sizeof(int) * nc, cudaMemcpyDeviceToHost, bs);

@@ -98,3 +98,35 @@ def test_pole_in_a_stack_layer_and_redo_in_a_batch():
     for i, c in enumerate(cells):
         one, _ = capi.rcwa_batch([capi.rcwa_cell(**c)])
         assert abs(res[2 * i]["tx0"] - one[0]["tx0"]) <= TOL
+
+
+@pytest.mark.parametrize("shape", [capi.SHAPE_RECT, capi.SHAPE_ELLIPSE, capi.SHAPE_CROSS, capi.SHAPE_RING])
+@pytest.mark.parametrize("grid,Mx,My,fx,fy,param", [
+    (128, 2, 2, 0.55, 0.55, 0.5), (100, 2, 1, 0.6, 0.35, 0.4), (37, 1, 3, 0.31, 0.77, 0.3), (3, 2, 2, 0.7, 0.7, 0.5),
+    (64, 3, 2, 1.0, 1.0, 0.9), (48, 2, 2, 1.3, 0.5, 1.2), (33, 2, 2, 0.5, 0.5, 0.0), (256, 1, 1, 1e-3, 0.6, 0.5),
+])
+def test_raster_sample_intervals(shape, grid, Mx, My, fx, fy, param):
+    """Parity-class operators of rasterised shapes from sample intervals and prefix sums:
+    odd and tiny rasters (an order a multiple of the raster size), fills of nothing and of
+    more than the cell, cross and ring parameters of 0 and above 1."""
+    eps_p = complex(5.0, 0.1) if grid == 100 else 5.0
+    cell = dict(Mx=Mx, My=My, shape=shape, grid=grid, force_laurent=1, fill_x=fx, fill_y=fy, shape_param=param,
+                eps_pillar=eps_p)
+    eps = RO.rasterize_eps(eps_p, 1.0, grid, grid, shape, fx, fy, param, 0.0)
+    if np.linalg.cond(RO.laurent_toeplitz(eps, grid, grid, Mx, My)) > 1e12:
+        # fewer raster points than orders: the Laurent matrix is singular and no solution
+        # is defined (the oracle's inverse raises or is rounding noise); the call returns
+        _, info = capi.rcwa_batch([capi.rcwa_cell(**dict(BASE, **cell))])
+        assert info.shape == (1,)
+    elif np.ptp(eps.real) == 0.0 and np.ptp(eps.imag) == 0.0:
+        # the shape covers nothing or everything: a uniform layer, whose degenerate
+        # eigenvectors leave the oracle's numbers undefined; the Airy formula holds
+        n1, h = np.sqrt(eps[0, 0] + 0j), BASE["thickness_um"]
+        r12, r23 = (1.0 - n1) / (1.0 + n1), (n1 - 1.46) / (n1 + 1.46)
+        e2 = np.exp(4j * np.pi * n1 * h / BASE["wavelength_um"])
+        R = abs((r12 + r23 * e2) / (1 + r12 * r23 * e2)) ** 2
+        res, info = capi.rcwa_batch([capi.rcwa_cell(**dict(BASE, **cell))])
+        assert info[0] == 0
+        assert all(abs(q["R"] - R) <= TOL for q in res)
+    else:
+        check(cell)
