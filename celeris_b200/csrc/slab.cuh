@@ -50,7 +50,7 @@ constexpr int kMaxDoublings = 40;
 // end costs more, so it waits for a larger loss.
 constexpr int kMaxRest = 3;
 __device__ __forceinline__ double growth_limit(int rest) {
-    return rest == 0 ? 64.0 : rest == 1 ? 1e3 : 5e3;
+    return rest == 0 ? 64.0 : 3e3;
 }
 
 // ---- scalars: double or complex ---------------------------------------------------------
