@@ -1208,6 +1208,24 @@ int check_status_and_reset(cudaStream_t stream) {
     return CELERIS_OK;
 }
 
+// Device address of a stream's status word (resolved once per device), for reading it
+// behind the stream's work instead of with a synchronous copy after it.
+int status_address(cudaStream_t st, const int** out) {
+    static std::mutex mu;
+    static int* base[64] = {};
+    int dev = 0;
+    CEL_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return set_error(CELERIS_ERR_TOO_LARGE, "device index %d", dev);
+    std::lock_guard<std::mutex> lk(mu);
+    if (!base[dev]) {
+        void* p = nullptr;
+        CEL_CUDA(cudaGetSymbolAddress(&p, g_ff_status));
+        base[dev] = static_cast<int*>(p);
+    }
+    *out = base[dev] + status_slot(st);
+    return CELERIS_OK;
+}
+
 Geom psf_geom(double cx, double cy, double z, int n, double W) {
     Geom g;
     g.mode = GEOM_PSF;
@@ -1592,6 +1610,12 @@ constexpr size_t kPiece = (size_t)4 << 20;
 // (per-thread events 1, 2, ...).
 int download(void* dst, char* stage, const void* src, size_t bytes, cudaStream_t st) {
     if (!dst || bytes == 0) return CELERIS_OK;
+    if (bytes <= kPiece) {
+        CEL_CUDA(cudaMemcpyAsync(stage, src, bytes, cudaMemcpyDeviceToHost, st));
+        CEL_CUDA(cudaStreamSynchronize(st));
+        std::memcpy(dst, stage, bytes);
+        return CELERIS_OK;
+    }
     const size_t np = (bytes + kPiece - 1) / kPiece;
     for (size_t i = 0; i < np; ++i) {
         const size_t o = i * kPiece, b = std::min(kPiece, bytes - o);
@@ -1652,7 +1676,8 @@ int ff_host(int form, const double* px, const double* py, const double* pt, int 
     const size_t idx_bytes = sidx.size() * sizeof(int);
     const size_t pin_bytes = celeris_rt::align256(in_bytes) + celeris_rt::align256(fld_bytes) +
                              celeris_rt::align256(int_bytes) + celeris_rt::align256(idx_bytes);
-    // pinned: the device I/O layout, then the accumulator words of the error check
+    // pinned: the device I/O layout, then the accumulator words of the error check and
+    // the two streams' status words
     char* pin = static_cast<char*>(celeris_rt::pinned_staging(pin_bytes + 256));
     if (!pin) return set_error(CELERIS_ERR_OOM, "pinned staging of %zu bytes failed", pin_bytes);
 
@@ -1680,7 +1705,14 @@ int ff_host(int form, const double* px, const double* py, const double* pt, int 
                               reinterpret_cast<const char*>(pt)};
         const size_t len[3] = {npil * sizeof(double), npil * sizeof(double), npil * 2 * sizeof(double)};
         size_t off = 0;
-        for (int a = 0; a < 3; ++a) {
+        if (in_bytes <= kPiece) {  // one transfer (the three arrays are contiguous on the device)
+            for (int a = 0; a < 3; ++a) {
+                std::memcpy(pin + off, src[a], len[a]);
+                off += len[a];
+            }
+            CEL_CUDA(cudaMemcpyAsync(d, pin, in_bytes, cudaMemcpyHostToDevice, st));
+        }
+        for (int a = 0; a < 3 && in_bytes > kPiece; ++a) {
             for (size_t o = 0; o < len[a]; o += kPiece) {
                 const size_t b = std::min(kPiece, len[a] - o);
                 std::memcpy(pin + off + o, src[a] + o, b);
@@ -1714,6 +1746,15 @@ int ff_host(int form, const double* px, const double* py, const double* pt, int 
         CEL_TRY(ff_check_enqueue(d_px, d_py, d_pt, npil, g, k, d_fld, d_idx, want_err ? (int)sidx.size() : 0,
                                  want_bound, h_acc, st2));
     }
+    int* h_status = reinterpret_cast<int*>(pin + pin_bytes + 128);
+    h_status[0] = h_status[1] = 0;
+    const int* d_status = nullptr;
+    CEL_TRY(status_address(st, &d_status));
+    CEL_CUDA(cudaMemcpyAsync(h_status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (stated) {
+        CEL_TRY(status_address(st2, &d_status));
+        CEL_CUDA(cudaMemcpyAsync(h_status + 1, d_status, sizeof(int), cudaMemcpyDeviceToHost, st2));
+    }
     const int rd = download(field_out, h_fld, d_fld, field_out ? fld_bytes : 0, st);
     const int ri = rd == CELERIS_OK ? download(int_out, h_int, d_int, int_out ? int_bytes : 0, st) : rd;
     cudaError_t e1 = cudaStreamSynchronize(st);
@@ -1723,8 +1764,8 @@ int ff_host(int form, const double* px, const double* py, const double* pt, int 
     CEL_CUDA(e2);
     if (want_err) *err_out = check_ratio(h_acc);
     if (want_bound) *bound_out = bound_ratio(h_acc, npil);
-    const int s1 = check_status_and_reset(st);
-    const int s2 = stated ? check_status_and_reset(st2) : CELERIS_OK;
+    const int s1 = h_status[0] ? check_status_and_reset(st) : CELERIS_OK;
+    const int s2 = stated && h_status[1] ? check_status_and_reset(st2) : CELERIS_OK;
     return s1 != CELERIS_OK ? s1 : s2;
 }
 

@@ -3152,6 +3152,15 @@ int run_stacks_qr(const celeris_rcwa_cell* layers, const std::vector<std::pair<i
     return CELERIS_OK;
 }
 
+// Device memory of one layer and of one stack of order n on the two-port path.
+size_t layer_bytes(int n) {
+    const size_t N = n / 2;
+    return (5 * (size_t)n * n + slab::work_size(n) + 3 * N * N) * sizeof(cplx) + 4096;
+}
+size_t stack_bytes(int n, int nexc) {
+    return (slab::work_size(n) + 10 * (size_t)n) * sizeof(cplx) + (size_t)nexc * n * sizeof(double) + 4096;
+}
+
 // The same through the layers' two-ports (rcwa_slab, rcwa_stack_port). info_out (required):
 // 0 or kInfoRedo per stack; results of flagged stacks are not written.
 int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair<int, int>>& stacks, const double* exc,
@@ -3170,16 +3179,27 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
         const celeris_rcwa_cell& f = layers[stacks[s].first];
         groups[{f.Mx, f.My}].push_back(s);
     }
-    size_t free_b = 0, total_b = 0;
-    CEL_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const size_t budget = (free_b + ws.capacity()) / 2;
     const size_t c16 = sizeof(cplx);
+    // the budget matters only when the arena must grow: the driver's query (a call that
+    // can take milliseconds) is left out while every group fits the arena that is there
+    size_t most = 0;
+    for (auto& g : groups) {
+        const int N = (2 * g.first.first + 1) * (2 * g.first.second + 1), n = 2 * N;
+        size_t all = 0;
+        for (int k : g.second) all += stack_bytes(n, nexc) + layer_bytes(n) * stacks[k].second;
+        most = std::max(most, all + ((size_t)1 << 22));
+    }
+    size_t budget = ws.capacity();
+    if (most > budget) {
+        size_t free_b = 0;
+        CEL_TRY(query_free_memory(dev, &free_b));
+        budget = (free_b + ws.capacity()) / 2;
+    }
     for (auto& g : groups) {
         const int Mx = g.first.first, My = g.first.second;
         const int N = (2 * Mx + 1) * (2 * My + 1), n = 2 * N;
         const size_t s_nn = (size_t)n * n, s_n = (size_t)n, s_NN = (size_t)N * N, s_w = slab::work_size(n);
-        const size_t per_layer = (5 * s_nn + s_w + 3 * s_NN) * c16 + 4096;
-        const size_t per_stack = (s_w + 10 * s_n) * c16 + (size_t)nexc * N * 2 * sizeof(double) + 4096;
+        const size_t per_layer = layer_bytes(n), per_stack = stack_bytes(n, nexc);
         size_t c0 = 0;
         while (c0 < g.second.size()) {
             std::vector<int> ids;
@@ -3192,14 +3212,13 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
             }
             const int ns = (int)ids.size();
             std::vector<HostCell> sub;
+            std::vector<CellDev> head;
             std::vector<int2> hs(ns);
-            std::vector<CellDev> hc(ns);
-            std::vector<int> hinfo(ns, 0);
             for (int k = 0; k < ns; ++k) {
                 const auto& sp = stacks[ids[k]];
                 const double* e = exc + 4 * (size_t)ids[k];
                 hs[k] = make_int2(sp.second, (int)sub.size());
-                hc[k] = make_cell(layers[sp.first], ids[k], e[0], e[1], e[2], e[3], nexc).d;
+                head.push_back(make_cell(layers[sp.first], ids[k], e[0], e[1], e[2], e[3], nexc).d);
                 for (int l = 0; l < sp.second; ++l)
                     sub.push_back(make_cell(layers[sp.first + l], (int)sub.size(), 1.0, 0.0, 0.0, 0.0, 2));
             }
@@ -3207,19 +3226,28 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
             // buckets by raster: (ng, cells)
             std::map<int, std::vector<int>> by_ng;
             for (int i = 0; i < nslot; ++i) by_ng[sub[i].ng].push_back(i);
+            // one block up (descriptors), one block down (results, status words), the rest
+            size_t up_bytes = a256(ns * sizeof(CellDev)) + a256(ns * sizeof(int2));
+            size_t down_bytes = a256(ns * nexc * sizeof(celeris_rcwa_result)) + a256(ns * sizeof(int));
+            if (ord_out) down_bytes += a256((size_t)ns * nexc * N * 2 * sizeof(double));
             size_t fixed = 3 * a256(s_nn * nslot * c16) + a256(s_w * ns * c16) + a256(10 * s_n * ns * c16) +
-                           a256(ns * sizeof(int)) + a256(nslot * sizeof(int)) + a256(ns * sizeof(CellDev)) +
-                           a256(ns * sizeof(int2)) +
-                           a256(ns * nexc * sizeof(celeris_rcwa_result));
-            if (ord_out) fixed += a256((size_t)ns * nexc * N * 2 * sizeof(double));
+                           a256(nslot * sizeof(int));
             for (auto& kv : by_ng) {
                 const size_t nc = kv.second.size(), ng = (size_t)std::max(kv.first, 0);
-                fixed += a256(nc * sizeof(CellDev)) + 2 * a256(s_nn * nc * c16) + a256(s_w * nc * c16) +
-                         3 * a256(s_NN * nc * c16) + a256(s_n * nc * sizeof(int)) + 2 * a256(nc * sizeof(int));
+                up_bytes += a256(nc * sizeof(CellDev)) + a256(nc * sizeof(int));
+                down_bytes += a256(nc * sizeof(int));
+                fixed += 2 * a256(s_nn * nc * c16) + a256(s_w * nc * c16) + 3 * a256(s_NN * nc * c16) +
+                         a256(s_n * nc * sizeof(int));
                 if (ng > 0) fixed += a256((4 * Mx + 1) * ng * c16) + a256((4 * My + 1) * ng * c16);
             }
-            CEL_TRY(ws.reserve(st, fixed));
-            Bump mem{static_cast<char*>(ws.take(fixed)), fixed};
+            CEL_TRY(ws.reserve(st, up_bytes + down_bytes + fixed));
+            char* region = static_cast<char*>(ws.take(up_bytes + down_bytes + fixed));
+            char* pin = static_cast<char*>(celeris_rt::pinned_staging(up_bytes + down_bytes));
+            if (!pin) return set_error(CELERIS_ERR_OOM, "pinned staging of %zu bytes failed", up_bytes + down_bytes);
+            Bump up{region, up_bytes}, down{region + up_bytes, down_bytes};
+            Bump mem{region + up_bytes + down_bytes, fixed};
+            // the host copy of a pointer into the up or down block
+            auto host = [&](const void* d) { return pin + (static_cast<const char*>(d) - region); };
             StackPort sp;
             std::memset(&sp, 0, sizeof(sp));
             sp.Mx = Mx;
@@ -3234,26 +3262,22 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
             CEL_TRY(mem.get(&sp.lK, s_nn * nslot));
             CEL_TRY(mem.get(&sp.work, s_w * ns));
             CEL_TRY(mem.get(&sp.vec, 10 * s_n * ns));
-            CEL_TRY(mem.get(&sp.info, (size_t)ns));
+            CEL_TRY(down.get(&sp.info, (size_t)ns));
             int* lrest;
             CEL_TRY(mem.get(&lrest, (size_t)nslot));
             sp.lrest = lrest;
             CellDev* scells;
             int2* sstacks;
             celeris_rcwa_result* dres;
-            CEL_TRY(mem.get(&scells, (size_t)ns));
-            CEL_TRY(mem.get(&sstacks, (size_t)ns));
-            CEL_TRY(mem.get(&dres, (size_t)ns * nexc));
+            CEL_TRY(up.get(&scells, (size_t)ns));
+            CEL_TRY(up.get(&sstacks, (size_t)ns));
+            CEL_TRY(down.get(&dres, (size_t)ns * nexc));
             sp.cells = scells;
             sp.stacks = sstacks;
-            CEL_CUDA(cudaMemcpyAsync(scells, hc.data(), sizeof(CellDev) * ns, cudaMemcpyHostToDevice, st));
-            CEL_CUDA(cudaMemcpyAsync(sstacks, hs.data(), sizeof(int2) * ns, cudaMemcpyHostToDevice, st));
-            CEL_CUDA(cudaMemsetAsync(sp.info, 0, sizeof(int) * ns, st));
-            CEL_CUDA(cudaMemsetAsync(lrest, 0, sizeof(int) * nslot, st));
-            // the layers, one bucket per raster class
-            std::vector<std::vector<CellDev>> hd;
-            std::vector<std::vector<int>> hlinfo;
-            std::vector<int*> dlinfo;
+            std::memcpy(host(scells), head.data(), sizeof(CellDev) * ns);
+            std::memcpy(host(sstacks), hs.data(), sizeof(int2) * ns);
+            // the layers' buckets, one per raster class
+            std::vector<Bucket> buckets;
             for (auto& kv : by_ng) {
                 const int ng = kv.first, nc = (int)kv.second.size();
                 if (ng > 0 && laurent_smem(Mx, My, ng) + 1024 > (size_t)smem_optin)
@@ -3277,7 +3301,7 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
                 b.lrest = lrest;
                 CellDev* dcells;
                 int* dslot;
-                CEL_TRY(mem.get(&dcells, (size_t)nc));
+                CEL_TRY(up.get(&dcells, (size_t)nc));
                 CEL_TRY(mem.get(&b.H, s_nn * nc));
                 CEL_TRY(mem.get(&b.Kp, s_nn * nc));
                 CEL_TRY(mem.get(&b.slab, s_w * nc));
@@ -3285,8 +3309,8 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
                 CEL_TRY(mem.get(&b.Exx, s_NN * nc));
                 CEL_TRY(mem.get(&b.Eyy, s_NN * nc));
                 CEL_TRY(mem.get(&b.piv, s_n * nc));
-                CEL_TRY(mem.get(&b.info, (size_t)nc));
-                CEL_TRY(mem.get(&dslot, (size_t)nc));
+                CEL_TRY(down.get(&b.info, (size_t)nc));
+                CEL_TRY(up.get(&dslot, (size_t)nc));
                 if (ng > 0) {
                     cplx *phx, *phy;
                     CEL_TRY(mem.get(&phx, (size_t)(4 * Mx + 1) * ng));
@@ -3296,18 +3320,19 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
                 }
                 b.cells = dcells;
                 b.lslot = dslot;
-                hd.emplace_back(nc);
-                for (int i = 0; i < nc; ++i) hd.back()[i] = sub[kv.second[i]].d;
-                CEL_CUDA(cudaMemcpyAsync(dcells, hd.back().data(), sizeof(CellDev) * nc, cudaMemcpyHostToDevice, st));
-                CEL_CUDA(cudaMemcpyAsync(dslot, kv.second.data(), sizeof(int) * nc, cudaMemcpyHostToDevice, st));
+                CellDev* hd = reinterpret_cast<CellDev*>(host(dcells));
+                for (int i = 0; i < nc; ++i) hd[i] = sub[kv.second[i]].d;
+                std::memcpy(host(dslot), kv.second.data(), sizeof(int) * nc);
                 SmemNeeds needs;
                 needs.add(Mx, My, ng, n, 0, 0);
                 CEL_TRY(set_smem_limits(needs));
-                launch_bucket(b, uniform_cfg(256), st, nullptr, false);
-                CEL_CUDA(cudaGetLastError());
-                dlinfo.push_back(b.info);
-                hlinfo.emplace_back(nc);
+                buckets.push_back(b);
             }
+            CEL_CUDA(cudaMemcpyAsync(region, pin, up_bytes, cudaMemcpyHostToDevice, st));
+            CEL_CUDA(cudaMemsetAsync(region + up_bytes, 0, down_bytes, st));  // status words, results
+            CEL_CUDA(cudaMemsetAsync(lrest, 0, sizeof(int) * nslot, st));
+            for (const Bucket& b : buckets) launch_bucket(b, uniform_cfg(256), st, nullptr, false);
+            CEL_CUDA(cudaGetLastError());
             CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_stack_port), slab::shared_bytes(n)));
             rcwa_stack_port<<<ns, 512, slab::shared_bytes(n), st>>>(sp);
             Bucket eb;
@@ -3323,29 +3348,21 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
             eb.res = dres;
             eb.s_n = s_n;
             eb.s_nn = s_nn;
-            if (ord_out) CEL_TRY(mem.get(&eb.ord, (size_t)ns * nexc * N * 2));
+            if (ord_out) CEL_TRY(down.get(&eb.ord, (size_t)ns * nexc * N * 2));
             rcwa_epilogue<<<ns, kRT, 0, st>>>(eb);
             count_launch(2);
             CEL_CUDA(cudaGetLastError());
-            std::vector<celeris_rcwa_result> hres((size_t)ns * nexc);
-            CEL_CUDA(cudaMemcpyAsync(hres.data(), dres, sizeof(celeris_rcwa_result) * ns * nexc,
-                                     cudaMemcpyDeviceToHost, st));
-            CEL_CUDA(cudaMemcpyAsync(hinfo.data(), sp.info, sizeof(int) * ns, cudaMemcpyDeviceToHost, st));
-            for (size_t k = 0; k < dlinfo.size(); ++k)
-                CEL_CUDA(cudaMemcpyAsync(hlinfo[k].data(), dlinfo[k], sizeof(int) * hlinfo[k].size(),
-                                         cudaMemcpyDeviceToHost, st));
-            std::vector<double> hord;
-            if (ord_out) {
-                hord.resize((size_t)ns * nexc * N * 2);
-                CEL_CUDA(cudaMemcpyAsync(hord.data(), eb.ord, sizeof(double) * hord.size(), cudaMemcpyDeviceToHost,
-                                         st));
-            }
+            CEL_CUDA(cudaMemcpyAsync(pin + up_bytes, region + up_bytes, down_bytes, cudaMemcpyDeviceToHost, st));
             CEL_CUDA(cudaStreamSynchronize(st));
+            const auto* hres = reinterpret_cast<const celeris_rcwa_result*>(host(dres));
+            const int* hinfo = reinterpret_cast<const int*>(host(sp.info));
+            const double* hord = ord_out ? reinterpret_cast<const double*>(host(eb.ord)) : nullptr;
             // a flagged layer flags its stack (its part of the layer store was not written)
             std::vector<char> bad(nslot, 0);
             size_t k = 0;
             for (auto& kv : by_ng) {
-                for (size_t i = 0; i < kv.second.size(); ++i) bad[kv.second[i]] = hlinfo[k][i] != 0;
+                const int* li = reinterpret_cast<const int*>(host(buckets[k].info));
+                for (size_t i = 0; i < kv.second.size(); ++i) bad[kv.second[i]] = li[i] != 0;
                 ++k;
             }
             for (int i = 0; i < ns; ++i) {
@@ -3356,7 +3373,7 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
                 if (f != 0) continue;
                 for (int e = 0; e < nexc; ++e) out[(size_t)ids[i] * nexc + e] = hres[(size_t)i * nexc + e];
                 if (ord_out)
-                    std::memcpy(ord_out + (size_t)ids[i] * nexc * N * 2, hord.data() + (size_t)i * nexc * N * 2,
+                    std::memcpy(ord_out + (size_t)ids[i] * nexc * N * 2, hord + (size_t)i * nexc * N * 2,
                                 sizeof(double) * nexc * N * 2);
             }
         }
