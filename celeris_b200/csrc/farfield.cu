@@ -498,6 +498,9 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     return d;
 }
 
+// The sign bits on the integer pipe, which these kernels leave idle.
+__device__ __forceinline__ f32x2 neg2(f32x2 a) { return a ^ 0x8000000080000000ull; }
+
 // Knuth TwoSum: s + c += x with the rounding error of s + x kept in c.
 __device__ __forceinline__ void two_sum_acc(float& s, float& c, float x) {
     const float t = s + x;
@@ -507,6 +510,10 @@ __device__ __forceinline__ void two_sum_acc(float& s, float& c, float x) {
     s = t;
 }
 
+// The SFU (three approximations a term) bounds the kernel. Eight pillars per loop round:
+// their records' loads and the SFU results of one overlap the arithmetic of the next
+// (785,456 pillars x 512^2: 150.0 ms at two per round, 145.3 ms, 1.42e12 terms/s, here;
+// 70,688 x 161^2: 1.40 -> 1.355 ms). The order of the sums is the same.
 template <bool ZLO>
 __global__ void __launch_bounds__(kThreads, 3) rs_f32c_kernel(const float4* __restrict__ rec,
                                                            int npil, int chunk_len, Geom g,
@@ -574,7 +581,7 @@ __global__ void __launch_bounds__(kThreads, 3) rs_f32c_kernel(const float4* __re
             f32x2 er[kPairs], ei[kPairs];
 #pragma unroll
             for (int h = 0; h < kPairs; ++h) er[h] = ei[h] = 0ull;
-#pragma unroll 2
+#pragma unroll 8
             for (int p = 0; p < cnt; ++p) {
                 const float4 r = tile[p];  // {x, y, |t|, arg t / 2pi}
                 // s0 = base - x, sy = fy - y (grid values: only bits of x, y
@@ -632,7 +639,9 @@ __global__ void __launch_bounds__(kThreads, 3) rs_f32c_kernel(const float4* __re
 // ---- precision-form adjoint: out_j = e^{-ikz} sum_p (1/R) e^{-2 pi i (R - z)/lambda} v_p
 // The forward kernel's arithmetic with the roles swapped: each thread owns
 // kAdjPPT32 pillars (packed pairs), pixel records stream through the tiles; the
-// product with v is conj(g) v = (1/R) [(c vr + s vi) + i (c vi - s vr)].
+// product with v is conj(g) v = (1/R) [(c vr + s vi) + i (c vi - s vr)]. The FP32 pipe
+// bounds it (25 packed operations a pair against the SFU's time of 24): signs are turned
+// on the integer pipe (70,688 pillars x 161^2: 1.77 -> 1.67 ms, the same values).
 __global__ void __launch_bounds__(kThreads, 3) rs_adj_f32c_kernel(const float4* __restrict__ pix, int npix,
                                                                   int chunk_len, const double* __restrict__ px,
                                                                   const double* __restrict__ py, int npil, Geom g,
@@ -649,7 +658,7 @@ __global__ void __launch_bounds__(kThreads, 3) rs_adj_f32c_kernel(const float4* 
         xj[h] = pk2((float)(px[a] - g.ox), (float)(px[b] - g.ox));
         yj[h] = pk2((float)(py[a] - g.oy), (float)(py[b] - g.oy));
     }
-    const f32x2 NEG1 = dup2(-1.0f), NZ = dup2(-z), Z2X = dup2(2.0f * z), NHALF = dup2(-0.5f);
+    const f32x2 NZ = dup2(-z), Z2X = dup2(2.0f * z), NHALF = dup2(-0.5f);
     const f32x2 Z2 = dup2(z * z), ILHI = dup2(il_hi), NILHI = dup2(-il_hi), ILLO = dup2(il_lo);
     const f32x2 MAGIC = dup2(12582912.0f);
     const f32x2 TWOPI = dup2(6.28318530717958647692f);
@@ -670,16 +679,15 @@ __global__ void __launch_bounds__(kThreads, 3) rs_adj_f32c_kernel(const float4* 
             f32x2 er[kPairs], ei[kPairs];
 #pragma unroll
             for (int h = 0; h < kPairs; ++h) er[h] = ei[h] = 0ull;
-#pragma unroll 2
+#pragma unroll 8
             for (int p = 0; p < cnt; ++p) {
                 const float4 r = tile[p];  // {fx, fy, Re v, Im v}
                 const f32x2 FX = dup2(r.x), FY = dup2(r.y), VR = dup2(r.z), VI = dup2(r.w), NVR = dup2(-r.z);
 #pragma unroll
                 for (int h = 0; h < kPairs; ++h) {
-                    const f32x2 dx = fma2(xj[h], NEG1, FX), ndx = fma2(FX, NEG1, xj[h]);
-                    const f32x2 dy = fma2(yj[h], NEG1, FY), ndy = fma2(FY, NEG1, yj[h]);
+                    const f32x2 dx = sub2(FX, xj[h]), dy = sub2(FY, yj[h]);
                     const f32x2 u = fma2(dx, dx, fma2(dy, dy, Z2));         // R^2 (seed only)
-                    const f32x2 ns = fma2(dx, ndx, mul2(dy, ndy));          // -rho^2
+                    const f32x2 ns = neg2(fma2(dx, dx, mul2(dy, dy)));      // -rho^2
                     float ua, ub;
                     upk2(u, ua, ub);
                     const f32x2 ri = pk2(rsqrt_approx(ua), rsqrt_approx(ub));  // ~1/R
@@ -690,8 +698,8 @@ __global__ void __launch_bounds__(kThreads, 3) rs_adj_f32c_kernel(const float4* 
                     const f32x2 np = mul2(d, NILHI);
                     const f32x2 rp = fma2(d, ILHI, np);
                     const f32x2 t = fma2(d, ILLO, rp);
-                    const f32x2 w = fma2(add2(np, MAGIC), NEG1, MAGIC);
-                    const f32x2 ang = mul2(fma2(add2(np, w), NEG1, t), TWOPI);
+                    const f32x2 w = sub2(MAGIC, add2(np, MAGIC));
+                    const f32x2 ang = mul2(sub2(t, add2(np, w)), TWOPI);
                     float aa, ab;
                     upk2(ang, aa, ab);
                     const f32x2 pr = mul2(ri, pk2(cos_approx(aa), cos_approx(ab)));
