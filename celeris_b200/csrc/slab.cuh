@@ -39,18 +39,22 @@ namespace slab {
 
 constexpr int kMaxOrder = 512;        // largest order of the routines here
 constexpr int kNB = 16;               // Gauss-Jordan panel width
-constexpr int kGs = 20;               // row stride of the staged panel (4 mod 16: fragment reads do not conflict)
+// Row stride of the staged panel: 64 bytes mod 128, so that the fragment reads (16 bytes a
+// lane, two rows per quarter-warp) do not conflict.
+constexpr int kGs = 20, kGsReal = 24;
 constexpr double kSpectral = 2.2;     // largest spectral radius of Q y of the series
 constexpr double kPhaseMax = 2.5;     // largest q x of a propagating mode at S^-1 (sin q x = 0 at pi)
 constexpr int kMaxAngles = 2;         // double-angle steps
 constexpr int kMaxDoublings = 40;
 // Largest max |X| of the doubling that leaves r more (r >= 0): beyond it the doublings
-// stop (r + 1 <= kMaxRest), or the layer is given up. 64 keeps the error at the level of
-// the eigendecomposition's (1e-14 to 1e-13 against long double); a stop further from the
-// end costs more, so it waits for a larger loss.
+// stop (r + 1 <= kMaxRest), or the layer is given up. At 1000 a cell's error against long
+// double stays at the eigendecomposition's level (1e-14 to 1e-13 of its fields); every stop
+// costs complex solves that hold up the whole batch (96 oblique cells, one stop among
+// them: 7.0 ms instead of 5.2), so a lower limit is not worth the digits, and a stop further
+// from the end waits for a larger loss.
 constexpr int kMaxRest = 3;
 __device__ __forceinline__ double growth_limit(int rest) {
-    return rest == 0 ? 64.0 : 3e3;
+    return rest == 0 ? 1e3 : 3e3;
 }
 
 // ---- scalars: double or complex ---------------------------------------------------------
@@ -409,6 +413,10 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 // finished panel G goes to s.pan (over the column buffers): the update of every other
 // column is row <- row + G (old pivot rows), with the pivot rows themselves replaced
 // (trailing()).
+template <class T>
+__host__ __device__ constexpr int panel_stride() {
+    return sizeof(T) == sizeof(double) ? kGsReal : kGs;
+}
 constexpr unsigned kFlagPolls = 1u << 22;  // bound of a wait for a column
 __device__ __forceinline__ int wait_column(const int* flag) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(flag);
@@ -537,7 +545,7 @@ __device__ __noinline__ void panel(int n, int k0, int kb, const T* Wm, int ld, c
 #pragma unroll
         for (int r = 0; r < RA; ++r) {
             const int row = lane + 32 * r;
-            if (row < n) pan[row * kGs + warp + PW * q] = a[q][r];  // zero in the columns past kb
+            if (row < n) pan[row * panel_stride<T>() + warp + PW * q] = a[q][r];  // zero in the columns past kb
         }
 }
 
@@ -585,6 +593,82 @@ __device__ __forceinline__ void trailing_units(int n, int c0, int cn, T* Wm, int
         }
     }
 }
+// The same in real arithmetic with 16-byte accesses throughout (36 instead of 16 shared and
+// global accesses per 16 tensor instructions otherwise; 64 cells M = 3: 0.345 -> 0.333 ms a
+// call): units of 8 R x 32, two k of G and two columns of the pivot rows
+// and of Wm per access, as in gemm_units_real. c0 and ld are even.
+template <int R>
+__device__ __forceinline__ void trailing_units_real(int n, int c0, int cn, double* Wm, int ld, const Shared& s, int k0,
+                                                    int ldp) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const double* pan = as<double>(s.pan) + 2 * t4;
+    const double* pr = as<double>(s.prow);
+    const int rt = (n + 8 * R - 1) / (8 * R), units = rt * ((cn + 31) >> 5);
+    for (int u = warp; u < units; u += nwarp) {
+        const int i0 = (u % rt) * (8 * R), j0 = (u / rt) * 32;
+        Acc<false> acc[R][4];
+        double* wrow[R];
+        const double* grow[R];
+        bool live[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int row = i0 + 8 * r + g, rowc = min(row, n - 1);
+            live[r] = row < n;
+            const bool keep = live[r] && s.pos[rowc] < k0;  // pos >= k0: a pivot row of this panel
+            wrow[r] = Wm + (size_t)rowc * ld + c0 + j0 + 4 * t4;
+            grow[r] = pan + rowc * kGsReal;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {  // columns j0 + 16 q + 4 t4 .. + 3: tiles 2 q, 2 q + 1
+                const int c = j0 + 16 * q + 4 * t4;
+                double2 lo = make_double2(0.0, 0.0), hi = lo;
+                if (keep && c < cn) lo = *reinterpret_cast<const double2*>(wrow[r] + 16 * q);
+                if (keep && c + 2 < cn) hi = *reinterpret_cast<const double2*>(wrow[r] + 16 * q + 2);
+                acc[r][2 * q].r[0] = lo.x;
+                acc[r][2 * q + 1].r[0] = lo.y;
+                acc[r][2 * q].r[1] = hi.x;
+                acc[r][2 * q + 1].r[1] = hi.y;
+            }
+        }
+#pragma unroll
+        for (int ks = 0; ks < kNB; ks += 8) {
+            double2 av[R], bv[2][2];
+#pragma unroll
+            for (int r = 0; r < R; ++r) av[r] = *reinterpret_cast<const double2*>(grow[r] + ks);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    bv[h][q] = *reinterpret_cast<const double2*>(pr + (ks + 2 * t4 + h) * ldp + j0 + 16 * q + 2 * g);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const double a = h == 0 ? av[r].x : av[r].y;
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        mma(acc[r][2 * q], a, bv[h][q].x);
+                        mma(acc[r][2 * q + 1], a, bv[h][q].y);
+                    }
+                }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (!live[r]) continue;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int c = j0 + 16 * q + 4 * t4;
+                if (c < cn)
+                    *reinterpret_cast<double2*>(wrow[r] + 16 * q) =
+                        make_double2(acc[r][2 * q].r[0], acc[r][2 * q + 1].r[0]);
+                if (c + 2 < cn)
+                    *reinterpret_cast<double2*>(wrow[r] + 16 * q + 2) =
+                        make_double2(acc[r][2 * q].r[1], acc[r][2 * q + 1].r[1]);
+            }
+        }
+    }
+}
+
 template <class T>
 __device__ void trailing(int n, int c0, int c1, T* Wm, int ld, const Shared& s, int k0, int kb) {
     constexpr bool CP = sizeof(T) == sizeof(cplx);
@@ -592,12 +676,18 @@ __device__ void trailing(int n, int c0, int c1, T* Wm, int ld, const Shared& s, 
     const int cmax = CP ? s.chunk : 2 * s.chunk;  // staged columns
     for (int c = c0; c < c1; c += cmax) {
         const int cn = min(cmax, c1 - c);
-        const int ldp = cmax + (CP ? 2 : 4);  // fragment reads of the staged rows do not conflict
+        const int ldp = cmax + 2;  // fragment reads of the staged rows do not conflict
         for (int e = threadIdx.x; e < kNB * cn; e += blockDim.x) {
             const int l = e / cn, j = e - l * cn;
             pr[l * ldp + j] = l < kb ? Wm[(size_t)s.perm[k0 + l] * ld + c + j] : zero_of(T());
         }
         __syncthreads();
+        if constexpr (!CP) {
+            if (unit_cost(n, cn, 2, 4) < unit_cost(n, cn, 1, 4)) trailing_units_real<2>(n, c, cn, Wm, ld, s, k0, ldp);
+            else trailing_units_real<1>(n, c, cn, Wm, ld, s, k0, ldp);
+            __syncthreads();
+            continue;
+        }
         const int w = unit_width((n + 7) >> 3, (cn + 7) >> 3);
         if (w == 4) trailing_units<T, 4>(n, c, cn, Wm, ld, s, k0, ldp);
         else if (w == 2) trailing_units<T, 2>(n, c, cn, Wm, ld, s, k0, ldp);
@@ -606,7 +696,8 @@ __device__ void trailing(int n, int c0, int c1, T* Wm, int ld, const Shared& s, 
     }
 }
 
-// Gauss-Jordan on the n x ncol matrix Wm = [A | R] (A its first n columns): afterwards row
+// Gauss-Jordan on the n x ncol matrix Wm = [A | R] (A its first n columns, in real
+// arithmetic R from the next even column, ld even): afterwards row
 // s.perm[k] of the right part holds row k of A^-1 R. inverse: A's part becomes A^-1 in
 // place, its entry (k, perm[l]) stored at (row perm[k], column l). Returns false (in
 // every thread) at a zero or non-finite pivot. Starts and ends on a barrier.
@@ -630,13 +721,13 @@ __device__ bool gauss_jordan(int n, int ncol, T* Wm, int ld, bool inverse, const
         if (*s.bad) return false;
         if (threadIdx.x < kNB) s.flag[threadIdx.x] = 0;  // a barrier follows before the next panel
         const long long t1 = clock64();
-        const int c1 = k0 + kb;
+        const int c1 = sizeof(T) == sizeof(double) ? (k0 + kb + 1) & ~1 : k0 + kb;
         if (inverse) {
             if (k0 > 0) trailing(n, 0, k0, Wm, ld, s, k0, kb);
             const T* pan = as<T>(s.pan);
             for (int e = threadIdx.x; e < n * kb; e += blockDim.x) {
                 const int i = e / kb, j = e - i * kb;
-                Wm[(size_t)i * ld + k0 + j] = pan[i * kGs + j];
+                Wm[(size_t)i * ld + k0 + j] = pan[i * panel_stride<T>() + j];
             }
         }
         if (c1 < ncol) trailing(n, c1, ncol, Wm, ld, s, k0, kb);
