@@ -24,7 +24,8 @@
 //   37 -> 13 ms; 96 oblique cells M = 4 26 -> 7 ms; 64 two-layer stacks M = 3 15.5 -> 3.4 ms
 //
 // The eigendecomposition's sequence remains for what the two-port does not take (needs_qr)
-// or flags (kInfoRedo), and for celeris_eig_general; it runs in the order basis:
+// or flags (kInfoRedo), and for celeris_eig_general; it runs in the order basis, or on the
+// class operators of a mirror-symmetric cell (hess, schur, vec, then rcwa_sym_smat):
 //   rcwa_build_M  M = ep2 kp - kkT using the diagonal Kx, Ky (two N^3 GEMMs)
 //   rcwa_hess     Householder reduction to Hessenberg form H = Q^H M Q (in
 //                 shared memory for n <= 112, blocked compact-WY panels above)
@@ -113,6 +114,9 @@ struct Bucket {
     // per solved class (matrix ncls * cell + class): M and kp in the class basis,
     // and the amplitudes aN | b0 (2 m)
     cplx *cM, *cKp, *cvec;
+    // QR path in the classes: eigen-stage buffers (m^2 each), q and the eigensolve's info
+    cplx *sZ, *sX, *sW, *sA, *sq;
+    int* sinfo;
     // the layer two-port (slab.cuh): work area of a full-order cell (s_w complex), kp
     cplx *slab, *Kp;
     size_t s_w;
@@ -1980,8 +1984,103 @@ __global__ void __launch_bounds__(512, 1) rcwa_stack_port(StackPort sp) {
     if (!ok && tid == 0) sp.info[st] = kInfoRedo;
 }
 
+// QR path of one excited class: the reference's two-interface recursion restricted to the
+// class (rcwa2d.cpp:376-411), from the eigenvectors W and q of its M. With Y of the incident
+// and substrate half-spaces (half_entry) and D = diag(exp(i q h)):
+//   A = kp W,  P = Yi A diag(1/q),  T11 = (W + P)/2,  T12 = (W - P)/2,
+//   [S12 | u] = T11^-1 [-T12 D | a0],  R = diag(q) (Ys A)^-1 W,
+//   (I + R - D S12 + D S12 R) y = 2 D u,  aN = W y,
+//   y2 = (y - R y)/2,  b0 = T12 (u + S12 y2) + T11 D y2.
+// A class matrix costs 1/64 of the order basis, which is what a thick or thin layer that
+// the two-port does not take would otherwise pay (64 cells, thin or beyond 100 rad: M = 3 9.4 -> 0.75 ms,
+// M = 5 48 -> 4.8 ms a call). A zero pivot sends the cell to
+// the order basis (kInfoAsym).
+__global__ void __launch_bounds__(512, 1) rcwa_sym_smat(Bucket b) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int skip;
+    const int mi = blockIdx.x, cell = mi / b.ncls, cc = mi - cell * b.ncls, c = b.cls0 + cc, n = b.m;
+    const int tid = threadIdx.x, nt = blockDim.x, Mx = b.Mx, My = b.My;
+    if (tid == 0) skip = b.info[cell] != 0 || b.sinfo[mi] != 0;
+    __syncthreads();
+    if (skip) return;
+    const CellDev cd = b.cells[cell];
+    const size_t nn = (size_t)n * n;
+    const cplx *W = b.sW + nn * mi, *Kp = b.cKp + nn * mi, *q = b.sq + (size_t)mi * n;
+    const slab::Shared s = slab::carve(smem, n);
+    const slab::Work w = slab::carve_work(at(cc ? b.X : b.Z, b.s_nn, cell), n);
+    const int n2 = 2 * n, lq = n2 + 1, lc = n + 1;
+    cplx *A = w.w0, *T12 = w.w1, *Cm = w.w2, *G = w.p;
+    cplx* S = w.q;  // [T11 | -T12 D | a0], n x lq: w.q and the start of w.e[0] behind it
+    cplx *T11 = w.e[1], *S12 = w.e[2], *R = w.w0;
+    slab::gemm(n, n, n, Kp, n, W, n, nullptr, [=](int r, int j, cplx v) { A[(size_t)r * n + j] = v; });
+    HalfTable t = half_table(Mx, My, cd, cd.n_inc, c, n, s);
+    for (int e = tid; e < n * n; e += nt) {
+        const int r = e / n, j = e - r * n;
+        const cplx pv = cmul(t.times(A, n, r, j), cinv(q[j])), wv = W[e];
+        const cplx t11 = cscale(cadd(wv, pv), 0.5), t12 = cscale(csub(wv, pv), 0.5);
+        T11[e] = t11;
+        T12[e] = t12;
+        S[(size_t)r * lq + j] = t11;
+        S[(size_t)r * lq + n + j] = cneg(cmul(t12, cexpi(cscale(q[j], cd.h))));
+    }
+    for (int r = tid; r < n; r += nt) S[(size_t)r * lq + n2] = C(excitation(Mx, My, c, r, 0), 0.0);
+    t = half_table(Mx, My, cd, cd.n_sub, c, n, s);
+    for (int e = tid; e < n * n; e += nt) {
+        const int r = e / n, j = e - r * n;
+        G[(size_t)r * n2 + j] = t.times(A, n, r, j);
+        G[(size_t)r * n2 + n + j] = W[e];
+    }
+    bool ok = slab::gauss_jordan(n, lq, S, lq, false, s);
+    cplx *y = w.v, *v1 = y + n2, *v2 = v1 + n2, *v3 = v2 + n2;
+    if (ok) {
+        for (int e = tid; e < n * n; e += nt) S12[e] = S[(size_t)s.perm[e / n] * lq + n + e % n];
+        for (int r = tid; r < n; r += nt) v3[2 * r] = S[(size_t)s.perm[r] * lq + n2];  // u
+        ok = slab::gauss_jordan(n, n2, G, n2, false, s);
+    }
+    if (ok) {
+        for (int e = tid; e < n * n; e += nt) R[e] = cmul(q[e / n], G[(size_t)s.perm[e / n] * n2 + n + e % n]);
+        __syncthreads();
+        slab::gemm(n, n, n, (const cplx*)S12, n, (const cplx*)R, n, nullptr, [=](int r, int j, cplx v) {
+            const size_t e = (size_t)r * n + j;
+            const cplx x = cadd(R[e], cmul(cexpi(cscale(q[r], cd.h)), csub(v, S12[e])));
+            Cm[(size_t)r * lc + j] = r == j ? C(x.x + 1.0, x.y) : x;
+        });
+        for (int r = tid; r < n; r += nt)
+            Cm[(size_t)r * lc + n] = cscale(cmul(cexpi(cscale(q[r], cd.h)), v3[2 * r]), 2.0);
+        ok = slab::gauss_jordan(n, lc, Cm, lc, false, s);
+    }
+    if (!ok) {
+        if (tid == 0) atomicCAS(&b.info[cell], 0, kInfoAsym);
+        return;
+    }
+    for (int r = tid; r < n; r += nt) y[2 * r] = Cm[(size_t)s.perm[r] * lc + n];
+    __syncthreads();
+    cplx *aN = b.cvec + (size_t)mi * 2 * n, *b0 = aN + n;
+    auto same = [](int r) { return r; };
+    matvec_rows2(n, 1, W, n, same, y, v1);
+    matvec_rows2(n, 1, R, n, same, y, v2);
+    __syncthreads();
+    for (int r = tid; r < n; r += nt) {
+        aN[r] = v1[2 * r];
+        v2[2 * r] = cscale(csub(y[2 * r], v2[2 * r]), 0.5);  // y2
+    }
+    __syncthreads();
+    matvec_rows2(n, 1, S12, n, same, v2, v1);
+    __syncthreads();
+    for (int r = tid; r < n; r += nt) {
+        y[2 * r] = cadd(v3[2 * r], v1[2 * r]);                              // u + S12 y2
+        v2[2 * r] = cmul(cexpi(cscale(q[r], cd.h)), v2[2 * r]);             // D y2
+    }
+    __syncthreads();
+    matvec_rows2(n, 1, T12, n, same, y, v1);
+    matvec_rows2(n, 1, T11, n, same, v2, v3);
+    __syncthreads();
+    for (int r = tid; r < n; r += nt) b0[r] = cadd(v1[2 * r], v3[2 * r]);
+}
+
 // aN and b0 of both excitations into the full basis (the vector area the
-// epilogue reads: aN_X, aN_Y, b0_X, b0_Y).
+// epilogue reads: aN_X, aN_Y, b0_X, b0_Y). QR path: a class eigensolve's failure becomes
+// the cell's info.
 __global__ void __launch_bounds__(kRT) rcwa_sym_expand(Bucket b) {
     const int cell = blockIdx.x;
     const int N = b.N, n = b.n, Mx = b.Mx, My = b.My, m = b.m, ny = 2 * My + 1;
@@ -2018,6 +2117,31 @@ __global__ void __launch_bounds__(kRT) rcwa_sym_expand(Bucket b) {
             vec[3 * b.s_n + rk] = cscale(vec[2 * b.s_n + k], sg);
         }
     }
+    if (b.sinfo && tid == 0 && b.info[cell] != kInfoAsym)
+        for (int cc = 0; cc < b.ncls && b.info[cell] == 0; ++cc) b.info[cell] = b.sinfo[b.ncls * cell + cc];
+}
+
+// The eigen stages' bucket of a mirror-symmetric bucket's class matrices.
+Bucket sym_eig_bucket(const Bucket& b) {
+    Bucket e;
+    std::memset(&e, 0, sizeof(e));
+    e.Mx = b.Mx;
+    e.My = b.My;
+    e.n = b.m;
+    e.N = b.m / 2;
+    e.ncell = b.ncls * b.ncell;
+    e.cells = b.cells;
+    e.H = b.cM;
+    e.Z = b.sZ;
+    e.X = b.sX;
+    e.W = b.sW;
+    e.A = b.sA;
+    e.q1 = b.sq;
+    e.info = b.sinfo;
+    e.dbg = b.dbg;
+    e.s_nn = (size_t)e.n * e.n;
+    e.s_n = (size_t)e.n;
+    return e;
 }
 
 // ---- host side ------------------------------------------------------------------------------------
@@ -2125,7 +2249,6 @@ HostCell make_cell(const celeris_rcwa_cell& c, int index, double ex_re, double e
     h.sym = !sym_eligible(c) ? 0
             : (c.period_x_um == c.period_y_um && c.Mx == c.My && c.fill_x == c.fill_y) ? 2 : 1;
     h.qr = needs_qr(c) ? 1 : 0;
-    if (h.qr) h.sym = 0;
     return h;
 }
 
@@ -2233,20 +2356,27 @@ size_t sym_g1_size(int Mx, int My, int ng) {
     const size_t nx = 2 * Mx + 1, ny = 2 * My + 1;
     return std::max(nx * (size_t)ng, nx * nx + ny * ny);
 }
-// Device memory of one mirror-symmetric cell: Z and X of full order (the class build's
-// scratch, then the two-port's work areas), the raster's row transform, the vector
-// area; per solved class M, kp and 2 m amplitudes.
-size_t sym_per_cell_bytes(int Mx, int My, int ng, int nexc, int ncls) {
+// Z and X of one mirror-symmetric cell: the class build's scratch (full order), then a
+// class's work area each, which is the larger one at Mx = My = 1.
+size_t sym_scratch(int Mx, int My) {
+    const size_t n = 2 * (size_t)(2 * Mx + 1) * (2 * My + 1);
+    return std::max(n * n, slab::work_size(sym_class_size(Mx, My, 0)));
+}
+// Device memory of one mirror-symmetric cell: Z and X, the raster's row transform, the
+// vector area; per solved class M, kp and 2 m amplitudes; QR path: the eigen stages'
+// four matrices and q per class.
+size_t sym_per_cell_bytes(int Mx, int My, int ng, int nexc, int ncls, int qr) {
     const size_t n = 2 * (size_t)(2 * Mx + 1) * (2 * My + 1);
     const size_t m = (size_t)sym_class_size(Mx, My, 0);
-    return (2 * n * n + sym_g1_size(Mx, My, ng) + 10 * n + ncls * (2 * m * m + 2 * m)) * sizeof(cplx) + sizeof(int) +
-           sizeof(celeris_rcwa_result) * nexc + sizeof(CellDev) + 16 * 256;
+    return (2 * sym_scratch(Mx, My) + sym_g1_size(Mx, My, ng) + 10 * n +
+            ncls * (2 * m * m + 2 * m + (qr ? 4 * m * m + m : 0))) * sizeof(cplx) + (1 + ncls) * sizeof(int) +
+           sizeof(celeris_rcwa_result) * nexc + sizeof(CellDev) + 24 * 256;
 }
 
 // The largest dynamic shared memory each stage kernel needs over a wave's
 // buckets; raised once per wave, outside any capture.
 struct SmemNeeds {
-    size_t laurent = 0, rect = 0, hess_s = 0, hess_g = 0, smat = 0, slab = 0, ops = 0;
+    size_t laurent = 0, rect = 0, hess_s = 0, hess_g = 0, smat = 0, slab = 0, ops = 0, sym_smat = 0;
     bool aed = false;
     void add_eig(int n) {
         if (n <= kSmemEigMaxN) hess_s = std::max(hess_s, ((size_t)n * n + 2 * n) * sizeof(cplx));
@@ -2256,6 +2386,7 @@ struct SmemNeeds {
     void add(int Mx, int My, int ng, int n, int sym = 0, int qr = 1) {
         if (sym) {
             ops = std::max(ops, sym_ops_smem(Mx, My, ng));
+            if (qr) sym_smat = std::max(sym_smat, slab::shared_bytes(sym_class_size(Mx, My, 0)));
         } else if (ng > 0) {
             laurent = std::max(laurent, laurent_smem(Mx, My, ng));
         } else {
@@ -2265,8 +2396,8 @@ struct SmemNeeds {
         if (!qr) {
             slab = std::max(slab, slab_smem(sym ? sym_class_size(Mx, My, 0) : n, 512));
         } else {
-            add_eig(n);
-            smat = std::max(smat, lu_stage_bytes(n));
+            add_eig(sym ? sym_class_size(Mx, My, 0) : n);
+            if (!sym) smat = std::max(smat, lu_stage_bytes(n));
         }
     }
 };
@@ -2304,6 +2435,7 @@ int set_smem_limits(const SmemNeeds& s) {
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_smat1), s.smat));
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_smat2), s.smat));
     }
+    if (s.sym_smat) CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_sym_smat), s.sym_smat));
     if (s.ops) {
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_sym_ops<256>), s.ops));
         CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_sym_ops<512>), s.ops));
@@ -2318,7 +2450,7 @@ int set_smem_limits(const SmemNeeds& s) {
 // Launch the stage sequence of one bucket on `st`. ev (ST_COUNT + 1 events) is
 // optional: stage boundaries are recorded into it.
 // eig_only: stop after the eigenvectors (the layers of a multi-layer stack).
-// qr: through the eigendecomposition (order basis), else through the layer two-port.
+// qr: through the eigendecomposition, else through the layer two-port.
 void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEvent_t* ev, bool qr,
                    bool eig_only = false) {
     const int nc = b.ncell, n = b.n;
@@ -2345,14 +2477,14 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
         count_launch(1);
     }
     if (ev) cudaEventRecord(ev[1], st);
+    if (b.sym) {  // class operators
+        const size_t sm = sym_ops_smem(b.Mx, b.My, b.ng);
+        if (slab_threads(1, nc) == 512) rcwa_sym_ops<512><<<nc, 512, sm, st>>>(b);
+        else rcwa_sym_ops<256><<<nc, 256, sm, st>>>(b);
+    }
     if (!qr) {
-        // the layer two-port: class operators first for mirror-symmetric cells, then one
-        // kernel (timed as smat1), the amplitudes into the order basis, the outputs
-        if (b.sym) {
-            const size_t sm = sym_ops_smem(b.Mx, b.My, b.ng);
-            if (slab_threads(1, nc) == 512) rcwa_sym_ops<512><<<nc, 512, sm, st>>>(b);
-            else rcwa_sym_ops<256><<<nc, 256, sm, st>>>(b);
-        }
+        // the layer two-port: one kernel (timed as smat1), the amplitudes of
+        // mirror-symmetric cells into the order basis, the outputs
         if (ev)
             for (int i = 2; i <= 5; ++i) cudaEventRecord(ev[i], st);
         const int m = b.sym ? b.m : n, count = b.sym ? b.ncls * nc : nc;
@@ -2368,21 +2500,31 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
         count_launch((b.sym ? 3 : 1) + (b.lA ? 0 : 1));
         return;
     }
-    rcwa_build_M<<<nc, T[ST_BUILD], 0, st>>>(b, b.ng > 0 ? 1 : 0);
+    const Bucket e = b.sym ? sym_eig_bucket(b) : b;
+    if (b.sym) cudaMemsetAsync(e.info, 0, sizeof(int) * e.ncell, st);
+    else rcwa_build_M<<<nc, T[ST_BUILD], 0, st>>>(b, b.ng > 0 ? 1 : 0);
     if (ev) cudaEventRecord(ev[2], st);
-    if (n <= kSmemEigMaxN) {
-        const size_t sm = ((size_t)n * n + 2 * n) * sizeof(cplx);
-        rcwa_hess<true><<<nc, hess_smem_threads(n, T[ST_HESS]), sm, st>>>(b);
-        if (ev) cudaEventRecord(ev[3], st);
-        rcwa_schur<<<nc, kSchurThreads, schur_smem(nc), st>>>(b);
+    if (e.n <= kSmemEigMaxN) {
+        const size_t sm = ((size_t)e.n * e.n + 2 * e.n) * sizeof(cplx);
+        rcwa_hess<true><<<e.ncell, hess_smem_threads(e.n, T[ST_HESS]), sm, st>>>(e);
     } else {
-        rcwa_hess<false><<<nc, T[ST_HESS], hess_stage_bytes(n), st>>>(b);
-        if (ev) cudaEventRecord(ev[3], st);
-        rcwa_schur<<<nc, kSchurThreads, schur_smem(nc), st>>>(b);
+        rcwa_hess<false><<<e.ncell, T[ST_HESS], hess_stage_bytes(e.n), st>>>(e);
     }
+    if (ev) cudaEventRecord(ev[3], st);
+    rcwa_schur<<<e.ncell, kSchurThreads, schur_smem(e.ncell), st>>>(e);
     if (ev) cudaEventRecord(ev[4], st);
-    rcwa_vec<<<nc, T[ST_VEC], 0, st>>>(b);
+    rcwa_vec<<<e.ncell, T[ST_VEC], 0, st>>>(e);
     if (ev) cudaEventRecord(ev[5], st);
+    if (b.sym) {
+        rcwa_sym_smat<<<e.ncell, 512, slab::shared_bytes(e.n), st>>>(b);
+        if (ev) cudaEventRecord(ev[6], st);
+        rcwa_sym_expand<<<nc, T[ST_SMAT2], 0, st>>>(b);
+        if (ev) cudaEventRecord(ev[7], st);
+        rcwa_epilogue<<<nc, T[ST_EPI], 0, st>>>(b);
+        if (ev) cudaEventRecord(ev[8], st);
+        count_launch(7);
+        return;
+    }
     if (eig_only) {
         count_launch(4);
         return;
@@ -2563,9 +2705,9 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             p.n = 2 * p.N;
             if (p.ng > 0 && laurent_smem(p.Mx, p.My, p.ng) + 1024 > (size_t)smem_optin)
                 return set_error(CELERIS_ERR_TOO_LARGE, "raster %d with M=(%d,%d) exceeds shared memory", p.ng, p.Mx, p.My);
-            p.per_cell = p.qr    ? per_cell_bytes(p.n, nexc)
-                         : p.sym ? sym_per_cell_bytes(p.Mx, p.My, p.ng, nexc, p.sym == 2 ? 1 : 2)
-                                 : slab_per_cell_bytes(p.n, nexc);
+            p.per_cell = p.sym  ? sym_per_cell_bytes(p.Mx, p.My, p.ng, nexc, p.sym == 2 ? 1 : 2, p.qr)
+                         : p.qr ? per_cell_bytes(p.n, nexc)
+                                : slab_per_cell_bytes(p.n, nexc);
             // split buckets that alone exceed the budget
             const size_t max_cells = std::max<size_t>(1, budget / std::max<size_t>(1, p.per_cell));
             for (size_t c0 = 0; c0 < kv.second.size(); c0 += max_cells) {
@@ -2664,7 +2806,8 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             CellDev* dcells = static_cast<CellDev*>(ws.take(sizeof(CellDev) * nc));
             b.cells = dcells;
             auto take = [&](size_t count) { return static_cast<cplx*>(ws.take(sizeof(cplx) * count)); };
-            if (p.qr) {
+            if (p.sym) b.s_nn = sym_scratch(p.Mx, p.My);  // Z and X are its only square buffers
+            if (p.qr && !p.sym) {
                 cplx** mats[] = {&b.H, &b.Z, &b.X, &b.W, &b.A, &b.T11, &b.T11lu, &b.T12};
                 for (cplx** m : mats) *m = take(b.s_nn * nc);
                 b.S12 = take(b.s_ns * nc);
@@ -2705,6 +2848,11 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                 b.cM = take(m * m * nm);
                 b.cKp = take(m * m * nm);
                 b.cvec = take(2 * m * nm);
+                if (p.qr) {
+                    for (cplx** x : {&b.sZ, &b.sX, &b.sW, &b.sA}) *x = take(m * m * nm);
+                    b.sq = take(m * nm);
+                    b.sinfo = static_cast<int*>(ws.take(sizeof(int) * nm));
+                }
             }
             hdesc[w] = reinterpret_cast<CellDev*>(pin);
             pin += celeris_rt::align256(sizeof(CellDev) * nc);
@@ -2871,8 +3019,8 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
         std::vector<HostCell> sub;
         for (size_t j = 0; j < redo.size(); ++j) {
             HostCell h = cells[pos[redo[j]]];
-            h.sym = 0;
-            h.qr = h.qr || hinfo[redo[j]] == kInfoRedo || 2 * (2 * h.Mx + 1) * (2 * h.My + 1) > slab::kMaxOrder;
+            if (hinfo[redo[j]] == kInfoAsym) h.sym = 0;
+            h.qr = h.qr || hinfo[redo[j]] == kInfoRedo || (!h.sym && 2 * (2 * h.Mx + 1) * (2 * h.My + 1) > slab::kMaxOrder);
             h.index = (int)j;
             sub.push_back(h);
         }
