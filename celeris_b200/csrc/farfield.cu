@@ -1821,6 +1821,7 @@ int ff_run_noalloc(int form, const double* d_px, const double* d_py, const doubl
     // device (creating the array) and caches the array's device address.
     void* base = nullptr;
     CEL_TRY(noalloc_scratch(&base));
+    CEL_TRY(prepare64());  // kernel attributes too: nothing of the set-up is left to a captured call
     const long npix = (long)g.nx * g.ny;
     if (npix <= 0) return CELERIS_OK;
     if (npix > (1L << 30)) return set_error(CELERIS_ERR_TOO_LARGE, "grid too large (%ld pixels)", npix);
@@ -1845,7 +1846,6 @@ int ff_run_noalloc(int form, const double* d_px, const double* d_py, const doubl
         ctas_pix = (int)((spr * g.ny + kThreads - 1) / kThreads);
         plan_chunks(ctas_pix, npil, kTile32, 3, &nchunk, &chunk_len);
     } else {
-        CEL_TRY(prepare64());
         p64 = plan_field64(g, npil);
         nchunk = p64.nchunk;
         chunk_len = p64.chunk_len;
