@@ -20,8 +20,8 @@
 //   rcwa_epilogue Poynting flux and order-0 field for each requested excitation
 // Stacks run rcwa_slab per layer and rcwa_stack_port (one CTA per stack).
 // Measured (one B200, whole calls, against the eigendecomposition's sequence below):
-//   one M = 5 cell 4.6 -> 0.9 ms; 64 cells M = 3 0.99 -> 0.49 ms; 512 rasterised cells M = 3..7
-//   37 -> 13 ms; 96 oblique cells M = 4 26 -> 7 ms; 64 two-layer stacks M = 3 15.5 -> 3.4 ms
+//   one M = 5 cell 4.7 -> 0.55 ms; 64 cells M = 3 0.98 -> 0.40 ms; 512 rasterised cells M = 3..7
+//   37 -> 10.7 ms; 96 oblique cells M = 4 26 -> 7.2 ms; 64 two-layer stacks M = 3 15.6 -> 3.8 ms
 //
 // The eigendecomposition's sequence remains for what the two-port does not take (needs_qr)
 // or flags (kInfoRedo), and for celeris_eig_general; it runs in the order basis, or on the

@@ -46,16 +46,15 @@ constexpr double kSpectral = 2.2;     // largest spectral radius of Q y of the s
 constexpr double kPhaseMax = 2.5;     // largest q x of a propagating mode at S^-1 (sin q x = 0 at pi)
 constexpr int kMaxAngles = 2;         // double-angle steps
 constexpr int kMaxDoublings = 40;
-// Largest max |X| of the doubling that leaves r more (r >= 0): beyond it the doublings
-// stop (r + 1 <= kMaxRest), or the layer is given up. At 1000 a cell's error against long
-// double stays at the eigendecomposition's level (1e-14 to 1e-13 of its fields); every stop
-// costs complex solves that hold up the whole batch (96 oblique cells, one stop among
-// them: 7.0 ms instead of 5.2), so a lower limit is not worth the digits, and a stop further
-// from the end waits for a larger loss.
-constexpr int kMaxRest = 3;
-__device__ __forceinline__ double growth_limit(int rest) {
-    return rest == 0 ? 1e3 : 3e3;
-}
+// Largest max |X| of a doubling: beyond it the doublings stop where at most kMaxRest are left
+// (1 << kMaxRest slabs), or the layer is given up. The error grows as eps |X|^2. Largest
+// difference from the eigendecomposition over 6000 mirror-symmetric cells M = 1 .. 3 and 1000
+// oblique cells M = 1: 6e-11 and 3.4e-9 at a limit of 1000, 2e-12 and 6e-11 at 100, 2e-12 and
+// 6e-12 at 30, what is left being resonances of both. A stop costs complex solves that
+// hold up the batch (limit 1000 -> 30: 64 cells M = 3 0.33 -> 0.40 ms, 512 rasterised cells 6.3 ->
+// 10.7 ms, 96 oblique cells M = 4 5.0 -> 7.2 ms, 64 stacks 2.5 -> 3.8 ms); that is the price of the digits.
+constexpr int kMaxRest = 5;
+constexpr double kGrowthLimit = 30.0;
 
 // ---- scalars: double or complex ---------------------------------------------------------
 __device__ __forceinline__ double zero_of(double) { return 0.0; }
@@ -916,7 +915,7 @@ __device__ __noinline__ bool two_port(int n, cplx* Mc, double h, double qmax, co
         // X = A^-1 B in the right half of Q (rows by s.perm)
         const bool ok = gauss_jordan(n, nw, Q, n2, false, s);
         const int left = ns - 1 - i;
-        if (!ok || !(max_entry(n, Q, n2, ln, s.red) <= growth_limit(left))) {  // NaN too
+        if (!ok || !(max_entry(n, Q, n2, ln, s.red) <= kGrowthLimit)) {  // NaN too
             if (left + 1 > kMaxRest) return false;
             *rest = left + 1;
             break;
