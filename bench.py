@@ -307,26 +307,38 @@ def rcwa_flops(cell, method="run"):
     """Algorithmic FP64 flops of one cell solve.
     method="reference": 240 n^3 (n = 2N, diagonal-aware count of the reference
     method: ep2 kp 4n^3, eigensolve 100n^3, interfaces 136n^3).
-    method="run": the method this library runs. A mirror-symmetric cell at
-    normal incidence (unrotated shape, theta = 0, Mx, My >= 1) solves the same
-    steps in its two excited parity classes of order m = (Mx+1)(My+1) + Mx My:
-    2 x 240 m^3, plus building M at full order (2 n^3) and projecting it, the
-    layer kp and the half-space operators (4 x 16 x 8 m^2 per class). Other
-    cells run the reference method.
-    Both add n^3 for the Laurent inverse and the raster DFT on rasterised cells."""
+    method="run": the method this library runs, one two-port per matrix of order m
+    (an oblique or rotated cell: m = n; a mirror-symmetric one: its two excited parity
+    classes of order m = (Mx+1)(My+1) + Mx My, one if it is C4-symmetric). With the usual
+    two double angles and three doublings: powers and series 14 m^3, double angles 8,
+    [S^-1 | S^-1 C] 4, doublings 15 (all times 4 where the layer's M is complex), between
+    the half-spaces 20 (24 complex); operators 4 m^3 per class, 2 n^3 in the order basis.
+    Rasterised cells add the Laurent inverse (n^3; by class N^3 / 2) and the transform."""
     Mx, My = cell["Mx"], cell.get("My", cell["Mx"])
     N = (2 * Mx + 1) * (2 * My + 1)
     n = 2 * N
     sym = (cell.get("theta_rad", 0.0) == 0.0 and cell.get("rotation_rad", 0.0) == 0.0 and Mx >= 1 and My >= 1)
-    if method == "run" and sym:
-        m = (Mx + 1) * (My + 1) + Mx * My
-        f = 2 * 240.0 * m ** 3 + 2.0 * n ** 3 + 2 * 4 * 16 * 8.0 * m * m
-    else:
+    laurent = cell.get("force_laurent") or cell.get("shape", 0) != 0
+    ng = cell.get("grid") or max(128, 8 * (2 * Mx + 1))
+    M4 = 4 * Mx + 1
+    if method != "run":
         f = 240.0 * n ** 3
-    if cell.get("force_laurent") or cell.get("shape", 0) != 0:
-        ng = cell.get("grid") or max(128, 8 * (2 * Mx + 1))
-        M4 = 4 * Mx + 1
-        f += n ** 3 + 8.0 * ng * ng * M4 + 8.0 * M4 * M4 * ng
+        if laurent:
+            f += n ** 3 + 8.0 * ng * ng * M4 + 8.0 * M4 * M4 * ng
+        return f
+    real = all(complex(cell.get(k, 1.0)).imag == 0.0 for k in ("eps_pillar", "eps_bg"))
+    per = 41.0 + 20.0 if real else 164.0 + 24.0
+    if sym:
+        m = (Mx + 1) * (My + 1) + Mx * My
+        c4 = (Mx == My and cell.get("period_x_um", 0) == cell.get("period_y_um", cell.get("period_x_um", 0))
+              and cell["fill_x"] == cell.get("fill_y", cell["fill_x"]))
+        f = (1 if c4 else 2) * (per + 4.0) * m ** 3
+        if laurent:
+            f += 0.5 * N ** 3 + 2.0 * ng * (2 * Mx + 1) * (2 * My + 1)
+    else:
+        f = per * n ** 3 + 2.0 * n ** 3
+        if laurent:
+            f += n ** 3 + 8.0 * ng * ng * M4 + 8.0 * M4 * M4 * ng
     return f
 
 
@@ -427,7 +439,7 @@ def measure_rcwa(peaks, quick=False, with_cpu=True, sampler=None):
                             "batched_over_per_cell": per_cell / (dt / 64),
                             "roofline": {"bound": "fp64", "achieved": fl / dt, "peak": p_fp64, "unit": "FLOP/s",
                                          "frac": fl / dt / p_fp64,
-                                         "flops": "of the method run (parity-class solve of mirror-symmetric cells)"},
+                                         "flops": "of the method run (layer two-ports, in parity classes for mirror-symmetric cells)"},
                             "reference_method_flops_per_s": fl_ref / dt,
                             # per-call spread and host CPU time (process, all threads): a wall time far
                             # above the CPU time is time the calling thread spent waiting, not working
@@ -460,7 +472,7 @@ def measure_rcwa(peaks, quick=False, with_cpu=True, sampler=None):
             "max_abs_R_plus_T_minus_1": float(max(abs(r["R"] + r["T"] - 1.0) for r in res)),
             "roofline": {"bound": "fp64", "achieved": fl2 / dt2, "peak": p_fp64, "unit": "FLOP/s",
                          "frac": fl2 / dt2 / p_fp64,
-                         "flops": "of the method run (parity-class solve of mirror-symmetric cells)"},
+                         "flops": "of the method run (layer two-ports, in parity classes for mirror-symmetric cells)"},
             "reference_method_flops_per_s": fl2_ref / dt2}
         if with_cpu:
             try:
