@@ -135,7 +135,7 @@ struct Prod<double, double> {
 // (8-byte fragments: 56 % of L1 and 25 % of the tensor pipe busy at order 162), so they
 // load 16 bytes per lane: two k of A at a time (the order of k within a step of 8
 // is free) and two columns of B, and a warp's unit is 8 R x 8 W with the R, W that leave
-// the least to the busiest warp (96 oblique cells of order 162: 7.0 -> 5.6 ms a call). Real operands have even leading dimensions and
+// the least to the busiest warp (96 oblique cells of order 162, growth limit 1000: 7.0 -> 5.6 ms a call). Real operands have even leading dimensions and
 // 16-byte-aligned bases. bmap (shared, may be NULL): row r of B is stored at row bmap[r].
 template <class TB, int R, int W, class Epi>
 __device__ __forceinline__ void gemm_units_real(int m, int n, int k, const double* A, int lda, const TB* B, int ldb,
@@ -593,7 +593,7 @@ __device__ __forceinline__ void trailing_units(int n, int c0, int cn, T* Wm, int
     }
 }
 // The same in real arithmetic with 16-byte accesses throughout (36 instead of 16 shared and
-// global accesses per 16 tensor instructions otherwise; 64 cells M = 3: 0.345 -> 0.333 ms a
+// global accesses per 16 tensor instructions otherwise; 64 cells M = 3, growth limit 1000: 0.345 -> 0.333 ms a
 // call): units of 8 R x 32, two k of G and two columns of the pivot rows
 // and of Wm per access, as in gemm_units_real. c0 and ld are even.
 template <int R>
