@@ -60,6 +60,7 @@
 #include "cblas_block.cuh"
 #include "schur_aed.cuh"
 #include "slab.cuh"
+#include "slab_check.cuh"
 #include "runtime.cuh"
 
 namespace {

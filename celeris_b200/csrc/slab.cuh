@@ -464,6 +464,9 @@ __device__ __noinline__ void panel(int n, int k0, int kb, const T* Wm, int ld, c
             key = max(key, ((unsigned)__double2hiint(pivot_size(c[r])) & keep[r]) | (unsigned)row);
         }
         key = __reduce_max_sync(0xffffffffu, key);
+        // a warp reduction does not order memory: without this, lane 0's release would cover
+        // its own rows of the column only
+        __syncwarp();
         if (lane == 0) {
             const int p = (int)(key & kRow);
             // zero (or denormal), infinite and NaN pivots: the high word's exponent field

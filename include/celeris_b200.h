@@ -256,6 +256,12 @@ int celeris_debug_fail_alloc(int count);
  * non-convergence report (CELERIS_ERR_EIG_NOCONV, per-cell info > 0 like
  * LAPACK's). Applies to the current device. */
 int celeris_debug_qr_iteration_cap(int cap);
+/* New: the RCWA layers' block elimination alone, one block of `threads` (256 for
+ * n <= 256, or 512): x = a^-1 b, and ainv = a^-1 when `inverse`. a, ainv: n x n,
+ * b, x: n x nrhs, row-major host arrays (interleaved re, im when is_complex),
+ * n <= 512. *ok = 0 (x and ainv not written) when a column had no pivot. */
+int celeris_debug_slab_solve(int n, int nrhs, int is_complex, int inverse, int threads, const double* a,
+                             const double* b, double* x, double* ainv, int* ok);
 
 /* ---- RCWA ------------------------------------------------------------------ */
 

@@ -1,0 +1,56 @@
+"""The block elimination of the RCWA layers on its own, against numpy: orders around its
+panel (16), lane (32, 64, 128, 256) and warp counts, in both block sizes, real and
+complex, with and without the inverse.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+from celeris_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+U = np.finfo(np.float64).eps / 2
+P = ctypes.POINTER(ctypes.c_double)
+
+
+def solve(a, b, inverse=False, threads=512):
+    """(ok, x, ainv) of a x = b through celeris_debug_slab_solve."""
+    n, nrhs, cplx = a.shape[0], b.shape[1], np.iscomplexobj(a)
+    a, b = np.ascontiguousarray(a), np.ascontiguousarray(b)
+    x, inv, ok = np.zeros_like(b), np.zeros_like(a), ctypes.c_int(-1)
+    ptr = lambda v: v.ctypes.data_as(P)  # noqa: E731
+    capi.check(capi.load().celeris_debug_slab_solve(n, nrhs, int(cplx), int(inverse), threads, ptr(a), ptr(b), ptr(x),
+                                                    ptr(inv), ctypes.byref(ok)))
+    return ok.value, x, inv
+
+
+def unitary(n, cplx, seed):
+    rng = np.random.default_rng(seed)
+    a = rng.standard_normal((n, n))
+    if cplx:
+        a = a + 1j * rng.standard_normal((n, n))
+    return np.linalg.qr(a)[0]
+
+
+@pytest.mark.parametrize("n", [1, 2, 5, 15, 16, 17, 31, 32, 33, 49, 61, 64, 65, 98, 127, 128, 129, 162, 255, 256, 257,
+                               481, 512])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("threads", [256, 512])
+def test_elimination(n, cplx, threads):
+    """A handed-over column that is read before all of it is written shows here as a wrong
+    solution. Unitary matrices (condition 1): Gauss-Jordan's forward error is within 2 n u times the
+    growth of the pivots, taken as n."""
+    if threads == 256 and n > 256:
+        pytest.skip("orders above 256 take sixteen warps")
+    a = unitary(n, cplx, n)
+    tol = 2.0 * (n + 4) ** 2 * U
+    for nrhs, inverse in ((1, False), (n, True), (2, True)):
+        b = unitary(max(n, nrhs), cplx, 7 * n + nrhs)[:n, :nrhs]
+        ok, x, inv = solve(a, b, inverse, threads)
+        assert ok == 1
+        want = a.conj().T @ b
+        assert np.linalg.norm(x - want) <= tol * np.linalg.norm(want)
+        if inverse:
+            assert np.linalg.norm(inv - a.conj().T) <= tol * np.sqrt(n)
