@@ -138,7 +138,7 @@ def load(path: str = LIB_PATH):
         "celeris_device_wait_selftest": (_I, [ctypes.c_uint]),
         "celeris_debug_fail_alloc": (_I, [_I]),
         "celeris_debug_qr_iteration_cap": (_I, [_I]),
-        "celeris_debug_slab_solve": (_I, [_I, _I, _I, _I, _I, _P, _P, _P, _P, _PI]),
+        "celeris_debug_slab_solve": (_I, [_I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _PI]),
         "celeris_set_kernel_timing": (_I, [_I]),
         "celeris_last_kernel_ms": (_I, [_P]),
         "celeris_solve_rcwa_2d": (_I, [ctypes.POINTER(RcwaCell), _P, _P, ctypes.POINTER(RcwaResult)]),

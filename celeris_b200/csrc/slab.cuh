@@ -46,6 +46,7 @@ constexpr double kSpectral = 2.2;     // largest spectral radius of Q y of the s
 constexpr double kPhaseMax = 2.5;     // largest q x of a propagating mode at S^-1 (sin q x = 0 at pi)
 constexpr int kMaxAngles = 2;         // double-angle steps
 constexpr int kMaxDoublings = 40;
+constexpr unsigned kFlagPolls = 1u << 22;  // bound of a panel's wait for a column
 // Largest max |X| of a doubling: beyond it the doublings stop where at most kMaxRest are left
 // (1 << kMaxRest slabs), or the layer is given up. The error grows as eps |X|^2. Largest
 // difference from the eigendecomposition over 6000 mirror-symmetric cells M = 1 .. 3 and 1000
@@ -338,9 +339,10 @@ struct Shared {
     int* pos;     // [n] variable of row r, -1 while it has none
     int* perm2;   // [n] a kept copy of perm
     int* flag;    // [kNB] of a panel's columns: 0, or 1 + the pivot's row, or -1 (no pivot)
-    int* bad;     // set when a column had no pivot
+    int* bad;     // set when a column had no pivot, or a warp's wait for one ran out
     double* red;  // [32]
     int chunk;    // columns staged at a time
+    unsigned polls;  // bound of a wait for a column
     long long* prof;  // optional clock64 sums: [0] panels, [1] updates of the other columns, [2] whole kernel
 };
 __host__ __device__ inline size_t pad16(size_t b) { return (b + 15) & ~size_t(15); }
@@ -364,6 +366,7 @@ __device__ __forceinline__ Shared carve(unsigned char* p, int n) {
     Shared s;
     s.prof = nullptr;
     s.chunk = chunk_of(n);
+    s.polls = kFlagPolls;
     s.pan = reinterpret_cast<cplx*>(p);
     p += panel_elems(n) * 16;
     s.prow = reinterpret_cast<cplx*>(p);
@@ -416,11 +419,10 @@ template <class T>
 __host__ __device__ constexpr int panel_stride() {
     return sizeof(T) == sizeof(double) ? kGsReal : kGs;
 }
-constexpr unsigned kFlagPolls = 1u << 22;  // bound of a wait for a column
-__device__ __forceinline__ int wait_column(const int* flag) {
+__device__ __forceinline__ int wait_column(const int* flag, unsigned polls) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(flag);
     int v = 0;
-    for (unsigned i = 0; i < kFlagPolls && v == 0; ++i)
+    for (unsigned i = 0; i < polls && v == 0; ++i)
         asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v == 0 ? -1 : v;
 }
@@ -483,7 +485,7 @@ __device__ __noinline__ void panel(int n, int k0, int kb, const T* Wm, int ld, c
         for (int wo = 0; wo < PW; ++wo) {
             const int j = qo * PW + wo;
             if (j >= kb) break;
-            const int got = wait_column(flag + j);
+            const int got = wait_column(flag + j, s.polls);
             if (got < 0) {
                 ok = false;
                 break;
@@ -538,7 +540,7 @@ __device__ __noinline__ void panel(int n, int k0, int kb, const T* Wm, int ld, c
     used = mask;
     panel_barrier<PW * 32>();  // the column buffers are read; G overlays them
     if (!ok) {
-        if (threadIdx.x == 0) *s.bad = 1;
+        if (lane == 0) *s.bad = 1;  // any warp's: its columns of G are missing
         return;
     }
     T* pan = as<T>(s.pan);

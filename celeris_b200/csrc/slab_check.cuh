@@ -13,11 +13,14 @@
 
 namespace {
 
-// W (n x ncol, ld) <- its elimination (gauss_jordan); ok, perm: its result.
+// W (n x ncol, ld) <- its elimination (gauss_jordan); ok, perm: its result. lost_warp >= 0: that
+// warp gives up its waits at once.
 template <class T>
-__global__ void __launch_bounds__(512) slab_check_solve(int n, int ncol, int ld, T* W, int inverse, int* perm, int* ok) {
+__global__ void __launch_bounds__(512) slab_check_solve(int n, int ncol, int ld, T* W, int inverse, int lost_warp,
+                                                        int* perm, int* ok) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const cb::slab::Shared s = cb::slab::carve(smem, n);
+    cb::slab::Shared s = cb::slab::carve(smem, n);
+    if ((int)(threadIdx.x >> 5) == lost_warp) s.polls = 0;
     const bool got = cb::slab::gauss_jordan(n, ncol, W, ld, inverse != 0, s);
     __syncthreads();
     if (got)
@@ -26,7 +29,7 @@ __global__ void __launch_bounds__(512) slab_check_solve(int n, int ncol, int ld,
 }
 
 template <class T>
-int run_solve(int n, int nrhs, int inverse, int threads, const T* a, const T* b, T* x, T* ainv, int* ok_out) {
+int run_solve(int n, int nrhs, int inverse, int threads, int lost_warp, const T* a, const T* b, T* x, T* ainv, int* ok_out) {
     const int c1 = sizeof(T) == sizeof(double) ? (n + 1) & ~1 : n;  // first right-hand side's column
     const int ncol = c1 + nrhs, ld = (ncol + 1) & ~1;
     std::vector<T> h((size_t)n * ld);
@@ -46,7 +49,7 @@ int run_solve(int n, int nrhs, int inverse, int threads, const T* a, const T* b,
         CEL_CUDA(cudaMemset(dperm, 0, words * sizeof(int)));
         const size_t smem = cb::slab::shared_bytes(n);
         CEL_CUDA(cudaFuncSetAttribute(slab_check_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        slab_check_solve<T><<<1, threads, smem>>>(n, ncol, ld, dW, inverse, dperm, dperm + n);
+        slab_check_solve<T><<<1, threads, smem>>>(n, ncol, ld, dW, inverse, lost_warp, dperm, dperm + n);
         celeris_rt::count_launch(1);
         CEL_CUDA(cudaGetLastError());
         CEL_CUDA(cudaMemcpy(h.data(), dW, bytes, cudaMemcpyDeviceToHost));
@@ -72,8 +75,8 @@ int run_solve(int n, int nrhs, int inverse, int threads, const T* a, const T* b,
 
 }  // namespace
 
-extern "C" int celeris_debug_slab_solve(int n, int nrhs, int is_complex, int inverse, int threads, const double* a,
-                                        const double* b, double* x, double* ainv, int* ok) {
+extern "C" int celeris_debug_slab_solve(int n, int nrhs, int is_complex, int inverse, int threads, int lost_warp,
+                                        const double* a, const double* b, double* x, double* ainv, int* ok) {
     CEL_TRY(celeris_rt::require_device());
     // above order 256 the panel takes sixteen warps
     if (n < 1 || n > cb::slab::kMaxOrder || nrhs < 1 || (threads != 512 && (threads != 256 || n > 256)) || !a || !b ||
@@ -81,7 +84,7 @@ extern "C" int celeris_debug_slab_solve(int n, int nrhs, int is_complex, int inv
         return celeris_rt::set_error(CELERIS_ERR_INVALID_ARG, "n in [1, %d], threads 256 (n <= 256) or 512",
                                      cb::slab::kMaxOrder);
     if (is_complex)
-        return run_solve(n, nrhs, inverse, threads, reinterpret_cast<const cb::cplx*>(a), reinterpret_cast<const cb::cplx*>(b),
-                         reinterpret_cast<cb::cplx*>(x), reinterpret_cast<cb::cplx*>(ainv), ok);
-    return run_solve(n, nrhs, inverse, threads, a, b, x, ainv, ok);
+        return run_solve(n, nrhs, inverse, threads, lost_warp, reinterpret_cast<const cb::cplx*>(a),
+                         reinterpret_cast<const cb::cplx*>(b), reinterpret_cast<cb::cplx*>(x), reinterpret_cast<cb::cplx*>(ainv), ok);
+    return run_solve(n, nrhs, inverse, threads, lost_warp, a, b, x, ainv, ok);
 }

@@ -15,14 +15,14 @@ U = np.finfo(np.float64).eps / 2
 P = ctypes.POINTER(ctypes.c_double)
 
 
-def solve(a, b, inverse=False, threads=512):
+def solve(a, b, inverse=False, threads=512, lost_warp=-1):
     """(ok, x, ainv) of a x = b through celeris_debug_slab_solve."""
     n, nrhs, cplx = a.shape[0], b.shape[1], np.iscomplexobj(a)
     a, b = np.ascontiguousarray(a), np.ascontiguousarray(b)
     x, inv, ok = np.zeros_like(b), np.zeros_like(a), ctypes.c_int(-1)
     ptr = lambda v: v.ctypes.data_as(P)  # noqa: E731
-    capi.check(capi.load().celeris_debug_slab_solve(n, nrhs, int(cplx), int(inverse), threads, ptr(a), ptr(b), ptr(x),
-                                                    ptr(inv), ctypes.byref(ok)))
+    capi.check(capi.load().celeris_debug_slab_solve(n, nrhs, int(cplx), int(inverse), threads, lost_warp, ptr(a), ptr(b),
+                                                    ptr(x), ptr(inv), ctypes.byref(ok)))
     return ok.value, x, inv
 
 
@@ -54,3 +54,15 @@ def test_elimination(n, cplx, threads):
         assert np.linalg.norm(x - want) <= tol * np.linalg.norm(want)
         if inverse:
             assert np.linalg.norm(inv - a.conj().T) <= tol * np.sqrt(n)
+
+
+@pytest.mark.parametrize("warp", [0, 1, 3, 7])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_a_warp_that_gives_up_is_reported(warp, cplx):
+    """One warp's wait runs out while the others' do not (order 1: one column, whose owner, warp
+    0, hands it over before it waits). The elimination reports it, from whichever warp: that warp's
+    columns are missing from the update."""
+    a = unitary(1, cplx, 1)
+    ok, x, _ = solve(a, a, lost_warp=warp)
+    assert ok == 0 and not np.any(x)
+    assert solve(a, a)[0] == 1
