@@ -473,9 +473,12 @@ __device__ __noinline__ void panel(int n, int k0, int kb, const T* Wm, int ld, c
             const int p = (int)(key & kRow);
             // zero (or denormal), infinite and NaN pivots: the high word's exponent field
             const unsigned e = (key >> 20) & 0x7ffu;
-            raise_column(flag + j, e == 0u || e == 0x7ffu ? -1 : p + 1);
-            perm[j] = p;
-            pos[p] = k0 + j;
+            const bool none = e == 0u || e == 0x7ffu;
+            raise_column(flag + j, none ? -1 : p + 1);
+            if (!none) {  // else p may be a lane's row past the matrix
+                perm[j] = p;
+                pos[p] = k0 + j;
+            }
         }
     };
     if (warp == 0) hand_over(a[0], 0);

@@ -14,18 +14,31 @@
 namespace {
 
 // W (n x ncol, ld) <- its elimination (gauss_jordan); ok, perm: its result. lost_warp >= 0: that
-// warp gives up its waits at once.
+// warp gives up its waits at once. intact: a failed elimination left what it does not own in
+// shared memory as it was (perm2, and the flags of the columns behind the one without a pivot).
 template <class T>
 __global__ void __launch_bounds__(512) slab_check_solve(int n, int ncol, int ld, T* W, int inverse, int lost_warp,
-                                                        int* perm, int* ok) {
+                                                        int* perm, int* ok, int* intact) {
     extern __shared__ __align__(16) unsigned char smem[];
     cb::slab::Shared s = cb::slab::carve(smem, n);
     if ((int)(threadIdx.x >> 5) == lost_warp) s.polls = 0;
+    constexpr int kMark = 0x5a5a5a5a;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) s.perm2[i] = kMark;
     const bool got = cb::slab::gauss_jordan(n, ncol, W, ld, inverse != 0, s);
     __syncthreads();
     if (got)
         for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = s.perm[i];
     ok[threadIdx.x] = got;
+    if (threadIdx.x == 0) {
+        int fine = 1;
+        for (int i = 0; i < n; ++i) fine &= s.perm2[i] == kMark;
+        bool behind = false;
+        for (int j = 0; j < cb::slab::kNB; ++j) {
+            if (behind) fine &= s.flag[j] == 0;
+            behind = behind || (!got && s.flag[j] < 0);
+        }
+        *intact = fine;
+    }
 }
 
 template <class T>
@@ -38,7 +51,7 @@ int run_solve(int n, int nrhs, int inverse, int threads, int lost_warp, const T*
         std::copy(a + (size_t)i * n, a + (size_t)(i + 1) * n, h.begin() + (size_t)i * ld);
         std::copy(b + (size_t)i * nrhs, b + (size_t)(i + 1) * nrhs, h.begin() + (size_t)i * ld + c1);
     }
-    const size_t bytes = h.size() * sizeof(T), words = (size_t)n + threads;
+    const size_t bytes = h.size() * sizeof(T), words = (size_t)n + threads + 1;
     char* d = nullptr;
     CEL_TRY(celeris_rt::device_alloc(reinterpret_cast<void**>(&d), bytes + words * sizeof(int), "slab check"));
     T* dW = reinterpret_cast<T*>(d);
@@ -49,7 +62,8 @@ int run_solve(int n, int nrhs, int inverse, int threads, int lost_warp, const T*
         CEL_CUDA(cudaMemset(dperm, 0, words * sizeof(int)));
         const size_t smem = cb::slab::shared_bytes(n);
         CEL_CUDA(cudaFuncSetAttribute(slab_check_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        slab_check_solve<T><<<1, threads, smem>>>(n, ncol, ld, dW, inverse, lost_warp, dperm, dperm + n);
+        slab_check_solve<T><<<1, threads, smem>>>(n, ncol, ld, dW, inverse, lost_warp, dperm, dperm + n,
+                                                   dperm + n + threads);
         celeris_rt::count_launch(1);
         CEL_CUDA(cudaGetLastError());
         CEL_CUDA(cudaMemcpy(h.data(), dW, bytes, cudaMemcpyDeviceToHost));
@@ -63,6 +77,7 @@ int run_solve(int n, int nrhs, int inverse, int threads, int lost_warp, const T*
     *ok_out = ok[0];
     for (int t = 1; t < threads; ++t)
         if (ok[t] != ok[0]) return celeris_rt::set_error(CELERIS_ERR_CUDA, "threads disagree on the elimination's result");
+    if (!ok[threads]) return celeris_rt::set_error(CELERIS_ERR_CUDA, "the elimination wrote outside its own arrays");
     if (!ok[0]) return CELERIS_OK;
     for (int k = 0; k < n; ++k) {
         const T* row = h.data() + (size_t)hw[k] * ld;

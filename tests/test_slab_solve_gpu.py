@@ -66,3 +66,15 @@ def test_a_warp_that_gives_up_is_reported(warp, cplx):
     ok, x, _ = solve(a, a, lost_warp=warp)
     assert ok == 0 and not np.any(x)
     assert solve(a, a)[0] == 1
+
+
+@pytest.mark.parametrize("n,col", [(1, 0), (5, 2), (5, 4), (9, 3), (9, 8), (17, 16), (25, 7), (33, 20), (61, 40), (100, 99),
+                                   (162, 17), (300, 299)])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_a_column_without_a_pivot_writes_nothing_outside(n, col, cplx):
+    """A zero column ends the elimination, and the row its search falls on, which may lie past the
+    matrix, is not recorded (the call checks the neighbouring arrays and reports an error)."""
+    a = unitary(n, cplx, n)
+    a[:, col] = 0.0
+    ok, x, _ = solve(a, unitary(n, cplx, n)[:, :1])
+    assert ok == 0 and not np.any(x)
