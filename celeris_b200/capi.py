@@ -57,6 +57,7 @@ EXPORTED = [
     "celeris_probe_mufu_accuracy", "celeris_rs_field_bounded", "celeris_rs_error_bound_dev",
     "celeris_rs_field_rows_dev", "celeris_rs_adjoint_rows_dev", "celeris_device_wait_selftest",
     "celeris_debug_fail_alloc", "celeris_debug_qr_iteration_cap", "celeris_debug_slab_solve",
+    "celeris_debug_slab_max",
 ]
 
 
@@ -139,6 +140,7 @@ def load(path: str = LIB_PATH):
         "celeris_debug_fail_alloc": (_I, [_I]),
         "celeris_debug_qr_iteration_cap": (_I, [_I]),
         "celeris_debug_slab_solve": (_I, [_I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _PI]),
+        "celeris_debug_slab_max": (_I, [_I, _I, _P, _P]),
         "celeris_set_kernel_timing": (_I, [_I]),
         "celeris_last_kernel_ms": (_I, [_P]),
         "celeris_solve_rcwa_2d": (_I, [ctypes.POINTER(RcwaCell), _P, _P, ctypes.POINTER(RcwaResult)]),

@@ -1364,9 +1364,9 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) rcwa_sym_ops(Bucket b) 
         for (int e = tid; e < (4 * Mx + 1) * (4 * My + 1); e += nt) {
             const int dp = e / (4 * My + 1) - 2 * Mx, dq = e % (4 * My + 1) - 2 * My;
             const cplx v = Ge(dp, dq);
-            dev = fmax(dev, fmax(cabs(csub(v, Ge(-dp, dq))), cabs(csub(v, Ge(dp, -dq)))));
-            if (b.ncls == 1) dev = fmax(dev, cabs(csub(v, Ge(-dq, dp))));
-            mag = fmax(mag, cabs(v));
+            dev = slab::nan_max(slab::nan_max(dev, cabs(csub(v, Ge(-dp, dq)))), cabs(csub(v, Ge(dp, -dq))));
+            if (b.ncls == 1) dev = slab::nan_max(dev, cabs(csub(v, Ge(-dq, dp))));
+            mag = slab::nan_max(mag, cabs(v));
         }
         dev = slab::block_max(dev, red);
         mag = slab::block_max(mag, red);
@@ -1808,8 +1808,8 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) rcwa_slab(Bucket b) {
     if (real) {
         double re = 0.0, im = 0.0;
         for (int e = threadIdx.x; e < n * n; e += NT) {
-            re = fmax(re, fabs(M[e].x));
-            im = fmax(im, fabs(M[e].y));
+            re = slab::nan_max(re, fabs(M[e].x));
+            im = slab::nan_max(im, fabs(M[e].y));
         }
         re = slab::block_max(re, s.red);
         im = slab::block_max(im, s.red);

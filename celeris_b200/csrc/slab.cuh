@@ -389,14 +389,16 @@ __device__ __forceinline__ T* as(cplx* p) {
     return reinterpret_cast<T*>(p);
 }
 
-// Largest value over the block, the same in every thread.
+// The larger of m and v, NaN if either is (fmax would drop it).
+__device__ __forceinline__ double nan_max(double m, double v) { return v > m || v != v ? v : m; }
+// Largest value over the block, the same in every thread; NaN if any is.
 __device__ __forceinline__ double block_max(double v, double* red) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = nan_max(v, __shfl_xor_sync(0xffffffffu, v, o));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
     double m = red[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = nan_max(m, red[w]);
     return m;
 }
 
@@ -783,7 +785,7 @@ __device__ double norm_inf(int n, const T* A, int ld, double* red) {
         double t = 0.0;
         for (int j = lane; j < n; j += 32) t += size1(A[(size_t)i * ld + j]);
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        best = t > best || t != t ? t : best;  // NaN sticks
+        best = nan_max(best, t);
     }
     return block_max(best, red);
 }
@@ -794,8 +796,7 @@ __device__ double max_entry(int n, const T* A, int ld, int c0, double* red) {
     double best = 0.0;
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
         const int i = e / n, j = e - i * n;
-        const double v = size1(A[(size_t)i * ld + c0 + j]);
-        best = v > best || v != v ? v : best;
+        best = nan_max(best, size1(A[(size_t)i * ld + c0 + j]));
     }
     return block_max(best, red);
 }

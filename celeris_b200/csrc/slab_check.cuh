@@ -1,5 +1,5 @@
-// The block elimination of slab.cuh on its own, for tests of its edges: orders around
-// its panel and lane counts and matrices without a pivot. Not part of any result path.
+// The block elimination and norms of slab.cuh on their own, for tests of their edges: orders
+// around the panel and lane counts, matrices without a pivot, NaN. Not part of any result path.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -88,7 +88,51 @@ int run_solve(int n, int nrhs, int inverse, int threads, int lost_warp, const T*
     return CELERIS_OK;
 }
 
+// out: norm_inf and max_entry of the n x n matrix A, as every thread has them (NaN if they differ).
+__global__ void __launch_bounds__(512) slab_check_max(int n, const double* A, double* out) {
+    __shared__ double red[32];
+    __shared__ int differ;
+    if (threadIdx.x == 0) differ = 0;
+    const double a = cb::slab::norm_inf(n, A, n, red), b = cb::slab::max_entry(n, A, n, 0, red);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        out[0] = a;
+        out[1] = b;
+    }
+    __syncthreads();
+    const auto same = [](double x, double y) { return x == y || (x != x && y != y); };
+    if (!same(out[0], a) || !same(out[1], b)) atomicOr(&differ, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) out[2] = differ;
+}
+
 }  // namespace
+
+extern "C" int celeris_debug_slab_max(int n, int threads, const double* a, double* out) {
+    CEL_TRY(celeris_rt::require_device());
+    if (n < 1 || n > cb::slab::kMaxOrder || (threads != 256 && threads != 512) || !a || !out)
+        return celeris_rt::set_error(CELERIS_ERR_INVALID_ARG, "n in [1, %d], threads 256 or 512", cb::slab::kMaxOrder);
+    const size_t bytes = (size_t)n * n * sizeof(double);
+    double* d = nullptr;
+    double h[3];
+    CEL_TRY(celeris_rt::device_alloc(reinterpret_cast<void**>(&d), bytes + sizeof(h), "slab check"));
+    auto call = [&]() -> int {
+        double* dout = d + (size_t)n * n;
+        CEL_CUDA(cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice));
+        slab_check_max<<<1, threads>>>(n, d, dout);
+        celeris_rt::count_launch(1);
+        CEL_CUDA(cudaGetLastError());
+        CEL_CUDA(cudaMemcpy(h, dout, sizeof(h), cudaMemcpyDeviceToHost));
+        return CELERIS_OK;
+    };
+    const int status = call();
+    cudaFree(d);
+    CEL_TRY(status);
+    if (h[2] != 0.0) return celeris_rt::set_error(CELERIS_ERR_CUDA, "threads disagree on a block's maximum");
+    out[0] = h[0];
+    out[1] = h[1];
+    return CELERIS_OK;
+}
 
 extern "C" int celeris_debug_slab_solve(int n, int nrhs, int is_complex, int inverse, int threads, int lost_warp,
                                         const double* a, const double* b, double* x, double* ainv, int* ok) {

@@ -264,6 +264,9 @@ int celeris_debug_qr_iteration_cap(int cap);
  * at once (-1: none). */
 int celeris_debug_slab_solve(int n, int nrhs, int is_complex, int inverse, int threads, int lost_warp,
                              const double* a, const double* b, double* x, double* ainv, int* ok);
+/* New: out[0] = the largest row sum of |a|, out[1] = its largest entry (n x n, n <= 512), as
+ * one block of 256 or 512 threads has them for the checks of a layer: NaN if an entry is. */
+int celeris_debug_slab_max(int n, int threads, const double* a, double* out);
 
 /* ---- RCWA ------------------------------------------------------------------ */
 

@@ -78,3 +78,22 @@ def test_a_column_without_a_pivot_writes_nothing_outside(n, col, cplx):
     a[:, col] = 0.0
     ok, x, _ = solve(a, unitary(n, cplx, n)[:, :1])
     assert ok == 0 and not np.any(x)
+
+
+@pytest.mark.parametrize("n", [1, 7, 33, 98])
+@pytest.mark.parametrize("threads", [256, 512])
+def test_block_maxima_keep_nan(n, threads):
+    """One NaN among numbers shows in the norm and in the largest entry, wherever it lies."""
+    a = np.random.default_rng(n).standard_normal((n, n))
+    out = np.zeros(2)
+
+    def maxima(m):
+        capi.check(capi.load().celeris_debug_slab_max(n, threads, m.ctypes.data_as(P), out.ctypes.data_as(P)))
+        return out.copy()
+
+    got = maxima(a)
+    assert abs(got[0] - np.abs(a).sum(axis=1).max()) <= 2 * n * U * got[0] and got[1] == np.abs(a).max()
+    for e in {0, n * n // 3, n * n - 1}:
+        b = a.copy()
+        b.flat[e] = np.nan
+        assert np.all(np.isnan(maxima(b)))
