@@ -2174,6 +2174,12 @@ double symmetry_tolerance() {
     const char* e = std::getenv("CELERIS_RCWA_SYM_TOL");
     return e ? std::atof(e) : 1e-9;
 }
+// Every bit of v (std::to_string keeps six decimals).
+std::string exact_text(double v) {
+    char t[40];
+    std::snprintf(t, sizeof(t), "%a", v);
+    return t;
+}
 bool sym_eligible(const celeris_rcwa_cell& c) {
     return c.theta_rad == 0.0 && c.rotation_rad == 0.0 && c.Mx >= 1 && c.My >= 1 && symmetry_enabled();
 }
@@ -2875,7 +2881,8 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
             for (int i = 0; i < nc; ++i) hdesc[w][i] = cells[p.ids[i]].d;
             needs.add(p.Mx, p.My, p.ng, p.n, p.sym, p.qr);
             sig += "|" + std::to_string(p.Mx) + "," + std::to_string(p.My) + "," + std::to_string(p.ng) + "," +
-                   std::to_string(p.sym) + "," + std::to_string(p.qr) + "," + std::to_string(nc) + "," + std::to_string(b.sym_tol);
+                   std::to_string(p.sym) + "," + std::to_string(p.qr) + "," + std::to_string(nc) + "," +
+                   exact_text(b.sym_tol);  // the tolerance is an argument of the captured kernels
         }
         CEL_TRY(set_smem_limits(needs));
         // ---- tune unseen bucket shapes (descriptors must be on the device)

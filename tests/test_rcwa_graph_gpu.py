@@ -1,0 +1,40 @@
+"""What a cached graph of celeris_rcwa_batch holds: a batch of a shape seen before, with another
+symmetry tolerance, does not replay the old one's graph.
+"""
+import os
+
+import pytest
+
+from celeris_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+BASE = dict(period_um=0.4, wavelength_um=0.633, n_inc=1.0, n_sub=1.46, eps_pillar=4.0, eps_bg=1.0, thickness_um=0.6)
+
+
+def launches(cells):
+    """Kernels that one batch launches, once its shape is known (tuned and captured)."""
+    arr = [capi.rcwa_cell(**c) for c in cells]
+    lib = capi.load()
+    for _ in range(2):
+        before = lib.celeris_launch_count()
+        res, info = capi.rcwa_batch(arr)
+        assert not info.any()
+    return lib.celeris_launch_count() - before, res
+
+
+@pytest.mark.parametrize("grid", [0, 64])
+def test_symmetry_tolerance_of_a_known_shape(grid):
+    """Tolerance 0 sends every cell to the order basis: more kernels, the same results. The
+    default and 0 agree in their first six decimals."""
+    cells = [dict(BASE, Mx=2, fill_x=0.3 + 0.1 * i, shape=1 if grid else 0, grid=grid) for i in range(5)]
+    count, res = launches(cells)
+    os.environ["CELERIS_RCWA_SYM_TOL"] = "0"
+    try:
+        redo, res0 = launches(cells)
+    finally:
+        del os.environ["CELERIS_RCWA_SYM_TOL"]
+    assert redo > count
+    assert launches(cells)[0] == count
+    for a, b in zip(res, res0):
+        assert abs(a["tx0"] - b["tx0"]) <= 1e-10 and abs(a["R"] - b["R"]) <= 1e-10
