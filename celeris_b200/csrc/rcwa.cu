@@ -2465,6 +2465,14 @@ int set_smem_limits(const SmemNeeds& s) {
     return CELERIS_OK;
 }
 
+// Kernels that launch_bucket launches (layer: of a stack, through the two-port).
+int bucket_kernels(bool sym, int ng, bool qr, bool eig_only = false, bool layer = false) {
+    const int operators = sym ? (ng > 0 ? 2 : 1) : (ng > 0 ? 3 : 1);
+    if (!qr) return operators + 1 + (sym ? 1 : 0) + (layer ? 0 : 1);  // slab, expand, epilogue
+    // build (order basis), hess, schur, vec; smat1 and smat2, or the classes' smat and expand; epilogue
+    return operators + (sym ? 6 : eig_only ? 4 : 7);
+}
+
 // Launch the stage sequence of one bucket on `st`. ev (ST_COUNT + 1 events) is
 // optional: stage boundaries are recorded into it.
 // eig_only: stop after the eigenvectors (the layers of a multi-layer stack).
@@ -2474,6 +2482,7 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
     const int nc = b.ncell, n = b.n;
     const int* T = cfg.threads;
     if (ev) cudaEventRecord(ev[0], st);
+    count_launch(bucket_kernels(b.sym != 0, b.ng, qr, eig_only, b.lA != nullptr));
     cudaMemsetAsync(b.info, 0, sizeof(int) * nc, st);
     if (b.sym) {
         if (b.ng > 0) {
@@ -2481,18 +2490,15 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
             rcwa_prefix_table<<<((mmax + 1) * (b.ng + 1) + 255) / 256, 256, 0, st>>>(
                 b.ng, mmax, const_cast<cplx*>(b.phx), const_cast<cplx*>(b.pcx));
         }
-        count_launch(b.ng > 0 ? 1 : 0);
     } else if (b.ng > 0) {
         const int Mx = b.Mx, My = b.My, ng = b.ng;
         rcwa_phase_table<<<((4 * Mx + 1) * ng + 255) / 256, 256, 0, st>>>(ng, 2 * Mx, const_cast<cplx*>(b.phx));
         rcwa_phase_table<<<((4 * My + 1) * ng + 255) / 256, 256, 0, st>>>(ng, 2 * My, const_cast<cplx*>(b.phy));
         rcwa_fourier_laurent<<<nc, T[ST_FOURIER], laurent_smem(Mx, My, ng), st>>>(b);
-        count_launch(3);
     } else {
         const int nx = 2 * b.Mx + 1, ny = 2 * b.My + 1;
         const size_t sm = ((size_t)2 * (nx * nx + ny * ny) + 2 * std::max(nx, ny)) * sizeof(cplx);
         rcwa_fourier_rect<<<nc, T[ST_FOURIER], sm, st>>>(b);
-        count_launch(1);
     }
     if (ev) cudaEventRecord(ev[1], st);
     if (b.sym) {  // class operators
@@ -2515,7 +2521,6 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
         if (ev) cudaEventRecord(ev[7], st);
         if (!b.lA) rcwa_epilogue<<<nc, T[ST_EPI], 0, st>>>(b);
         if (ev) cudaEventRecord(ev[8], st);
-        count_launch((b.sym ? 3 : 1) + (b.lA ? 0 : 1));
         return;
     }
     const Bucket e = b.sym ? sym_eig_bucket(b) : b;
@@ -2540,13 +2545,9 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
         if (ev) cudaEventRecord(ev[7], st);
         rcwa_epilogue<<<nc, T[ST_EPI], 0, st>>>(b);
         if (ev) cudaEventRecord(ev[8], st);
-        count_launch(7);
         return;
     }
-    if (eig_only) {
-        count_launch(4);
-        return;
-    }
+    if (eig_only) return;
     const size_t sm_stage = lu_stage_bytes(n);
     rcwa_smat1<<<nc, T[ST_SMAT1], sm_stage, st>>>(b);
     if (ev) cudaEventRecord(ev[6], st);
@@ -2554,7 +2555,6 @@ void launch_bucket(const Bucket& b, const StageCfg& cfg, cudaStream_t st, cudaEv
     if (ev) cudaEventRecord(ev[7], st);
     rcwa_epilogue<<<nc, T[ST_EPI], 0, st>>>(b);
     if (ev) cudaEventRecord(ev[8], st);
-    count_launch(7);
 }
 
 // Time each stage at every candidate size on (up to) the first 2 x SMs cells
@@ -2994,7 +2994,7 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                     cudaMemcpyAsync(const_cast<CellDev*>(p.b.cells), hdesc[w], sizeof(CellDev) * nc,
                                     cudaMemcpyHostToDevice, bs);
                     launch_bucket(p.b, cfgs[w], bs, nullptr, p.qr != 0);
-                    nk += p.sym ? (p.ng > 0 ? 5 : 4) : (p.ng > 0 ? 3 : 1) + (p.qr ? 7 : 2);
+                    nk += bucket_kernels(p.sym != 0, p.ng, p.qr != 0);
                     cudaMemcpyAsync(hres_pin[w], p.b.res, sizeof(celeris_rcwa_result) * nexc * nc,
                                     cudaMemcpyDeviceToHost, bs);
                     cudaMemcpyAsync(hinfo_pin[w], p.b.info, sizeof(int) * nc, cudaMemcpyDeviceToHost, bs);

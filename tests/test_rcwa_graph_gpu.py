@@ -1,5 +1,5 @@
 """What a cached graph of celeris_rcwa_batch holds: a batch of a shape seen before, with another
-symmetry tolerance, does not replay the old one's graph.
+symmetry tolerance, does not replay the old one's graph; and its kernels are counted.
 """
 import os
 
@@ -38,3 +38,17 @@ def test_symmetry_tolerance_of_a_known_shape(grid):
     assert launches(cells)[0] == count
     for a, b in zip(res, res0):
         assert abs(a["tx0"] - b["tx0"]) <= 1e-10 and abs(a["R"] - b["R"]) <= 1e-10
+
+
+@pytest.mark.parametrize("extra,kernels", [
+    (dict(), 4),  # class operators, two-port, expansion, outputs
+    (dict(shape=1, grid=64), 5),  # and the phase table
+    (dict(theta_rad=0.2), 3),  # operators, two-port, outputs
+    (dict(theta_rad=0.2, shape=1, grid=64), 5),  # two phase tables
+    (dict(thickness_um=5e-4), 7),  # class operators, three eigen stages, class S-matrix, expansion, outputs
+    (dict(thickness_um=5e-4, shape=1, grid=64), 8),
+    (dict(thickness_um=5e-4, theta_rad=0.2), 8),  # operators, M, three eigen stages, two S-matrix stages, outputs
+    (dict(thickness_um=5e-4, theta_rad=0.2, shape=1, grid=64), 10),
+])
+def test_launch_count_of_a_bucket(extra, kernels):
+    assert launches([dict(BASE, Mx=2, fill_x=0.5, **extra)])[0] == kernels
