@@ -72,7 +72,7 @@ using celeris_rt::Workspace;
 
 constexpr double PI = 3.14159265358979323846;
 constexpr int kRT = 256;            // threads per CTA
-constexpr int kDbgSlots = 24;       // diagnostic counters per cell
+constexpr int kDbgSlots = 16;       // diagnostic counters per cell
 constexpr int kSmemEigMaxN = 116;   // Hessenberg reduction in shared memory up to this n ((n^2 + 2n) 16 B <= 227 KB)
 
 struct CellDev {
@@ -2165,8 +2165,8 @@ bool symmetry_enabled() {
     const char* e = std::getenv("CELERIS_RCWA_SYMMETRY");
     return !(e && e[0] == '0');
 }
-// Mirror-asymmetry tolerance of the class split, relative to the largest entry
-// of each eps operator (Exx, Eyy, Einv and the Laurent coefficients): rounding
+// Mirror-asymmetry tolerance of the class split, relative to the largest Laurent
+// coefficient of a rasterised cell (an analytic rectangle is symmetric exactly): rounding
 // leaves ~1e-15; one raster sample on the other side of a shape boundary
 // ~1e-6. CELERIS_RCWA_SYM_TOL overrides it (the test is strict, so 0 sends
 // every cell to the full order through the fallback, for tests of that path).
@@ -2957,17 +2957,14 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                 }
                 char buf[64];
                 std::snprintf(buf, sizeof(buf), " | sweeps/cell %.1f", sw / nc);
-                char buf2[640];
+                char buf2[512];
                 std::snprintf(buf2, sizeof(buf2), " | schur Mcycles/cell: aed %.2f (qr %.2f, %.0f rot) aed_far %.2f sweep %.2f (%.0f steps) sweep_far %.2f small %.2f"
                               " | hess Mcycles/cell: columns %.2f (matvec %.2f) updates %.2f"
-                              " | small QR Mcycles/cell: aed chase %.2f deferred %.2f, block chase %.2f deferred %.2f"
-                              " | class smat Mcycles/cell: kpW+C0A %.2f LU(T11) %.2f solve %.2f KsW %.2f LU(A) %.2f solve %.2f S12Q %.2f rest %.2f\n",
+                              " | small QR Mcycles/cell: aed chase %.2f deferred %.2f, block chase %.2f deferred %.2f\n",
                               ph[0] / nc * 1e-6, ph[5] / nc * 1e-6, ph[8] / nc, ph[1] / nc * 1e-6, ph[2] / nc * 1e-6,
                               ph[7] / nc, ph[3] / nc * 1e-6, ph[4] / nc * 1e-6, ph[9] / nc * 1e-6, ph[10] / nc * 1e-6,
                               ph[11] / nc * 1e-6, ph[12] / nc * 1e-6, ph[13] / nc * 1e-6, ph[14] / nc * 1e-6,
-                              ph[15] / nc * 1e-6, ph[16] / nc * 1e-6, ph[17] / nc * 1e-6, ph[18] / nc * 1e-6,
-                              ph[19] / nc * 1e-6, ph[20] / nc * 1e-6, ph[21] / nc * 1e-6, ph[22] / nc * 1e-6,
-                              ph[23] / nc * 1e-6);
+                              ph[15] / nc * 1e-6);
                 std::fprintf(stderr, "%s%s%s", line.c_str(), buf, buf2);
                 for (auto& e : ev) cudaEventDestroy(e);
                 cudaFree(dbg);
