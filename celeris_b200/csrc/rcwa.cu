@@ -2184,12 +2184,27 @@ bool sym_eligible(const celeris_rcwa_cell& c) {
     return c.theta_rad == 0.0 && c.rotation_rad == 0.0 && c.Mx >= 1 && c.My >= 1 && symmetry_enabled();
 }
 
-// Cells the two-port does not take: orders above its limit; layers thinner than k0 h =
+// Largest optical phase k0 h sqrt(max |eps|) of a layer of this order that goes through the
+// two-port. A pole leaves the last doublings out, at most r of them below a phase of 2^(r+1) pi / 2
+// (a growth of 30 is met within 1/47 of the pole), and each makes the complex recursion twice as long; the
+// batch waits for its slowest cell. Whole calls, the eigendecomposition's time over the two-port's, at
+// r <= 4 and 5: mirror-symmetric M = 2, 3, 4, 7, 64 cells, 1.13, 1.33, 1.56, 1.82 and 0.74, 0.81, 0.90, 1.02;
+// oblique M = 1 .. 4 1.36, 1.73, 1.79, 1.28 and 0.86, 0.98, 0.98, 0.68. Above order 256 (12 cells) at r <= 3 and 4:
+// oblique M = 6 1.29 and 0.73, classes of M = 15 1.22 and 0.71; with complex doublings at
+// r <= 2, 3 and 4: oblique M = 6 1.70, 0.97 and 0.61.
+double phase_limit(int order, bool real) {
+    if (order <= 200) return 48.0;
+    if (order <= 256) return real ? 48.0 : 24.0;
+    return real ? 24.0 : 12.0;
+}
+
+// Cells of `order` (of their parity class, or of the order basis) the two-port does not take: orders
+// above its limit; layers thinner than k0 h =
 // 0.4 (40 nm at 633 nm; A and B are ~1 / h and only their difference counts, so
 // digits go as 1 / (k0 h): against 50 digits, 48 cells of M = 1, 2 per range of k0 h, median error
 // here and by the eigendecomposition 7.1e-15, 2.8e-16 in 0.01 .. 0.02, 1.1e-15, 4.4e-16 in 0.1 .. 0.2,
-// 5.7e-16, 4.0e-16 in 0.2 .. 0.4, 4.7e-16, 6.1e-16 in 0.4 .. 1), zero and negative thicknesses with them; layers of more than
-// 100 rad of optical phase (every doubling past pi / 2 may meet a mode's pole); layers with a
+// 5.7e-16, 4.0e-16 in 0.2 .. 0.4, 4.7e-16, 6.1e-16 in 0.4 .. 1), zero and negative thicknesses with them; layers
+// of more optical phase than phase_limit; layers with a
 // permittivity of negative real part, whose plasmon modes pass the bulk's q (up to 355 times over
 // 4400 random metal cells M = 1..3, so the series' slab may be at sin(q x) = 0) and whose two-port is
 // less exact even where it is regular (against 50 digits, 90 % of 110 cells below 1.6e-13, the
@@ -2197,13 +2212,17 @@ bool sym_eligible(const celeris_rcwa_cell& c) {
 // cell while the QR iteration cap of the failure-path tests is set (the cap is about
 // the eigendecomposition).
 std::atomic<int> g_qr_cap_set{0};
-bool needs_qr(const celeris_rcwa_cell& c) {
-    const int n = 2 * (2 * c.Mx + 1) * (2 * c.My + 1);
-    const int order = sym_eligible(c) ? sym_class_size(c.Mx, c.My, 0) : n;
+bool needs_qr(const celeris_rcwa_cell& c, int order) {
     const double kh = 2.0 * PI / c.wavelength_um * c.thickness_um;
     const double eps = std::max(std::hypot(c.eps_pillar[0], c.eps_pillar[1]), std::hypot(c.eps_bg[0], c.eps_bg[1]));
     const bool metal = !(c.eps_pillar[0] > 0.0 && c.eps_bg[0] > 0.0);
-    return metal || order > slab::kMaxOrder || !(kh >= 0.4) || !(kh * std::sqrt(eps) <= 100.0) || g_qr_cap_set.load() != 0;
+    const bool real = c.eps_pillar[1] == 0.0 && c.eps_bg[1] == 0.0 && (c.n_inc[1] == 0.0 || c.theta_rad == 0.0);
+    return metal || order > slab::kMaxOrder || !(kh >= 0.4) || !(kh * std::sqrt(eps) <= phase_limit(order, real)) ||
+           g_qr_cap_set.load() != 0;
+}
+int full_order(int Mx, int My) { return 2 * (2 * Mx + 1) * (2 * My + 1); }
+bool needs_qr(const celeris_rcwa_cell& c) {
+    return needs_qr(c, sym_eligible(c) ? sym_class_size(c.Mx, c.My, 0) : full_order(c.Mx, c.My));
 }
 
 int validate(const celeris_rcwa_cell& c) {
@@ -3555,7 +3574,7 @@ int run_stacks(const celeris_rcwa_cell* layers, const std::vector<std::pair<int,
         bool qr = false;
         for (int l = 0; l < stacks[s].second; ++l) {
             const celeris_rcwa_cell& c = layers[stacks[s].first + l];
-            qr = qr || needs_qr(c) || 2 * (2 * c.Mx + 1) * (2 * c.My + 1) > slab::kMaxOrder;
+            qr = qr || needs_qr(c, full_order(c.Mx, c.My));  // stacks are solved in the order basis
         }
         (qr ? rest : direct).push_back(s);
     }

@@ -54,7 +54,7 @@ constexpr unsigned kFlagPolls = 1u << 22;  // bound of a panel's wait for a colu
 // 6e-12 at 30, what is left being resonances of both. A stop costs complex solves that
 // hold up the batch (limit 1000 -> 30: 64 cells M = 3 0.33 -> 0.40 ms, 512 rasterised cells 6.3 ->
 // 10.7 ms, 96 oblique cells M = 4 5.0 -> 7.2 ms, 64 stacks 2.5 -> 3.8 ms); that is the price of the digits.
-constexpr int kMaxRest = 5;
+constexpr int kMaxRest = 4;
 constexpr double kGrowthLimit = 30.0;
 
 // ---- scalars: double or complex ---------------------------------------------------------
