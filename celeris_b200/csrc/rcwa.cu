@@ -2614,7 +2614,8 @@ struct BatchCtx {
     int dev = -1;
     cudaStream_t main = nullptr;
     std::vector<cudaStream_t> side;
-    std::vector<cudaEvent_t> fork, join;
+    cudaEvent_t fork = nullptr;
+    std::vector<cudaEvent_t> join;
     void* pinned = nullptr;
     size_t pinned_cap = 0;
     cudaGraphExec_t exec = nullptr;
@@ -2636,11 +2637,11 @@ struct BatchCtx {
             Workspace::release_stream(s);
             cudaStreamDestroy(s);
         }
-        for (cudaEvent_t e : fork) cudaEventDestroy(e);
+        if (fork) cudaEventDestroy(fork);
+        fork = nullptr;
         for (cudaEvent_t e : join) cudaEventDestroy(e);
         cudaStreamDestroy(main);
         side.clear();
-        fork.clear();
         join.clear();
         main = nullptr;
         dev = -1;
@@ -2661,17 +2662,22 @@ int ensure_streams(int nb) {
     CEL_CUDA(cudaGetDevice(&cur));
     if (c.main && c.dev != cur) c.drop_device_objects();
     if (!c.main) {
-        CEL_CUDA(cudaStreamCreateWithFlags(&c.main, cudaStreamNonBlocking));
+        CEL_CUDA(cudaEventCreateWithFlags(&c.fork, cudaEventDisableTiming));
+        const cudaError_t e = cudaStreamCreateWithFlags(&c.main, cudaStreamNonBlocking);
+        if (e != cudaSuccess) {
+            cudaEventDestroy(c.fork);
+            c.fork = nullptr;
+            c.main = nullptr;
+            return celeris_rt::cuda_error(e, "stream of the RCWA batch");
+        }
         c.dev = cur;
     }
     while ((int)c.side.size() < nb) {
         cudaStream_t s;
-        cudaEvent_t f, j;
+        cudaEvent_t j;
         CEL_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        CEL_CUDA(cudaEventCreateWithFlags(&f, cudaEventDisableTiming));
         CEL_CUDA(cudaEventCreateWithFlags(&j, cudaEventDisableTiming));
         c.side.push_back(s);
-        c.fork.push_back(f);
         c.join.push_back(j);
     }
     return CELERIS_OK;
@@ -3001,12 +3007,14 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                 CEL_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
                 celeris_rt::set_launch_counting(false);
                 uint64_t nk = 0;
+                // one fork before the first bucket and the joins behind the last: a join in
+                // between would hold the next bucket's fork back until the buckets before it are done
+                cudaEventRecord(ctx.fork, st);
                 for (size_t w = 0; w < wave.size(); ++w) {
                     const BucketPlan& p = plans[wave[w]];
                     const int nc = (int)p.ids.size();
                     cudaStream_t bs = ctx.side[w];
-                    cudaEventRecord(ctx.fork[w], st);
-                    cudaStreamWaitEvent(bs, ctx.fork[w], 0);
+                    cudaStreamWaitEvent(bs, ctx.fork, 0);
                     cudaMemcpyAsync(const_cast<CellDev*>(p.b.cells), hdesc[w], sizeof(CellDev) * nc,
                                     cudaMemcpyHostToDevice, bs);
                     launch_bucket(p.b, cfgs[w], bs, nullptr, p.qr != 0);
@@ -3015,8 +3023,8 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                                     cudaMemcpyDeviceToHost, bs);
                     cudaMemcpyAsync(hinfo_pin[w], p.b.info, sizeof(int) * nc, cudaMemcpyDeviceToHost, bs);
                     cudaEventRecord(ctx.join[w], bs);
-                    cudaStreamWaitEvent(st, ctx.join[w], 0);
                 }
+                for (size_t w = 0; w < wave.size(); ++w) cudaStreamWaitEvent(st, ctx.join[w], 0);
                 const cudaError_t ce = cudaStreamEndCapture(st, &graph);
                 celeris_rt::set_launch_counting(true);
                 if (ce != cudaSuccess) return celeris_rt::cuda_error(ce, "capture of the RCWA batch");

@@ -1,8 +1,11 @@
 """What a cached graph of celeris_rcwa_batch holds: a batch of a shape seen before, with another
-symmetry tolerance, does not replay the old one's graph; and its kernels are counted.
+symmetry tolerance, does not replay the old one's graph; its kernels are counted; and the
+buckets of a batch (cells of one size and path) run beside one another.
 """
 import os
+import time
 
+import numpy as np
 import pytest
 
 from celeris_b200 import capi
@@ -52,3 +55,20 @@ def test_symmetry_tolerance_of_a_known_shape(grid):
 ])
 def test_launch_count_of_a_bucket(extra, kernels):
     assert launches([dict(BASE, Mx=2, fill_x=0.5, **extra)])[0] == kernels
+
+
+def test_buckets_run_side_by_side():
+    """Twenty thin M = 4 cells (eigendecomposition, ~1.5 ms) and twenty M = 5 cells (two-port,
+    ~0.8 ms) leave most of the chip idle alone: together they take less than one after the other."""
+    def median_time(cells):
+        arr, t = [capi.rcwa_cell(**c) for c in cells], []
+        for _ in range(15):
+            t0 = time.perf_counter()
+            capi.rcwa_batch(arr)
+            t.append(time.perf_counter() - t0)
+        return float(np.median(t[3:]))
+
+    thin = [dict(BASE, Mx=4, fill_x=0.2 + 0.03 * i, thickness_um=2e-3) for i in range(20)]
+    thick = [dict(BASE, Mx=5, fill_x=0.2 + 0.03 * i) for i in range(20)]
+    a, b, both = (median_time(c) for c in (thin, thick, thin + thick))
+    assert both <= 0.85 * (a + b), (a, b, both)
