@@ -118,10 +118,12 @@ struct Bucket {
     // QR path in the classes: eigen-stage buffers (m^2 each), q and the eigensolve's info
     cplx *sZ, *sX, *sW, *sA, *sq;
     int* sinfo;
-    // the layer two-port (slab.cuh): work area of a full-order cell (s_w complex), kp
-    cplx *slab, *Kp;
+    // the layer two-port (slab.cuh): work area of a full-order cell (s_w complex), kp. The
+    // Fourier operators (s_NN = s_w) and the scratch of their LU lie in parts of the work area
+    // that the two-port has not reached when they are read
+    cplx *slab, *Kp, *lu;
     size_t s_w;
-    // layers of a stack: A, B and kp of cell i go to slot lslot[i] (s_nn each)
+    // layers of a stack: A, B and kp of cell i go to slot lslot[i] (s_nn each; no Kp)
     cplx *lA, *lB, *lK;
     const int* lslot;
     int* lrest;  // log2 of the slabs (A, B) the layer consists of
@@ -396,7 +398,7 @@ __global__ void __launch_bounds__(kRT) rcwa_fourier_laurent(Bucket b) {
     __syncthreads();
     // Laurent Toeplitz (rcwa2d.cpp:191-198); Exx = Eyy = epsT
     cplx* Exx = at(b.Exx, b.s_NN, cell);
-    cplx* lu = at(b.H, b.s_nn, cell);  // scratch for the LU of epsT
+    cplx* lu = b.lu ? at(b.lu, b.s_w, cell) : at(b.H, b.s_nn, cell);  // scratch for the LU of epsT
     cplx* Einv = at(b.Einv, b.s_NN, cell);
     for (int e = tid; e < N * N; e += nt) {
         const int r = e / N, col = e % N;
@@ -1643,7 +1645,7 @@ __device__ __noinline__ bool slab_port(int Mx, int My, const CellDev& cd, int c,
                                        cplx* aN, cplx* b0, size_t stride) {
     const int tid = threadIdx.x, nt = blockDim.x, nr = c < 0 ? 2 : 1, n2 = 2 * n, ldg = n + 2,
               ln = slab::ld_of(n);
-    cplx *Q = w.q, *G = w.w2, *L = w.e[0], *P = w.e[1], *Pn = w.e[2];
+    cplx *Q = w.q, *G = w.e[0], *L = w.e[0], *P = w.e[1], *Pn = w.e[2];
     HalfTable ys = half_table(Mx, My, cd, cd.n_sub, c, n, s);
     HalfTable yi;
     for (int k = slabs; k >= 1; --k) {
@@ -1791,9 +1793,9 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) rcwa_slab(Bucket b) {
         Kp = b.cKp + (size_t)mi * n * n;
         base = at(cc ? b.X : b.Z, b.s_nn, cell);  // the class build's scratch, free now
     } else {
-        M = at(b.H, b.s_nn, cell);
-        Kp = at(b.Kp, b.s_nn, cell);
         base = b.slab + b.s_w * cell;
+        M = base + slab::work_q(n);
+        Kp = b.lA ? b.lK + b.s_nn * b.lslot[cell] : at(b.Kp, b.s_nn, cell);
     }
     slab::Shared s = slab::carve(smem, n);
     if (b.dbg) s.prof = b.dbg + kDbgSlots * (size_t)mi;
@@ -1843,7 +1845,6 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) rcwa_slab(Bucket b) {
             const size_t p = (size_t)(e / n) * slab::ld_of(n) + e % n;
             b.lA[o + e] = slab::as_cplx(A[p]);
             b.lB[o + e] = slab::as_cplx(B[p]);
-            b.lK[o + e] = Kp[e];
         }
         return true;
     };
@@ -1891,7 +1892,7 @@ __global__ void __launch_bounds__(512, 1) rcwa_stack_port(StackPort sp) {
     const int nl = sp.stacks[st].x, slot0 = sp.stacks[st].y;
     const slab::Shared s = slab::carve(smem, n);
     const slab::Work w = slab::carve_work(sp.work + sp.s_w * st, n);
-    cplx *Q = w.q, *G = w.w2, *Yin = w.w0, *L = w.w1;
+    cplx *Q = w.q, *G = w.e[0], *Yin = w.p, *L = w.w1;
     bool ok = true;
     for (int l = nl - 1; l >= 0; --l) {
         cplx *A = sp.lA + sp.s_nn * (slot0 + l), *B = sp.lB + sp.s_nn * (slot0 + l);
@@ -1905,7 +1906,7 @@ __global__ void __launch_bounds__(512, 1) rcwa_stack_port(StackPort sp) {
             __syncthreads();
         }
         const int slabs = 1 << sp.lrest[slot0 + l];
-        cplx *P = w.e[0], *Pn = w.e[1];
+        cplx *P = w.e[1], *Pn = w.e[2];
         for (int k = slabs; k >= 1; --k) {
             const cplx* load = k == slabs ? L : Yin;
             for (int e = tid; e < n * n; e += nt) {
@@ -2014,9 +2015,10 @@ __global__ void __launch_bounds__(512, 1) rcwa_sym_smat(Bucket b) {
     const slab::Shared s = slab::carve(smem, n);
     const slab::Work w = slab::carve_work(at(cc ? b.X : b.Z, b.s_nn, cell), n);
     const int n2 = 2 * n, lq = n2 + 1, lc = n + 1;
-    cplx *A = w.w0, *T12 = w.w1, *Cm = w.w2, *G = w.p;
-    cplx* S = w.q;  // [T11 | -T12 D | a0], n x lq: w.q and the start of w.e[0] behind it
-    cplx *T11 = w.e[1], *S12 = w.e[2], *R = w.w0;
+    cplx *A = w.e[0], *T12 = w.w1, *G = w.p;
+    cplx* S = w.q;  // [T11 | -T12 D | a0], n x lq
+    cplx *T11 = w.e[1], *S12 = w.e[2];
+    cplx *R = A, *Cm = S;  // where A and S are no longer needed
     slab::gemm(n, n, n, Kp, n, W, n, nullptr, [=](int r, int j, cplx v) { A[(size_t)r * n + j] = v; });
     HalfTable t = half_table(Mx, My, cd, cd.n_inc, c, n, s);
     for (int e = tid; e < n * n; e += nt) {
@@ -2380,11 +2382,10 @@ size_t per_cell_bytes(int n, int nexc) {
            celeris_rt::align256(sizeof(CellDev)) + 14 * 256;
 }
 
-// Device memory of one order-basis cell solved through its two-port: M, kp, the
-// two-port's work area, the Fourier operators, the vector area and pivots.
+// Device memory of one order-basis cell solved through its two-port: kp, the two-port's
+// work area (M, the Fourier operators and their LU scratch in it), the vector area and pivots.
 size_t slab_per_cell_bytes(int n, int nexc) {
-    const size_t N = n / 2, s_nn = (size_t)n * n;
-    return (2 * s_nn + slab::work_size(n) + 3 * N * N + 10 * (size_t)n) * sizeof(cplx) + (size_t)n * sizeof(int) +
+    return ((size_t)n * n + slab::work_size(n) + 10 * (size_t)n) * sizeof(cplx) + (size_t)n * sizeof(int) +
            sizeof(int) + sizeof(celeris_rcwa_result) * nexc + sizeof(CellDev) + 16 * 256;
 }
 
@@ -2490,6 +2491,16 @@ int bucket_kernels(bool sym, int ng, bool qr, bool eig_only = false, bool layer 
     if (!qr) return operators + 1 + (sym ? 1 : 0) + (layer ? 0 : 1);  // slab, expand, epilogue
     // build (order basis), hess, schur, vec; smat1 and smat2, or the classes' smat and expand; epilogue
     return operators + (sym ? 6 : eig_only ? 4 : 7);
+}
+
+// The Fourier operators of a two-port bucket into e[0] of the work areas, their LU scratch into q.
+void place_operators(Bucket& b) {
+    const size_t NN = (size_t)b.N * b.N;
+    b.Einv = b.slab + slab::work_e(b.n);
+    b.Exx = b.Einv + NN;
+    b.Eyy = b.Exx + NN;
+    b.s_NN = b.s_w;
+    b.lu = b.slab + slab::work_q(b.n);
 }
 
 // Launch the stage sequence of one bucket on `st`. ev (ST_COUNT + 1 events) is
@@ -2860,13 +2871,14 @@ int run_cells(std::vector<HostCell>& cells, celeris_rcwa_result* out, int* info_
                 b.s_g1 = sym_g1_size(p.Mx, p.My, p.ng);
                 b.G1 = take(b.s_g1 * nc);
             } else {
-                b.H = take(b.s_nn * nc);
                 b.Kp = take(b.s_nn * nc);
                 b.s_w = slab::work_size(p.n);
                 b.slab = take(b.s_w * nc);
+                place_operators(b);
             }
             if (!p.sym) {
-                for (cplx** m : {&b.Einv, &b.Exx, &b.Eyy}) *m = take(b.s_NN * nc);
+                if (p.qr)
+                    for (cplx** m : {&b.Einv, &b.Exx, &b.Eyy}) *m = take(b.s_NN * nc);
                 b.piv = static_cast<int*>(ws.take(sizeof(int) * b.s_n * nc));
             }
             b.vec = take(10 * b.s_n * nc);
@@ -3343,13 +3355,13 @@ int run_stacks_qr(const celeris_rcwa_cell* layers, const std::vector<std::pair<i
     return CELERIS_OK;
 }
 
-// Device memory of one layer and of one stack of order n on the two-port path.
-size_t layer_bytes(int n) {
-    const size_t N = n / 2;
-    return (5 * (size_t)n * n + slab::work_size(n) + 3 * N * N) * sizeof(cplx) + 4096;
-}
-size_t stack_bytes(int n, int nexc) {
-    return (slab::work_size(n) + 10 * (size_t)n) * sizeof(cplx) + (size_t)nexc * n * sizeof(double) + 4096;
+// Device memory of `ns` stacks of `nslot` layers in all, of order n, on the two-port path: three
+// matrices a layer, and work areas for the layers or the stacks that run at a time. Up to eight layers
+// per SM run in one launch: at one or two blocks per SM, more of them would save little.
+size_t work_areas(size_t ns, size_t nslot, int sms) { return std::min(nslot, std::max(ns, (size_t)8 * sms)); }
+size_t stacks_bytes(size_t ns, size_t nslot, int n, int nexc, int sms) {
+    return (3 * (size_t)n * n * nslot + slab::work_size(n) * work_areas(ns, nslot, sms) + 10 * (size_t)n * ns) * sizeof(cplx) +
+           (size_t)nexc * n * sizeof(double) * ns + 4096 * (ns + nslot);
 }
 
 // The same through the layers' two-ports (rcwa_slab, rcwa_stack_port). info_out (required):
@@ -3357,9 +3369,10 @@ size_t stack_bytes(int n, int nexc) {
 int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair<int, int>>& stacks, const double* exc,
                     celeris_rcwa_result* out, int* info_out, int nexc, double* ord_out) {
     CEL_TRY(celeris_rt::require_device());
-    int dev = 0, smem_optin = 0;
+    int dev = 0, smem_optin = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     static thread_local celeris_rt::ThreadStream t_slab_st;
     cudaStream_t st = nullptr;
     CEL_TRY(t_slab_st.get(&st));
@@ -3376,9 +3389,9 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
     size_t most = 0;
     for (auto& g : groups) {
         const int N = (2 * g.first.first + 1) * (2 * g.first.second + 1), n = 2 * N;
-        size_t all = 0;
-        for (int k : g.second) all += stack_bytes(n, nexc) + layer_bytes(n) * stacks[k].second;
-        most = std::max(most, all + ((size_t)1 << 22));
+        size_t nslot = 0;
+        for (int k : g.second) nslot += stacks[k].second;
+        most = std::max(most, stacks_bytes(g.second.size(), nslot, n, nexc, sms) + ((size_t)1 << 22));
     }
     size_t budget = ws.capacity();
     if (most > budget) {
@@ -3389,17 +3402,16 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
     for (auto& g : groups) {
         const int Mx = g.first.first, My = g.first.second;
         const int N = (2 * Mx + 1) * (2 * My + 1), n = 2 * N;
-        const size_t s_nn = (size_t)n * n, s_n = (size_t)n, s_NN = (size_t)N * N, s_w = slab::work_size(n);
-        const size_t per_layer = layer_bytes(n), per_stack = stack_bytes(n, nexc);
+        const size_t s_nn = (size_t)n * n, s_n = (size_t)n, s_w = slab::work_size(n);
         size_t c0 = 0;
         while (c0 < g.second.size()) {
             std::vector<int> ids;
-            size_t bytes = 0;
+            size_t slots = 0;
             while (c0 < g.second.size()) {
-                const size_t need = per_stack + per_layer * stacks[g.second[c0]].second;
-                if (!ids.empty() && bytes + need > budget) break;
+                const size_t more = slots + stacks[g.second[c0]].second;
+                if (!ids.empty() && stacks_bytes(ids.size() + 1, more, n, nexc, sms) > budget) break;
                 ids.push_back(g.second[c0++]);
-                bytes += need;
+                slots = more;
             }
             const int ns = (int)ids.size();
             std::vector<HostCell> sub;
@@ -3421,14 +3433,13 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
             size_t up_bytes = a256(ns * sizeof(CellDev)) + a256(ns * sizeof(int2));
             size_t down_bytes = a256(ns * nexc * sizeof(celeris_rcwa_result)) + a256(ns * sizeof(int));
             if (ord_out) down_bytes += a256((size_t)ns * nexc * N * 2 * sizeof(double));
-            size_t fixed = 3 * a256(s_nn * nslot * c16) + a256(s_w * ns * c16) + a256(10 * s_n * ns * c16) +
-                           a256(nslot * sizeof(int));
+            const size_t areas = work_areas(ns, nslot, sms);
+            size_t fixed = 3 * a256(s_nn * nslot * c16) + a256(s_w * areas * c16) + a256(10 * s_n * ns * c16) +
+                           a256(nslot * sizeof(int)) + a256(s_n * areas * sizeof(int));
             for (auto& kv : by_ng) {
                 const size_t nc = kv.second.size(), ng = (size_t)std::max(kv.first, 0);
                 up_bytes += a256(nc * sizeof(CellDev)) + a256(nc * sizeof(int));
                 down_bytes += a256(nc * sizeof(int));
-                fixed += 2 * a256(s_nn * nc * c16) + a256(s_w * nc * c16) + 3 * a256(s_NN * nc * c16) +
-                         a256(s_n * nc * sizeof(int));
                 if (ng > 0) fixed += a256((4 * Mx + 1) * ng * c16) + a256((4 * My + 1) * ng * c16);
             }
             CEL_TRY(ws.reserve(st, up_bytes + down_bytes + fixed));
@@ -3451,7 +3462,9 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
             CEL_TRY(mem.get(&sp.lA, s_nn * nslot));
             CEL_TRY(mem.get(&sp.lB, s_nn * nslot));
             CEL_TRY(mem.get(&sp.lK, s_nn * nslot));
-            CEL_TRY(mem.get(&sp.work, s_w * ns));
+            CEL_TRY(mem.get(&sp.work, s_w * areas));  // the layers', then the stacks'
+            int* piv;
+            CEL_TRY(mem.get(&piv, s_n * areas));
             CEL_TRY(mem.get(&sp.vec, 10 * s_n * ns));
             CEL_TRY(down.get(&sp.info, (size_t)ns));
             int* lrest;
@@ -3483,9 +3496,11 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
                 b.ng = ng;
                 b.ncell = nc;
                 b.s_nn = s_nn;
-                b.s_NN = s_NN;
                 b.s_n = s_n;
                 b.s_w = s_w;
+                b.slab = sp.work;
+                place_operators(b);
+                b.piv = piv;
                 b.lA = sp.lA;
                 b.lB = sp.lB;
                 b.lK = sp.lK;
@@ -3493,13 +3508,6 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
                 CellDev* dcells;
                 int* dslot;
                 CEL_TRY(up.get(&dcells, (size_t)nc));
-                CEL_TRY(mem.get(&b.H, s_nn * nc));
-                CEL_TRY(mem.get(&b.Kp, s_nn * nc));
-                CEL_TRY(mem.get(&b.slab, s_w * nc));
-                CEL_TRY(mem.get(&b.Einv, s_NN * nc));
-                CEL_TRY(mem.get(&b.Exx, s_NN * nc));
-                CEL_TRY(mem.get(&b.Eyy, s_NN * nc));
-                CEL_TRY(mem.get(&b.piv, s_n * nc));
                 CEL_TRY(down.get(&b.info, (size_t)nc));
                 CEL_TRY(up.get(&dslot, (size_t)nc));
                 if (ng > 0) {
@@ -3522,7 +3530,15 @@ int run_stacks_slab(const celeris_rcwa_cell* layers, const std::vector<std::pair
             CEL_CUDA(cudaMemcpyAsync(region, pin, up_bytes, cudaMemcpyHostToDevice, st));
             CEL_CUDA(cudaMemsetAsync(region + up_bytes, 0, down_bytes, st));  // status words, results
             CEL_CUDA(cudaMemsetAsync(lrest, 0, sizeof(int) * nslot, st));
-            for (const Bucket& b : buckets) launch_bucket(b, uniform_cfg(256), st, nullptr, false);
+            for (const Bucket& b : buckets)
+                for (int i = 0; i < b.ncell; i += (int)areas) {
+                    Bucket part = b;
+                    part.ncell = std::min(b.ncell - i, (int)areas);
+                    part.cells += i;
+                    part.lslot += i;
+                    part.info += i;
+                    launch_bucket(part, uniform_cfg(256), st, nullptr, false);
+                }
             CEL_CUDA(cudaGetLastError());
             CEL_TRY(raise_dyn_smem(reinterpret_cast<const void*>(rcwa_stack_port), slab::shared_bytes(n)));
             rcwa_stack_port<<<ns, 512, slab::shared_bytes(n), st>>>(sp);

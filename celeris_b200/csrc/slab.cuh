@@ -750,27 +750,31 @@ __device__ bool gauss_jordan(int n, int ncol, T* Wm, int ld, bool inverse, const
 }
 
 // ---- the layer's two-port ------------------------------------------------------------------
-// Work area of one matrix: kAreas buffers of order x ld_of(order) complex plus 10 order (the
-// third carries two right-hand-side columns; four vectors of two columns). In real
-// arithmetic the same buffers hold doubles.
-constexpr int kAreas = 10;
+// Work area of one matrix: kAreas buffers of order x ld_of(order) complex plus 12 order (the
+// padding of q and e[0] takes right-hand-side columns; four vectors of two columns). In real
+// arithmetic the same buffers hold doubles. Routines share buffers by lifetime:
+//   two_port       e[2] M, w1 M^2 and then a B, e[0..1] [M^3 | M^4], p and q the series and
+//                  [S | C], p then A | B, q the doublings' systems
+//   slab_port      q [A + L | B], e[0] the load L and at last the incident system, e[1], e[2] the
+//                  product of the slabs' X (A and B stay in p and w1)
+constexpr int kAreas = 8;
 // Leading dimension of the n x n matrices in the work area (real products load pairs).
 __host__ __device__ inline int ld_of(int n) { return (n + 1) & ~1; }
-__host__ __device__ inline size_t work_size(int n) { return (size_t)kAreas * n * ld_of(n) + 10 * (size_t)n; }
+__host__ __device__ inline size_t work_size(int n) { return (size_t)kAreas * n * ld_of(n) + 12 * (size_t)n; }
 struct Work {
-    cplx *w0, *w1, *w2, *p, *q, *v;  // w2: n (n + 2); p, q: 2 n^2 each; v: 8 n
-    cplx* e[3];                      // n^2 each: the recursion's load and products
+    cplx *w1, *p, *q, *v;  // p: 2 n^2, q: 2 n (n + 1); v: 8 n
+    cplx* e[3];            // n^2 each, e[0]: n (n + 2)
 };
+__host__ __device__ inline size_t work_q(int n) { return 3 * (size_t)n * ld_of(n); }                        // q
+__host__ __device__ inline size_t work_e(int n) { return 5 * (size_t)n * ld_of(n) + 2 * (size_t)n; }  // e[0]
 __device__ __forceinline__ Work carve_work(cplx* base, int n) {
     const size_t nn = (size_t)n * ld_of(n);
     Work w;
-    w.w0 = base;
-    w.w1 = w.w0 + nn;
-    w.w2 = w.w1 + nn;
-    w.p = w.w2 + nn + 2 * (size_t)n;
-    w.q = w.p + 2 * nn;
-    w.e[0] = w.q + 2 * nn;
-    w.e[1] = w.e[0] + nn;
+    w.w1 = base;
+    w.p = w.w1 + nn;
+    w.q = base + work_q(n);
+    w.e[0] = base + work_e(n);
+    w.e[1] = w.e[0] + nn + 2 * (size_t)n;
     w.e[2] = w.e[1] + nn;
     w.v = w.e[2] + nn;
     return w;
@@ -804,33 +808,29 @@ __device__ double max_entry(int n, const T* A, int ld, int c0, double* red) {
 // A, B of the slab of thickness h / 2^*rest from M (n x n), *rest = 0 unless the last
 // doublings are ill conditioned. In real arithmetic (T double) M's real part is used.
 // qmax bounds the propagating modes' q. Returns false (in every thread) when S or an earlier
-// doubling is ill conditioned too. A and B point into the work area (w.q, w.w2 and w.e free). M may be overwritten.
+// doubling is ill conditioned too. A and B point into the work area (w.q and w.e free). M may lie in w.q.
 template <class T>
 __device__ __noinline__ bool two_port(int n, cplx* Mc, double h, double qmax, const Work& w, const Shared& s, T** Aout, T** Bout,
                                       int* rest) {
     // matrices of leading dimension ln; pairs [. | .] side by side, the right one from column ln
     const int tid = threadIdx.x, nt = blockDim.x, ln = ld_of(n), n2 = 2 * ln, nw = ln + n;
-    T* M1;
-    int l1 = ln;  // M1's
-    if constexpr (sizeof(T) == sizeof(double)) {
-        M1 = as<T>(w.w0);
-        for (int e = tid; e < n * n; e += nt) M1[(e / n) * ln + e % n] = Mc[e].x;
-    } else {
-        M1 = Mc;
-        l1 = n;
+    T* M1 = as<T>(w.e[2]);
+    for (int e = tid; e < n * n; e += nt) {
+        if constexpr (sizeof(T) == sizeof(double)) M1[(e / n) * ln + e % n] = Mc[e].x;
+        else M1[(e / n) * ln + e % n] = Mc[e];
     }
     T *M2 = as<T>(w.w1), *M34 = as<T>(w.e[0]), *P = as<T>(w.p), *Q = as<T>(w.q);
     T* A = P;
     T* B0 = P + (size_t)n * ln;
     __syncthreads();
     // M^2, then [M^3 | M^4] (side by side, ld 2 n)
-    gemm(n, n, n, M1, l1, M1, l1, nullptr, [=](int r, int c, T v) { M2[(size_t)r * ln + c] = v; });
+    gemm(n, n, n, M1, ln, M1, ln, nullptr, [=](int r, int c, T v) { M2[(size_t)r * ln + c] = v; });
     __syncthreads();
-    gemm(n, n, n, M2, ln, M1, l1, nullptr, [=](int r, int c, T v) { M34[(size_t)r * n2 + c] = v; });
+    gemm(n, n, n, M2, ln, M1, ln, nullptr, [=](int r, int c, T v) { M34[(size_t)r * n2 + c] = v; });
     gemm(n, n, n, M2, ln, M2, ln, nullptr, [=](int r, int c, T v) { M34[(size_t)r * n2 + ln + c] = v; });
     __syncthreads();
     // spectral radius of Q: from ||M||, or ||M^2||, ||M^4|| (every power's root bounds it)
-    const double b1 = norm_inf(n, M1, l1, s.red), b2 = norm_inf(n, M2, ln, s.red),
+    const double b1 = norm_inf(n, M1, ln, s.red), b2 = norm_inf(n, M2, ln, s.red),
                  b4 = norm_inf(n, M34 + ln, n2, s.red);
     const double rho = sqrt(fmin(b1, fmin(sqrt(b2), sqrt(sqrt(b4)))));
     if (!isfinite(b1 + b2 + b4) || !(h > 0.0)) return false;
@@ -853,7 +853,7 @@ __device__ __noinline__ bool two_port(int n, cplx* Mc, double h, double qmax, co
     const double y2 = y * y, y4 = y2 * y2, y6 = y4 * y2, y8 = y4 * y4;
     auto group = [=](int r, int c, double f0, double f1, double f2, double f3) {
         // f0 I + f1 M y^2 + f2 M^2 y^4 + f3 M^3 y^6
-        T v = scale(M1[(size_t)r * l1 + c], f1 * y2);
+        T v = scale(M1[(size_t)r * ln + c], f1 * y2);
         v = add(v, scale(M2[(size_t)r * ln + c], f2 * y4));
         v = add(v, scale(M34[(size_t)r * n2 + c], f3 * y6));
         return r == c ? plus_real(v, f0) : v;
