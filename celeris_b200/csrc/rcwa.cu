@@ -21,7 +21,7 @@
 // Stacks run rcwa_slab per layer and rcwa_stack_port (one CTA per stack).
 // Measured (one B200, whole calls, against the eigendecomposition's sequence below):
 //   one M = 5 cell 4.7 -> 0.55 ms; 64 cells M = 3 0.98 -> 0.40 ms; 512 rasterised cells M = 3..7
-//   37 -> 10.7 ms; 96 oblique cells M = 4 26 -> 7.2 ms; 64 two-layer stacks M = 3 15.6 -> 3.8 ms
+//   37 -> 6.0 ms; 96 oblique cells M = 4 26 -> 7.2 ms; 64 two-layer stacks M = 3 15.6 -> 3.8 ms
 //
 // The eigendecomposition's sequence remains for what the two-port does not take (needs_qr)
 // or flags (kInfoRedo), and for celeris_eig_general; it runs in the order basis, or on the
@@ -1183,7 +1183,8 @@ __device__ __forceinline__ double orbit_factor(int p, int pp) {
 // function of |x| that does not decrease away from x = 0 (with the reference's own
 // roundings) with a bound. So a row is two binary searches, and its sum over the samples is a
 // difference of prefix sums of the phase factors: nothing is summed over the pixels. 512
-// cells on 256^2 rasters, M = 3..7, growth limit 1000, 11.9 -> 6.9 ms a call; the operators of 102 M = 7 cells
+// cells on 256^2 rasters, M = 3..7, 11.9 -> 6.9 ms a call when doublings stopped at a growth of 1000
+// (30 today) and buckets ran one after another; the operators of 102 M = 7 cells
 // 2.1 -> 0.2 ms, of one M = 5 rectangle 0.30 -> 0.08 ms.
 //
 // Tables of a bucket, m = 0 .. 2 M: ph[m][i] = exp(-2 pi i m xf_i) / ng of pixel i, and
@@ -1765,7 +1766,7 @@ __device__ void slab_build_full(const Bucket& b, const CellDev& c, int cell, cpl
 
 // Orders whose whole work area fits in shared memory beside the routines' own: every
 // product and copy there waits on a load or two, ~30 cycles instead of ~300 from L2
-// (64 cells M = 3, growth limit 1000: 0.40 -> 0.36 ms a call).
+// (64 cells M = 3: 0.40 -> 0.36 ms a call when doublings stopped at a growth of 1000, 30 today).
 constexpr int kSmemWork = 31;
 size_t slab_smem(int n, int threads) {
     return slab::shared_bytes(n) + (threads >= 512 && n <= kSmemWork ? slab::work_size(n) * sizeof(cplx) : 0);

@@ -53,7 +53,7 @@ constexpr unsigned kFlagPolls = 1u << 22;  // bound of a panel's wait for a colu
 // oblique cells M = 1: 6e-11 and 3.4e-9 at a limit of 1000, 2e-12 and 6e-11 at 100, 2e-12 and
 // 6e-12 at 30, what is left being resonances of both. A stop costs complex solves that
 // hold up the batch (limit 1000 -> 30: 64 cells M = 3 0.33 -> 0.40 ms, 512 rasterised cells 6.3 ->
-// 10.7 ms, 96 oblique cells M = 4 5.0 -> 7.2 ms, 64 stacks 2.5 -> 3.8 ms); that is the price of the digits.
+// 10.7 ms with the buckets one after another, 6.0 side by side, 96 oblique cells M = 4 5.0 -> 7.2 ms, 64 stacks 2.5 -> 3.8 ms); that is the price of the digits.
 constexpr int kMaxRest = 4;
 constexpr double kGrowthLimit = 30.0;
 
@@ -136,7 +136,8 @@ struct Prod<double, double> {
 // (8-byte fragments: 56 % of L1 and 25 % of the tensor pipe busy at order 162), so they
 // load 16 bytes per lane: two k of A at a time (the order of k within a step of 8
 // is free) and two columns of B, and a warp's unit is 8 R x 8 W with the R, W that leave
-// the least to the busiest warp (96 oblique cells of order 162, growth limit 1000: 7.0 -> 5.6 ms a call). Real operands have even leading dimensions and
+// the least to the busiest warp (96 oblique cells of order 162: 7.0 -> 5.6 ms a call when doublings
+// stopped at a growth of 1000, 30 today). Real operands have even leading dimensions and
 // 16-byte-aligned bases. bmap (shared, may be NULL): row r of B is stored at row bmap[r].
 template <class TB, int R, int W, class Epi>
 __device__ __forceinline__ void gemm_units_real(int m, int n, int k, const double* A, int lda, const TB* B, int ldb,
@@ -342,7 +343,7 @@ struct Shared {
     int* bad;     // set when a column had no pivot, or a warp's wait for one ran out
     double* red;  // [32]
     int chunk;    // columns staged at a time
-    unsigned polls;  // bound of a wait for a column
+    int lost;     // a warp whose waits for a column count as run out (tests; -1: none)
     long long* prof;  // optional clock64 sums: [0] panels, [1] updates of the other columns, [2] whole kernel
 };
 __host__ __device__ inline size_t pad16(size_t b) { return (b + 15) & ~size_t(15); }
@@ -366,7 +367,7 @@ __device__ __forceinline__ Shared carve(unsigned char* p, int n) {
     Shared s;
     s.prof = nullptr;
     s.chunk = chunk_of(n);
-    s.polls = kFlagPolls;
+    s.lost = -1;
     s.pan = reinterpret_cast<cplx*>(p);
     p += panel_elems(n) * 16;
     s.prow = reinterpret_cast<cplx*>(p);
@@ -412,7 +413,7 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 // 0.1 % of the largest) and raises the column's flag with the row; every warp then
 // forms the reciprocal itself. The owner of the next column brings that one up to date and
 // hands it over before it touches its others. Cycles per column at 25 / 61 / 113 / 162
-// rows, real: 565, 682, 880, 1241 (complex 763, 878, 1195, 2030); one column per warp
+// rows, real: 646, 740, 950, 1396 (complex 865, 960, 1330, 2240); one column per warp
 // behind block-wide barriers took 830, 1109, 1537, 2065 (1006, 1477, 2166, 2926). The
 // finished panel G goes to s.pan (over the column buffers): the update of every other
 // column is row <- row + G (old pivot rows), with the pivot rows themselves replaced
@@ -421,10 +422,10 @@ template <class T>
 __host__ __device__ constexpr int panel_stride() {
     return sizeof(T) == sizeof(double) ? kGsReal : kGs;
 }
-__device__ __forceinline__ int wait_column(const int* flag, unsigned polls) {
+__device__ __forceinline__ int wait_column(const int* flag) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(flag);
     int v = 0;
-    for (unsigned i = 0; i < polls && v == 0; ++i)
+    for (unsigned i = 0; i < kFlagPolls && v == 0; ++i)
         asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v == 0 ? -1 : v;
 }
@@ -484,13 +485,14 @@ __device__ __noinline__ void panel(int n, int k0, int kb, const T* Wm, int ld, c
         }
     };
     if (warp == 0) hand_over(a[0], 0);
-    bool ok = true;
+    bool ok = warp != s.lost;
 #pragma unroll
     for (int qo = 0; qo < CPW; ++qo) {
+        if (!ok) break;
         for (int wo = 0; wo < PW; ++wo) {
             const int j = qo * PW + wo;
             if (j >= kb) break;
-            const int got = wait_column(flag + j, s.polls);
+            const int got = wait_column(flag + j);
             if (got < 0) {
                 ok = false;
                 break;
@@ -540,7 +542,6 @@ __device__ __noinline__ void panel(int n, int k0, int kb, const T* Wm, int ld, c
                 }
             }
         }
-        if (!ok) break;
     }
     used = mask;
     panel_barrier<PW * 32>();  // the column buffers are read; G overlays them
@@ -603,8 +604,8 @@ __device__ __forceinline__ void trailing_units(int n, int c0, int cn, T* Wm, int
     }
 }
 // The same in real arithmetic with 16-byte accesses throughout (36 instead of 16 shared and
-// global accesses per 16 tensor instructions otherwise; 64 cells M = 3, growth limit 1000: 0.345 -> 0.333 ms a
-// call): units of 8 R x 32, two k of G and two columns of the pivot rows
+// global accesses per 16 tensor instructions otherwise; 64 cells M = 3: 0.345 -> 0.333 ms a call when
+// doublings stopped at a growth of 1000, 30 today): units of 8 R x 32, two k of G and two columns of the pivot rows
 // and of Wm per access, as in gemm_units_real. c0 and ld are even.
 template <int R>
 __device__ __forceinline__ void trailing_units_real(int n, int c0, int cn, double* Wm, int ld, const Shared& s, int k0,

@@ -14,14 +14,14 @@
 namespace {
 
 // W (n x ncol, ld) <- its elimination (gauss_jordan); ok, perm: its result. lost_warp >= 0: that
-// warp gives up its waits at once. intact: a failed elimination left what it does not own in
+// warp's waits count as run out. intact: a failed elimination left what it does not own in
 // shared memory as it was (perm2, and the flags of the columns behind the one without a pivot).
 template <class T>
 __global__ void __launch_bounds__(512) slab_check_solve(int n, int ncol, int ld, T* W, int inverse, int lost_warp,
                                                         int* perm, int* ok, int* intact) {
     extern __shared__ __align__(16) unsigned char smem[];
     cb::slab::Shared s = cb::slab::carve(smem, n);
-    if ((int)(threadIdx.x >> 5) == lost_warp) s.polls = 0;
+    s.lost = lost_warp;
     constexpr int kMark = 0x5a5a5a5a;
     for (int i = threadIdx.x; i < n; i += blockDim.x) s.perm2[i] = kMark;
     const bool got = cb::slab::gauss_jordan(n, ncol, W, ld, inverse != 0, s);

@@ -260,8 +260,8 @@ int celeris_debug_qr_iteration_cap(int cap);
  * n <= 256, or 512): x = a^-1 b, and ainv = a^-1 when `inverse`. a, ainv: n x n,
  * b, x: n x nrhs, row-major host arrays (interleaved re, im when is_complex),
  * n <= 512. *ok = 0 (x and ainv not written) when a column had no pivot, or a warp's
- * bounded wait for a column ran out; lost_warp >= 0 makes that warp's waits run out
- * at once (-1: none). */
+ * bounded wait for a column ran out; lost_warp >= 0: that warp's waits count as run
+ * out (-1: none). */
 int celeris_debug_slab_solve(int n, int nrhs, int is_complex, int inverse, int threads, int lost_warp,
                              const double* a, const double* b, double* x, double* ainv, int* ok);
 /* New: out[0] = the largest row sum of |a|, out[1] = its largest entry (n x n, n <= 512), as
