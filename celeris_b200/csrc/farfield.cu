@@ -886,11 +886,22 @@ __global__ void __launch_bounds__(kThreads, 2) rs_adj_f64_kernel(const double4* 
         if (j0 + q < npil) partial[(size_t)blockIdx.y * npil + j0 + q] = make_double2(gr[q], gi[q]);
 }
 
+template <bool SPLIT>
 __global__ void chunk_sum_kernel(const double2* __restrict__ partial, int nchunk, int n,
                                  double2* __restrict__ out) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     double r = 0.0, i = 0.0;
-    if (split_chunk_sum(partial, nchunk, n, j, r, i)) out[j] = make_double2(r, i);
+    if constexpr (SPLIT) {
+        if (!split_chunk_sum(partial, nchunk, n, j, r, i)) return;
+    } else {
+        if (j >= n) return;
+        for (int c = 0; c < nchunk; ++c) {
+            const double2 v = partial[(size_t)c * n + j];
+            r += v.x;
+            i += v.y;
+        }
+    }
+    out[j] = make_double2(r, i);
 }
 
 // ---- stated error of the precision form ------------------------------------------
@@ -1447,8 +1458,11 @@ int ff_adjoint(const double* d_px, const double* d_py, int npil, const Geom& g0,
         rs_adj_f64_kernel<1><<<grid, kThreads, kSmem64, st>>>(rec, (int)npix, p64.chunk_len, d_px, d_py, npil, g.z, ph,
                                                               g.slot, partial);
     timer_end(st);
-    chunk_sum_kernel<<<(npil + 31) / 32, dim3(32, kSplitY), 0, st>>>(partial, p64.nchunk, npil,
-                                                                     reinterpret_cast<double2*>(d_out));
+    double2* out = reinterpret_cast<double2*>(d_out);
+    if (p64.nchunk >= 2 * kSplitY)
+        chunk_sum_kernel<true><<<(npil + 31) / 32, dim3(32, kSplitY), 0, st>>>(partial, p64.nchunk, npil, out);
+    else
+        chunk_sum_kernel<false><<<(npil + 255) / 256, 256, 0, st>>>(partial, p64.nchunk, npil, out);
     count_launch(3);
     CEL_CUDA(cudaGetLastError());
     return CELERIS_OK;
