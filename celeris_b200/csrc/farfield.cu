@@ -268,10 +268,11 @@ struct TilePipe {
 //    minimax; |error| < 2e-16) and e^{2 pi i n / 512} from a table in shared memory. Each
 //    lane of a quarter-warp reads its own copy of the table (8 copies, 16 B x 8 =
 //    one full bank row per entry), so the 16-byte lookups never conflict.
-// Domain: all coordinates and z within 1e9 um, |k| <= 4e3 rad/um (R il < 2^50) and
-// |z| >= 1e-100; outside it (or for NaN) tile_general evaluates the direct form.
+// Domain: all coordinates and z within 4e12 / |k| (R il < 2^50 then, in any unit of length) and
+// 1e100, and |z| >= 1e-100; outside it (or for NaN) tile_general evaluates the direct form. (With
+// limits of 1e9 um and 4e3 rad/um a lens given in metres took it: 70,688 x 161^2 14.0 ms.)
 // Measured (B200, 70,688 pillars x 161^2): 7.35 ms with sqrt, sincos and a division
-// per term, 3.41 ms (5.4e11 terms/s) here, the FP64 pipe 84 % busy; 125,676 pillars x
+// per term, 3.37 ms (5.4e11 terms/s) here, the FP64 pipe 85 % busy; 125,676 pillars x
 // 321^2: 5.65e11 terms/s. Four pixels per thread at two CTAs per SM; three CTAs, two
 // pixels, or the pillar loop unrolled by two measured 1-10 % slower. Error against
 // long double on lattice apertures (2-norm, relative): 5.8e-15, 4.0e-15, 2.3e-15 at
@@ -286,13 +287,12 @@ constexpr double kC2 = -7.529910584122855e-05, kC4 = 9.44985951974752e-10;
 // quadratic Chebyshev part on that interval is folded into the two coefficients;
 // what remains is below 5e-19.
 constexpr double kF0 = 0.5 + 4.03e-13, kF1 = 0.375 + 3.39e-7;
-constexpr double kCoordMax = 1e9, kWaveMax = 4e3, kZMin = 1e-100;
+constexpr double kPhaseCoordMax = 4e12, kCoordMax = 1e100, kZMin = 1e-100;
 
 // Phase constants of a launch: 512 k / 2 pi = il + il_lo (the adjoint negates
-// both), and whether z and k are in the domain above.
+// both), and the largest coordinate of the domain above.
 struct Phase64 {
-    double il, il_lo, k;
-    int ok;
+    double il, il_lo, k, cmax;
 };
 
 __device__ __forceinline__ double rsqrt_seed(double x) {
@@ -362,10 +362,10 @@ constexpr size_t kSmem64 = (size_t)kTab * kTabCopies * sizeof(double2) + (size_t
 
 // Every thread looks at the tile's record of its own index; the block takes the
 // direct form for the tile if any is out of the domain.
-__device__ __forceinline__ bool tile_in_domain(const double4* tile, int cnt, bool ok) {
+__device__ __forceinline__ bool tile_in_domain(const double4* tile, int cnt, bool ok, double cmax) {
     bool in = ok;
     for (int p = threadIdx.x; p < cnt; p += blockDim.x)
-        in = in && fabs(tile[p].x) <= kCoordMax && fabs(tile[p].y) <= kCoordMax;
+        in = in && fabs(tile[p].x) <= cmax && fabs(tile[p].y) <= cmax;
     return __syncthreads_and(in);
 }
 
@@ -390,9 +390,9 @@ __global__ void __launch_bounds__(kThreads, 2) rs_f64_kernel(const double4* __re
 #pragma unroll
     for (int q = 0; q < PPT; ++q) pixel_pos(g, min(i0 + q, g.nx - 1), jj, fx[q], fy, fz);
     const double z2 = fz * fz;
-    bool ok = ph.ok && fabs(fz) >= kZMin && fabs(fz) <= kCoordMax && fabs(fy) <= kCoordMax;
+    bool ok = fabs(fz) >= kZMin && fabs(fz) <= ph.cmax && fabs(fy) <= ph.cmax;
 #pragma unroll
-    for (int q = 0; q < PPT; ++q) ok = ok && fabs(fx[q]) <= kCoordMax;
+    for (int q = 0; q < PPT; ++q) ok = ok && fabs(fx[q]) <= ph.cmax;
 
     TilePipe<double4, kTile64> pipe;
     const int lo = blockIdx.y * chunk_len;
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kThreads, 2) rs_f64_kernel(const double4* __re
         const bool got = pipe.wait(t);
         const double4* tile = buf[t % kStages];
         const int cnt = got ? pipe.count(t) : 0;
-        if (tile_in_domain(tile, cnt, ok)) {  // (also orders the table before its first use)
+        if (tile_in_domain(tile, cnt, ok, ph.cmax)) {  // (also orders the table before its first use)
 #pragma unroll 1
             for (int p = 0; p < cnt; ++p) {
                 const double4 r = tile[p];
@@ -828,13 +828,13 @@ __global__ void __launch_bounds__(kThreads, 2) rs_adj_f64_kernel(const double4* 
 
     const int j0 = (blockIdx.x * kThreads + threadIdx.x) * PPT;
     double x[PPT], y[PPT];
-    bool ok = ph.ok && fabs(z) >= kZMin && fabs(z) <= kCoordMax;
+    bool ok = fabs(z) >= kZMin && fabs(z) <= ph.cmax;
 #pragma unroll
     for (int q = 0; q < PPT; ++q) {
         const int jq = min(j0 + q, npil - 1);
         x[q] = px[jq];
         y[q] = py[jq];
-        ok = ok && fabs(x[q]) <= kCoordMax && fabs(y[q]) <= kCoordMax;
+        ok = ok && fabs(x[q]) <= ph.cmax && fabs(y[q]) <= ph.cmax;
     }
     const double z2 = z * z;
 
@@ -852,7 +852,7 @@ __global__ void __launch_bounds__(kThreads, 2) rs_adj_f64_kernel(const double4* 
         const bool got = pipe.wait(t);
         const double4* tile = buf[t % kStages];
         const int cnt = got ? pipe.count(t) : 0;
-        if (tile_in_domain(tile, cnt, ok)) {
+        if (tile_in_domain(tile, cnt, ok, ph.cmax)) {
 #pragma unroll 1
             for (int p = 0; p < cnt; ++p) {
                 const double4 r = tile[p];  // {fx, fy, |v|, arg v}
@@ -1151,7 +1151,7 @@ Plan64 plan_field64(const Geom& g, int npil) {
     return plan64([&](int ppt) { return ((long)((g.nx + ppt - 1) / ppt) * g.ny + kThreads - 1) / kThreads; }, npil);
 }
 
-Phase64 phase64(double z, double k, bool adjoint) {
+Phase64 phase64(double k, bool adjoint) {
     Phase64 p;
     // 512 k / 2 pi as a pair: the product's rounding by FMA, and 512 / 2 pi's own
     const double c_lo = -5.037741228846716e-15;  // 512 / (2 pi) - kTabPerRad
@@ -1160,7 +1160,8 @@ Phase64 phase64(double z, double k, bool adjoint) {
     p.il = adjoint ? -il : il;
     p.il_lo = adjoint ? -lo : lo;
     p.k = k;
-    p.ok = std::fabs(k) <= kWaveMax && std::fabs(z) <= kCoordMax;
+    const double c = kPhaseCoordMax / std::fabs(k);
+    p.cmax = c < kCoordMax ? c : (c >= kCoordMax ? kCoordMax : -1.0);  // a NaN k: no coordinate is within it
     return p;
 }
 
@@ -1186,7 +1187,7 @@ int prepare64() {
 void launch_f64(const Plan64& p, cudaStream_t st, const double4* rec, int npil, const Geom& g, double k,
                 double2* partial) {
     const dim3 grid(p.ctas, p.nchunk);
-    const Phase64 ph = phase64(g.mode == GEOM_PSF ? g.z : 0.0, k, false);  // ZX: the kernel checks each row's z
+    const Phase64 ph = phase64(k, false);
     if (p.ppt == 4) rs_f64_kernel<4><<<grid, kThreads, kSmem64, st>>>(rec, npil, p.chunk_len, g, ph, partial);
     else if (p.ppt == 2) rs_f64_kernel<2><<<grid, kThreads, kSmem64, st>>>(rec, npil, p.chunk_len, g, ph, partial);
     else rs_f64_kernel<1><<<grid, kThreads, kSmem64, st>>>(rec, npil, p.chunk_len, g, ph, partial);
@@ -1446,7 +1447,7 @@ int ff_adjoint(const double* d_px, const double* d_py, int npil, const Geom& g0,
     double2* partial = static_cast<double2*>(ws.take(part_bytes));
     ff_pack_pix<<<(int)((npix + 255) / 256), 256, 0, st>>>(g, reinterpret_cast<const double2*>(d_v), rec);
     const dim3 grid(p64.ctas, p64.nchunk);
-    const Phase64 ph = phase64(g.z, k, true);
+    const Phase64 ph = phase64(k, true);
     timer_begin(st);
     if (p64.ppt == 4)
         rs_adj_f64_kernel<4><<<grid, kThreads, kSmem64, st>>>(rec, (int)npix, p64.chunk_len, d_px, d_py, npil, g.z, ph,

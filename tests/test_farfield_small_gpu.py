@@ -1,6 +1,7 @@
 """Far-field sums of few terms: few pillars on large grids, few pixels under many pillars (sums with
-fewer and with more chunks than the split reductions take), FP64 form, against the oracle; tolerance as
-derived in test_farfield_fp64_gpu.py.
+fewer and with more chunks than the split reductions take); and lengths in other units than um, up
+to the limits of the FP64 form's phase table. FP64 form, against the oracle; tolerance as derived in
+test_farfield_fp64_gpu.py.
 """
 import ctypes
 
@@ -10,7 +11,7 @@ import torch
 
 from celeris_b200 import capi, torch_ops as T
 from oracle import farfield as F
-from test_farfield_fp64_gpu import inputs, tolerance
+from test_farfield_fp64_gpu import EPS, inputs, tolerance
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +52,43 @@ def test_few_terms_do_not_wait_for_the_phase_table():
     finally:
         capi.check(lib.celeris_set_kernel_timing(0))
     assert max(times) < 23.0, times
+
+
+@pytest.mark.parametrize("unit", [1e-6, 1e3, 1e-40, 1e40])
+def test_other_units_of_length(unit):
+    x, y, t = inputs(1009, 9)
+    x, y, z, W, k = x * unit, y * unit, 30.0 * unit, 3.0 * unit, 2 * np.pi / 0.55 / unit
+    E, _, _ = capi.rs_field(x, y, t, 0.0, 0.0, z, k, 41, W)
+    Eo = F.rs_field(x, y, t, 0.0, 0.0, z, k, 41, W)
+    assert np.max(np.abs(E - Eo)) <= tolerance(x, y, z, k, np.abs(t).sum(), W)
+
+
+@pytest.mark.parametrize("k,far", [(5e12, 0.0), (11.0, 8e11), (0.0, 3e101), (4.0e-9, 2e21)])
+def test_beyond_the_phase_tables_domain(k, far):
+    """Phases above 2^50 table steps take the direct form. The phase of a term is only known to half an
+    ulp of k R there, which may be many turns, so one pillar at a time is summed and amplitudes are
+    compared: |E| = |t| / R."""
+    x, y, t = inputs(5, 11)
+    x = x + far
+    for j in range(5):
+        E, _, _ = capi.rs_field(x[j:j + 1], y[j:j + 1], t[j:j + 1], 0.0, 0.0, 30.0, k, 3, 3.0)
+        g = np.linspace(-3.0, 3.0, 3)
+        R = np.sqrt((g[None, :] - x[j]) ** 2 + (g[:, None] - y[j]) ** 2 + 900.0)
+        assert np.all(np.abs(np.abs(E) - np.abs(t[j]) / R) <= 16 * EPS * np.abs(t[j]) / R)
+
+
+def test_metres_take_the_time_of_micrometres():
+    def ms(unit):
+        x, y, t = (torch.tensor(a, device="cuda") for a in inputs(20000, 3))
+        x, y, grid = x * unit, y * unit, T.FarFieldGrid(128, 3.0 * unit, 30.0 * unit, 0.55 * unit)
+        out = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            T.rs_field_dev(x, y, t, grid, capi.FORM_PLAIN_F64, want_intensity=True)
+            b.record()
+            b.synchronize()
+            out.append(a.elapsed_time(b))
+        return float(np.median(out[2:]))
+
+    assert ms(1e-6) <= 1.3 * ms(1.0)
